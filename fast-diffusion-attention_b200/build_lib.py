@@ -1,4 +1,5 @@
-"""Build libfda_sm100.so in-tree with nvcc, for sm_100a only.
+"""Build libfda_sm100.so in-tree with nvcc, for sm_100a only, and beside it _fda_torch.so, the C++ host path of the
+Python functions, against the torch that runs this script.
 
     python build_lib.py            # incremental
     python build_lib.py --force    # rebuild everything
@@ -18,12 +19,13 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "fast_diffusion_attention", "libfda_sm100.so")
+TORCH_SRC = os.path.join(CSRC, "torch_binding.cpp")
+TORCH_EXT = os.path.join(HERE, "fast_diffusion_attention", "_fda_torch.so")
 SOURCES = ["abi.cu", "fwd_sm100.cu", "bwd_sm100.cu", "bwd_fused_sm100.cu", "selftest_sm100.cu", "varlen_list.cu"]
 
 
 def _nvcc():
-    cuda_home = os.environ.get("CUDA_HOME", "/usr/local/cuda")
-    cand = os.path.join(cuda_home, "bin", "nvcc")
+    cand = os.path.join(_cuda_home(), "bin", "nvcc")
     return cand if os.path.exists(cand) else "nvcc"
 
 
@@ -31,6 +33,28 @@ def _headers():
     out = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     out.append(os.path.join(HERE, "..", "include", "fda.h"))
     return out
+
+
+def _cuda_home():
+    return os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+
+def _torch_command():
+    """g++ line of the host path. The torch libraries are already loaded when the module is imported, so it carries no
+    run path."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           os.path.join(_cuda_home(), "include"), sysconfig.get_paths()["include"]]
+    libs = ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python",
+            # the shared C++ runtime that torch uses: some toolchains carry only a static one, and a second copy of the
+            # stream classes in one process crashes on the first exception text that goes through both
+            "-nostdlib++", "-l:libstdc++.so.6", "-lm"]
+    return ([os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+             f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + ["-I" + i for i in inc] +
+            [TORCH_SRC, "-o", TORCH_EXT, "-L" + os.path.join(root, "lib")] + libs)
 
 
 def _stale(target, deps):
@@ -64,11 +88,14 @@ def build(force=False, verbose=False):
         if verbose or r.returncode != 0 or os.environ.get("FDA_RESOURCE_USAGE", "0") == "1":
             sys.stderr.write(" ".join(cmd) + "\n" + r.stdout + r.stderr)
         if r.returncode != 0:
-            raise RuntimeError("nvcc failed for " + cmd[2])
+            raise RuntimeError("compilation failed: " + " ".join(cmd))
 
+    links = list(jobs)
+    if force or _stale(TORCH_EXT, [TORCH_SRC, os.path.join(HERE, "..", "include", "fda.h")]):
+        jobs.append(_torch_command())
     with ThreadPoolExecutor(max_workers=int(os.environ.get("MAX_JOBS", "4"))) as ex:
         list(ex.map(run, jobs))
-    if force or jobs or _stale(LIB, objs):
+    if force or links or _stale(LIB, objs):
         run([_nvcc(), "-shared", "-o", LIB] + objs + ["-cudart", "static"])
     return LIB
 

@@ -47,6 +47,8 @@ struct BwdParams {
   int n_long_kv, n_long_q;  // of the 2 * tiles_per_half items of a (sample, head): how many count as long
   int* ticket_kv;      // work counters of the two persistent kernels, zeroed before each launch
   int* ticket_q;
+  int* zero_tickets;   // the preprocess zeroes the counters (kTicketInts from here) when the stages run in one call
+  int64_t zero_acc16;  // ... and this many 16-byte pieces of the dQ accumulator
   float* dq_acc;     // single-pass backward: fp32 dQ accumulator, [heads][acc_tiles][head dim][64 queries]
   int acc_tiles;     // 64-row accumulator tiles per query head
   int64_t acc_floats;   // size of the accumulator

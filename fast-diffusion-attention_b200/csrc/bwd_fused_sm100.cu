@@ -624,7 +624,9 @@ int launch_fused_instance(const BwdParams& p, int sm_count, unsigned stages, cud
     static PerDeviceFlags smem_set;
     const int rc = set_dynamic_smem(kernel, Cfg::kSmemBytes, smem_set);
     if (rc) return rc;
-    FDA_CUDA_TRY(cudaMemsetAsync(p.dq_acc, 0, static_cast<size_t>(p.heads) * p.acc_tiles * 64 * kHeadDim * 4, stream));
+    if (p.zero_acc16 == 0) {
+      FDA_CUDA_TRY(cudaMemsetAsync(p.dq_acc, 0, static_cast<size_t>(p.heads) * p.acc_tiles * 64 * kHeadDim * 4, stream));
+    }
     const int items = bwd_item_bound(p, p.heads_k);
     const int grid = items < sm_count ? items : sm_count;
     kernel<<<grid, kDkdvThreads, Cfg::kSmemBytes, stream>>>(p);

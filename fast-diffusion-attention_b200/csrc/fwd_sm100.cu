@@ -888,7 +888,6 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
   if (p.total_items <= 0) return FDA_OK;
   if (!a.workspace || a.workspace_bytes < fwd_workspace_bytes(pr)) return FDA_ERR_WORKSPACE;
   p.ticket = static_cast<int*>(a.workspace);
-  FDA_CUDA_TRY(cudaMemsetAsync(p.ticket, 0, 256, stream));
   int grid = info.sm_count - (pr.sm_margin > 0 ? pr.sm_margin : 0);
   if (grid < 1) grid = 1;
   // the shortest eighths of every (sample, head) run at the end; few items per CTA: rank for rank over all of them
@@ -897,14 +896,17 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
     // the work list is built on the device from cu_seqlens (no host synchronisation): the host only knows an upper
     // bound of the number of items, blocks beyond the real number find no work and leave
     int* list = reinterpret_cast<int*>(static_cast<uint8_t*>(a.workspace) + 256);
-    const int rc = launch_varlen_prepare(pr.cu_seqlens, pr.batch, q_tiles * kBlockM, list, stream);
+    const int rc = launch_varlen_prepare(pr.cu_seqlens, pr.batch, q_tiles * kBlockM, list, p.ticket, stream);
     if (rc) return rc;
     p.vl.base = list;
     p.vl.batch = pr.batch;
     const int64_t bound = (static_cast<int64_t>(pr.total) / (2 * q_tiles * kBlockM) + pr.batch) * 2 * pr.heads;
     if (grid > bound) grid = static_cast<int>(bound);
-  } else if (grid > p.total_items) {
-    grid = p.total_items;
+  } else if (grid >= p.total_items) {
+    grid = p.total_items;   // a block for every item: no work counter, nothing to zero
+    p.ticket = nullptr;
+  } else {
+    FDA_CUDA_TRY(cudaMemsetAsync(p.ticket, 0, kTicketInts * 4, stream));
   }
   const bool bf16 = pr.dtype == FDA_BF16;
   if (fp8) {

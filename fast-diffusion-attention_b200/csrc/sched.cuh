@@ -37,7 +37,10 @@ __device__ __forceinline__ void sched_init(SchedMailbox* m, int consumer_arrival
 __device__ __forceinline__ int sched_take(SchedMailbox* m, uint32_t it, int* ticket, volatile int* abort_flag) {
   const uint32_t slot = it & 1u;
   if (!ptx::mbar_wait(&m->empty[slot], ((it >> 1) & 1u) ^ 1u, abort_flag, 5)) return -1;
-  return (it == 0) ? static_cast<int>(blockIdx.x) : static_cast<int>(gridDim.x) + atomicAdd(ticket, 1);
+  if (it == 0) return static_cast<int>(blockIdx.x);
+  // a launch with a block for every item passes no counter (nothing to zero beforehand): one item each
+  if (ticket == nullptr) return 0x7fffffff;
+  return static_cast<int>(gridDim.x) + atomicAdd(ticket, 1);
 }
 __device__ __forceinline__ void sched_publish(SchedMailbox* m, uint32_t it, int idx) {
   const uint32_t slot = it & 1u;

@@ -6,7 +6,8 @@
 namespace fda {
 
 __global__ void __launch_bounds__(256) varlen_prepare_kernel(const int32_t* __restrict__ cu_seqlens, int batch,
-                                                             int unit_rows, int* out) {
+                                                             int unit_rows, int* out, int* tickets) {
+  if (threadIdx.x < kTicketInts) tickets[threadIdx.x] = 0;
   int* order = out + 1;
   int* cum = out + 1 + batch;
   // rank of a sample = number of samples that come before it: longer ones, and equally long ones with a smaller
@@ -34,8 +35,8 @@ __global__ void __launch_bounds__(256) varlen_prepare_kernel(const int32_t* __re
   }
 }
 
-int launch_varlen_prepare(const int32_t* cu_seqlens, int batch, int unit_rows, int* out, void* stream) {
-  varlen_prepare_kernel<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(cu_seqlens, batch, unit_rows, out);
+int launch_varlen_prepare(const int32_t* cu_seqlens, int batch, int unit_rows, int* out, int* tickets, void* stream) {
+  varlen_prepare_kernel<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(cu_seqlens, batch, unit_rows, out, tickets);
   FDA_CUDA_TRY(cudaGetLastError());
   return FDA_OK;
 }

@@ -46,8 +46,11 @@ __device__ __forceinline__ VarlenPos varlen_locate(const VarlenList& vl, int idx
 }
 
 // One block. unit_rows = rows of a half that one unit covers (128-row tiles in the backward, the forward's item).
-__global__ void varlen_prepare_kernel(const int32_t* __restrict__ cu_seqlens, int batch, int unit_rows, int* out);
+// Also zeroes the kTicketInts work counters at `tickets` (one launch less than a separate fill).
+constexpr int kTicketInts = 64;
+__global__ void varlen_prepare_kernel(const int32_t* __restrict__ cu_seqlens, int batch, int unit_rows, int* out,
+                                      int* tickets);
 
-int launch_varlen_prepare(const int32_t* cu_seqlens, int batch, int unit_rows, int* out, void* stream);
+int launch_varlen_prepare(const int32_t* cu_seqlens, int batch, int unit_rows, int* out, int* tickets, void* stream);
 
 }  // namespace fda

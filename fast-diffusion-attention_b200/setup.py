@@ -34,7 +34,7 @@ setup(
     name="fast_diffusion_attention",
     version=__version__,  # noqa: F821
     packages=["fast_diffusion_attention"],
-    package_data={"fast_diffusion_attention": ["libfda_sm100.so"]},
+    package_data={"fast_diffusion_attention": ["libfda_sm100.so", "_fda_torch.so"]},
     cmdclass={"build_ext": BuildLib},
     python_requires=">=3.9",
 )

@@ -54,7 +54,7 @@ struct FusedCfg {
   static_assert(kHeadDim == 64 || kHeadDim == 128, "the single-pass backward covers head dimensions up to 128");
   static_assert(kOffStat % 1024 == 0, "tiles stay 1024-byte aligned for the swizzle");
   static_assert(kSmemBytes <= 232448, "shared memory budget");
-  static_assert((12 + 2 * kSlots + 2 * kDoSlots) * 8 + 8 + 16 + 16 * kSlots <= 384, "barrier area");
+  static_assert((14 + 2 * kSlots + 2 * kDoSlots) * 8 + 8 + 16 + 16 * kSlots <= 384, "barrier area");
 };
 
 // 768 threads start with 80 registers each. The compute warps hold a step's 32 probabilities per thread across the
@@ -129,7 +129,11 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
   uint64_t* ds_free = dp_free + 1;             // dQ^T and dK have read dS^T: the next step may overwrite it
   uint64_t* acc_full = ds_free + 1;
   uint64_t* acc_free = acc_full + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 1);
+  // [2] The step's description for the drain warps is in dq_desc[g & 1]. They do not wait for ds_full: where dQ^T has its
+  // own columns, dS^T of step g + 1 can be complete before they look for step g, and a wait by parity that is one whole
+  // round late waits for ever. A barrier for even and one for odd steps cannot be lapped (step g + 2 needs dp_free of g).
+  uint64_t* desc_full = acc_free + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(desc_full + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* dq_desc = reinterpret_cast<volatile int*>(tmem_slot + 2);   // [2][2]: {flags, first accumulator row}
   volatile int* hdr = reinterpret_cast<volatile int*>(tmem_slot + 6);       // [kSlots][4]
@@ -167,6 +171,8 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
     ptx::mbar_init(ds_free, 1);
     ptx::mbar_init(acc_full, 1);
     ptx::mbar_init(acc_free, 4);
+    ptx::mbar_init(&desc_full[0], 1);
+    ptx::mbar_init(&desc_full[1], 1);
     ptx::fence_mbar_init();
   }
   if (warp == kLoadWarpB) {
@@ -199,8 +205,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
       if (!it.valid) continue;
       for (bool last = false; alive && !last; ++gd) {
         const uint32_t par = gd & 1u;
-        // the compute warps' barrier orders their description of the step before our read of it
-        if (!ptx::mbar_wait(ds_full, par, abort_flag, 63)) { alive = false; break; }
+        if (!ptx::mbar_wait(&desc_full[par], (gd >> 1) & 1u, abort_flag, 63)) { alive = false; break; }
         const int flags = dq_desc[2 * par];
         const int acc_row = dq_desc[2 * par + 1];
         last = (flags & 1) != 0;
@@ -572,6 +577,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
         if (threadIdx.x == 0) {
           dq_desc[2 * par] = hdr0 & ~6;
           dq_desc[2 * par + 1] = hdr2;
+          ptx::mbar_arrive(&desc_full[par]);
         }
         ptx::fence_async_smem();
         ptx::tc_fence_before();

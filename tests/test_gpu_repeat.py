@@ -90,3 +90,19 @@ def test_sm_margin_changes_the_grid_not_the_result():
             assert_same_gradients(f"{name} with sm_margin={margin}, deterministic", a, b, exact=True)
     torch.cuda.synchronize()
     assert _lib.device_status()[0] == 0
+
+
+@pytest.mark.parametrize("heads,heads_k,d", [(32, 8, 64), (8, 8, 64), (32, 8, 128)])
+def test_no_wait_expires_over_many_backward_passes(heads, heads_k, d):
+    """The roles of the single-pass backward run a step apart; where one of them can be lapped by another, a wait by
+    parity misses its phase now and then (a few launches in a thousand) and gives up after two seconds."""
+    torch.manual_seed(10)
+    n = 2048
+    q = torch.randn(4, 2 * n, heads, d, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    k = torch.randn(4, 2 * n, heads_k, d, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    v = torch.randn(4, 2 * n, heads_k, d, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    do = torch.randn_like(q)
+    for _ in range(400):
+        torch.autograd.grad(diffusion_attn_func(q, k, v, 64), (q, k, v), do)
+    torch.cuda.synchronize()
+    assert _lib.device_status()[0] == 0

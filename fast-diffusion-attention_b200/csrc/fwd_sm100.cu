@@ -37,7 +37,9 @@ namespace {
 
 
 constexpr int kBlockM = 128;  // query rows per tile (= tensor-memory lanes)
-constexpr int kBlockN = 128;  // keys per tile
+constexpr int kSubKeys = 64;  // keys per sub-step (columns of one S buffer)
+constexpr int kBufs = 2;      // S buffers per query tile
+constexpr int kQPanelBytes = kBlockM * 128;
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kLn2 = 0.6931471805599453f;
 constexpr float kRescaleThreshold = 8.0f;  // in log2 units
@@ -122,13 +124,13 @@ __device__ __forceinline__ Item decode_item(const FwdParams& p, int idx) {
 struct TileSpans {
   Span half[2];
   // selects instead of half[kh]: a run-time index would put the spans in local memory
-  __device__ __forceinline__ int classify(int kh, int kt) const {
+  __device__ __forceinline__ int classify(int kh, int k0) const {
     Span s;
     s.lo_first = kh ? half[1].lo_first : half[0].lo_first;
     s.hi_first = kh ? half[1].hi_first : half[0].hi_first;
     s.lo_last = kh ? half[1].lo_last : half[0].lo_last;
     s.hi_last = kh ? half[1].hi_last : half[0].hi_last;
-    return s.classify(kt * kBlockN, kBlockN);
+    return s.classify(k0, kSubKeys);
   }
 };
 
@@ -155,74 +157,85 @@ struct ItemDesc {
   TileSpans spans[2];
 };
 
-template <int kHeadDim, int kQTiles, int kStages, int kType, bool kSoftcap>
+// kType: 0 bf16, 1 fp16, 2 fp8 e4m3 (forward only; the output is bf16)
+template <int kHeadDim, int kQTiles, int kType, bool kSoftcap>
 struct FwdConfig {
-  // kType: 0 bf16, 1 fp16, 2 fp8 e4m3 (forward only; the output is bf16)
   static constexpr bool kFp8 = kType == 2;
   static constexpr int kElemBytes = kFp8 ? 1 : 2;
-  static constexpr int kTileBytes = kBlockN * kHeadDim * kElemBytes;  // one 128-row tile of Q, K or V
+  static constexpr int kTileBytes = kBlockM * kHeadDim * kElemBytes;  // one query tile
   static constexpr int kPanelElems = 128 / kElemBytes;                // elements per 128-byte panel row
   static constexpr int kPanels = kHeadDim / kPanelElems;
-  static constexpr int kPanelBytes = 128 * 128;
   static constexpr int kStepElems = 32 / kElemBytes;                  // reduction elements per MMA (32 bytes)
-  static constexpr int kPCols = kBlockN * kElemBytes / 4;             // tensor-memory columns of the packed P
   static_assert(kHeadDim % kPanelElems == 0, "head dimension must fill whole 128-byte panels");
+  // K and V travel in slots of kSlotKeys keys. 16-bit rows of 256 leave room for four slots of 64 keys only.
+  static constexpr int kSlotKeys = kTileBytes > 32768 ? 64 : 128;
+  static constexpr int kSlotBytes = kSlotKeys * kHeadDim * kElemBytes;
+  static constexpr int kSlotPanelBytes = kSlotKeys * 128;
+  static constexpr int kHalves = kSlotKeys / kSubKeys;                // sub-steps per slot
   // Two query tiles: the two softmax warpgroups need more registers than an even split of the file gives them
   // (168 per thread with the block rounded up to whole warpgroups), so the block is padded to three whole
-  // warpgroups and the third (TMA warp, MMA warp, two idle warps) hands most of its registers to the other two.
+  // warpgroups and the third (TMA warp, MMA warp, two idle warps) hands registers to the other two.
   static constexpr bool kRegRealloc = kQTiles == 2;
   static constexpr int kThreads = kRegRealloc ? 384 : 128 * kQTiles + 64;
-  static constexpr uint32_t kSoftmaxRegs = 216, kProducerRegs = 72;
-  // the pool is what the block got at launch, 384 threads x 168 registers: 2 * 128 * 216 + 128 * 72 = 384 * 168.
+  static constexpr uint32_t kSoftmaxRegs = 200, kProducerRegs = 104;
+  // the pool is what the block got at launch, 384 threads x 168 registers: 2 * 128 * 200 + 128 * 104 = 384 * 168.
   // Asking for more than the pool holds would block the warpgroup for ever.
   static_assert(2 * 128 * kSoftmaxRegs + 128 * kProducerRegs <= 384 * 168, "register pool");
   static constexpr int kLoadWarp = 4 * kQTiles;
-  static constexpr int kMmaWarp = 4 * kQTiles + 1;
+  static constexpr int kMmaWarp = 4 * kQTiles + 1;                    // one issuing warp per query tile
   // epilogue staging: per query tile one [128 rows][64 columns] 16-bit tile, stored to out as a whole
   static constexpr int kStageOBytes = kBlockM * 128;
-  static constexpr int kSmemBytes = (kQTiles + kStages) * kTileBytes + kQTiles * kStageOBytes +
-                                    1024 /*alignment slack*/ + 1024 /*barriers, mailbox, item descriptions*/;
-  static_assert(kSmemBytes <= 232448, "shared memory budget");
-  static constexpr int kTmemS = 0;                  // S_t at t*128
-  static constexpr int kTmemO = 128 * kQTiles;      // O_t at kTmemO + t*kHeadDim
+  static constexpr int kFixedBytes = kQTiles * (kTileBytes + kStageOBytes) + 1024 /*alignment slack*/ +
+                                     1024 /*barriers, mailbox, item descriptions*/;
+  static constexpr int kFit = (232448 - kFixedBytes) / (2 * kSlotBytes);
+  static constexpr int kPairs = kFit < 4 ? kFit : 4;                  // the ring holds pairs of a K and a V slot
+  static_assert(kPairs >= 2, "two V slots owed to P V and the K slots ahead of them");
+  static constexpr int kSmemBytes = kFixedBytes + 2 * kPairs * kSlotBytes;
+  // tensor memory: S of query tile t, buffer b at (t * kBufs + b) * 64 (P over its first columns), O behind
+  static constexpr int kTmemO = kQTiles * kBufs * kSubKeys;
   static_assert(kTmemO + kQTiles * kHeadDim <= 512, "tensor memory budget");
-  // Where columns are left over (head dimensions up to 64) the packed P gets columns of its own instead of
-  // overwriting S, and every query tile gets its own MMA issuer. The next S of a tile is then issued as soon as its
-  // softmax warps have read this one and runs under their arithmetic; with P in place of S it has to wait for the
-  // P V product, and the chain softmax -> P V -> S -> softmax sets the pace. (One issuer for both tiles is held in
-  // the issue of 24 small MMAs per step for longer than a softmax takes.)
-  static constexpr bool kOwnP = kQTiles == 2 && kQTiles * (128 + kHeadDim + kPCols) <= 512;
-  static constexpr int kTmemP = kOwnP ? kTmemO + kQTiles * kHeadDim : kTmemS;   // P_t at kTmemP + t*kPStride
-  static constexpr int kPStride = kOwnP ? kPCols : 128;
-  // (Two issuers with P in place of S, as head dimension 128 would need, are slower than one: 0.38 against 0.31 ms
-  // on the benchmark shape, the two threads' products interleave in the pipe and every one of them takes longer.)
-  static constexpr int kIssuers = kOwnP ? kQTiles : 1;
+  static constexpr int kPCols = kSubKeys * kElemBytes / 4;            // tensor-memory columns of the packed P
 };
 
-template <int kHeadDim, int kQTiles, int kStages, int kType, bool kSoftcap>
+// The keys advance in sub-steps of 64 and every query tile has two 64-column S buffers (kBufs), used in turn, P written
+// over the S it came from. While the softmax warps turn one buffer into P, the tensor pipe runs P V of the other and
+// then the S product that refills it, so neither waits for the other's latency. With ONE 128-column buffer per tile the
+// chain S -> softmax -> P V -> next S was serial and set the pace: 3700 cycles for two query tiles against 128 keys of
+// head dimension 128, of which the tensor pipe has 2048 and the special-function unit 2048 to do. The price is the
+// shared-memory traffic of N = 64 products (6 KB per 32 cycles of arithmetic, 48 cycles at 128 bytes per clock):
+// about 2600 cycles.
+//
+// Every query tile has its own issuing warp, and that warp does next to nothing but wait and issue: the TMA warp, which
+// has time, walks the geometry and leaves one word of flags beside every K slot. (A single thread that decoded items and
+// classified tiles between the products spent 1200 cycles a round on that while the pipe ran dry; the whole warp takes
+// part in waits and loop control, one elected lane issues, which keeps descriptors and counters in uniform registers.)
+constexpr uint32_t kInfoFirst = 16, kInfoLast = 32, kInfoHalf1 = 64, kInfoStop = 128, kInfoTile0 = 256;  // bit 2 t + h: tile t sees half h
+
+template <int kHeadDim, int kQTiles, int kType, bool kSoftcap>
 __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fwd_kernel(const __grid_constant__ FwdParams p) {
-  using Cfg = FwdConfig<kHeadDim, kQTiles, kStages, kType, kSoftcap>;
+  using Cfg = FwdConfig<kHeadDim, kQTiles, kType, kSoftcap>;
+  constexpr int kStages = 2 * Cfg::kPairs;         // slot 2 i: K of pair i, slot 2 i + 1: its V
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
   uint8_t* sKV = smem + kQTiles * Cfg::kTileBytes;
-  uint8_t* sStageO = sKV + kStages * Cfg::kTileBytes;
+  uint8_t* sStageO = sKV + kStages * Cfg::kSlotBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sStageO + kQTiles * Cfg::kStageOBytes);
-  uint64_t* q_full = bars;                       // 1
-  uint64_t* q_empty = bars + 1;                  // 1
-  uint64_t* kv_full = bars + 2;                  // kStages
-  uint64_t* kv_empty = kv_full + kStages;        // kStages
-  uint64_t* s_full = kv_empty + kStages;         // kQTiles
-  uint64_t* p_full = s_full + kQTiles;           // kQTiles
-  uint64_t* o_full = p_full + kQTiles;           // kQTiles
-  uint64_t* s_free = o_full + kQTiles;           // kQTiles; used where P has its own columns: S is in registers
-  uint64_t* p_free = s_free + kQTiles;           // kQTiles; likewise: P V has read P (and updated O)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(p_free + kQTiles);
-  static_assert((2 + 2 * kStages + 5 * kQTiles) * 8 + 8 <= 256, "barrier area");
+  uint64_t* q_full = bars;                         // 1
+  uint64_t* q_empty = bars + 1;                    // 1
+  uint64_t* kv_full = bars + 2;                    // kStages
+  uint64_t* kv_empty = kv_full + kStages;          // kStages
+  uint64_t* s_full = kv_empty + kStages;           // [kQTiles][kBufs] S complete
+  uint64_t* p_full = s_full + kQTiles * kBufs;     // [kQTiles][kBufs] P written over it
+  uint64_t* pv_done = p_full + kQTiles * kBufs;    // [kQTiles][kBufs] P V has updated O
+  uint64_t* o_full = pv_done + kQTiles * kBufs;    // kQTiles
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + kQTiles);
+  static_assert((2 + 2 * kStages + 3 * kQTiles * kBufs + kQTiles) * 8 + 8 + 16 <= 320, "barrier area");
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  SchedMailbox* mbox = reinterpret_cast<SchedMailbox*>(reinterpret_cast<uint8_t*>(bars) + 256);
+  volatile uint32_t* slot_info = tmem_slot + 2;    // one word per pair
+  SchedMailbox* mbox = reinterpret_cast<SchedMailbox*>(reinterpret_cast<uint8_t*>(bars) + 320);
   ItemDesc* desc = reinterpret_cast<ItemDesc*>(reinterpret_cast<uint8_t*>(bars) + 512);  // two slots
-  static_assert(2 * sizeof(ItemDesc) <= 512, "item descriptions");
+  static_assert(Cfg::kMmaWarp + kQTiles <= Cfg::kThreads / 32 && sizeof(SchedMailbox) <= 192 && 2 * sizeof(ItemDesc) <= 512, "mailbox and item descriptions");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -230,20 +243,19 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    sched_init(mbox, 4 * kQTiles + Cfg::kIssuers);
+    sched_init(mbox, 4 * kQTiles);
     ptx::mbar_init(q_full, 1);
-    ptx::mbar_init(q_empty, Cfg::kIssuers);
+    ptx::mbar_init(q_empty, kQTiles);
     for (int i = 0; i < kStages; ++i) {
       ptx::mbar_init(&kv_full[i], 1);
-      ptx::mbar_init(&kv_empty[i], Cfg::kIssuers);   // every issuer lets go of the tile
+      ptx::mbar_init(&kv_empty[i], kQTiles);   // every issuer lets go of every slot
     }
-    for (int t = 0; t < kQTiles; ++t) {
-      ptx::mbar_init(&s_full[t], 1);
-      ptx::mbar_init(&p_full[t], 4);  // one arrival per softmax warp
-      ptx::mbar_init(&o_full[t], 1);
-      ptx::mbar_init(&s_free[t], 4);
-      ptx::mbar_init(&p_free[t], 1);
+    for (int i = 0; i < kQTiles * kBufs; ++i) {
+      ptx::mbar_init(&s_full[i], 1);
+      ptx::mbar_init(&p_full[i], 4);  // one arrival per softmax warp
+      ptx::mbar_init(&pv_done[i], 1);
     }
+    for (int t = 0; t < kQTiles; ++t) ptx::mbar_init(&o_full[t], 1);
     ptx::fence_mbar_init();
   }
   if (warp == Cfg::kLoadWarp) {
@@ -268,257 +280,202 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
   if (warp == Cfg::kLoadWarp) {
     // ------------------------------------------------------------------------------------------- TMA producer
     if (lane == 0) {
-      uint32_t slot = 0, n_item = 0;
+      uint32_t pair = 0, empty_par = 1, n_item = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
         const int idx = sched_take(mbox, n_sched, p.ticket, abort_flag);
         if (idx < 0) break;
         if (idx >= total_items) {
           sched_publish(mbox, n_sched, idx);
+          if (ptx::mbar_wait(&kv_empty[2 * pair], empty_par, abort_flag, 11)) {
+            slot_info[pair] = kInfoStop;
+            ptx::mbar_arrive(&kv_full[2 * pair]);
+          }
           break;
         }
         const Item it = decode_item<kQTiles>(p, idx);
         KeyPlan plan{};
+        TileSpans spans[kQTiles];
         {
           ItemDesc& d = desc[n_sched & 1u];
           d.it = it;
           if (it.valid) {
-            plan = make_key_plan(it.qh, it.qa, it.qb, it.n, bs, kBlockN);
+            plan = make_key_plan(it.qh, it.qa, it.qb, it.n, bs, Cfg::kSlotKeys);
             d.plan = plan;
 #pragma unroll
-            for (int t = 0; t < kQTiles; ++t) d.spans[t] = make_tile_spans(it, t, bs);
+            for (int t = 0; t < kQTiles; ++t) {
+              spans[t] = make_tile_spans(it, t, bs);
+              d.spans[t] = spans[t];
+            }
           }
         }
         sched_publish(mbox, n_sched, idx);
         if (!it.valid) continue;
-        const int steps = plan.steps();
+        const int tiles = plan.steps();
         const int q_row = it.row0 + it.qh * it.n + it.qa;
         const int ntiles = ceil_div(it.qb - it.qa, kBlockM);
-        for (int s = 0; s < steps && alive; ++s) {
+        auto visible = [&](int s, int sub) -> uint32_t {   // bit 2 t + sub: tile t sees these 64 keys of slot s
           int kh, kt;
           plan.step(s, kh, kt);
-          const int k_row = it.row0 + kh * it.n + kt * kBlockN;
-          for (int which = 0; which < 2; ++which) {  // 0: K tile, 1: V tile
-            const uint32_t stage = slot % kStages;
-            if (!ptx::mbar_wait(&kv_empty[stage], ((slot / kStages) & 1) ^ 1, abort_flag, 11)) { alive = false; break; }
-            ptx::mbar_expect_tx(&kv_full[stage], Cfg::kTileBytes);
-            uint8_t* dst = sKV + stage * Cfg::kTileBytes;
+          const int k0 = kt * Cfg::kSlotKeys + (Cfg::kHalves == 2 ? sub * kSubKeys : 0);
+          uint32_t bits = 0;
+#pragma unroll
+          for (int t = 0; t < kQTiles; ++t) bits |= spans[t].classify(kh, k0) != kTileSkip ? 1u << (2 * t + sub) : 0u;
+          return bits;
+        };
+        for (int s = 0; s < tiles && alive; ++s) {
+          int kh, kt;
+          plan.step(s, kh, kt);
+          const int k_row = it.row0 + kh * it.n + kt * Cfg::kSlotKeys;
+          for (int which = 0; which < 2; ++which) {  // 0: K, 1: V
+            const uint32_t slot = 2 * pair + which;
+            if (!ptx::mbar_wait(&kv_empty[slot], empty_par, abort_flag, 11)) { alive = false; break; }
+            if (which == 0 && (Cfg::kHalves == 2 || (s & 1) == 0)) {
+              // flags of the two sub-steps that start here: both halves of this slot, or this slot and the next
+              const bool two = Cfg::kHalves == 2 || s + 1 < tiles;
+              uint32_t w = visible(s, 0);
+              if (two) w |= visible(Cfg::kHalves == 2 ? s : s + 1, 1) | kInfoHalf1;
+              if (s == 0) w |= kInfoFirst;
+              if (s + (Cfg::kHalves == 2 ? 1 : 2) >= tiles) w |= kInfoLast;
+              w |= ((1u << ntiles) - 1u) * kInfoTile0;
+              slot_info[pair] = w;
+            }
+            ptx::mbar_expect_tx(&kv_full[slot], Cfg::kSlotBytes);
+            uint8_t* dst = sKV + slot * Cfg::kSlotBytes;
             const CUtensorMap* tm = which == 0 ? &p.tm_k : &p.tm_v;
 #pragma unroll
             for (int c = 0; c < Cfg::kPanels; ++c) {
-              ptx::tma_load_4d(dst + c * Cfg::kPanelBytes, tm, &kv_full[stage], c * Cfg::kPanelElems, k_row, it.hk,
+              ptx::tma_load_4d(dst + c * Cfg::kSlotPanelBytes, tm, &kv_full[slot], c * Cfg::kPanelElems, k_row, it.hk,
                                it.bcoord);
             }
-            ++slot;
             if (s == 0 && which == 0) {
-              // Q after the first K tile: the first MMA needs both, the previous item may still own Q.
+              // Q after the first K slot: the first MMA needs both, the previous item may still own Q.
               if (!ptx::mbar_wait(q_empty, (n_item & 1) ^ 1, abort_flag, 12)) { alive = false; break; }
               ptx::mbar_expect_tx(q_full, ntiles * Cfg::kTileBytes);
               for (int t = 0; t < ntiles; ++t) {
 #pragma unroll
                 for (int c = 0; c < Cfg::kPanels; ++c) {
-                  ptx::tma_load_4d(sQ + t * Cfg::kTileBytes + c * Cfg::kPanelBytes, &p.tm_q, q_full, c * Cfg::kPanelElems,
+                  ptx::tma_load_4d(sQ + t * Cfg::kTileBytes + c * kQPanelBytes, &p.tm_q, q_full, c * Cfg::kPanelElems,
                                    q_row + t * kBlockM, it.h, it.bcoord);
                 }
               }
             }
           }
+          if (++pair == Cfg::kPairs) { pair = 0; empty_par ^= 1; }
         }
         ++n_item;
       }
       if (*abort_flag) __nanosleep(100000);  // let copies in flight land before the CTA exits
     }
-  } else if (Cfg::kOwnP && warp >= Cfg::kMmaWarp && warp < Cfg::kMmaWarp + Cfg::kIssuers) {
+  } else if (warp < Cfg::kMmaWarp + kQTiles) {
     // ------------------------------------------------------------------------------- MMA issuer of one query tile
-    // P has its own columns: S of step s is issued as soon as the softmax warps hold S of step s - 1 (s_free), P V of
-    // step s - 1 when they have written P (p_full). Every issuer waits for every K / V tile and lets go of it, also
-    // where its own query tile skips the step: an issuer can then never be a whole ring ahead of the other.
-    if (lane == 0) {
-      const int t = warp - Cfg::kMmaWarp;
-      constexpr int kFmt = kType == 0 ? 1 : 0;
-      const uint32_t idesc_s = ptx::make_idesc(kBlockM, kBlockN, kFmt, false, false);
-      const uint32_t idesc_o = ptx::make_idesc(kBlockM, kHeadDim, kFmt, false, true);
-      constexpr uint32_t kDescHi = ptx::smem_desc_hi(1024);
-      const uint32_t q_lo = ptx::smem_desc_lo(ptx::smem_u32(sQ), 16) + t * (Cfg::kTileBytes >> 4);
-      const uint32_t k_lo0 = ptx::smem_desc_lo(ptx::smem_u32(sKV), 16);
-      const uint32_t v_lo0 = ptx::smem_desc_lo(ptx::smem_u32(sKV), Cfg::kPanelBytes);
-      const uint32_t tmem_s_t = tmem + Cfg::kTmemS + t * 128;
-      const uint32_t tmem_p_t = tmem + Cfg::kTmemP + t * Cfg::kPStride;
-      const uint32_t tmem_o_t = tmem + Cfg::kTmemO + t * kHeadDim;
-      uint32_t slot = 0, n_item = 0, cnt_p = 0, cnt_s = 0;
-      bool alive = true;
-      for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = sched_peek(mbox, n_sched, abort_flag);
-        if (idx < 0 || idx >= total_items) break;
-        const Item it = desc[n_sched & 1u].it;
-        const KeyPlan plan = desc[n_sched & 1u].plan;
-        const TileSpans spans = desc[n_sched & 1u].spans[t];
-        sched_release<false>(mbox, n_sched);
-        if (!it.valid) continue;
-        const int steps = plan.steps();
-        if (!ptx::mbar_wait(q_full, n_item & 1, abort_flag, 21)) { alive = false; break; }
-        bool pend = false, o_acc = false;
-        for (int s = 0; s <= steps && alive; ++s) {
-          const uint32_t slot_k = slot + 2 * s;        // K tile of step s
-          const uint32_t slot_v = slot + 2 * s - 1;    // V tile of step s-1
-          bool vis = false;
-          if (s < steps) {
-            int kh, kt;
-            plan.step(s, kh, kt);
-            vis = spans.classify(kh, kt) != kTileSkip;
-          }
-          // S of step s
-          auto do_s = [&]() -> bool {
-            if (s >= steps) return true;
-            if (!ptx::mbar_wait(&kv_full[slot_k % kStages], (slot_k / kStages) & 1, abort_flag, 22)) return false;
-            if (vis) {
-              if (!ptx::mbar_wait(&s_free[t], (cnt_s & 1) ^ 1, abort_flag, 25)) return false;
-              ++cnt_s;
-              ptx::tc_fence_after();
-              const uint32_t b_lo = k_lo0 + (slot_k % kStages) * (Cfg::kTileBytes >> 4);
-#pragma unroll
-              for (int kk = 0; kk < kHeadDim / Cfg::kStepElems; ++kk) {
-                const uint32_t off = ((kk / 4) * Cfg::kPanelBytes + (kk % 4) * 32) >> 4;
-                if (Cfg::kFp8) ptx::umma_ss_f8_lh(tmem_s_t, q_lo + off, b_lo + off, kDescHi, idesc_s, kk > 0);
-                else ptx::umma_ss_f16_lh(tmem_s_t, q_lo + off, b_lo + off, kDescHi, idesc_s, kk > 0);
-              }
-              ptx::umma_commit(&s_full[t]);
-            }
-            // arrives when this thread's products so far are complete (at once if it issued none on the tile)
-            ptx::umma_commit(&kv_empty[slot_k % kStages]);
-            if (s == steps - 1) ptx::umma_commit(q_empty);   // Q is read by the S products only
-            return true;
-          };
-          // P V of step s - 1
-          auto do_pv = [&]() -> bool {
-            if (s == 0) return true;
-            if (!ptx::mbar_wait(&kv_full[slot_v % kStages], (slot_v / kStages) & 1, abort_flag, 23)) return false;
-            if (pend) {
-              if (!ptx::mbar_wait(&p_full[t], cnt_p & 1, abort_flag, 24)) return false;
-              ++cnt_p;
-              ptx::tc_fence_after();
-              const uint32_t b_lo = v_lo0 + (slot_v % kStages) * (Cfg::kTileBytes >> 4);
-#pragma unroll
-              for (int kk = 0; kk < kBlockN / Cfg::kStepElems; ++kk) {
-                const uint32_t b = b_lo + kk * ((Cfg::kStepElems * 128) >> 4);
-                const uint32_t acc = (o_acc || kk > 0) ? 1u : 0u;
-                if (Cfg::kFp8) ptx::umma_ts_f8_lh(tmem_o_t, tmem_p_t + kk * 8, b, kDescHi, idesc_o, acc);
-                else ptx::umma_ts_f16_lh(tmem_o_t, tmem_p_t + kk * 8, b, kDescHi, idesc_o, acc);
-              }
-              ptx::umma_commit(&p_free[t]);
-              o_acc = true;
-            }
-            ptx::umma_commit(&kv_empty[slot_v % kStages]);
-            return true;
-          };
-          // S first: it only needs the previous S to have been read
-          if (!do_s() || !do_pv()) { alive = false; break; }
-          pend = vis;
-        }
-        if (!alive) break;
-        if (steps == 0) ptx::umma_commit(q_empty);
-        if (it.qa + t * kBlockM < it.qb) ptx::umma_commit(&o_full[t]);
-        slot += 2 * steps;
-        ++n_item;
+    // Two sub-steps of 64 keys a round: P V of the last round's half h, then S of this round's half h into the buffer
+    // that this P V has read (the products of one thread run in order).
+    constexpr int kFmt = kType == 0 ? 1 : 0;  // kind::f16: 1 = bf16, 0 = f16; kind::f8f6f4: 0 = e4m3
+    constexpr uint32_t kIdescS = ptx::make_idesc(kBlockM, kSubKeys, kFmt, false, false);
+    constexpr uint32_t kIdescO = ptx::make_idesc(kBlockM, kHeadDim, kFmt, false, true);
+    constexpr uint32_t kDescHi = ptx::smem_desc_hi(1024);
+    const int t = __shfl_sync(0xffffffffu, warp, 0) - Cfg::kMmaWarp;
+    // descriptor low words of slot 0; a slot adds its bytes / 16, a k-step a constant
+    const uint32_t q_lo = ptx::smem_desc_lo(ptx::smem_u32(sQ), 16) + t * (Cfg::kTileBytes >> 4);
+    const uint32_t k_lo0 = ptx::smem_desc_lo(ptx::smem_u32(sKV), 16);
+    const uint32_t v_lo0 = ptx::smem_desc_lo(ptx::smem_u32(sKV), Cfg::kSlotPanelBytes);
+    const uint32_t tmem_st = tmem + t * kBufs * kSubKeys;
+    const uint32_t tmem_ot = tmem + Cfg::kTmemO + t * kHeadDim;
+    uint64_t* s_full_t = s_full + t * kBufs;
+    uint64_t* p_full_t = p_full + t * kBufs;
+    uint64_t* pv_done_t = pv_done + t * kBufs;
+
+    uint32_t pair = 0, par = 0;            // ring position of the next K
+    uint32_t v_pair[2] = {0, 0}, v_par[2] = {0, 0};
+    uint32_t p_par[2] = {0, 0}, q_par = 0;
+    bool owed[2] = {false, false};         // a V slot of the last round waits for its release ...
+    bool pend[2] = {false, false};         // ... and a P V for being issued
+    bool o_acc = false, alive = true;
+
+    auto do_pv = [&](int h) {
+      if (!owed[h]) return;
+      const uint32_t slot = 2 * v_pair[h] + 1;
+      if (Cfg::kHalves == 1 || h == 0) {
+        if (!ptx::mbar_wait(&kv_full[slot], v_par[h], abort_flag, 23)) { alive = false; return; }
       }
-    }
-  } else if (!Cfg::kOwnP && warp == Cfg::kMmaWarp) {
-    // --------------------------------------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr int kFmt = kType == 0 ? 1 : 0;  // kind::f16: 1 = bf16, 0 = f16; kind::f8f6f4: 0 = e4m3
-      const uint32_t idesc_s = ptx::make_idesc(kBlockM, kBlockN, kFmt, false, false);
-      const uint32_t idesc_o = ptx::make_idesc(kBlockM, kHeadDim, kFmt, false, true);
-      uint32_t slot = 0, n_item = 0;
-      uint32_t cnt_p[kQTiles];
+      if (pend[h]) {
+        if (!ptx::mbar_wait(&p_full_t[h], p_par[h], abort_flag, 24)) { alive = false; return; }
+        p_par[h] ^= 1;
+        ptx::tc_fence_after();
+        const uint32_t b_lo = v_lo0 + slot * (Cfg::kSlotBytes >> 4) + (Cfg::kHalves == 2 ? h * ((kSubKeys * 128) >> 4) : 0);
+        if (ptx::elect_one()) {
 #pragma unroll
-      for (int t = 0; t < kQTiles; ++t) cnt_p[t] = 0;
-      bool alive = true;
-
-      // descriptor low words of stage 0 / tile 0; a stage or tile step adds kTileBytes / 16, a k-step a constant
-      constexpr uint32_t kDescHi = ptx::smem_desc_hi(1024);
-      const uint32_t q_lo0 = ptx::smem_desc_lo(ptx::smem_u32(sQ), 16);
-      const uint32_t k_lo0 = ptx::smem_desc_lo(ptx::smem_u32(sKV), 16);
-      const uint32_t v_lo0 = ptx::smem_desc_lo(ptx::smem_u32(sKV), Cfg::kPanelBytes);
-      auto issue_s = [&](int t, uint32_t k_stage) {
-        const uint32_t a_lo = q_lo0 + t * (Cfg::kTileBytes >> 4);
-        const uint32_t b_lo = k_lo0 + k_stage * (Cfg::kTileBytes >> 4);
-#pragma unroll
-        for (int kk = 0; kk < kHeadDim / Cfg::kStepElems; ++kk) {
-          const uint32_t off = ((kk / 4) * Cfg::kPanelBytes + (kk % 4) * 32) >> 4;
-          if (Cfg::kFp8) ptx::umma_ss_f8_lh(tmem + Cfg::kTmemS + t * 128, a_lo + off, b_lo + off, kDescHi, idesc_s, kk > 0);
-          else ptx::umma_ss_f16_lh(tmem + Cfg::kTmemS + t * 128, a_lo + off, b_lo + off, kDescHi, idesc_s, kk > 0);
+          for (int kk = 0; kk < kSubKeys / Cfg::kStepElems; ++kk) {
+            // one MMA consumes 32 bytes of every P row (8 columns) and kStepElems rows of V (128 bytes each)
+            const uint32_t b = b_lo + kk * ((Cfg::kStepElems * 128) >> 4);
+            const uint32_t acc = (kk > 0 || o_acc) ? 1u : 0u;
+            if (Cfg::kFp8) ptx::umma_ts_f8_lh(tmem_ot, tmem_st + h * kSubKeys + kk * 8, b, kDescHi, kIdescO, acc);
+            else ptx::umma_ts_f16_lh(tmem_ot, tmem_st + h * kSubKeys + kk * 8, b, kDescHi, kIdescO, acc);
+          }
+          ptx::umma_commit(&pv_done_t[h]);
+          if (Cfg::kHalves == 1 || h == 1) ptx::umma_commit(&kv_empty[slot]);
         }
-      };
-      auto issue_pv = [&](int t, uint32_t v_stage, bool accumulate) {
-        const uint32_t b_lo = v_lo0 + v_stage * (Cfg::kTileBytes >> 4);
-#pragma unroll
-        for (int kk = 0; kk < kBlockN / Cfg::kStepElems; ++kk) {
-          // one MMA consumes 32 bytes of every P row (8 columns) and kStepElems rows of V (128 bytes each)
-          const uint32_t a_t = tmem + Cfg::kTmemS + t * 128 + kk * 8;
-          const uint32_t b = b_lo + kk * ((Cfg::kStepElems * 128) >> 4);
-          if (Cfg::kFp8) ptx::umma_ts_f8_lh(tmem + Cfg::kTmemO + t * kHeadDim, a_t, b, kDescHi, idesc_o, (accumulate || kk > 0) ? 1u : 0u);
-          else ptx::umma_ts_f16_lh(tmem + Cfg::kTmemO + t * kHeadDim, a_t, b, kDescHi, idesc_o, (accumulate || kk > 0) ? 1u : 0u);
-        }
-      };
+        o_acc = true;
+        pend[h] = false;
+      } else if (Cfg::kHalves == 1 || h == 1) {
+        if (ptx::elect_one()) ptx::umma_commit(&kv_empty[slot]);
+      }
+      owed[h] = false;
+    };
 
-      for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = sched_peek(mbox, n_sched, abort_flag);
-        if (idx < 0 || idx >= total_items) break;
-        const Item it = desc[n_sched & 1u].it;
-        const KeyPlan plan = desc[n_sched & 1u].plan;
-        TileSpans spans[kQTiles];
+    while (alive) {
+      if (!ptx::mbar_wait(&kv_full[2 * pair], par, abort_flag, 22)) break;
+      const uint32_t info = __shfl_sync(0xffffffffu, slot_info[pair], 0);
+      if (info & kInfoStop) break;
+      if (info & kInfoFirst) {
+        if (!ptx::mbar_wait(q_full, q_par, abort_flag, 21)) break;
+        q_par ^= 1;
+        o_acc = false;
+      }
 #pragma unroll
-        for (int t = 0; t < kQTiles; ++t) spans[t] = desc[n_sched & 1u].spans[t];
-        sched_release<false>(mbox, n_sched);
-        if (!it.valid) continue;
-        const int steps = plan.steps();
-        if (!ptx::mbar_wait(q_full, n_item & 1, abort_flag, 21)) { alive = false; break; }
-        bool pend[kQTiles], o_acc[kQTiles];
+      for (int h = 0; h < 2; ++h) {
+        do_pv(h);
+        if (!alive) break;
+        if (Cfg::kHalves == 1 && h == 1) {
+          if (!(info & kInfoHalf1)) break;
+          if (!ptx::mbar_wait(&kv_full[2 * pair], par, abort_flag, 22)) { alive = false; break; }
+        }
+        const bool vis = (info >> (2 * t + h)) & 1u;
+        const uint32_t slot = 2 * pair;
+        const uint32_t b_lo = k_lo0 + slot * (Cfg::kSlotBytes >> 4) + (Cfg::kHalves == 2 ? h * ((kSubKeys * 128) >> 4) : 0);
+        const bool ends = (info & kInfoLast) != 0 && (h == 1 || !(info & kInfoHalf1));
+        ptx::tc_fence_after();
+        if (ptx::elect_one()) {
+          if (vis) {
 #pragma unroll
-        for (int t = 0; t < kQTiles; ++t) { pend[t] = false; o_acc[t] = false; }
-        for (int s = 0; s <= steps && alive; ++s) {
-          const uint32_t slot_k = slot + 2 * s;        // K tile of step s
-          const uint32_t slot_v = slot + 2 * s - 1;    // V tile of step s-1
-          int kh = 0, kt = 0;
-          if (s < steps) {
-            plan.step(s, kh, kt);
-            if (!ptx::mbar_wait(&kv_full[slot_k % kStages], (slot_k / kStages) & 1, abort_flag, 22)) { alive = false; break; }
-          }
-          if (s > 0) {
-            if (!ptx::mbar_wait(&kv_full[slot_v % kStages], (slot_v / kStages) & 1, abort_flag, 23)) { alive = false; break; }
-          }
-          ptx::tc_fence_after();
-#pragma unroll
-          for (int t = 0; t < kQTiles; ++t) {
-            if (pend[t]) {
-              if (!ptx::mbar_wait(&p_full[t], cnt_p[t] & 1, abort_flag, 24)) { alive = false; break; }
-              ++cnt_p[t];
-              ptx::tc_fence_after();
-              issue_pv(t, slot_v % kStages, o_acc[t]);
-              o_acc[t] = true;
-              pend[t] = false;
+            for (int kk = 0; kk < kHeadDim / Cfg::kStepElems; ++kk) {
+              const uint32_t a = q_lo + (((kk / 4) * kQPanelBytes + (kk % 4) * 32) >> 4);
+              const uint32_t b = b_lo + (((kk / 4) * Cfg::kSlotPanelBytes + (kk % 4) * 32) >> 4);
+              if (Cfg::kFp8) ptx::umma_ss_f8_lh(tmem_st + h * kSubKeys, a, b, kDescHi, kIdescS, kk > 0);
+              else ptx::umma_ss_f16_lh(tmem_st + h * kSubKeys, a, b, kDescHi, kIdescS, kk > 0);
             }
-            if (s < steps && spans[t].classify(kh, kt) != kTileSkip) {
-              issue_s(t, slot_k % kStages);
-              ptx::umma_commit(&s_full[t]);
-              pend[t] = true;
-            }
+            ptx::umma_commit(&s_full_t[h]);
           }
-          if (!alive) break;
-          if (s > 0) ptx::umma_commit(&kv_empty[slot_v % kStages]);
-          if (s < steps) ptx::umma_commit(&kv_empty[slot_k % kStages]);
+          if (Cfg::kHalves == 1 || h == 1) ptx::umma_commit(&kv_empty[slot]);
           // Q is read by the S products only: after the last of them the next item's Q may load, while the last
           // P V products and the epilogue of this item still run
-          if (s == steps - 1) ptx::umma_commit(q_empty);
+          if (ends) ptx::umma_commit(q_empty);
         }
+        pend[h] = vis;
+        owed[h] = true;
+        v_pair[h] = pair;
+        v_par[h] = par;
+        if (Cfg::kHalves == 1 || h == 1) {
+          if (++pair == Cfg::kPairs) { pair = 0; par ^= 1; }
+        }
+      }
+      if (!alive) break;
+      if (info & kInfoLast) {
+        do_pv(0);
+        if (alive) do_pv(1);
         if (!alive) break;
-        if (steps == 0) ptx::umma_commit(q_empty);
-#pragma unroll
-        for (int t = 0; t < kQTiles; ++t) {
-          if (it.qa + t * kBlockM < it.qb) ptx::umma_commit(&o_full[t]);
-        }
-        slot += 2 * steps;
-        ++n_item;
+        if ((info & (kInfoTile0 << t)) && ptx::elect_one()) ptx::umma_commit(&o_full[t]);
       }
     }
   }
@@ -529,10 +486,10 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
     const int quad = warp & 3;                     // tensor-memory lane quadrant of this warp
     const int row = quad * 32 + lane;              // row inside the tile
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t tmem_s = tmem + Cfg::kTmemS + t * 128 + lane_addr;
+    const uint32_t tmem_s = tmem + t * kBufs * kSubKeys + lane_addr;
     const uint32_t tmem_o = tmem + Cfg::kTmemO + t * kHeadDim + lane_addr;
-    const uint32_t tmem_p = tmem + Cfg::kTmemP + t * Cfg::kPStride + lane_addr;
-    uint32_t cnt_s = 0, cnt_o = 0;
+    uint32_t s_par = 0;   // bit b: parity of the next S in buffer b
+    uint32_t cnt_o = 0;
     bool alive = true;
     uint8_t* stage_o = sStageO + t * Cfg::kStageOBytes;
     for (uint32_t n_sched = 0; alive; ++n_sched) {
@@ -545,7 +502,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       if (!it.valid) continue;
       const int ta = it.qa + t * kBlockM;
       if (ta >= it.qb) continue;
-      const int steps = plan.steps();
+      const int subs = plan.steps() * Cfg::kHalves;
       const int r = ta + row;                      // position in the half
       const bool row_valid = r < it.n;
       const int r_eff = row_valid ? r : it.n - 1;
@@ -566,79 +523,75 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
           lse_scale *= qk;
         }
       }
-      // P is rounded to e4m3 for FP8: keep it in (0, 2^8] by advancing the maximum at every increase and shifting
-      // the exponent by 8 (the reference's Max_offset = 8, softmax.h:67-69 there); 16-bit P may run up to 2^8
-      // above 1 before the maximum is advanced.
-      constexpr float kThreshold = Cfg::kFp8 ? 0.f : kRescaleThreshold;
+      // P is rounded to e4m3 for FP8: the exponent is shifted by 8 (the reference's Max_offset = 8, softmax.h:67-69
+      // there) and the maximum advances when it grew by more than 0.8, so P stays below 2^8.8 = 445.8 of the type's
+      // 448. (Advancing it at every increase, as the reference does, rescales O several times as often: a warp's 32
+      // rows hardly ever all keep their maximum.) 16-bit P may run up to 2^8 above 1 before the maximum is advanced.
+      constexpr float kThreshold = Cfg::kFp8 ? 0.8f : kRescaleThreshold;
       constexpr float kPShift = Cfg::kFp8 ? 8.f : 0.f;
       float m_run = -INFINITY;  // reference maximum (unscaled scores, or tanh values with softcap)
       float l_run = 0.f;
       bool o_started = false;
-      for (int s = 0; s < steps && alive; ++s) {
+      int buf = 0;
+      for (int u = 0; u < subs && alive; ++u, buf = buf + 1 == kBufs ? 0 : buf + 1) {
         int kh, kt;
-        plan.step(s, kh, kt);
-        const int cls = spans.classify(kh, kt);
+        plan.step(u / Cfg::kHalves, kh, kt);
+        const int k0 = kt * Cfg::kSlotKeys + (u % Cfg::kHalves) * kSubKeys;
+        const int cls = spans.classify(kh, k0);
         if (cls == kTileSkip) continue;
-        if (!ptx::mbar_wait(&s_full[t], cnt_s & 1, abort_flag, 31)) { alive = false; break; }
-        ++cnt_s;
+        if (!ptx::mbar_wait(&s_full[t * kBufs + buf], (s_par >> buf) & 1u, abort_flag, 31)) { alive = false; break; }
+        s_par ^= 1u << buf;
         ptx::tc_fence_after();
-        float v[kBlockN];
+        const uint32_t tmem_sb = tmem_s + buf * kSubKeys;
+        float v[kSubKeys];
         {
-          uint32_t* u = reinterpret_cast<uint32_t*>(v);
+          uint32_t* w = reinterpret_cast<uint32_t*>(v);
 #pragma unroll
-          for (int c = 0; c < kBlockN / 32; ++c) ptx::tmem_ld32(tmem_s + c * 32, u + c * 32);
+          for (int c = 0; c < kSubKeys / 32; ++c) ptx::tmem_ld32(tmem_sb + c * 32, w + c * 32);
           ptx::tmem_wait_ld();
-        }
-        // cnt_s - 1 tiles came before this one. With P in its own columns: S may be overwritten from here on, and
-        // the P V product of the previous tile must have completed before O is rescaled or P is overwritten (with P
-        // in place of S the S product of this tile already followed it through the pipe).
-        bool pv_done = !Cfg::kOwnP;
-        auto wait_pv = [&]() -> bool {
-          if (pv_done) return true;
-          pv_done = true;
-          if (!ptx::mbar_wait(&p_free[t], cnt_s & 1, abort_flag, 33)) return false;
-          ptx::tc_fence_after();
-          return true;
-        };
-        if (Cfg::kOwnP) {
-          ptx::tc_fence_before();
-          ptx::mbar_arrive_warp(&s_free[t]);
         }
         if (kSoftcap) {
 #pragma unroll
-          for (int c = 0; c < kBlockN; ++c) v[c] = ptx::tanh_fast(v[c] * softcap_pre);
+          for (int c = 0; c < kSubKeys; ++c) v[c] = ptx::tanh_fast(v[c] * softcap_pre);
         }
         if (cls == kTileMasked) {
           int lo, hi;
           if (it.qh == 1) { lo = 0; hi = blk1; }
           else if (kh == 1) { lo = 0; hi = blk0; }
           else { lo = blk0; hi = blk1; }
-          lo -= kt * kBlockN;
-          hi -= kt * kBlockN;
+          lo -= k0;
+          hi -= k0;
 #pragma unroll
-          for (int c = 0; c < kBlockN; ++c) {
+          for (int c = 0; c < kSubKeys; ++c) {
             if (c < lo || c >= hi) v[c] = -INFINITY;
           }
         }
-        // eight independent running maxima (a single chain of 127 dependent max operations costs more than the
-        // exponentials that follow)
+        // eight independent running maxima (one chain of dependent max operations costs more than the exponentials
+        // that follow)
         float mx[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) mx[i] = fmaxf(v[2 * i], v[2 * i + 1]);
 #pragma unroll
-        for (int c = 16; c < kBlockN; c += 16) {
+        for (int c = 16; c < kSubKeys; c += 16) {
 #pragma unroll
           for (int i = 0; i < 8; ++i) mx[i] = ptx::max3(mx[i], v[c + 2 * i], v[c + 2 * i + 1]);
         }
-        const float m_tile = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])),
-                                   fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7])));
+        const float m_tile = fmaxf(ptx::max3(mx[0], mx[1], mx[2]), ptx::max3(ptx::max3(mx[3], mx[4], mx[5]), mx[6], mx[7]));
         const float m_new = fmaxf(m_run, m_tile);
         // advance the reference maximum only when it grew by more than the threshold (always on the first tile)
         const bool need = (m_new - m_run) * scale_log2 > kThreshold;
         if (__any_sync(0xffffffffu, need)) {
           const float factor = need ? ptx::ex2((m_run - m_new) * scale_log2) : 1.f;
           if (o_started) {
-            if (!wait_pv()) { alive = false; break; }
+            // every P V of this tile so far must have updated O. In this buffer it has: S followed it through the
+            // pipe. In the others the last one may still run (an unused buffer's barrier passes at once).
+#pragma unroll
+            for (int b = 0; b < kBufs; ++b) {
+              if (b == buf) continue;
+              if (!ptx::mbar_wait(&pv_done[t * kBufs + b], ((s_par >> b) & 1u) ^ 1u, abort_flag, 33)) { alive = false; break; }
+            }
+            if (!alive) break;
+            ptx::tc_fence_after();
 #pragma unroll
             for (int c = 0; c < kHeadDim / 32; ++c) {
               uint32_t o[32];
@@ -658,7 +611,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
         uint32_t pk[Cfg::kPCols];
         if (Cfg::kFp8) {
 #pragma unroll
-          for (int c = 0; c < kBlockN; c += 4) {
+          for (int c = 0; c < kSubKeys; c += 4) {
             const float p0 = ptx::ex2(fmaf(v[c], scale_log2, neg_m));
             const float p1 = ptx::ex2(fmaf(v[c + 1], scale_log2, neg_m));
             const float p2 = ptx::ex2(fmaf(v[c + 2], scale_log2, neg_m));
@@ -670,7 +623,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
           // two elements per FMA and per ADD: the sums run as four pairs of partial sums
           float sumb[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-          for (int c = 0; c < kBlockN; c += 2) {
+          for (int c = 0; c < kSubKeys; c += 2) {
             float y0, y1;
             ptx::fma2(y0, y1, v[c], v[c + 1], scale_log2, scale_log2, neg_m, neg_m);
             const float p0 = ptx::ex2(y0);
@@ -682,12 +635,11 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
           for (int i = 0; i < 4; ++i) sum4[i] += sumb[i];
         }
         l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
-        if (!wait_pv()) { alive = false; break; }
-#pragma unroll
-        for (int c = 0; c < Cfg::kPCols / 32; ++c) ptx::tmem_st32(tmem_p + c * 32, pk + c * 32);
+        if (Cfg::kPCols == 32) ptx::tmem_st32(tmem_sb, pk);
+        else ptx::tmem_st16(tmem_sb, pk);
         ptx::tmem_wait_st();
         ptx::tc_fence_before();
-        ptx::mbar_arrive_warp(&p_full[t]);
+        ptx::mbar_arrive_warp(&p_full[t * kBufs + buf]);
         o_started = true;
       }
       if (!alive) break;
@@ -773,10 +725,10 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
   if (warp == Cfg::kLoadWarp) ptx::tmem_dealloc(tmem, 512);
 }
 
-template <int kHeadDim, int kQTiles, int kStages, int kType, bool kSoftcap>
+template <int kHeadDim, int kQTiles, int kType, bool kSoftcap>
 int launch_fwd_instance(const FwdParams& p, int grid, cudaStream_t stream) {
-  using Cfg = FwdConfig<kHeadDim, kQTiles, kStages, kType, kSoftcap>;
-  auto kernel = fwd_kernel<kHeadDim, kQTiles, kStages, kType, kSoftcap>;
+  using Cfg = FwdConfig<kHeadDim, kQTiles, kType, kSoftcap>;
+  auto kernel = fwd_kernel<kHeadDim, kQTiles, kType, kSoftcap>;
   static PerDeviceFlags smem_set;
   const int rc = set_dynamic_smem(kernel, Cfg::kSmemBytes, smem_set);
   if (rc) return rc;
@@ -785,20 +737,20 @@ int launch_fwd_instance(const FwdParams& p, int grid, cudaStream_t stream) {
   return FDA_OK;
 }
 
-template <int kHeadDim, int kQTiles, int kStages>
+template <int kHeadDim, int kQTiles>
 int dispatch_fwd(const FwdParams& p, int grid, bool bf16, bool softcap, cudaStream_t stream) {
   if (bf16) {
-    return softcap ? launch_fwd_instance<kHeadDim, kQTiles, kStages, 0, true>(p, grid, stream)
-                   : launch_fwd_instance<kHeadDim, kQTiles, kStages, 0, false>(p, grid, stream);
+    return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 0, true>(p, grid, stream)
+                   : launch_fwd_instance<kHeadDim, kQTiles, 0, false>(p, grid, stream);
   }
-  return softcap ? launch_fwd_instance<kHeadDim, kQTiles, kStages, 1, true>(p, grid, stream)
-                 : launch_fwd_instance<kHeadDim, kQTiles, kStages, 1, false>(p, grid, stream);
+  return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 1, true>(p, grid, stream)
+                 : launch_fwd_instance<kHeadDim, kQTiles, 1, false>(p, grid, stream);
 }
 
-template <int kHeadDim, int kQTiles, int kStages>
+template <int kHeadDim, int kQTiles>
 int dispatch_fwd_fp8(const FwdParams& p, int grid, bool softcap, cudaStream_t stream) {
-  return softcap ? launch_fwd_instance<kHeadDim, kQTiles, kStages, 2, true>(p, grid, stream)
-                 : launch_fwd_instance<kHeadDim, kQTiles, kStages, 2, false>(p, grid, stream);
+  return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 2, true>(p, grid, stream)
+                 : launch_fwd_instance<kHeadDim, kQTiles, 2, false>(p, grid, stream);
 }
 
 }  // namespace
@@ -819,7 +771,7 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
   const bool fp8 = pr.dtype == FDA_E4M3;
   // FP8 rows are padded to whole 128-byte panels, so the smallest FP8 kernel is the 128-wide one
   const int d_round = (d <= 64 && !fp8) ? 64 : (d <= 128 ? 128 : 256);
-  const int q_tiles = d_round <= 128 ? 2 : 1;
+  const int slot_keys = (d_round == 256 && !fp8) ? 64 : 128;   // FwdConfig::kSlotKeys
   const int eb = fp8 ? 1 : 2;
   const int box_cols = 128 / eb;
   const bool varlen = pr.cu_seqlens != nullptr;
@@ -827,16 +779,26 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
   const int tma_batch = varlen ? 1 : pr.batch;
   const bool fp16 = pr.dtype == FDA_FP16;
 
+  int grid = info.sm_count - (pr.sm_margin > 0 ? pr.sm_margin : 0);
+  if (grid < 1) grid = 1;
+  // Items of two query tiles share the K and V they read. Where even items of one tile find an SM each, one tile per
+  // item halves the time of the longest item instead. (Packed batches: by the upper bound that the host knows.)
+  auto item_bound = [&](int tiles) -> int64_t {
+    if (varlen) return (static_cast<int64_t>(pr.total) / (2 * tiles * kBlockM) + pr.batch) * 2 * pr.heads;
+    return static_cast<int64_t>(ceil_div(pr.seqlen / 2, tiles * kBlockM)) * 2 * pr.heads * pr.batch;
+  };
+  const int q_tiles = d_round > 128 || item_bound(1) <= grid ? 1 : 2;
+
   FwdParams p;
   memset(&p, 0, sizeof(p));
   rc = encode_tile_map(&p.tm_q, a.q.ptr, eb, fp8, fp16, d, rows, pr.heads, tma_batch, a.q.row_stride,
                        a.q.head_stride, a.q.batch_stride, box_cols, kBlockM);
   if (rc) return rc;
   rc = encode_tile_map(&p.tm_k, a.k.ptr, eb, fp8, fp16, d, rows, pr.heads_k, tma_batch, a.k.row_stride,
-                       a.k.head_stride, a.k.batch_stride, box_cols, kBlockN);
+                       a.k.head_stride, a.k.batch_stride, box_cols, slot_keys);
   if (rc) return rc;
   rc = encode_tile_map(&p.tm_v, a.v.ptr, eb, fp8, fp16, d, rows, pr.heads_k, tma_batch, a.v.row_stride,
-                       a.v.head_stride, a.v.batch_stride, box_cols, kBlockN);
+                       a.v.head_stride, a.v.batch_stride, box_cols, slot_keys);
   if (rc) return rc;
   if (fp8) {
     p.q_descale = a.q_descale;
@@ -888,8 +850,6 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
   if (p.total_items <= 0) return FDA_OK;
   if (!a.workspace || a.workspace_bytes < fwd_workspace_bytes(pr)) return FDA_ERR_WORKSPACE;
   p.ticket = static_cast<int*>(a.workspace);
-  int grid = info.sm_count - (pr.sm_margin > 0 ? pr.sm_margin : 0);
-  if (grid < 1) grid = 1;
   // the shortest eighths of every (sample, head) run at the end; few items per CTA: rank for rank over all of them
   p.n_long = order_n_long(2 * p.items_per_half, FDA_SHORT8_FWD, p.total_items, grid);
   if (varlen) {
@@ -900,8 +860,7 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
     if (rc) return rc;
     p.vl.base = list;
     p.vl.batch = pr.batch;
-    const int64_t bound = (static_cast<int64_t>(pr.total) / (2 * q_tiles * kBlockM) + pr.batch) * 2 * pr.heads;
-    if (grid > bound) grid = static_cast<int>(bound);
+    if (grid > item_bound(q_tiles)) grid = static_cast<int>(item_bound(q_tiles));
   } else if (grid >= p.total_items) {
     grid = p.total_items;   // a block for every item: no work counter, nothing to zero
     p.ticket = nullptr;
@@ -910,15 +869,15 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
   }
   const bool bf16 = pr.dtype == FDA_BF16;
   if (fp8) {
-    if (d_round == 128) return dispatch_fwd_fp8<128, 2, 6>(p, grid, softcap, stream);
-    return dispatch_fwd_fp8<256, 1, 4>(p, grid, softcap, stream);
+    if (d_round == 256) return dispatch_fwd_fp8<256, 1>(p, grid, softcap, stream);
+    return q_tiles == 2 ? dispatch_fwd_fp8<128, 2>(p, grid, softcap, stream) : dispatch_fwd_fp8<128, 1>(p, grid, softcap, stream);
   }
-  if (d_round == 64) return dispatch_fwd<64, 2, 6>(p, grid, bf16, softcap, stream);
-  if (d_round == 128) return dispatch_fwd<128, 2, 4>(p, grid, bf16, softcap, stream);
-  return dispatch_fwd<256, 1, 2>(p, grid, bf16, softcap, stream);
+  if (d_round == 256) return dispatch_fwd<256, 1>(p, grid, bf16, softcap, stream);
+  if (d_round == 128) {
+    return q_tiles == 2 ? dispatch_fwd<128, 2>(p, grid, bf16, softcap, stream) : dispatch_fwd<128, 1>(p, grid, bf16, softcap, stream);
+  }
+  return q_tiles == 2 ? dispatch_fwd<64, 2>(p, grid, bf16, softcap, stream) : dispatch_fwd<64, 1>(p, grid, bf16, softcap, stream);
 }
-
-
 
 int read_status_fwd(int32_t* out4) {
   int zero[4] = {0, 0, 0, 0};

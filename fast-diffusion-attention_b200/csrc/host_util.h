@@ -70,9 +70,19 @@ inline int encode_tile_map(CUtensorMap* map, const void* ptr, int elem_bytes, bo
   cuuint32_t estride[4] = {1, 1, 1, 1};
   CUtensorMapDataType dt = is_fp8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                                   : (is_fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16);
-  CUresult r = enc(map, dt, 4, const_cast<void*>(ptr), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&]() {
+    return enc(map, dt, 4, const_cast<void*>(ptr), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // A thread whose first CUDA work this is (an autograd thread whose allocations came out of the cache) has no current
+    // context yet: the driver call wants one, and nothing of the runtime has bound it. cudaSetDevice does.
+    int dev = 0;
+    FDA_CUDA_TRY(cudaGetDevice(&dev));
+    FDA_CUDA_TRY(cudaSetDevice(dev));
+    r = encode();
+  }
   if (r != CUDA_SUCCESS) {
     snprintf(cuda_error_buf(), 256, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
     return FDA_ERR_CUDA;

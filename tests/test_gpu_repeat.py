@@ -106,3 +106,22 @@ def test_no_wait_expires_over_many_backward_passes(heads, heads_k, d):
         torch.autograd.grad(diffusion_attn_func(q, k, v, 64), (q, k, v), do)
     torch.cuda.synchronize()
     assert _lib.device_status()[0] == 0
+
+
+def test_first_call_of_a_new_thread():
+    """A thread that has done no CUDA work has no current context, and with every allocation out of the cache nothing
+    binds one before the tensor maps are encoded. Autograd threads are such threads."""
+    import threading
+    torch.manual_seed(11)
+    q, k, v = (torch.randn(1, 512, 2, 64, device=DEV, dtype=torch.bfloat16) for _ in range(3))
+    want = diffusion_attn_func(q, k, v, 32)
+    del want
+    torch.cuda.synchronize()
+    want = diffusion_attn_func(q, k, v, 32)
+    spare = diffusion_attn_func(q, k, v, 32)
+    del spare   # the thread's output comes from here
+    got = []
+    thread = threading.Thread(target=lambda: got.append(diffusion_attn_func(q, k, v, 32)))
+    thread.start()
+    thread.join()
+    assert len(got) == 1 and torch.equal(got[0], want)

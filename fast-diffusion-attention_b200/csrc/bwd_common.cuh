@@ -120,7 +120,7 @@ static_assert(kCols == 32, "one 32-column tensor-memory load per operand and war
 // P and dS of kN columns for one thread. `s`/`dp` hold the raw accumulators; the results are packed 16-bit.
 // lse2 / delta are per column (kPerColumn, read from shared memory) or per thread. kMasked is a template
 // parameter so that the common fully-visible tile carries no per-element compare/select at all.
-template <int kN, bool kBf16, bool kSoftcap, bool kPerColumn, bool kMasked, bool kNeedP>
+template <int kN, bool kBf16, bool kSoftcap, bool kPerColumn, bool kMasked, bool kNeedP, bool kNeedDs = true>
 __device__ __forceinline__ void softmax_backward_cols(const uint32_t* s, const uint32_t* dp, const float* lse2_col,
                                                       const float* delta_col, float lse2_row, float delta_row,
                                                       float scale_log2, float softcap_pre, int lo, int hi,
@@ -142,7 +142,7 @@ __device__ __forceinline__ void softmax_backward_cols(const uint32_t* s, const u
       float pr = ptx::ex2(fmaf(x, scale_log2, -l2));
       // the derivative of the cap goes onto P first: the single-pass backward computes P (1 - tanh^2) in the first
       // half of its arithmetic and meets dP only in the second, and both forms round alike
-      float d = (kSoftcap ? pr * dt : pr) * (__uint_as_float(dp[col]) - dl);
+      float d = kNeedDs ? (kSoftcap ? pr * dt : pr) * (__uint_as_float(dp[col]) - dl) : 0.f;
       if (kMasked && (col < lo || col >= hi)) {
         pr = 0.f;
         d = 0.f;
@@ -151,7 +151,7 @@ __device__ __forceinline__ void softmax_backward_cols(const uint32_t* s, const u
       dsv[e] = d;
     }
     if (kNeedP) pk_p[c / 2] = ptx::pack2<kBf16>(pv[0], pv[1]);
-    pk_ds[c / 2] = ptx::pack2<kBf16>(dsv[0], dsv[1]);
+    if (kNeedDs) pk_ds[c / 2] = ptx::pack2<kBf16>(dsv[0], dsv[1]);
   }
 }
 

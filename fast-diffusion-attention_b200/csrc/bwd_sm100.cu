@@ -22,6 +22,8 @@
 // Numerics kept from the reference: P = exp2(S*c - LSE2) from the saved LSE, dS = P * (dP - delta)
 // [* (1 - tanh^2) with softcap, before masking], P and dS rounded to the input dtype before the second GEMMs,
 // dK and dQ scaled by softmax_scale once at the end (mainloop_bwd...hpp:836-893, :1009).
+#include <type_traits>
+
 #include "bwd_common.cuh"
 
 namespace fda {
@@ -125,19 +127,29 @@ struct DkdvCfg {
   using T = TileCfg<kHeadDim>;
   static constexpr int kSubTileBytes = kSub * kHeadDim * 2;     // Q or dO sub-tile
   static constexpr int kSubPanelBytes = kSub * 128;             // one 64-column panel of a sub-tile
-  static constexpr int kStageBytes = 2 * kSubTileBytes + 1024;  // Q sub-tile, dO sub-tile, lse2[64], delta[64], header
-  static constexpr int kHeaderOffset = 2 * kSubTileBytes + 512;
-  static constexpr int kSmemBytes = 2 * T::kTileBytes + kStages * kStageBytes + 1024 + 512;
   static constexpr int kThreads = kDkdvThreads;
   // buffer u: S^T at u*128, dP^T at u*128 + 64; accumulators behind
-  // head dimensions above 128 do not leave room for both accumulators next to the S^T / dP^T buffers: the key
-  // tile is then processed in kPasses passes, each producing kAccDim columns of dK and dV
-  static constexpr int kAccDim = kHeadDim > 128 ? 128 : kHeadDim;
-  static constexpr int kPasses = kHeadDim / kAccDim;
-  static constexpr int kLookahead = kStages >= 2 ? 2 : 1;  // S^T / dP^T sub-steps issued ahead of dV / dK
-  static constexpr int kTmemDK = 256, kTmemDV = 256 + kAccDim;
-  static_assert(256 + 2 * kAccDim <= 512, "tensor memory budget");
-  static_assert(kStageBytes % 1024 == 0, "sub-tiles must stay 1024-byte aligned for the 128-byte swizzle");
+  // Head dimensions above 128 do not leave room for both accumulators next to the S^T / dP^T buffers: every key tile is
+  // two items, one for dK (three products: S^T, dP^T, dS^T Q) and one for dV (two: S^T, P^T dO). Halving the columns of
+  // both instead takes S^T and dP^T twice, six products for five. (Backward of 2 x 16384 tokens, 8 heads of 256, blocks of
+  // 256: 7.34 -> 4.97 ms with the rings below.)
+  static constexpr int kPasses = kHeadDim > 128 ? 2 : 1;
+  static constexpr int kTmemDK = 256, kTmemDV = kPasses == 2 ? 256 : 256 + kHeadDim;
+  static_assert(kTmemDV + kHeadDim <= 512, "tensor memory budget");
+  // Rings of Q and dO sub-tiles of their own. With 128 KB of K and V there is room for three of 32 KB: two for Q, one for
+  // dO, so that the next sub-step's tiles load while this one's are in use (one slot for both left the pipe waiting for
+  // every load).
+  static constexpr int kQSlots = kPasses == 2 ? 2 : kStages, kDoSlots = kPasses == 2 ? 1 : kStages;
+  // lse2[64], delta[64] and the header of a sub-step. The slot of step x is written when Q of step x - 2 is done with,
+  // which for dV means S^T of x - 2 complete, so that step x - 4 is the last that every role has certainly left.
+  static constexpr int kStatSlots = kPasses == 2 ? 4 : kStages;
+  static constexpr int kHeaderOffset = 2 * kSub * 4, kStatBytes = kHeaderOffset + 32;
+  static constexpr int kOffQ = 2 * T::kTileBytes, kOffDo = kOffQ + kQSlots * kSubTileBytes;
+  static constexpr int kOffStat = kOffDo + kDoSlots * kSubTileBytes;
+  static constexpr int kOffBar = kOffStat + kStatSlots * kStatBytes;
+  static constexpr int kSmemBytes = kOffBar + 512;
+  static_assert(kSmemBytes <= 232448 && kOffBar % 16 == 0, "shared memory budget");
+  static_assert((11 + 2 * kQSlots + 2 * kDoSlots + kStatSlots) * 8 + 8 <= 384, "barrier area");
 };
 
 // Sub-steps of one item: query heads of the group x visible 128-row query tiles x two 64-row halves; a half
@@ -145,35 +157,56 @@ template <int kHeadDim, int kStages, bool kBf16, bool kSoftcap>
 __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_constant__ BwdParams p) {
   using Cfg = DkdvCfg<kHeadDim, kStages>;
   using T = TileCfg<kHeadDim>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  // The tiles need 1024-byte alignment for the 128-byte swizzle. Dynamic shared memory starts at the beginning of the
+  // block's window, which is aligned that far; head dimension 256 leaves no room to round the base up, so a base that is
+  // not aligned is reported through the status word instead.
+  extern __shared__ __align__(1024) uint8_t smem_dkdv[];
+  uint8_t* smem = smem_dkdv;
   uint8_t* sK = smem;
   uint8_t* sV = smem + T::kTileBytes;
-  uint8_t* sStage = smem + 2 * T::kTileBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStage + kStages * Cfg::kStageBytes);
+  uint8_t* sQ = smem + Cfg::kOffQ;
+  uint8_t* sDo = smem + Cfg::kOffDo;
+  uint8_t* sStat = smem + Cfg::kOffStat;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBar);
   uint64_t* kv_full = bars;
   uint64_t* kv_empty = bars + 1;
-  uint64_t* st_full = bars + 2;
-  uint64_t* st_empty = st_full + kStages;
-  uint64_t* sdp_full = st_empty + kStages;   // [2]
+  uint64_t* q_full = bars + 2;                    // [kQSlots]
+  uint64_t* q_empty = q_full + Cfg::kQSlots;
+  uint64_t* do_full = q_empty + Cfg::kQSlots;     // [kDoSlots]
+  uint64_t* do_empty = do_full + Cfg::kDoSlots;
+  uint64_t* stat_full = do_empty + Cfg::kDoSlots; // [kStatSlots] statistics and header
+  uint64_t* sdp_full = stat_full + Cfg::kStatSlots;   // [2]
   uint64_t* pds_full = sdp_full + 2;         // [2]
   uint64_t* acc_full = pds_full + 2;
   uint64_t* buf_free = acc_full + 1;         // [2]
   uint64_t* acc_free = buf_free + 2;         // the epilogue warps have the accumulators in registers
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_free + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  SchedMailbox* mbox = reinterpret_cast<SchedMailbox*>(reinterpret_cast<uint8_t*>(bars) + 256);
+  SchedMailbox* mbox = reinterpret_cast<SchedMailbox*>(reinterpret_cast<uint8_t*>(bars) + 384);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if ((ptx::smem_u32(smem) & 1023u) != 0) {
+    if (threadIdx.x == 0 && atomicCAS(&g_fda_status[0], 0, 120) == 0) {
+      g_fda_status[1] = static_cast<int>(blockIdx.x);
+      g_fda_status[2] = 0;
+      g_fda_status[3] = static_cast<int>(ptx::smem_u32(smem) & 1023u);
+    }
+    return;
+  }
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     sched_init(mbox, 4 * kCmpWG + 2 + 4);   // compute warps, two MMA issuers, four epilogue warps
     ptx::mbar_init(kv_full, 1);
     ptx::mbar_init(kv_empty, 1);
-    for (int i = 0; i < kStages; ++i) {
-      ptx::mbar_init(&st_full[i], 1);
-      ptx::mbar_init(&st_empty[i], 1);
+    for (int i = 0; i < Cfg::kQSlots; ++i) {
+      ptx::mbar_init(&q_full[i], 1);
+      ptx::mbar_init(&q_empty[i], 1);
     }
+    for (int i = 0; i < Cfg::kDoSlots; ++i) {
+      ptx::mbar_init(&do_full[i], 1);
+      ptx::mbar_init(&do_empty[i], 1);
+    }
+    for (int i = 0; i < Cfg::kStatSlots; ++i) ptx::mbar_init(&stat_full[i], 1);
     for (int u = 0; u < 2; ++u) {
       ptx::mbar_init(&sdp_full[u], 1);
       ptx::mbar_init(&pds_full[u], 4 * kCmpWG);
@@ -194,6 +227,9 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
   const int bs = p.block_size;
   const int group = p.heads / p.heads_k;
   const int total_items = kv_item_count(p) * Cfg::kPasses;
+  // what the item with this index makes
+  auto makes_dk = [](int idx) { return Cfg::kPasses == 1 || (idx & 1) == 0; };
+  auto makes_dv = [](int idx) { return Cfg::kPasses == 1 || (idx & 1) == 1; };
 
   // Calls fn(SubStep) for every non-skipped sub-step of the item, in order; stops early when fn returns false.
   auto for_each_substep = [&](const KvItem& it, const QueryPlan& plan, const KvSpans& spans, auto&& fn) -> bool {
@@ -237,7 +273,6 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       if (idx < 0 || idx >= total_items) break;
       const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
       if (!it.valid) continue;
-      const int pass_col0 = (idx % Cfg::kPasses) * Cfg::kAccDim;
       const int kj = it.k0 + row;
       const int rows_valid = imax(0, imin(32, it.n - (it.k0 + quad * 32)));  // of this warp's 32 key rows
       const int64_t srow = static_cast<int64_t>(it.row0) + it.kh * it.n + kj;
@@ -246,12 +281,12 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       if (!ptx::mbar_wait(acc_full, n_item & 1, abort_flag, 62)) break;
       ++n_item;
       ptx::tc_fence_after();
-      // dK and dV sit side by side in tensor memory: 2 * d / 32 chunks of 32 columns
-      constexpr int kChunks = 2 * Cfg::kAccDim / 32;
+      // dK and dV sit side by side in tensor memory (or the item makes one of them): chunks of 32 columns
+      constexpr int kChunks = (Cfg::kPasses == 2 ? 1 : 2) * kHeadDim / 32;
 #pragma unroll 1
       for (int gidx = 0; gidx < kChunks; ++gidx) {
-        const bool is_dv = gidx * 32 >= Cfg::kAccDim;
-        const int col0 = pass_col0 + gidx * 32 - (is_dv ? Cfg::kAccDim : 0);
+        const bool is_dv = Cfg::kPasses == 2 ? makes_dv(idx) : gidx * 32 >= kHeadDim;
+        const int col0 = gidx * 32 - (Cfg::kPasses == 1 && is_dv ? kHeadDim : 0);
         uint32_t accv[32];
         ptx::tmem_ld32(tmem + Cfg::kTmemDK + lane_addr + gidx * 32, accv);
         ptx::tmem_wait_ld();
@@ -283,31 +318,38 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         const QueryPlan plan = make_query_plan(it.kh, it.k0, it.k1, it.n, bs, kTile);
         const KvSpans spans = make_kv_spans(it, bs);
         if (!ptx::mbar_wait(kv_empty, (n_item & 1) ^ 1, abort_flag, 41)) break;
-        ptx::mbar_expect_tx(kv_full, 2 * T::kTileBytes);
+        ptx::mbar_expect_tx(kv_full, (makes_dk(idx) ? 2 : 1) * T::kTileBytes);
         const int k_row = it.row0 + it.kh * it.n + it.k0;
         load_tile<kHeadDim>(sK, &p.tm_k, kv_full, k_row, it.hk, it.bcoord);
-        load_tile<kHeadDim>(sV, &p.tm_v, kv_full, k_row, it.hk, it.bcoord);
-        // The loader alone walks the item's geometry. Each stage carries a two-word header for the other roles:
+        if (makes_dk(idx)) load_tile<kHeadDim>(sV, &p.tm_v, kv_full, k_row, it.hk, it.bcoord);
+        // The loader alone walks the item's geometry. Each sub-step carries a two-word header for the other roles:
         // {bit 0 last sub-step of the item, bit 1 partially masked, bit 2 queries of the keys' own half; first row}.
         // A sub-step is sent when its successor is known, so that the last one can be marked.
         auto emit = [&](const SubStep& st, bool last) -> bool {
-          const uint32_t stage = gc % kStages;
-          if (!ptx::mbar_wait(&st_empty[stage], ((gc / kStages) & 1) ^ 1, abort_flag, 42)) return false;
-          uint8_t* base = sStage + stage * Cfg::kStageBytes;
-          volatile int* hdr = reinterpret_cast<volatile int*>(base + Cfg::kHeaderOffset);
+          const uint32_t qs = gc % Cfg::kQSlots, ds = gc % Cfg::kDoSlots, ss = gc % Cfg::kStatSlots;
+          if (!ptx::mbar_wait(&q_empty[qs], ((gc / Cfg::kQSlots) & 1) ^ 1, abort_flag, 42)) return false;
+          uint8_t* stat = sStat + ss * Cfg::kStatBytes;
+          volatile int* hdr = reinterpret_cast<volatile int*>(stat + Cfg::kHeaderOffset);
           hdr[0] = (last ? 1 : 0) | (st.cls == kTileMasked ? 2 : 0) | (st.qh == it.kh ? 4 : 0);
           hdr[1] = st.sa;
-          ptx::mbar_expect_tx(&st_full[stage], 2 * Cfg::kSubTileBytes + 512);
+          ptx::mbar_expect_tx(&stat_full[ss], 2 * kSub * 4);
+          const int64_t seg = stat_segment(p, it.b, st.h, st.qh) + st.sa;
+          ptx::bulk_load_1d(stat, p.lse2_pad + seg, kSub * 4, &stat_full[ss]);
+          ptx::bulk_load_1d(stat + kSub * 4, p.delta_pad + seg, kSub * 4, &stat_full[ss]);
           const int q_row = it.row0 + st.qh * it.n + st.sa;
+          ptx::mbar_expect_tx(&q_full[qs], Cfg::kSubTileBytes);
 #pragma unroll
           for (int c = 0; c < T::kPanels; ++c) {
-            ptx::tma_load_4d(base + c * Cfg::kSubPanelBytes, &p.tm_q64, &st_full[stage], c * 64, q_row, st.h, it.bcoord);
-            ptx::tma_load_4d(base + Cfg::kSubTileBytes + c * Cfg::kSubPanelBytes, &p.tm_do64, &st_full[stage], c * 64,
+            ptx::tma_load_4d(sQ + qs * Cfg::kSubTileBytes + c * Cfg::kSubPanelBytes, &p.tm_q64, &q_full[qs], c * 64, q_row,
+                             st.h, it.bcoord);
+          }
+          if (!ptx::mbar_wait(&do_empty[ds], ((gc / Cfg::kDoSlots) & 1) ^ 1, abort_flag, 43)) return false;
+          ptx::mbar_expect_tx(&do_full[ds], Cfg::kSubTileBytes);
+#pragma unroll
+          for (int c = 0; c < T::kPanels; ++c) {
+            ptx::tma_load_4d(sDo + ds * Cfg::kSubTileBytes + c * Cfg::kSubPanelBytes, &p.tm_do64, &do_full[ds], c * 64,
                              q_row, st.h, it.bcoord);
           }
-          const int64_t seg = stat_segment(p, it.b, st.h, st.qh) + st.sa;
-          ptx::bulk_load_1d(base + 2 * Cfg::kSubTileBytes, p.lse2_pad + seg, 256, &st_full[stage]);
-          ptx::bulk_load_1d(base + 2 * Cfg::kSubTileBytes + 256, p.delta_pad + seg, 256, &st_full[stage]);
           ++gc;
           return true;
         };
@@ -337,7 +379,8 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       constexpr uint32_t kHi = ptx::smem_desc_hi(1024);
       const uint32_t k_lo = ptx::smem_desc_lo(ptx::smem_u32(sK), 16);
       const uint32_t v_lo = ptx::smem_desc_lo(ptx::smem_u32(sV), 16);
-      const uint32_t st_lo_k = ptx::smem_desc_lo(ptx::smem_u32(sStage), 16);
+      const uint32_t q_lo = ptx::smem_desc_lo(ptx::smem_u32(sQ), 16);
+      const uint32_t do_lo = ptx::smem_desc_lo(ptx::smem_u32(sDo), 16);
       uint32_t n_item = 0, g = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
@@ -347,19 +390,38 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         if (!it.valid) continue;
         if (!ptx::mbar_wait(kv_full, n_item & 1, abort_flag, 51)) break;
         for (bool last = false; alive && !last; ++g) {
-          const uint32_t u = g & 1u, stage = g % kStages;
-          if (!ptx::mbar_wait(&st_full[stage], (g / kStages) & 1u, abort_flag, 52)) { alive = false; break; }
-          last = (*reinterpret_cast<const volatile int*>(sStage + stage * Cfg::kStageBytes + Cfg::kHeaderOffset) & 1) != 0;
+          const uint32_t u = g & 1u, qs = g % Cfg::kQSlots, ds = g % Cfg::kDoSlots, ss = g % Cfg::kStatSlots;
+          if (!ptx::mbar_wait(&stat_full[ss], (g / Cfg::kStatSlots) & 1u, abort_flag, 52)) { alive = false; break; }
+          last = (*reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset) & 1) != 0;
+          if (!ptx::mbar_wait(&q_full[qs], (g / Cfg::kQSlots) & 1u, abort_flag, 56)) { alive = false; break; }
           if (!ptx::mbar_wait(&buf_free[u], ((g >> 1) & 1u) ^ 1u, abort_flag, 54)) { alive = false; break; }
+          if (Cfg::kPasses == 1 &&
+              !ptx::mbar_wait(&do_full[ds], (g / Cfg::kDoSlots) & 1u, abort_flag, 58)) { alive = false; break; }
           ptx::tc_fence_after();
-          const uint32_t q_off = stage * (Cfg::kStageBytes >> 4);
-          const uint32_t do_off = q_off + (Cfg::kSubTileBytes >> 4);
-#pragma unroll
-          for (int kk = 0; kk < kHeadDim / 16; ++kk) {
+          const uint32_t q_off = qs * (Cfg::kSubTileBytes >> 4), do_off = ds * (Cfg::kSubTileBytes >> 4);
+          auto product = [&](int kk, uint32_t d_off, uint32_t a_lo, uint32_t b_lo) {
             const uint32_t a_off = ((kk / 4) * T::kPanelBytes + (kk % 4) * 32) >> 4;
             const uint32_t b_off = ((kk / 4) * Cfg::kSubPanelBytes + (kk % 4) * 32) >> 4;
-            ptx::umma_ss_f16_lh(tmem + u * 128, k_lo + a_off, st_lo_k + q_off + b_off, kHi, idesc_s, kk > 0);
-            ptx::umma_ss_f16_lh(tmem + u * 128 + 64, v_lo + a_off, st_lo_k + do_off + b_off, kHi, idesc_s, kk > 0);
+            ptx::umma_ss_f16_lh(tmem + u * 128 + d_off, a_lo + a_off, b_lo + b_off, kHi, idesc_s, kk > 0);
+          };
+          if (Cfg::kPasses == 1) {
+#pragma unroll
+            for (int kk = 0; kk < kHeadDim / 16; ++kk) {
+              product(kk, 0, k_lo, q_lo + q_off);
+              product(kk, 64, v_lo, do_lo + do_off);
+            }
+          } else {
+#pragma unroll
+            for (int kk = 0; kk < kHeadDim / 16; ++kk) product(kk, 0, k_lo, q_lo + q_off);
+            if (makes_dk(idx)) {
+              if (!ptx::mbar_wait(&do_full[ds], (g / Cfg::kDoSlots) & 1u, abort_flag, 58)) { alive = false; break; }
+              ptx::tc_fence_after();
+#pragma unroll
+              for (int kk = 0; kk < kHeadDim / 16; ++kk) product(kk, 64, v_lo, do_lo + do_off);
+              ptx::umma_commit(&do_empty[ds]);   // dK does not read dO
+            } else {
+              ptx::umma_commit(&q_empty[qs]);    // dV does not read Q
+            }
           }
           ptx::umma_commit(&sdp_full[u]);
         }
@@ -373,9 +435,10 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
     // ------------------------------------------------------------------- MMA issuer 2: dV += P^T dO, dK += dS^T Q
     if (lane == 0) {
       constexpr int kFmt = kBf16 ? 1 : 0;
-      const uint32_t idesc_g = ptx::make_idesc(kTile, Cfg::kAccDim, kFmt, false, true);
+      const uint32_t idesc_g = ptx::make_idesc(kTile, kHeadDim, kFmt, false, true);
       constexpr uint32_t kHi = ptx::smem_desc_hi(1024);
-      const uint32_t st_lo_mn = ptx::smem_desc_lo(ptx::smem_u32(sStage), Cfg::kSubPanelBytes);    // MN-major use
+      const uint32_t q_mn = ptx::smem_desc_lo(ptx::smem_u32(sQ), Cfg::kSubPanelBytes);    // MN-major use
+      const uint32_t do_mn = ptx::smem_desc_lo(ptx::smem_u32(sDo), Cfg::kSubPanelBytes);
       uint32_t g = 0, n_item_b = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
@@ -383,35 +446,36 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         if (idx < 0 || idx >= total_items) break;
         const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
         if (!it.valid) continue;
-        // descriptor offset of the first 64-column panel of this pass in a sub-tile
-        const uint32_t pass_panel_off = (idx % Cfg::kPasses) * (Cfg::kAccDim / 64) * (Cfg::kSubPanelBytes >> 4);
         bool acc = false;
         // the first products of an item overwrite the accumulators: the epilogue warps must have read the last item's
         if (!ptx::mbar_wait(acc_free, (n_item_b & 1u) ^ 1u, abort_flag, 57)) break;
         ++n_item_b;
         for (bool last = false; alive && !last; ++g) {
-          const uint32_t u = g & 1u, stage = g % kStages;
-          // the stage barrier orders the header and, through the other issuer's wait on it, nothing else here:
-          // the tiles themselves are read by the MMAs, after P^T / dS^T (pds_full) which follow S^T / dP^T
-          if (!ptx::mbar_wait(&st_full[stage], (g / kStages) & 1u, abort_flag, 55)) { alive = false; break; }
-          last = (*reinterpret_cast<const volatile int*>(sStage + stage * Cfg::kStageBytes + Cfg::kHeaderOffset) & 1) != 0;
+          const uint32_t u = g & 1u, qs = g % Cfg::kQSlots, ds = g % Cfg::kDoSlots, ss = g % Cfg::kStatSlots;
+          // the tiles are read after P^T / dS^T (pds_full), which follow products that have read them; only dO of an item
+          // that makes dV alone has not been waited for by anybody
+          if (!ptx::mbar_wait(&stat_full[ss], (g / Cfg::kStatSlots) & 1u, abort_flag, 55)) { alive = false; break; }
+          last = (*reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset) & 1) != 0;
           if (!ptx::mbar_wait(&pds_full[u], (g >> 1) & 1u, abort_flag, 53)) { alive = false; break; }
+          if (Cfg::kPasses == 2 && makes_dv(idx) &&
+              !ptx::mbar_wait(&do_full[ds], (g / Cfg::kDoSlots) & 1u, abort_flag, 59)) { alive = false; break; }
           ptx::tc_fence_after();
-          const uint32_t q_off = stage * (Cfg::kStageBytes >> 4);
-          const uint32_t do_off = q_off + (Cfg::kSubTileBytes >> 4);
+          const uint32_t q_off = qs * (Cfg::kSubTileBytes >> 4), do_off = ds * (Cfg::kSubTileBytes >> 4);
           const uint32_t st_t = tmem + u * 128, dpt_t = tmem + u * 128 + 64;
 #pragma unroll
           for (int kk = 0; kk < kSub / 16; ++kk) {
-            ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDV, st_t + kk * kSubCols,
-                                st_lo_mn + do_off + pass_panel_off + kk * (2048 >> 4), kHi, idesc_g,
-                                (acc || kk > 0) ? 1u : 0u);
-            ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDK, dpt_t + kk * kSubCols,
-                                st_lo_mn + q_off + pass_panel_off + kk * (2048 >> 4), kHi, idesc_g,
-                                (acc || kk > 0) ? 1u : 0u);
+            const uint32_t on = (acc || kk > 0) ? 1u : 0u;
+            if (makes_dv(idx)) {
+              ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDV, st_t + kk * kSubCols, do_mn + do_off + kk * (2048 >> 4), kHi, idesc_g, on);
+            }
+            if (makes_dk(idx)) {
+              ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDK, dpt_t + kk * kSubCols, q_mn + q_off + kk * (2048 >> 4), kHi, idesc_g, on);
+            }
           }
           acc = true;
           ptx::umma_commit(&buf_free[u]);
-          ptx::umma_commit(&st_empty[stage]);
+          if (makes_dk(idx)) ptx::umma_commit(&q_empty[qs]);
+          if (makes_dv(idx)) ptx::umma_commit(&do_empty[ds]);
         }
         if (!alive) break;
         ptx::umma_commit(acc_full);
@@ -431,7 +495,6 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       const int idx = sched_consume<true>(mbox, n_sched, abort_flag);
       if (idx < 0 || idx >= total_items) break;
       const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
-      const int pass_col0 = (idx % Cfg::kPasses) * Cfg::kAccDim;
       if (!it.valid) continue;
       const int kj = it.k0 + row;
       // queries that see this thread's key: same-half tiles and (clean keys only) noisy tiles of later blocks
@@ -439,11 +502,11 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       query_interval(it.kh, it.kh, kj, it.n, bs, same_lo, same_hi);
       query_interval(0, 1, kj, it.n, bs, cross_lo, cross_hi);
       for (bool last = false; alive && !last;) {
-        const uint32_t u = gc & 1u, stage = gc % kStages;
-        const uint8_t* stage_base = sStage + stage * Cfg::kStageBytes;
-        const float* stats = reinterpret_cast<const float*>(stage_base + 2 * Cfg::kSubTileBytes);
-        // wait on the stage barrier ourselves: it orders the header and the bulk copies of lse2 / delta before our reads
-        if (!ptx::mbar_wait(&st_full[stage], (gc / kStages) & 1u, abort_flag, 60)) { alive = false; break; }
+        const uint32_t u = gc & 1u, ss = gc % Cfg::kStatSlots;
+        const uint8_t* stage_base = sStat + ss * Cfg::kStatBytes;
+        const float* stats = reinterpret_cast<const float*>(stage_base);
+        // orders the header and the bulk copies of lse2 / delta before our reads
+        if (!ptx::mbar_wait(&stat_full[ss], (gc / Cfg::kStatSlots) & 1u, abort_flag, 60)) { alive = false; break; }
         int2 hdr;
         hdr.x = reinterpret_cast<const volatile int*>(stage_base + Cfg::kHeaderOffset)[0];
         hdr.y = reinterpret_cast<const volatile int*>(stage_base + Cfg::kHeaderOffset)[1];
@@ -468,25 +531,30 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         const uint32_t st_t = tmem + u * 128 + lane_addr + wg * kSubCols;
         const uint32_t dpt_t = st_t + 64;
         uint32_t sv[kSubCols], dpv[kSubCols];
-        ptx::tmem_ld16(st_t, sv);
-        ptx::tmem_ld16(dpt_t, dpv);
-        ptx::tmem_wait_ld();
+        const bool masked = (hdr.x & 2) != 0;
+        const int lo = ((hdr.x & 4) ? same_lo : cross_lo) - (hdr.y + wg * kSubCols);
+        const int hi = ((hdr.x & 4) ? same_hi : cross_hi) - (hdr.y + wg * kSubCols);
         uint32_t pk_p[kSubCols / 2], pk_ds[kSubCols / 2];
-        const float* l2 = l2r;
-        const float* dl = dlr;
-        if (hdr.x & 2) {
-          const int lo = ((hdr.x & 4) ? same_lo : cross_lo) - (hdr.y + wg * kSubCols);
-          const int hi = ((hdr.x & 4) ? same_hi : cross_hi) - (hdr.y + wg * kSubCols);
-          softmax_backward_cols<kSubCols, kBf16, kSoftcap, true, true, true>(sv, dpv, l2, dl, 0.f, 0.f, p.scale_log2,
-                                                                              p.softcap_pre, lo, hi, pk_p, pk_ds);
-        } else {
-          softmax_backward_cols<kSubCols, kBf16, kSoftcap, true, false, true>(sv, dpv, l2, dl, 0.f, 0.f, p.scale_log2,
-                                                                               p.softcap_pre, 0, 0, pk_p, pk_ds);
-        }
-        // a warp overwrites only columns it has itself already loaded: its packed P^T / dS^T pieces go to the
-        // start of its own kSubCols columns
-        ptx::tmem_st8(st_t, pk_p);
-        ptx::tmem_st8(dpt_t, pk_ds);
+        auto turn = [&](auto p_tag, auto ds_tag) {
+          constexpr bool kP = decltype(p_tag)::value, kDs = decltype(ds_tag)::value;
+          ptx::tmem_ld16(st_t, sv);
+          if (kDs) ptx::tmem_ld16(dpt_t, dpv);
+          ptx::tmem_wait_ld();
+          if (masked) {
+            softmax_backward_cols<kSubCols, kBf16, kSoftcap, true, true, kP, kDs>(sv, dpv, l2r, dlr, 0.f, 0.f, p.scale_log2,
+                                                                                  p.softcap_pre, lo, hi, pk_p, pk_ds);
+          } else {
+            softmax_backward_cols<kSubCols, kBf16, kSoftcap, true, false, kP, kDs>(sv, dpv, l2r, dlr, 0.f, 0.f, p.scale_log2,
+                                                                                   p.softcap_pre, 0, 0, pk_p, pk_ds);
+          }
+          // a warp overwrites only columns it has itself already loaded: its packed P^T / dS^T pieces go to the
+          // start of its own kSubCols columns
+          if (kP) ptx::tmem_st8(st_t, pk_p);
+          if (kDs) ptx::tmem_st8(dpt_t, pk_ds);
+        };
+        if (Cfg::kPasses == 1) turn(std::true_type{}, std::true_type{});
+        else if (makes_dk(idx)) turn(std::false_type{}, std::true_type{});
+        else turn(std::true_type{}, std::false_type{});
         ptx::tmem_wait_st();
         ptx::tc_fence_before();
         ptx::mbar_arrive_warp(&pds_full[u]);

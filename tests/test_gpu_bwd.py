@@ -155,3 +155,13 @@ def test_backward_padded_head_dims(bs, d):
     k = torch.randn(batch, 2 * n, heads_k, d, device=DEV, dtype=torch.bfloat16)
     v = torch.randn(batch, 2 * n, heads_k, d, device=DEV, dtype=torch.bfloat16)
     check_backward(q, k, v, bs)
+
+
+@pytest.mark.parametrize("d", [136, 256])
+@pytest.mark.parametrize("n,bs", [(1, 1), (63, 63), (64, 64), (65, 8), (129, 300), (700, 9)])
+def test_backward_wide_heads_sub_steps(n, bs, d):
+    """Head dimensions above 128: dK and dV are items of their own over sub-steps of 64 queries, with two slots for Q, one
+    for dO and four for the statistics. From one sub-step to more than the slots, whole and partial ones."""
+    torch.manual_seed(n + d)
+    q, k, v = (torch.randn(2, 2 * n, h, d, device=DEV, dtype=torch.bfloat16) for h in (4, 1, 1))
+    check_backward(q, k, v, bs)

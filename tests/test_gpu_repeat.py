@@ -125,3 +125,16 @@ def test_first_call_of_a_new_thread():
     thread.start()
     thread.join()
     assert len(got) == 1 and torch.equal(got[0], want)
+
+
+@pytest.mark.parametrize("heads,heads_k,d,deterministic", [(8, 2, 256, False), (8, 2, 128, True)])
+def test_no_wait_expires_over_many_split_backward_passes(heads, heads_k, d, deterministic):
+    torch.manual_seed(12)
+    n = 1500
+    q = torch.randn(2, 2 * n, heads, d, device=DEV, dtype=torch.bfloat16, requires_grad=True)
+    k, v = (torch.randn(2, 2 * n, heads_k, d, device=DEV, dtype=torch.bfloat16, requires_grad=True) for _ in range(2))
+    do = torch.randn_like(q)
+    for _ in range(300):
+        torch.autograd.grad(diffusion_attn_func(q, k, v, 48, deterministic=deterministic), (q, k, v), do)
+    torch.cuda.synchronize()
+    assert _lib.device_status()[0] == 0

@@ -14,9 +14,9 @@
 // dP^T (and the tail of the previous step) runs, dS^T while dV runs. The partial dQ^T of a step is added into an fp32
 // accumulator in global memory: the drain warps move it from tensor memory through a small shared-memory staging
 // area and out as 4 KB bulk reductions (cp.reduce.async.bulk add.f32); `bwd_dq_convert_kernel` then scales and
-// rounds the accumulator into dQ. About 30 bytes per clock leave an SM towards L2 whatever the instruction (plain
-// red, vector red and bulk reductions measured alike), so the 64 KB of a step take about 2200 cycles: the drain is
-// the long pole of the chain dP^T -> dS^T -> dQ^T -> drain -> next dP^T.
+// rounds the accumulator into dQ.
+// About 30 bytes per clock leave an SM towards L2 whatever the instruction, 2200 cycles for the 64 KB of a step, so the
+// drain runs under the next step's products.
 //
 // The reference does the same five GEMMs per pair with an fp32 dQ accumulator reduced through global memory
 // (csrc/fda/mainloop_bwd_sm90_tma_gmma_ws.hpp:815-984 `bwd_step`, :605-664 `store_dq`, there with
@@ -44,7 +44,7 @@ struct FusedCfg {
   static constexpr int kOffStage = kOffDs + kDsBytes;        // [4 warps][2 slots][kStageChunk]
   static constexpr int kOffStat = kOffStage + 4 * 2 * kStageChunk;
   static constexpr int kOffBar = kOffStat + kSlots * kStatBytes;
-  static constexpr int kSmemBytes = kOffBar + 512;
+  static constexpr int kSmemBytes = kOffBar + 768;   // barriers 384, mailbox 64, item descriptions
   // tensor memory: S^T / P^T at 0, dP^T / dQ^T at 128, dK and dV behind
   static constexpr int kTmemS = 0, kTmemDP = 128, kTmemDK = 256, kTmemDV = 256 + kHeadDim;
   // Head dimension 64 leaves 128 columns behind the accumulators: dQ^T gets them, and the next dP^T no longer waits
@@ -54,14 +54,38 @@ struct FusedCfg {
   static_assert(kHeadDim == 64 || kHeadDim == 128, "the single-pass backward covers head dimensions up to 128");
   static_assert(kOffStat % 1024 == 0, "tiles stay 1024-byte aligned for the swizzle");
   static_assert(kSmemBytes <= 232448, "shared memory budget");
-  static_assert((14 + 2 * kSlots + 2 * kDoSlots) * 8 + 8 + 16 + 16 * kSlots <= 384, "barrier area");
+  static_assert((17 + 2 * kSlots + 2 * kDoSlots) * 8 + 8 + 16 + 16 * kSlots <= 384, "barrier area");
 };
 
-// 768 threads start with 80 registers each. The compute warps hold a step's 32 probabilities per thread across the
-// two halves of the arithmetic; the producer warpgroup and the drain / epilogue warpgroup get by with less.
-constexpr uint32_t kFusedComputeRegs = 88, kFusedProducerRegs = 64, kFusedDrainRegs = 64;
-static_assert(kCmpThreads * kFusedComputeRegs + 128 * kFusedProducerRegs + 128 * kFusedDrainRegs <= kDkdvThreads * 80,
-              "register pool");
+// Warp roles: compute warpgroups (a thread = a key row and kCols query columns), a producer warpgroup (TMA warp, two
+// MMA warps, one idle), the drain and epilogue warpgroup. The register counts of a form add up to what its block has at
+// launch.
+//   Head dim 128: two compute warpgroups of 64 columns. 512 threads start with 128 registers, and the drain warps hold a
+//     whole dQ^T (128 columns): the buffer it shares with dP^T is free 250 cycles after the product instead of after 48
+//     of its 64 KB have left for L2. A step of the long loop takes 4300 cycles instead of 5300 (backward of 4 x 8192
+//     tokens, 32/8 heads of 128, blocks of 1024: 4.23 -> 3.9 ms). What bounds it now is shared memory: operands 2300
+//     cycles at 128 bytes a clock, the staging of dQ^T 1024, dS^T 256, the loads 512, statistics 250. Vector reductions
+//     straight from the registers would save the staging, but stall the load/store unit for the compute warps (their
+//     second half took 2100 cycles instead of 1150; 4.1 ms).
+//   Head dim 64: dQ^T has columns of its own, and the exponentials (and tanh) weigh more: four compute warpgroups of 32
+//     columns keep the special-function unit busier than two (4 x 8192 tokens, 32 heads, score cap: 2.8 against 3.2 ms).
+template <int kHeadDim>
+struct FusedRoles {
+  static constexpr int kCmpWG = kHeadDim == 128 ? 2 : 4;
+  static constexpr int kCols = kTile / kCmpWG;
+  static constexpr int kThreads = 128 * (kCmpWG + 2);
+  static constexpr int kLoadWarp = 4 * kCmpWG;
+  static constexpr int kMmaWarp = kLoadWarp + 1;
+  static constexpr int kEpiWarp0 = kLoadWarp + 4;
+  static constexpr int kLaunchRegs = kCmpWG == 2 ? 128 : 80;
+  static constexpr uint32_t kComputeRegs = kCmpWG == 2 ? 144 : 88;
+  static constexpr uint32_t kProducerRegs = 64;
+  static constexpr uint32_t kDrainRegs = kCmpWG == 2 ? 160 : 64;
+  static constexpr int kHold = kCmpWG == 2 ? 4 : 1;   // 32-column chunks of dQ^T that a drain warp holds at once
+  // A warp of its own works the items out ahead of the loader (head dim 64, scores capped: 2.77 ms with it, 2.72 without)
+  static constexpr bool kGeometryWarp = kHeadDim == 128;
+  static_assert(128 * (kCmpWG * kComputeRegs + kProducerRegs + kDrainRegs) <= kThreads * kLaunchRegs, "register pool");
+};
 
 // Rows of the dQ accumulator come in blocks of 64. Every half of every sample starts at its own block: the
 // "+ 2 b + qh" gives each of the 2 * batch halves one block of slack, so rounding the start down never lets two
@@ -71,10 +95,22 @@ __device__ __forceinline__ int acc_row_of(int grow0, int n, int b, int qh, int q
   return ((grow0 + qh * n) / 64 + 2 * b + qh) * 64 + qa;
 }
 
-// One step of an item: a visible 128-row query tile of one query head.
+// One step of an item: a visible 128-row query tile of one query head. At most `left` steps follow it.
 struct QStep {
-  int h, qh, qa, cls;
+  int h, qh, qa, cls, left;
 };
+
+// What the roles need to know about an item. At head dim 128 a warp of its own takes the items, works this out (some
+// twenty integer divisions and a ticket from global memory) while the last steps of the item before are under way, and
+// leaves it beside the mailbox; where items are short that counts (backward of 8 x 4096 tokens, 16 heads of 128, blocks of
+// 256: 1050 -> 1024 us). At head dim 64 the loader does it between its loads.
+struct FusedItem {
+  KvItem it;
+  QueryPlan plan;
+  KvSpans spans;
+  int grow0;   // first row of the sample in the packed row space
+};
+constexpr int kTicketSteps = 4;   // the next item is taken when at most this many steps of the current one are to be sent
 
 template <typename Fn>
 __device__ __forceinline__ bool for_each_qstep(const KvItem& it, const QueryPlan& plan, const KvSpans& spans, int group,
@@ -89,6 +125,7 @@ __device__ __forceinline__ bool for_each_qstep(const KvItem& it, const QueryPlan
       st.cls = spans.classify(st.qh, it.kh, st.qa, qb);
       if (st.cls == kTileSkip) continue;
       st.h = it.hk * group + g;
+      st.left = (group - 1 - g) * plan.steps() + plan.steps() - 1 - s;
       if (!fn(st)) return false;
     }
   }
@@ -96,9 +133,10 @@ __device__ __forceinline__ bool for_each_qstep(const KvItem& it, const QueryPlan
 }
 
 template <int kHeadDim, int kSlots, int kDoSlots, bool kBf16, bool kSoftcap>
-__global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid_constant__ BwdParams p) {
+__global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_kernel(const __grid_constant__ BwdParams p) {
   using Cfg = FusedCfg<kHeadDim, kSlots, kDoSlots>;
   using T = TileCfg<kHeadDim>;
+  using R = FusedRoles<kHeadDim>;
   // The tiles need 1024-byte alignment for the 128-byte swizzle. Dynamic shared memory starts at the beginning of the
   // block's window, which is aligned that far; the budget leaves no room to round the base up, so a base that is not
   // aligned is reported through the status word instead.
@@ -112,9 +150,11 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
   uint8_t* sStage = smem + Cfg::kOffStage;
   uint8_t* sStat = smem + Cfg::kOffStat;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kOffBar);
-  uint64_t* kv_full = bars;
-  uint64_t* kv_empty = bars + 1;
-  uint64_t* q_full = bars + 2;                 // [kSlots] Q tile, its statistics and the step header
+  uint64_t* k_full = bars;
+  uint64_t* k_empty = bars + 1;                // S^T and dQ^T of the item have read K
+  uint64_t* v_full = bars + 2;
+  uint64_t* v_empty = bars + 3;                // dP^T of the item has read V
+  uint64_t* q_full = bars + 4;                 // [kSlots] Q tile, its statistics and the step header
   uint64_t* q_empty = q_full + kSlots;
   uint64_t* do_full = q_empty + kSlots;        // [kDoSlots] dO tile
   uint64_t* do_empty = do_full + kDoSlots;
@@ -133,11 +173,14 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
   // own columns, dS^T of step g + 1 can be complete before they look for step g, and a wait by parity that is one whole
   // round late waits for ever. A barrier for even and one for odd steps cannot be lapped (step g + 2 needs dp_free of g).
   uint64_t* desc_full = acc_free + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(desc_full + 2);
+  uint64_t* go = desc_full + 2;                // the loader is about to send the last steps of its item
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(go + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   volatile int* dq_desc = reinterpret_cast<volatile int*>(tmem_slot + 2);   // [2][2]: {flags, first accumulator row}
   volatile int* hdr = reinterpret_cast<volatile int*>(tmem_slot + 6);       // [kSlots][4]
   SchedMailbox* mbox = reinterpret_cast<SchedMailbox*>(reinterpret_cast<uint8_t*>(bars) + 384);
+  FusedItem* items = reinterpret_cast<FusedItem*>(reinterpret_cast<uint8_t*>(bars) + 448);   // [2], like the mailbox
+  static_assert(sizeof(SchedMailbox) <= 64 && 2 * sizeof(FusedItem) <= 320, "mailbox and item descriptions");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if ((ptx::smem_u32(smem) & 1023u) != 0) {
@@ -150,9 +193,11 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
   }
   if (threadIdx.x == 0) {
     *abort_flag = 0;
-    sched_init(mbox, 4 * kCmpWG + 2 + 4);   // compute warps, two MMA issuers, four drain / epilogue warps
-    ptx::mbar_init(kv_full, 1);
-    ptx::mbar_init(kv_empty, 1);
+    sched_init(mbox, 4 * R::kCmpWG + (R::kGeometryWarp ? 3 : 2) + 4);   // compute, (loader,) two MMA, four drain warps
+    ptx::mbar_init(k_full, 1);
+    ptx::mbar_init(k_empty, 1);
+    ptx::mbar_init(v_full, 1);
+    ptx::mbar_init(v_empty, 1);
     for (int i = 0; i < kSlots; ++i) {
       ptx::mbar_init(&q_full[i], 1);
       ptx::mbar_init(&q_empty[i], 1);
@@ -163,8 +208,8 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
     }
     ptx::mbar_init(s_full, 1);
     ptx::mbar_init(dp_full, 1);
-    ptx::mbar_init(p_full, 4 * kCmpWG);
-    ptx::mbar_init(ds_full, 4 * kCmpWG);
+    ptx::mbar_init(p_full, 4 * R::kCmpWG);
+    ptx::mbar_init(ds_full, 4 * R::kCmpWG);
     ptx::mbar_init(s_free, 1);
     ptx::mbar_init(dq_full, 1);
     ptx::mbar_init(dp_free, 4);
@@ -173,9 +218,10 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
     ptx::mbar_init(acc_free, 4);
     ptx::mbar_init(&desc_full[0], 1);
     ptx::mbar_init(&desc_full[1], 1);
+    ptx::mbar_init(go, 1);
     ptx::fence_mbar_init();
   }
-  if (warp == kLoadWarpB) {
+  if (warp == R::kLoadWarp) {
     ptx::tmem_alloc(tmem_slot, 512);
     ptx::tmem_relinquish();
   }
@@ -187,22 +233,34 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
   const int group = p.heads / p.heads_k;
   const int total_items = kv_item_count(p);
 
-  if (warp >= kEpiWarp0) {
+  auto make_item = [&](int idx, FusedItem& d) -> bool {   // false: a tile that does not exist
+    const KvItem it = decode_kv_item(p, idx);
+    if (!it.valid) return false;
+    d.it = it;
+    d.plan = make_query_plan(it.kh, it.k0, it.k1, it.n, bs, kTile);
+    d.spans = make_kv_spans(it, bs);
+    d.grow0 = p.cu_seqlens != nullptr ? it.row0 : it.b * p.seqlen;
+    return true;
+  };
+
+  if (warp >= R::kEpiWarp0) {
     // ------------------------------------------------------------------------------------- dQ drain + dK/dV epilogue
     // Four warps, one per quarter of the tensor-memory lanes. Per step they add the partial dQ^T (lane = head-dim
     // row, 128 query columns) into the global accumulator; after the last step of an item they write dK and dV.
-    ptx::reg_release_to<kFusedDrainRegs>();
+    if (R::kHold > 1) ptx::reg_acquire_to<R::kDrainRegs>();
+    else ptx::reg_release_to<R::kDrainRegs>();
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const bool drain_rows = quad * 32 < kHeadDim;   // head dim 64: the upper two quarters hold nothing of dQ^T
+    const bool drain_rows = quad * 32 < p.head_dim;   // the quarters behind the head dimension hold nothing of dQ^T
     uint32_t n_item = 0, gd = 0, n_bulk = 0;
     bool alive = true;
     for (uint32_t n_sched = 0; alive; ++n_sched) {
-      const int idx = sched_consume<true>(mbox, n_sched, abort_flag);
+      const int idx = R::kGeometryWarp ? sched_peek(mbox, n_sched, abort_flag) : sched_consume<true>(mbox, n_sched, abort_flag);
       if (idx < 0 || idx >= total_items) break;
-      const KvItem it = decode_kv_item(p, idx);
-      if (!it.valid) continue;
+      const KvItem it = R::kGeometryWarp ? items[n_sched & 1u].it : decode_kv_item(p, idx);
+      if (R::kGeometryWarp) sched_release<true>(mbox, n_sched);
+      else if (!it.valid) continue;
       for (bool last = false; alive && !last; ++gd) {
         const uint32_t par = gd & 1u;
         if (!ptx::mbar_wait(&desc_full[par], (gd >> 1) & 1u, abort_flag, 63)) { alive = false; break; }
@@ -212,32 +270,45 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
         const int rows_left = flags >> 8;   // query rows of this tile that exist (1..128)
         if (!ptx::mbar_wait(dq_full, par, abort_flag, 64)) { alive = false; break; }
         ptx::tc_fence_after();
-        // Blocks of 32 query rows of the accumulator are stored as [head dim / 32][32 queries][32 head-dim values]: a
-        // warp's 32 x 32 piece of dQ^T goes through shared memory (a thread writes its head-dim value of each query,
-        // 32 lanes = 128 consecutive bytes) and out as ONE 4 KB bulk reduction, issued by lane 0. Two staging slots per
-        // warp alternate, so tensor memory is read out at shared-memory speed and the adds drain in the background.
+        // kHold chunks of 32 columns go to registers at once; when the last is there the columns are free and the adds
+        // follow behind the next step's products. Blocks of 32 query rows of the accumulator are stored as
+        // [head dim / 32][8 groups of 4 queries][32 head-dim values][4 queries]: a warp's 32 x 32 piece goes through
+        // shared memory (16 bytes a thread, a quarter of the store instructions of single values) and out as ONE 4 KB bulk
+        // reduction issued by lane 0. Two staging slots per warp alternate.
         float* dst = p.dq_acc + static_cast<size_t>(acc_row) * kHeadDim + quad * 1024;
-        if (drain_rows) {
 #pragma unroll 1
-          for (int c = 0; c < 4; ++c) {
-            uint32_t a[32];
-            ptx::tmem_ld32(tmem + Cfg::kTmemDQ + lane_addr + c * 32, a);
-            float* stage = reinterpret_cast<float*>(sStage + (quad * 2 + (n_bulk & 1u)) * Cfg::kStageChunk);
-            // the bulk reduction that last read this slot (two chunks ago) must have finished reading it
+        for (int c0 = 0; c0 < kTile / 32; c0 += R::kHold) {
+          uint32_t a[32 * R::kHold];
+#pragma unroll
+          for (int c = 0; c < R::kHold; ++c) ptx::tmem_ld32(tmem + Cfg::kTmemDQ + lane_addr + (c0 + c) * 32, a + c * 32);
+          if (R::kHold == 1) {   // the slot is waited for while the load is under way
             if (lane == 0) ptx::bulk_wait_group_read<1>();
             __syncwarp();
-            ptx::tmem_wait_ld();
-            if (c == 3) {
-              ptx::tc_fence_before();
-              ptx::mbar_arrive_warp(dp_free);
-            }
-            if (c * 32 < rows_left) {
+          }
+          ptx::tmem_wait_ld();
+          if (c0 + R::kHold == kTile / 32) {
+            ptx::tc_fence_before();
+            ptx::mbar_arrive_warp(dp_free);
+          }
+          if (!drain_rows) continue;
 #pragma unroll
-              for (int i = 0; i < 32; ++i) stage[i * 32 + lane] = __uint_as_float(a[i]);
+          for (int c = 0; c < R::kHold; ++c) {
+            if ((c0 + c) * 32 < rows_left) {
+              uint8_t* stage = sStage + (quad * 2 + (n_bulk & 1u)) * Cfg::kStageChunk;
+              // the bulk reduction that last read this slot (two chunks ago) must have finished reading it
+              if (R::kHold > 1) {
+                if (lane == 0) ptx::bulk_wait_group_read<1>();
+                __syncwarp();
+              }
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const uint32_t* x = a + c * 32 + i * 4;
+                ptx::st_shared_v4(stage + i * 512 + lane * 16, x[0], x[1], x[2], x[3]);
+              }
               ptx::fence_async_smem();
               __syncwarp();
               if (lane == 0) {
-                float* target = dst + c * (32 * kHeadDim);
+                float* target = dst + (c0 + c) * (32 * kHeadDim);
                 if (target >= p.dq_acc && target + 1024 <= p.dq_acc + p.acc_floats) {
                   ptx::bulk_reduce_add_f32(target, stage, Cfg::kStageChunk);
                   ptx::bulk_commit_group();
@@ -250,8 +321,6 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
               ++n_bulk;
             }
           }
-        } else {
-          ptx::mbar_arrive_warp(dp_free);
         }
       }
       if (!alive) break;
@@ -263,58 +332,97 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
       if (!ptx::mbar_wait(acc_full, n_item & 1, abort_flag, 62)) break;
       ++n_item;
       ptx::tc_fence_after();
-      constexpr int kChunks = 2 * kHeadDim / 32;   // dK and dV sit side by side in tensor memory
-#pragma unroll 1
-      for (int gidx = 0; gidx < kChunks; ++gidx) {
-        const bool is_dv = gidx * 32 >= kHeadDim;
-        const int col0 = gidx * 32 - (is_dv ? kHeadDim : 0);
-        uint32_t accv[32];
-        ptx::tmem_ld32(tmem + Cfg::kTmemDK + lane_addr + gidx * 32, accv);
-        ptx::tmem_wait_ld();
-        if (gidx == kChunks - 1) {
-          // everything is in registers: the first dV / dK products of the next item may overwrite the accumulators
-          ptx::tc_fence_before();
-          ptx::mbar_arrive_warp(acc_free);
-        }
+      // dK and dV sit side by side in tensor memory. With the registers for it (kHold > 1) both are rounded first, in three
+      // rounds of loads (a load is answered after 250 cycles and more while the products run, however wide it is), and
+      // the next item's products may overwrite them while the rows are stored. (Tile copies through the staging slots
+      // were slower: they queue behind the reductions.)
+      if constexpr (R::kHold > 1) {
+        uint32_t w[kHeadDim];
+        auto round = [&](auto cols_tag, int col0) {
+          constexpr int kN = decltype(cols_tag)::value;
+          uint32_t accv[kN];
+#pragma unroll
+          for (int c = 0; c < kN; c += 32) ptx::tmem_ld32(tmem + Cfg::kTmemDK + lane_addr + col0 + c, accv + c);
+          ptx::tmem_wait_ld();
+          const float sc = col0 >= kHeadDim ? 1.f : p.softmax_scale;
+#pragma unroll
+          for (int i = 0; i < kN / 2; ++i) {
+            w[col0 / 2 + i] = ptx::pack2<kBf16>(__uint_as_float(accv[2 * i]) * sc, __uint_as_float(accv[2 * i + 1]) * sc);
+          }
+        };
+        round(std::integral_constant<int, kHeadDim>{}, 0);
+        round(std::integral_constant<int, kHeadDim / 2>{}, kHeadDim);
+        round(std::integral_constant<int, kHeadDim / 2>{}, kHeadDim + kHeadDim / 2);
+        ptx::tc_fence_before();
+        ptx::mbar_arrive_warp(acc_free);
         if (lane < rows_valid) {
-          ptx::store_row32<kBf16>(is_dv ? dv_row : dk_row, col0, accv, is_dv ? 1.f : p.softmax_scale, p.head_dim,
-                                  p.wide_store != 0);
+#pragma unroll
+          for (int c = 0; c < 2 * kHeadDim; c += 32) {
+            ptx::store_row32_packed(c >= kHeadDim ? dv_row : dk_row, c % kHeadDim, w + c / 2, p.head_dim, p.wide_store != 0);
+          }
+        }
+      } else {
+        constexpr int kAccChunks = 2 * kHeadDim / 32;
+#pragma unroll 1
+        for (int c = 0; c < kAccChunks; ++c) {
+          const bool is_dv = c * 32 >= kHeadDim;
+          uint32_t accv[32];
+          ptx::tmem_ld32(tmem + Cfg::kTmemDK + lane_addr + c * 32, accv);
+          ptx::tmem_wait_ld();
+          if (c == kAccChunks - 1) {
+            ptx::tc_fence_before();
+            ptx::mbar_arrive_warp(acc_free);
+          }
+          if (lane < rows_valid) {
+            ptx::store_row32<kBf16>(is_dv ? dv_row : dk_row, c * 32 - (is_dv ? kHeadDim : 0), accv,
+                                    is_dv ? 1.f : p.softmax_scale, p.head_dim, p.wide_store != 0);
+          }
         }
       }
     }
     if (lane == 0) ptx::bulk_wait_group0();   // every reduction this warp issued has been performed
-  } else if (warp >= 4 * kCmpWG) {
-  ptx::reg_release_to<kFusedProducerRegs>();
-  if (warp == kLoadWarpB) {
+  } else if (warp >= R::kLoadWarp) {
+  ptx::reg_release_to<R::kProducerRegs>();
+  if (warp == R::kLoadWarp) {
     // ------------------------------------------------------------------------------------------------ producer
     if (lane == 0) {
       uint32_t n_item = 0, gc = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = sched_produce(mbox, n_sched, p.ticket_kv, abort_flag);
+        const int idx = R::kGeometryWarp ? sched_peek(mbox, n_sched, abort_flag)
+                                         : sched_produce(mbox, n_sched, p.ticket_kv, abort_flag);
         if (idx < 0 || idx >= total_items) break;
-        const KvItem it = decode_kv_item(p, idx);
-        if (!it.valid) continue;
-        const QueryPlan plan = make_query_plan(it.kh, it.k0, it.k1, it.n, bs, kTile);
-        const KvSpans spans = make_kv_spans(it, bs);
-        const int grow0 = p.cu_seqlens != nullptr ? it.row0 : it.b * p.seqlen;
-        if (!ptx::mbar_wait(kv_empty, (n_item & 1) ^ 1, abort_flag, 41)) break;
-        ptx::mbar_expect_tx(kv_full, 2 * T::kTileBytes);
+        FusedItem d;
+        if (R::kGeometryWarp) {
+          d = items[n_sched & 1u];
+          sched_release<false>(mbox, n_sched);
+        } else if (!make_item(idx, d)) {
+          continue;
+        }
+        const KvItem& it = d.it;
+        // V is free after the last item's last dP^T; K only after its last dQ^T, behind everything that the first step
+        // loads.
         const int k_row = it.row0 + it.kh * it.n + it.k0;
-        load_tile<kHeadDim>(sK, &p.tm_k, kv_full, k_row, it.hk, it.bcoord);
-        load_tile<kHeadDim>(sV, &p.tm_v, kv_full, k_row, it.hk, it.bcoord);
-        // The loader alone walks the item's geometry. Each step carries a header for the other roles:
+        if (!ptx::mbar_wait(v_empty, (n_item & 1) ^ 1, abort_flag, 41)) break;
+        ptx::mbar_expect_tx(v_full, T::kTileBytes);
+        load_tile<kHeadDim>(sV, &p.tm_v, v_full, k_row, it.hk, it.bcoord);
+        bool k_loaded = false, told = false;
+        // The loader alone walks the item's steps. Each carries a header for the other roles:
         // {bit 0 last step of the item, bit 1 partially masked, bit 2 queries of the keys' own half, bits 8.. the
         // number of query rows that exist; first query row; first accumulator row of the step's dQ}. A step is sent
         // when its successor is known, so that the last one can be marked.
         auto emit = [&](const QStep& st, bool last) -> bool {
           const uint32_t slot = gc % kSlots, par = ((gc / kSlots) & 1u) ^ 1u;
+          if (R::kGeometryWarp && !told && (last || st.left <= kTicketSteps)) {
+            told = true;
+            ptx::mbar_arrive(go);
+          }
           if (!ptx::mbar_wait(&q_empty[slot], par, abort_flag, 42)) return false;
           volatile int* h4 = hdr + 4 * slot;
           h4[0] = (last ? 1 : 0) | (st.cls == kTileMasked ? 2 : 0) | (st.qh == it.kh ? 4 : 0) |
                   (imin(kTile, it.n - st.qa) << 8);
           h4[1] = st.qa;
-          h4[2] = st.h * p.acc_tiles * 64 + acc_row_of(grow0, it.n, it.b, st.qh, st.qa);
+          h4[2] = st.h * p.acc_tiles * 64 + acc_row_of(d.grow0, it.n, it.b, st.qh, st.qa);
           ptx::mbar_expect_tx(&q_full[slot], T::kTileBytes + Cfg::kStatBytes);
           const int q_row = it.row0 + st.qh * it.n + st.qa;
           load_tile<kHeadDim>(sQ + slot * T::kTileBytes, &p.tm_q, &q_full[slot], q_row, st.h, it.bcoord);
@@ -326,11 +434,17 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
           ptx::mbar_expect_tx(&do_full[dslot], T::kTileBytes);
           load_tile<kHeadDim>(sDo + dslot * T::kTileBytes, &p.tm_do, &do_full[dslot], q_row, st.h, it.bcoord);
           ++gc;
+          if (!k_loaded) {
+            k_loaded = true;
+            if (!ptx::mbar_wait(k_empty, (n_item & 1) ^ 1, abort_flag, 44)) return false;
+            ptx::mbar_expect_tx(k_full, T::kTileBytes);
+            load_tile<kHeadDim>(sK, &p.tm_k, k_full, k_row, it.hk, it.bcoord);
+          }
           return true;
         };
         QStep pend{};
         bool have = false;
-        alive = for_each_qstep(it, plan, spans, group, [&](const QStep& st) -> bool {
+        alive = for_each_qstep(it, d.plan, d.spans, group, [&](const QStep& st) -> bool {
           if (have && !emit(pend, false)) return false;
           pend = st;
           have = true;
@@ -342,7 +456,19 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
       }
       if (*abort_flag) __nanosleep(100000);
     }
-  } else if (warp == kMmaWarpB) {
+  } else if (R::kGeometryWarp && warp == R::kMmaWarp + 2) {
+    // ---------------------------------------------------------------------------------------------- item geometry
+    if (lane == 0) {
+      for (uint32_t n = 0;; ++n) {
+        if (n > 0 && !ptx::mbar_wait(go, (n - 1) & 1u, abort_flag, 45)) break;
+        int idx = sched_take(mbox, n, p.ticket_kv, abort_flag);
+        if (idx < 0) break;
+        while (idx < total_items && !make_item(idx, items[n & 1u])) idx = sched_next(p.ticket_kv);
+        sched_publish(mbox, n, idx);
+        if (idx >= total_items) break;
+      }
+    }
+  } else if (warp == R::kMmaWarp) {
     // ------------------------------------------------------------------- MMA issuer 1: S^T = K Q^T, dP^T = V dO^T
     // Two threads issue the MMAs of this kernel, so that the barrier waits and commits of one overlap the MMAs of
     // the other. S^T of step g + 1 may overwrite P^T of step g once dV has read it (s_free); dP^T of step g + 1
@@ -361,9 +487,9 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
       for (uint32_t n_sched = 0; alive; ++n_sched) {
         const int idx = sched_consume<false>(mbox, n_sched, abort_flag);
         if (idx < 0 || idx >= total_items) break;
-        const KvItem it = decode_kv_item(p, idx);
-        if (!it.valid) continue;
-        if (!ptx::mbar_wait(kv_full, n_item & 1, abort_flag, 51)) break;
+        if (!R::kGeometryWarp && !decode_kv_item(p, idx).valid) continue;
+        if (!ptx::mbar_wait(k_full, n_item & 1, abort_flag, 51)) break;
+        bool first = true;
         for (bool last = false; alive && !last; ++g) {
           const uint32_t slot = g % kSlots, spar = (g / kSlots) & 1u;
           const uint32_t t_off = slot * (T::kTileBytes >> 4);
@@ -379,6 +505,8 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
           ptx::umma_commit(s_full);
           const uint32_t dslot = g % kDoSlots;
           if (!ptx::mbar_wait(&do_full[dslot], (g / kDoSlots) & 1u, abort_flag, 56)) { alive = false; break; }
+          if (first && !ptx::mbar_wait(v_full, n_item & 1, abort_flag, 69)) { alive = false; break; }
+          first = false;
           if (!ptx::mbar_wait(Cfg::kOwnDq ? ds_full : dp_free, (g & 1u) ^ 1u, abort_flag, 58)) { alive = false; break; }
           ptx::tc_fence_after();
 #pragma unroll
@@ -389,11 +517,12 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
           }
           ptx::umma_commit(dp_full);
           ptx::umma_commit(&do_empty[dslot]);
+          if (last) ptx::umma_commit(v_empty);
         }
         ++n_item;
       }
     }
-  } else if (warp == kMmaWarpB + 1) {
+  } else if (warp == R::kMmaWarp + 1) {
     // -------------------------------------------------- MMA issuer 2: dV += P^T dO, dQ^T = K^T dS^T, dK += dS^T Q
     if (lane == 0) {
       constexpr int kFmt = kBf16 ? 1 : 0;
@@ -410,8 +539,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
       for (uint32_t n_sched = 0; alive; ++n_sched) {
         const int idx = sched_consume<false>(mbox, n_sched, abort_flag);
         if (idx < 0 || idx >= total_items) break;
-        const KvItem it = decode_kv_item(p, idx);
-        if (!it.valid) continue;
+        if (!R::kGeometryWarp && !decode_kv_item(p, idx).valid) continue;
         bool acc = false;
         // the first dV / dK products of an item overwrite the accumulators: the epilogue must have read the last item's
         if (!ptx::mbar_wait(acc_free, (n_item_b & 1u) ^ 1u, abort_flag, 57)) break;
@@ -449,8 +577,9 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
           }
           ptx::umma_commit(dq_full);
           // K is read by S^T (complete for every step of this item by now) and by dQ^T: after the last dQ^T the next
-          // item's K and V may load
-          if (last) ptx::umma_commit(kv_empty);
+          // item's K may load. (The rows of dQ^T that come from V at head dim 64, where V may be changing by then, are
+          // the ones nobody reads.)
+          if (last) ptx::umma_commit(k_empty);
 #pragma unroll
           for (int kk = 0; kk < kTile / 16; ++kk) {
             ptx::umma_ss_f16_lh(tmem + Cfg::kTmemDK, ds_k + (((kk / 4) * Cfg::kDsPanelBytes + (kk % 4) * 32) >> 4),
@@ -466,25 +595,27 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
     }
   }
   } else {
-    ptx::reg_acquire_to<kFusedComputeRegs>();
+    ptx::reg_acquire_to<R::kComputeRegs>();
     // -------------------------------------------------------------------------------------- softmax backward
-    const int wg = warp >> 2;                  // which 32 query columns of the step
+    const int wg = warp >> 2;                  // which kCols query columns of the step
+    constexpr int kChunks = R::kCols / 32;
     const int quad = warp & 3;
     const int row = quad * 32 + lane;          // key row inside the tile
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t s_t = tmem + Cfg::kTmemS + lane_addr + wg * kCols;
-    const uint32_t dp_t = tmem + Cfg::kTmemDP + lane_addr + wg * kCols;
-    // this thread's row of the dS^T panel that holds its 32 queries: four 16-byte pieces starting at piece 4 (wg & 1)
-    // (128-byte swizzle: piece c of row r sits at c ^ (r & 7))
-    uint8_t* ds_row = sDs + (wg >> 1) * Cfg::kDsPanelBytes + row * 128;
-    const int ds_piece0 = 4 * (wg & 1);
+    const uint32_t s_t = tmem + Cfg::kTmemS + lane_addr + wg * R::kCols;
+    const uint32_t dp_t = tmem + Cfg::kTmemDP + lane_addr + wg * R::kCols;
+    // this thread's row of the dS^T panel that holds its queries: 16-byte pieces from ds_piece0 on (128-byte swizzle:
+    // piece c of row r sits at c ^ (r & 7))
+    uint8_t* ds_row = sDs + (wg * R::kCols / 64) * Cfg::kDsPanelBytes + row * 128;
+    const int ds_piece0 = R::kCols == 64 ? 0 : 4 * (wg & 1);
     uint32_t gc = 0;
     bool alive = true;
     for (uint32_t n_sched = 0; alive; ++n_sched) {
-      const int idx = sched_consume<true>(mbox, n_sched, abort_flag);
+      const int idx = R::kGeometryWarp ? sched_peek(mbox, n_sched, abort_flag) : sched_consume<true>(mbox, n_sched, abort_flag);
       if (idx < 0 || idx >= total_items) break;
-      const KvItem it = decode_kv_item(p, idx);
-      if (!it.valid) continue;
+      const KvItem it = R::kGeometryWarp ? items[n_sched & 1u].it : decode_kv_item(p, idx);
+      if (R::kGeometryWarp) sched_release<true>(mbox, n_sched);
+      else if (!it.valid) continue;
       const int kj = it.k0 + row;
       // queries that see this thread's key: same-half tiles and (clean keys only) noisy tiles of later blocks
       int same_lo, same_hi, cross_lo, cross_hi;
@@ -492,59 +623,63 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
       query_interval(0, 1, kj, it.n, bs, cross_lo, cross_hi);
       for (bool last = false; alive && !last; ++gc) {
         const uint32_t slot = gc % kSlots, par = gc & 1u;
-        const float* stats = reinterpret_cast<const float*>(sStat + slot * Cfg::kStatBytes) + wg * kCols;
+        const float* stats = reinterpret_cast<const float*>(sStat + slot * Cfg::kStatBytes) + wg * R::kCols;
         // the Q barrier orders the header and the bulk copies of lse2 / delta before our reads
         if (!ptx::mbar_wait(&q_full[slot], (gc / kSlots) & 1u, abort_flag, 60)) { alive = false; break; }
         const int hdr0 = hdr[4 * slot], hdr1 = hdr[4 * slot + 1], hdr2 = hdr[4 * slot + 2];
         last = (hdr0 & 1) != 0;
         const bool masked = (hdr0 & 2) != 0;
         // visible query columns of this thread's key, relative to its first column of the step
-        const int lo = ((hdr0 & 4) ? same_lo : cross_lo) - (hdr1 + wg * kCols);
-        const int hi = ((hdr0 & 4) ? same_hi : cross_hi) - (hdr1 + wg * kCols);
+        const int lo = ((hdr0 & 4) ? same_lo : cross_lo) - (hdr1 + wg * R::kCols);
+        const int hi = ((hdr0 & 4) ? same_hi : cross_hi) - (hdr1 + wg * R::kCols);
         {
           // First half, once S^T is complete: P^T (16-bit, back to tensor memory for dV) and, kept in registers, the
           // factor of the second half: P, or with the score cap P (1 - tanh^2).
-          float pr[kCols];
+          float pr[R::kCols];
           if (!ptx::mbar_wait(s_full, par, abort_flag, 61)) { alive = false; break; }
           ptx::tc_fence_after();
-          {
-            uint32_t sv[kCols], pk[kCols / 2];
-            ptx::tmem_ld16(s_t, sv);
-            ptx::tmem_ld16(s_t + 16, sv + 16);
-            ptx::tmem_wait_ld();
-            const float4* l2v = reinterpret_cast<const float4*>(stats);
-            // the fully visible tile (the common one) carries no per-element compare
-            auto first_half = [&](auto masked_tag) {
-              constexpr bool kMasked = decltype(masked_tag)::value;
 #pragma unroll
-              for (int i = 0; i < kCols / 4; ++i) {
-                const float4 l2 = l2v[i];
-                const float l2a[4] = {l2.x, l2.y, l2.z, l2.w};
-                float pv[4];
+          for (int half = 0; half < kChunks; ++half) ptx::tmem_ld32(s_t + 32 * half, reinterpret_cast<uint32_t*>(pr) + 32 * half);
+          ptx::tmem_wait_ld();
+          const float4* l2v = reinterpret_cast<const float4*>(stats);
+          // the fully visible tile (the common one) carries no per-element compare
+          auto first_half = [&](auto masked_tag) {
+            constexpr bool kMasked = decltype(masked_tag)::value;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const int c = 4 * i + j;
-                  float x = __uint_as_float(sv[c]);
-                  float dt = 1.f;
+            for (int half = 0; half < kChunks; ++half) {
+              uint32_t pk[16];
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                const float4 nl2 = l2v[8 * half + i];
+                const float nl2a[4] = {nl2.x, nl2.y, nl2.z, nl2.w};
+#pragma unroll
+                for (int j = 0; j < 4; j += 2) {
+                  const int c = 32 * half + 4 * i + j;
+                  float x0 = pr[c], x1 = pr[c + 1];
+                  float dt0 = 1.f, dt1 = 1.f;
                   if (kSoftcap) {
-                    x = ptx::tanh_fast(x * p.softcap_pre);
-                    dt = 1.f - x * x;
+                    x0 = ptx::tanh_fast(x0 * p.softcap_pre);
+                    x1 = ptx::tanh_fast(x1 * p.softcap_pre);
+                    dt0 = 1.f - x0 * x0;
+                    dt1 = 1.f - x1 * x1;
                   }
-                  float v = ptx::ex2(fmaf(x, p.scale_log2, -l2a[j]));
-                  if (kMasked && (c < lo || c >= hi)) v = 0.f;
-                  pv[j] = v;
-                  pr[c] = kSoftcap ? v * dt : v;
+                  float y0, y1;
+                  ptx::fma2(y0, y1, x0, x1, p.scale_log2, p.scale_log2, nl2a[j], nl2a[j + 1]);
+                  float v0 = ptx::ex2(y0), v1 = ptx::ex2(y1);
+                  if (kMasked && (c < lo || c >= hi)) v0 = 0.f;
+                  if (kMasked && (c + 1 < lo || c + 1 >= hi)) v1 = 0.f;
+                  pk[2 * i + j / 2] = ptx::pack2<kBf16>(v0, v1);
+                  pr[c] = kSoftcap ? v0 * dt0 : v0;
+                  pr[c + 1] = kSoftcap ? v1 * dt1 : v1;
                 }
-                pk[2 * i] = ptx::pack2<kBf16>(pv[0], pv[1]);
-                pk[2 * i + 1] = ptx::pack2<kBf16>(pv[2], pv[3]);
               }
-            };
-            if (masked) first_half(std::true_type{});
-            else first_half(std::false_type{});
-            // a warp overwrites only columns it has itself already loaded: the 16-bit P^T of its 32 queries goes to
-            // the first 16 of its own 32 columns
-            ptx::tmem_st16(s_t, pk);
-          }
+              // a warp overwrites only columns it has itself already loaded: the 16-bit P^T of 32 queries goes to the
+              // first 16 of their 32 columns
+              ptx::tmem_st16(s_t + 32 * half, pk);
+            }
+          };
+          if (masked) first_half(std::true_type{});
+          else first_half(std::false_type{});
           ptx::tmem_wait_st();
           ptx::tc_fence_before();
           ptx::mbar_arrive_warp(p_full);
@@ -552,26 +687,26 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
           // dQ^T and dK of the previous step have read the dS^T tile (long ago in the steady state)
           if (!ptx::mbar_wait(ds_free, par ^ 1u, abort_flag, 66)) { alive = false; break; }
           ptx::tc_fence_after();
-          {
-            uint32_t dpv[kCols];
-            ptx::tmem_ld16(dp_t, dpv);
-            ptx::tmem_ld16(dp_t + 16, dpv + 16);
-            ptx::tmem_wait_ld();
-            const float4* dlv = reinterpret_cast<const float4*>(stats + kTile);
-            // masked positions have P = 0, so dS = 0 there without another compare
+          const float4* dlv = reinterpret_cast<const float4*>(stats + kTile);
+          uint32_t dpv[R::kCols];
 #pragma unroll
-            for (int i = 0; i < kCols / 8; ++i) {
-              const float4 d0 = dlv[2 * i], d1 = dlv[2 * i + 1];
-              const float dl[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
-              uint32_t pk[4];
+          for (int half = 0; half < kChunks; ++half) ptx::tmem_ld32(dp_t + 32 * half, dpv + 32 * half);
+          ptx::tmem_wait_ld();
+          // masked positions have P = 0, so dS = 0 there without another compare
 #pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const int c = 8 * i + 2 * j;
-                pk[j] = ptx::pack2<kBf16>(pr[c] * (__uint_as_float(dpv[c]) - dl[2 * j]),
-                                          pr[c + 1] * (__uint_as_float(dpv[c + 1]) - dl[2 * j + 1]));
-              }
-              ptx::st_shared_v4(ds_row + (((ds_piece0 + i) ^ (row & 7)) << 4), pk[0], pk[1], pk[2], pk[3]);
+          for (int i = 0; i < R::kCols / 8; ++i) {
+            const float4 d0 = dlv[2 * i], d1 = dlv[2 * i + 1];
+            const float ndl[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+            uint32_t pk[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int c = 8 * i + 2 * j;
+              float t0, t1;
+              ptx::add2(t0, t1, __uint_as_float(dpv[c]), __uint_as_float(dpv[c + 1]), ndl[2 * j], ndl[2 * j + 1]);
+              ptx::mul2(t0, t1, t0, t1, pr[c], pr[c + 1]);
+              pk[j] = ptx::pack2<kBf16>(t0, t1);
             }
+            ptx::st_shared_v4(ds_row + (((ds_piece0 + i) ^ (row & 7)) << 4), pk[0], pk[1], pk[2], pk[3]);
           }
         }
         if (threadIdx.x == 0) {
@@ -587,7 +722,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_fused_kernel(const __grid
   }
   ptx::tc_fence_before();
   __syncthreads();
-  if (warp == kLoadWarpB) ptx::tmem_dealloc(tmem, 512);
+  if (warp == R::kLoadWarp) ptx::tmem_dealloc(tmem, 512);
 }
 
 // ------------------------------------------------------------------------------------------------------------
@@ -604,21 +739,33 @@ __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const __grid_consta
   const int grow0 = p.cu_seqlens != nullptr ? sm.row0 : b * p.seqlen;
   const float* src =
       p.dq_acc + (static_cast<size_t>(h) * p.acc_tiles * 64 + acc_row_of(grow0, sm.n, b, half, qa)) * kHeadDim;
-  // a thread turns 8 consecutive values of a row into one 16-byte store
+  // The accumulator is read in its own order ([head dim / 32][8 groups of 4 rows][32 values][4 rows] per 32 rows, 16 bytes
+  // a lane), rounded, transposed through shared memory and written in rows. The pad of 16 bytes keeps the row reads of 16
+  // bytes aligned and the 2-byte writes of a warp (32 neighbouring values of a row) free of conflicts.
+  constexpr int kRowElems = kHeadDim + 8;
+  __shared__ __align__(16) uint16_t tile[64 * kRowElems];
+  const float sc = p.softmax_scale;
+#pragma unroll
+  for (int i = threadIdx.x; i < 16 * kHeadDim; i += 256) {
+    const int e = i % 32, q4 = (i / 32) % 8, panel = (i / 256) % (kHeadDim / 32), q32 = i / (8 * kHeadDim);
+    if (panel * 32 >= p.head_dim) continue;
+    const float4 x = reinterpret_cast<const float4*>(src)[i];
+    const uint32_t w0 = ptx::pack2<kBf16>(x.x * sc, x.y * sc), w1 = ptx::pack2<kBf16>(x.z * sc, x.w * sc);
+    uint16_t* t = tile + (q32 * 32 + q4 * 4) * kRowElems + panel * 32 + e;
+    t[0] = static_cast<uint16_t>(w0);
+    t[kRowElems] = static_cast<uint16_t>(w0 >> 16);
+    t[2 * kRowElems] = static_cast<uint16_t>(w1);
+    t[3 * kRowElems] = static_cast<uint16_t>(w1 >> 16);
+  }
+  __syncthreads();
   constexpr int kPieces = kHeadDim / 8;
 #pragma unroll
   for (int i = threadIdx.x; i < 64 * kPieces; i += 256) {
     const int qr = i / kPieces, piece = i % kPieces;
     if (qa + qr >= sm.n || piece * 8 >= p.head_dim) continue;
-    // blocks of 32 rows are stored [head dim / 32][32 rows][32 values]
-    const float* s8 = src + (qr / 32) * (32 * kHeadDim) + (piece / 4) * 1024 + (qr % 32) * 32 + (piece % 4) * 8;
-    const float4 lo = *reinterpret_cast<const float4*>(s8);
-    const float4 hi = *reinterpret_cast<const float4*>(s8 + 4);
-    const float sc = p.softmax_scale;
     const int64_t srow = static_cast<int64_t>(sm.row0) + half * sm.n + qa + qr;
     uint16_t* dst = static_cast<uint16_t*>(p.dq) + sm.bcoord * p.dq_bs + srow * p.dq_rs + h * p.dq_hs + piece * 8;
-    *reinterpret_cast<uint4*>(dst) = make_uint4(ptx::pack2<kBf16>(lo.x * sc, lo.y * sc), ptx::pack2<kBf16>(lo.z * sc, lo.w * sc),
-                                                ptx::pack2<kBf16>(hi.x * sc, hi.y * sc), ptx::pack2<kBf16>(hi.z * sc, hi.w * sc));
+    *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(tile + qr * kRowElems + piece * 8);
   }
 }
 
@@ -635,7 +782,7 @@ int launch_fused_instance(const BwdParams& p, int sm_count, unsigned stages, cud
     }
     const int items = bwd_item_bound(p, p.heads_k);
     const int grid = items < sm_count ? items : sm_count;
-    kernel<<<grid, kDkdvThreads, Cfg::kSmemBytes, stream>>>(p);
+    kernel<<<grid, FusedRoles<kHeadDim>::kThreads, Cfg::kSmemBytes, stream>>>(p);
     FDA_CUDA_TRY(cudaGetLastError());
   }
   if (stages & 4u) {

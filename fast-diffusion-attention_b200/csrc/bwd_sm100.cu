@@ -103,16 +103,16 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
       const int r = r0 + u * kRowsPerWarp;
       if (r >= p.n_pad) continue;
       const bool valid = r < sm.n;
-      float lse2 = INFINITY;
+      float lse2 = -INFINITY;
       if (valid) {
         const int64_t srow = static_cast<int64_t>(sm.row0) + half * sm.n + r;
         const int64_t li = (p.cu_seqlens != nullptr)
                                ? static_cast<int64_t>(h) * p.total + srow
                                : (static_cast<int64_t>(b) * p.heads + h) * p.seqlen + (half * sm.n + r);
         const float lse = p.lse[li];
-        lse2 = (lse == -INFINITY) ? 0.f : lse * kLog2e;
+        lse2 = (lse == -INFINITY) ? 0.f : -lse * kLog2e;
       }
-      p.delta_pad[seg + r] = valid ? acc[u] : 0.f;
+      p.delta_pad[seg + r] = valid ? -acc[u] : 0.f;
       p.lse2_pad[seg + r] = lse2;
     }
   }

@@ -446,16 +446,19 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return kBf16 ? pack_bf16(lo, hi) : pack_f16(lo, hi);
 }
 
-// Store 32 fp32 accumulator values of one row as 16-bit after scaling: columns [col0, col0 + 32) of a row of
-// `head_dim` (a multiple of 8) elements. `wide` = the row pointer and head_dim allow 32-byte stores.
+// 32 fp32 accumulator values of one row, scaled and packed to 16 bits (16 words).
 template <bool kBf16>
-__device__ __forceinline__ void store_row32(uint16_t* row_ptr, int col0, const uint32_t* acc, float scale,
-                                            int head_dim, bool wide) {
-  uint32_t w[16];
+__device__ __forceinline__ void pack_row32(const uint32_t* acc, float scale, uint32_t* w) {
 #pragma unroll
   for (int i = 0; i < 16; ++i) {
     w[i] = pack2<kBf16>(__uint_as_float(acc[2 * i]) * scale, __uint_as_float(acc[2 * i + 1]) * scale);
   }
+}
+
+// Store such a row piece: columns [col0, col0 + 32) of a row of `head_dim` (a multiple of 8) elements. `wide` = the row
+// pointer and head_dim allow 32-byte stores.
+__device__ __forceinline__ void store_row32_packed(uint16_t* row_ptr, int col0, const uint32_t* w, int head_dim,
+                                                   bool wide) {
   if (wide) {
 #pragma unroll
     for (int i = 0; i < 32; i += 16) {
@@ -469,6 +472,15 @@ __device__ __forceinline__ void store_row32(uint16_t* row_ptr, int col0, const u
       }
     }
   }
+}
+
+// Both in one: scale, pack and store.
+template <bool kBf16>
+__device__ __forceinline__ void store_row32(uint16_t* row_ptr, int col0, const uint32_t* acc, float scale,
+                                            int head_dim, bool wide) {
+  uint32_t w[16];
+  pack_row32<kBf16>(acc, scale, w);
+  store_row32_packed(row_ptr, col0, w, head_dim, wide);
 }
 
 // The same 32 columns, but stored so that four neighbouring lanes write 64 contiguous bytes of ONE row: the four
@@ -513,14 +525,6 @@ __device__ __forceinline__ void store_rows32_grouped_packed(uint16_t* row_ptr, i
         *reinterpret_cast<uint4*>(dst) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
       }
     }
-  }
-}
-
-template <bool kBf16>
-__device__ __forceinline__ void pack_row32(const uint32_t* acc, float scale, uint32_t* w) {
-#pragma unroll
-  for (int i = 0; i < 16; ++i) {
-    w[i] = pack2<kBf16>(__uint_as_float(acc[2 * i]) * scale, __uint_as_float(acc[2 * i + 1]) * scale);
   }
 }
 

@@ -30,6 +30,13 @@ __device__ __forceinline__ void sched_init(SchedMailbox* m, int consumer_arrival
   }
 }
 
+// An item index that nobody else has, for the CTA's second item and later ones.
+__device__ __forceinline__ int sched_next(int* ticket) {
+  // a launch with a block for every item passes no counter (nothing to zero beforehand): one item each
+  if (ticket == nullptr) return 0x7fffffff;
+  return static_cast<int>(gridDim.x) + atomicAdd(ticket, 1);
+}
+
 // Producer side, one thread, in two halves so that the producer can leave a description of the item in shared
 // memory (two slots, indexed like the mailbox: it & 1) before the consumers see the index. `it` counts the
 // items this CTA has taken (0, 1, 2, ...). sched_take returns the item index (>= total means "no more work"), or
@@ -38,9 +45,7 @@ __device__ __forceinline__ int sched_take(SchedMailbox* m, uint32_t it, int* tic
   const uint32_t slot = it & 1u;
   if (!ptx::mbar_wait(&m->empty[slot], ((it >> 1) & 1u) ^ 1u, abort_flag, 5)) return -1;
   if (it == 0) return static_cast<int>(blockIdx.x);
-  // a launch with a block for every item passes no counter (nothing to zero beforehand): one item each
-  if (ticket == nullptr) return 0x7fffffff;
-  return static_cast<int>(gridDim.x) + atomicAdd(ticket, 1);
+  return sched_next(ticket);
 }
 __device__ __forceinline__ void sched_publish(SchedMailbox* m, uint32_t it, int idx) {
   const uint32_t slot = it & 1u;

@@ -165,3 +165,15 @@ def test_backward_wide_heads_sub_steps(n, bs, d):
     torch.manual_seed(n + d)
     q, k, v = (torch.randn(2, 2 * n, h, d, device=DEV, dtype=torch.bfloat16) for h in (4, 1, 1))
     check_backward(q, k, v, bs)
+
+
+@pytest.mark.parametrize("d", [96, 128])
+@pytest.mark.parametrize("bs", [5, 64])
+def test_backward_many_short_items(bs, d):
+    """Items of one or two steps, several per CTA: the next item is taken, worked out and its V loaded while the last steps of
+    the one before are still under way, and the drain warps go from one item's dK and dV to the next one's dQ."""
+    torch.manual_seed(bs + d)
+    ns = [(i * 37) % 131 + 1 for i in range(160)]
+    cu = torch.tensor([0] + list(torch.tensor([2 * x for x in ns]).cumsum(0)), device=DEV, dtype=torch.int32)
+    q, k, v = (torch.randn(2 * sum(ns), h, d, device=DEV, dtype=torch.bfloat16) for h in (4, 2, 2))
+    check_backward(q, k, v, bs, cu=cu)

@@ -63,7 +63,7 @@ struct FusedCfg {
 //   Head dim 128: two compute warpgroups of 64 columns. 512 threads start with 128 registers, and the drain warps hold a
 //     whole dQ^T (128 columns): the buffer it shares with dP^T is free 250 cycles after the product instead of after 48
 //     of its 64 KB have left for L2. A step of the long loop takes 4300 cycles instead of 5300 (backward of 4 x 8192
-//     tokens, 32/8 heads of 128, blocks of 1024: 4.23 -> 3.9 ms). What bounds it now is shared memory: operands 2300
+//     tokens, 32/8 heads of 128, blocks of 1024: 4.25 -> 3.98 ms). What bounds it now is shared memory: operands 2300
 //     cycles at 128 bytes a clock, the staging of dQ^T 1024, dS^T 256, the loads 512, statistics 250. Vector reductions
 //     straight from the registers would save the staging, but stall the load/store unit for the compute warps (their
 //     second half took 2100 cycles instead of 1150; 4.1 ms).

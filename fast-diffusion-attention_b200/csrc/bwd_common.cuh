@@ -38,8 +38,8 @@ struct BwdParams {
   int64_t dk_bs, dk_rs, dk_hs;
   int64_t dv_bs, dv_rs, dv_hs;
   const float* lse;
-  float* delta_pad;  // (batch, heads, 2, n_pad), negated: packed arithmetic adds and has no minus
-  float* lse2_pad;   // (batch, heads, 2, n_pad), negated likewise
+  float* delta_pad;  // (batch, heads, 2, n_pad); callers get this back as rowsum(dO * O)
+  float* lse2_pad;   // (batch, heads, 2, n_pad), negated: the exponent is one FMA, and a packed FMA has no minus
   const int32_t* cu_seqlens;
   int batch, seqlen, total, heads, heads_k, head_dim, block_size;
   int n_pad;           // round_up(max n, 128)
@@ -118,7 +118,7 @@ constexpr int kMmaWarpB = 4 * kCmpWG + 1;
 static_assert(kCols == 32, "one 32-column tensor-memory load per operand and warp");
 
 // P and dS of kN columns for one thread. `s`/`dp` hold the raw accumulators; the results are packed 16-bit.
-// lse2 / delta (both negated) are per column (kPerColumn, read from shared memory) or per thread. kMasked is a template
+// lse2 (negated) / delta are per column (kPerColumn, read from shared memory) or per thread. kMasked is a template
 // parameter so that the common fully-visible tile carries no per-element compare/select at all.
 template <int kN, bool kBf16, bool kSoftcap, bool kPerColumn, bool kMasked, bool kNeedP, bool kNeedDs = true>
 __device__ __forceinline__ void softmax_backward_cols(const uint32_t* s, const uint32_t* dp, const float* lse2_col,
@@ -142,7 +142,7 @@ __device__ __forceinline__ void softmax_backward_cols(const uint32_t* s, const u
       float pr = ptx::ex2(fmaf(x, scale_log2, l2));
       // the derivative of the cap goes onto P first: the single-pass backward computes P (1 - tanh^2) in the first
       // half of its arithmetic and meets dP only in the second, and both forms round alike
-      float d = kNeedDs ? (kSoftcap ? pr * dt : pr) * (__uint_as_float(dp[col]) + dl) : 0.f;
+      float d = kNeedDs ? (kSoftcap ? pr * dt : pr) * (__uint_as_float(dp[col]) - dl) : 0.f;
       if (kMasked && (col < lo || col >= hi)) {
         pr = 0.f;
         d = 0.f;

@@ -696,13 +696,14 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
 #pragma unroll
           for (int i = 0; i < R::kCols / 8; ++i) {
             const float4 d0 = dlv[2 * i], d1 = dlv[2 * i + 1];
-            const float ndl[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
+            const float dl[8] = {d0.x, d0.y, d0.z, d0.w, d1.x, d1.y, d1.z, d1.w};
             uint32_t pk[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const int c = 8 * i + 2 * j;
               float t0, t1;
-              ptx::add2(t0, t1, __uint_as_float(dpv[c]), __uint_as_float(dpv[c + 1]), ndl[2 * j], ndl[2 * j + 1]);
+              // dP - delta: there is no packed subtraction, the FMA with -1 rounds once like one
+              ptx::fma2(t0, t1, dl[2 * j], dl[2 * j + 1], -1.f, -1.f, __uint_as_float(dpv[c]), __uint_as_float(dpv[c + 1]));
               ptx::mul2(t0, t1, t0, t1, pr[c], pr[c + 1]);
               pk[j] = ptx::pack2<kBf16>(t0, t1);
             }

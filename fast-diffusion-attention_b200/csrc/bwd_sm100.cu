@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
         const float lse = p.lse[li];
         lse2 = (lse == -INFINITY) ? 0.f : -lse * kLog2e;
       }
-      p.delta_pad[seg + r] = valid ? -acc[u] : 0.f;
+      p.delta_pad[seg + r] = valid ? acc[u] : 0.f;
       p.lse2_pad[seg + r] = lse2;
     }
   }

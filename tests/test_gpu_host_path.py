@@ -1,0 +1,73 @@
+"""The eager host path against what the operators do: every input a caller may hold (expanded, strided and negated views),
+every context that wants to see the calls (modes, hooks on saved tensors, compiled autograd, threads), and the values the
+operators hand back. Where nothing but the route differs, results are compared bitwise (deterministic backward)."""
+
+import pytest
+import torch
+
+from fast_diffusion_attention import diffusion_attn_func, diffusion_attn_varlen_func
+from fast_diffusion_attention.interface import diffusion_attn_qkvpacked_func, diffusion_attn_varlen_qkvpacked_func
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+B, N, H, HK, D, BS = 2, 96, 4, 2, 64, 16
+LAYOUTS = ["batched", "varlen", "qkv", "varlen_qkv"]
+
+
+def _inputs(layout, seed=0, requires_grad=True):
+    """(leaves, cu, dout) of one small problem."""
+    g = torch.Generator(device=DEV).manual_seed(seed)
+
+    def normal(*shape):
+        return torch.randn(*shape, device=DEV, dtype=torch.bfloat16, generator=g)
+
+    lead = (B, 2 * N) if layout in ("batched", "qkv") else (B * 2 * N,)
+    leaves = [normal(*lead, H + 2 * HK, D)] if "qkv" in layout else [normal(*lead, h, D) for h in (H, HK, HK)]
+    cu = None if layout in ("batched", "qkv") else torch.arange(0, B * 2 * N + 1, 2 * N, device=DEV, dtype=torch.int32)
+    return [t.requires_grad_(requires_grad) for t in leaves], cu, normal(*lead, H, D)
+
+
+def _call(layout, leaves, cu, **kw):
+    kw.setdefault("deterministic", True)
+    if layout == "batched":
+        return diffusion_attn_func(*leaves, BS, **kw)
+    if layout == "varlen":
+        return diffusion_attn_varlen_func(*leaves, cu, cu, 2 * N, 2 * N, BS, **kw)
+    if layout == "qkv":
+        return diffusion_attn_qkvpacked_func(*leaves, BS, num_heads_q=H, **kw)
+    return diffusion_attn_varlen_qkvpacked_func(*leaves, cu, 2 * N, BS, num_heads_q=H, **kw)
+
+
+def _expected(layout):
+    leaves, cu, do = _inputs(layout)
+    out = _call(layout, leaves, cu)
+    return (out.detach(),) + torch.autograd.grad(out, leaves, do)
+
+
+def _assert_all_equal(got, want):
+    assert len(got) == len(want)
+    for i, (a, b) in enumerate(zip(got, want)):
+        assert torch.equal(a, b), i
+
+
+# ------------------------------------------------------------------------------------------ values handed back
+@pytest.mark.parametrize("varlen", [False, True])
+@pytest.mark.parametrize("d,deterministic", [(64, False), (128, False), (96, True), (256, False)])
+def test_backward_operator_returns_the_row_sums(d, deterministic, varlen):
+    """(batch, heads, 2, n_pad) of rowsum(dO * O), zero in the padding rows."""
+    torch.manual_seed(d)
+    n, n_pad, heads, heads_k = 150, 256, 4, 2
+    q, do = (torch.randn(B, 2 * n, heads, d, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    k, v = (torch.randn(B, 2 * n, heads_k, d, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    cu = max_len = None
+    if varlen:
+        q, k, v, do = (t.flatten(0, 1) for t in (q, k, v, do))
+        cu, max_len = torch.arange(0, B * 2 * n + 1, 2 * n, device=DEV, dtype=torch.int32), 2 * n
+    out, lse = torch.ops.fda._diffusion_attn_forward(q, k, v, 32, cu, max_len)
+    grads = [torch.empty_like(t) for t in (q, k, v)]
+    got = torch.ops.fda._diffusion_attn_backward(do, q, k, v, out, lse, *grads, 32, cu, max_len, deterministic=deterministic)
+    terms = (do.double() * out.double()).view(B, 2, n, heads, d).permute(0, 3, 1, 2, 4)
+    assert got.shape == (B, heads, 2, n_pad) and got.dtype == torch.float32
+    # fp32 sums of d exact products, in any order
+    assert ((got[..., :n] - terms.sum(-1)).abs() <= d * 2.0 ** -24 * terms.abs().sum(-1)).all()
+    assert (got[..., n:] == 0).all()

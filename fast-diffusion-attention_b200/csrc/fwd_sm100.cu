@@ -524,10 +524,12 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
         }
       }
       // P is rounded to e4m3 for FP8: the exponent is shifted by 8 (the reference's Max_offset = 8, softmax.h:67-69
-      // there) and the maximum advances when it grew by more than 0.8, so P stays below 2^8.8 = 445.8 of the type's
-      // 448. (Advancing it at every increase, as the reference does, rescales O several times as often: a warp's 32
-      // rows hardly ever all keep their maximum.) 16-bit P may run up to 2^8 above 1 before the maximum is advanced.
-      constexpr float kThreshold = Cfg::kFp8 ? 0.8f : kRescaleThreshold;
+      // there) and the maximum advances at every increase, so P stays in (0, 2^8] and the largest P of a row is 2^8
+      // itself, which e4m3 holds exactly. (P up to 2^8.8 would still fit below 448 and spare most of the rescales of O,
+      // 557 instead of 610 us on 4 x 8192 tokens, 16/4 heads of 128, but would round the probability that matters most,
+      // by up to 6 %, and the relative error of the output rises from 1.97e-2 to 2.06e-2.) 16-bit P may run up to 2^8
+      // above 1 before the maximum is advanced.
+      constexpr float kThreshold = Cfg::kFp8 ? 0.f : kRescaleThreshold;
       constexpr float kPShift = Cfg::kFp8 ? 8.f : 0.f;
       float m_run = -INFINITY;  // reference maximum (unscaled scores, or tanh values with softcap)
       float l_run = 0.f;
@@ -592,14 +594,20 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
             }
             if (!alive) break;
             ptx::tc_fence_after();
+            // A load is answered after some 250 cycles while products run, however wide it is. fp8 rescales often, and with
+            // one query tile has the registers for 128 columns a round (2 x 16384 tokens, 8 heads of 256: 1017 -> 948 us;
+            // with two tiles 64 are slower than 32, 646 against 610 us on 4 x 8192 tokens, 16/4 heads of 128).
+            constexpr int kRound = Cfg::kFp8 && kQTiles == 1 ? 128 : 32;
 #pragma unroll
-            for (int c = 0; c < kHeadDim / 32; ++c) {
-              uint32_t o[32];
-              ptx::tmem_ld32(tmem_o + c * 32, o);
+            for (int c0 = 0; c0 < kHeadDim; c0 += kRound) {
+              uint32_t o[kRound];
+#pragma unroll
+              for (int c = 0; c < kRound; c += 32) ptx::tmem_ld32(tmem_o + c0 + c, o + c);
               ptx::tmem_wait_ld();
 #pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
-              ptx::tmem_st32(tmem_o + c * 32, o);
+              for (int i = 0; i < kRound; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+#pragma unroll
+              for (int c = 0; c < kRound; c += 32) ptx::tmem_st32(tmem_o + c0 + c, o + c);
             }
           }
           l_run *= factor;

@@ -2,6 +2,8 @@
 every context that wants to see the calls (modes, hooks on saved tensors, compiled autograd, threads), and the values the
 operators hand back. Where nothing but the route differs, results are compared bitwise (deterministic backward)."""
 
+import math
+
 import pytest
 import torch
 
@@ -71,3 +73,22 @@ def test_backward_operator_returns_the_row_sums(d, deterministic, varlen):
     # fp32 sums of d exact products, in any order
     assert ((got[..., :n] - terms.sum(-1)).abs() <= d * 2.0 ** -24 * terms.abs().sum(-1)).all()
     assert (got[..., n:] == 0).all()
+
+
+@pytest.mark.parametrize("d", [64, 128, 256])
+def test_fp8_largest_probability_is_exact(d):
+    """The largest probability of a row is held as 2^8, which e4m3 has, also where the maximum creeps up by less than a
+    rounding step of the type: the row's result then errs by the rounding of the bf16 output (and of the fp32 sum)."""
+    n, small, big = 192, 0, 100                    # keys in different sub-steps, the larger score second
+    step = 0.09                                    # log2 of the ratio of the two probabilities
+    q = torch.zeros(1, 2 * n, 1, d, device=DEV)
+    k, v = torch.zeros_like(q), torch.zeros_like(q)
+    q[..., 0] = 1
+    k[..., 0] = -448                               # everything else: 2^-40 of the row
+    for half in (0, n):
+        k[:, half + small, :, 0] = 0
+        k[:, half + big, :, 0] = 1
+        v[:, half + big] = 1
+    out = diffusion_attn_func(*(t.to(torch.float8_e4m3fn) for t in (q, k, v)), n, softmax_scale=step * math.log(2))
+    want = 1 / (1 + 2.0 ** -step)
+    assert (out.double() - want).abs().max().item() <= want * 2.0 ** -8

@@ -533,7 +533,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       constexpr float kPShift = Cfg::kFp8 ? 8.f : 0.f;
       float m_run = -INFINITY;  // reference maximum (unscaled scores, or tanh values with softcap)
       float l_run = 0.f;
-      bool o_started = false;
+      bool o_started = false, settled = false;   // one sub-step, two sub-steps of this tile are done
       int buf = 0;
       for (int u = 0; u < subs && alive; ++u, buf = buf + 1 == kBufs ? 0 : buf + 1) {
         int kh, kt;
@@ -580,8 +580,11 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
         }
         const float m_tile = fmaxf(ptx::max3(mx[0], mx[1], mx[2]), ptx::max3(ptx::max3(mx[3], mx[4], mx[5]), mx[6], mx[7]));
         const float m_new = fmaxf(m_run, m_tile);
-        // advance the reference maximum only when it grew by more than the threshold (always on the first tile)
-        const bool need = (m_new - m_run) * scale_log2 > kThreshold;
+        // Advance the reference maximum only when it grew by more than the threshold. In the first two sub-steps at every
+        // increase: the largest of the first 128 scores then has P = 1 exactly, and few rows have a larger one after that.
+        // (Settling it on 64 keys saves a rescale of O an item, 289 instead of 298 us on 8 x 4096 tokens, 16 heads of 128,
+        // but the relative error of the output, over 24 drawn shapes in bf16, is 2.21e-3 instead of 2.17e-3.)
+        const bool need = (m_new - m_run) * scale_log2 > (settled ? kThreshold : 0.f);
         if (__any_sync(0xffffffffu, need)) {
           const float factor = need ? ptx::ex2((m_run - m_new) * scale_log2) : 1.f;
           if (o_started) {
@@ -648,6 +651,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
         ptx::tmem_wait_st();
         ptx::tc_fence_before();
         ptx::mbar_arrive_warp(&p_full[t * kBufs + buf]);
+        settled = o_started;
         o_started = true;
       }
       if (!alive) break;

@@ -92,3 +92,24 @@ def test_fp8_largest_probability_is_exact(d):
     out = diffusion_attn_func(*(t.to(torch.float8_e4m3fn) for t in (q, k, v)), n, softmax_scale=step * math.log(2))
     want = 1 / (1 + 2.0 ** -step)
     assert (out.double() - want).abs().max().item() <= want * 2.0 ** -8
+
+
+@pytest.mark.parametrize("dtype,digits", [(torch.bfloat16, 8), (torch.float16, 11)])
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("big", [40, 100])
+def test_largest_probability_of_the_first_keys_is_exact(d, dtype, digits, big):
+    """Where the largest score of a row is among its first 128 keys, its probability is held as 1: with one other key that
+    counts and has no value, the result errs by the rounding of the output alone."""
+    n = 192
+    step = torch.linspace(0.02, 0.98, n, device=DEV).to(dtype)     # log2 of the ratio of the two probabilities, by row
+    q = torch.zeros(1, 2 * n, 1, d, device=DEV, dtype=dtype)
+    k, v = torch.zeros_like(q), torch.zeros_like(q)
+    q[0, :, 0, 0] = step.repeat(2)
+    k[..., 0] = -10000                                             # everything else: 2^-200 of the row
+    for half in (0, n):
+        k[:, half, :, 0] = 0
+        k[:, half + big, :, 0] = 1
+        v[:, half + big] = 1
+    out = diffusion_attn_func(q, k, v, n, softmax_scale=math.log(2))[0, :, 0].double()
+    want = (1 / (1 + torch.exp2(-step.double()))).repeat(2)[:, None]
+    assert ((out - want).abs() <= want * 2.0 ** -digits * 1.001).all()

@@ -95,11 +95,23 @@ bool tile_copy_friendly(const Tensor& t) {
   return true;
 }
 
+// An expanded view: the gradient that a sum over tokens or heads hands back, keys that heads share. Tensor maps have no
+// stride of 0.
+bool repeats_itself(const Tensor& t) {
+  for (int64_t i = 0; i < t.dim(); ++i) {
+    if (t.size(i) > 1 && t.stride(i) == 0) return true;
+  }
+  return false;
+}
+
 // The reference copies an input only when its last dimension is strided (interface.py:17-18 there); a view whose base
-// or strides are not 16-byte multiples is copied as well, so that every call the reference accepts is accepted.
+// or strides are not 16-byte multiples, or with a stride of 0, is copied as well, so that every call the reference accepts
+// is accepted.
 Tensor maybe_contiguous(const Tensor& t) {
   if (!t.is_cuda()) return t;   // refused by the checks
-  if (t.dim() >= 1 && (t.stride(-1) != 1 || (t.dim() >= 3 && !tile_copy_friendly(t)))) return t.contiguous();
+  if (t.dim() >= 1 && (t.stride(-1) != 1 || (t.dim() >= 3 && (!tile_copy_friendly(t) || repeats_itself(t))))) {
+    return t.contiguous();
+  }
   return t;
 }
 

@@ -113,3 +113,35 @@ def test_largest_probability_of_the_first_keys_is_exact(d, dtype, digits, big):
     out = diffusion_attn_func(q, k, v, n, softmax_scale=math.log(2))[0, :, 0].double()
     want = (1 / (1 + torch.exp2(-step.double()))).repeat(2)[:, None]
     assert ((out - want).abs() <= want * 2.0 ** -digits * 1.001).all()
+
+
+# ------------------------------------------------------------------------------------------ views as inputs
+@pytest.mark.parametrize("layout", LAYOUTS)
+@pytest.mark.parametrize("axis", [-3, -2])
+def test_gradient_of_the_output_with_a_zero_stride(layout, axis):
+    """The gradient that a sum over tokens or heads hands back is an expanded view."""
+    grads = []
+    for expanded in (True, False):
+        leaves, cu, do = _inputs(layout)
+        w = do.select(axis, 0)
+        out = _call(layout, leaves, cu)
+        if expanded:
+            grads.append(torch.autograd.grad((out.sum(axis) * w).sum(), leaves))
+        else:
+            grads.append(torch.autograd.grad(out, leaves, w.unsqueeze(axis).expand_as(out).contiguous()))
+    _assert_all_equal(*grads)
+
+
+@pytest.mark.parametrize("layout", ["batched", "varlen"])
+@pytest.mark.parametrize("axis", [-2, -3])
+def test_expanded_keys_and_values(layout, axis):
+    results = []
+    for expanded in (True, False):
+        (q, k, v), cu, do = _inputs(layout, requires_grad=False)
+        k, v = (t.narrow(axis, 0, 1).clone().requires_grad_() for t in (k, v))
+        shape = list(k.shape)
+        shape[axis] = q.shape[axis]
+        ke, ve = (t.expand(shape) if expanded else t.expand(shape).contiguous() for t in (k, v))
+        out = _call(layout, (q, ke, ve), cu)
+        results.append((out.detach(),) + torch.autograd.grad(out, (k, v), do))
+    _assert_all_equal(*results)

@@ -115,6 +115,9 @@ Tensor maybe_contiguous(const Tensor& t) {
   return t;
 }
 
+// Offsets may be a strided view (a column of a table); forward and backward copy it alike.
+Tensor contiguous_offsets(const Tensor& cu) { return cu.defined() && cu.dim() == 1 && cu.is_cuda() ? cu.contiguous() : cu; }
+
 // The checks of the reference's check_inputs (csrc/fda/flash_api.cpp:92-139), same key words.
 Shape check_inputs(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& cu, const Options& o,
                    bool backward) {
@@ -209,7 +212,7 @@ std::pair<Tensor, Tensor> forward_impl(Tensor q, Tensor k, Tensor v, const Tenso
   q = maybe_contiguous(q);
   k = maybe_contiguous(k);
   v = maybe_contiguous(v);
-  const Tensor cu = cu_in.defined() && cu_in.dim() == 1 && cu_in.stride(0) != 1 ? cu_in.contiguous() : cu_in;
+  const Tensor cu = contiguous_offsets(cu_in);
   const Shape s = check_inputs(q, k, v, cu, o, false);
   const bool fp8 = !is_16bit(q);
   TORCH_CHECK(fp8 || !(descales[0].defined() || descales[1].defined() || descales[2].defined()),
@@ -254,7 +257,7 @@ int64_t padded_half(int64_t seqlen) { return (std::max<int64_t>(seqlen / 2, 1) +
 
 // Returns the workspace: it starts with rowsum(dO * O) in the padded (batch, heads, half, n_pad) layout.
 Tensor backward_impl(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor out, const Tensor& lse, const Tensor& dq,
-                     const Tensor& dk, const Tensor& dv, const Tensor& cu, const Options& o, Tensor workspace,
+                     const Tensor& dk, const Tensor& dv, const Tensor& cu_in, const Options& o, Tensor workspace,
                      unsigned stages, Shape* shape) {
   RECORD_FUNCTION("fda::_diffusion_attn_backward", c10::ArrayRef<const c10::IValue>{});
   dout = maybe_contiguous(dout);
@@ -262,6 +265,7 @@ Tensor backward_impl(Tensor dout, Tensor q, Tensor k, Tensor v, Tensor out, cons
   k = maybe_contiguous(k);
   v = maybe_contiguous(v);
   out = maybe_contiguous(out);
+  const Tensor cu = contiguous_offsets(cu_in);
   const Shape s = check_inputs(q, k, v, cu, o, true);
   if (shape) *shape = s;
   TORCH_CHECK(out.scalar_type() == q.scalar_type() && dout.scalar_type() == q.scalar_type(),

@@ -145,3 +145,10 @@ def test_expanded_keys_and_values(layout, axis):
         out = _call(layout, (q, ke, ve), cu)
         results.append((out.detach(),) + torch.autograd.grad(out, (k, v), do))
     _assert_all_equal(*results)
+
+
+@pytest.mark.parametrize("layout", ["varlen", "varlen_qkv"])
+def test_strided_offsets(layout):
+    leaves, cu, do = _inputs(layout)
+    out = _call(layout, leaves, torch.stack([cu, -cu], 1)[:, 0])
+    _assert_all_equal((out.detach(),) + torch.autograd.grad(out, leaves, do), _expected(layout))

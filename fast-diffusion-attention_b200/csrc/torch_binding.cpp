@@ -18,6 +18,7 @@
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
 #include <torch/csrc/jit/frontend/tracer.h>
+#include <torch/csrc/utils/object_ptr.h>
 
 #include <ATen/ATen.h>
 #include <ATen/core/LegacyTypeDispatch.h>
@@ -338,6 +339,34 @@ Tensor gradient_like(const Tensor& t) {
   return t.is_contiguous() ? empty_on(t.sizes(), t.scalar_type(), t) : at::empty_like(t);
 }
 
+// ---- who may be passed by -----------------------------------------------------------------------------------------
+// No dispatch mode, function transform or tracer wants to see the operators.
+bool plain_context() {
+  return !c10::impl::dispatch_mode_enabled() && !torch::jit::tracer::isTracing() &&
+         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+}
+
+// A CUDA tensor whose memory holds its values: no subclass, wrapper or lazily applied operation in between.
+bool plain_values(const Tensor& t) {
+  return t.is_cuda() && t.layout() == at::kStrided && !t.unsafeGetTensorImpl()->is_python_dispatch() &&
+         !t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
+                                                   c10::DispatchKey::Functionalize, c10::DispatchKey::Batched,
+                                                   c10::DispatchKey::ZeroTensor}));
+}
+
+// The Python layer's backward through the operators (interface.py `_gradients`), for calls that somebody wants to see.
+PyObject* operator_backward = nullptr;
+
+PyObject* none() {
+  Py_INCREF(Py_None);
+  return Py_None;
+}
+
+struct Gil {
+  PyGILState_STATE st = PyGILState_Ensure();
+  ~Gil() { PyGILState_Release(st); }
+};
+
 // ---- autograd node ----------------------------------------------------------------------------------------------
 // One node for separate q, k, v and for one packed projection, batched or packed samples. Saves q, k, v (or qkv), out,
 // lse and cu_seqlens, the set the reference saves (interface.py:158, :189 there).
@@ -362,10 +391,16 @@ struct DiffusionAttentionBackward : public torch::autograd::Node {
     const Tensor o = out.unpack(self), l = lse.unpack(self);
     TORCH_CHECK(!cu.defined() || cu._version() == cu_version,
                 "cu_seqlens has been modified by an inplace operation between the forward and the backward pass");
+    const Tensor dout = g[0].defined() ? g[0] : at::zeros_like(o);
     torch::autograd::variable_list r(n_in);
-    {
+    // The graph was built by an eager call, but the backward may run where a mode is on, or get a gradient that is more
+    // than its memory.
+    bool plain = plain_context() && plain_values(dout) && plain_values(o) && plain_values(l) && (!cu.defined() || plain_values(cu));
+    for (int i = 0; i < n_in; ++i) plain = plain && plain_values(x[i]);
+    if (!plain) {
+      by_operator(x, dout, o, l, &r);
+    } else {
       at::AutoDispatchBelowADInplaceOrView below;
-      const Tensor dout = g[0].defined() ? g[0] : at::zeros_like(o);
       if (n_in == 3) {
         for (int i = 0; i < 3; ++i) r[i] = gradient_like(x[i]);
         backward_impl(dout, x[0], x[1], x[2], o, l, r[0], r[1], r[2], cu, opts, Tensor(), 7u, nullptr);
@@ -385,6 +420,39 @@ struct DiffusionAttentionBackward : public torch::autograd::Node {
       }
     }
     return r;
+  }
+
+  // _gradients(inputs, dout, out, lse, cu_seqlens, num_heads_q, max_seqlen, block_size, softmax_scale, softcap,
+  //            deterministic, sm_margin) -> the inputs' gradients
+  void by_operator(const Tensor* x, const Tensor& dout, const Tensor& o, const Tensor& l, torch::autograd::variable_list* r) {
+    Gil gil;
+    auto own = [](PyObject* p) {
+      if (!p) {
+        python_error e;
+        e.persist();
+        throw e;
+      }
+      return THPObjectPtr(p);
+    };
+    auto integer = [](int64_t v) { return v < 0 ? none() : PyLong_FromLongLong(v); };
+    auto scale = [](double v) { return std::isnan(v) ? none() : PyFloat_FromDouble(v); };
+    THPObjectPtr inputs = own(PyTuple_New(n_in));
+    for (int i = 0; i < n_in; ++i) PyTuple_SET_ITEM(inputs.get(), i, own(THPVariable_Wrap(x[i])).release());
+    THPObjectPtr args = own(PyTuple_New(12));
+    int at = 0;
+    auto add = [&](PyObject* p) { PyTuple_SET_ITEM(args.get(), at++, own(p).release()); };
+    add(inputs.release());
+    for (const Tensor& t : {dout, o, l, cu}) add(THPVariable_Wrap(t));
+    add(integer(opts.heads_q));
+    add(integer(opts.max_seqlen));
+    add(PyLong_FromLongLong(opts.block_size));
+    add(scale(opts.softmax_scale));
+    add(PyFloat_FromDouble(opts.softcap));
+    add(PyBool_FromLong(opts.deterministic));
+    add(PyLong_FromLongLong(opts.sm_margin));
+    THPObjectPtr grads = own(PyObject_CallObject(operator_backward, args.get()));
+    TORCH_CHECK(PyTuple_Check(grads.get()) && PyTuple_GET_SIZE(grads.get()) == n_in, "one gradient for every input");
+    for (int i = 0; i < n_in; ++i) (*r)[i] = THPVariable_Unpack(PyTuple_GET_ITEM(grads.get(), i));
   }
 };
 
@@ -449,23 +517,11 @@ bool to_bool(PyObject* o, bool* out) {
 bool plain_tensor(PyObject* o, Tensor* out) {
   if (!THPVariable_CheckExact(o)) return false;
   const Tensor& t = THPVariable_Unpack(o);
-  if (!t.defined() || !t.is_cuda() || t.layout() != at::kStrided || t.unsafeGetTensorImpl()->is_python_dispatch()) return false;
-  if (t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
-                                               c10::DispatchKey::Functionalize, c10::DispatchKey::Batched,
-                                               c10::DispatchKey::ZeroTensor}))) {
-    return false;
-  }
-  if (t._fw_grad(0).defined()) return false;
+  if (!t.defined() || !plain_values(t) || t._fw_grad(0).defined()) return false;
   *out = t;
   return true;
 }
 bool optional_plain_tensor(PyObject* o, Tensor* out) { return o == Py_None || plain_tensor(o, out); }
-
-// No dispatch mode, function transform or tracer wants to see the operators.
-bool plain_context() {
-  return !c10::impl::dispatch_mode_enabled() && !torch::jit::tracer::isTracing() &&
-         !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
-}
 
 // softmax_scale None -> NaN
 bool to_scale(PyObject* o, double* out) {
@@ -622,9 +678,10 @@ PyObject* py_backward(PyObject*, PyObject* const* args, Py_ssize_t n) {
   END_HANDLE_TH_ERRORS
 }
 
-PyObject* py_bind(PyObject*, PyObject* arg) {
+PyObject* py_bind(PyObject*, PyObject* const* args, Py_ssize_t n) {
   HANDLE_TH_ERRORS
-  const char* path = PyUnicode_AsUTF8(arg);
+  TORCH_CHECK(n == 2, "bind takes 2 arguments");
+  const char* path = PyUnicode_AsUTF8(args[0]);
   if (!path) throw python_error();
   void* lib = dlopen(path, RTLD_NOW | RTLD_LOCAL);
   TORCH_CHECK(lib, "cannot load ", path, ": ", dlerror());
@@ -639,6 +696,8 @@ PyObject* py_bind(PyObject*, PyObject* arg) {
   abi.bwd_stages = reinterpret_cast<decltype(abi.bwd_stages)>(sym("fda_bwd_stages"));
   abi.strerror_ = reinterpret_cast<decltype(abi.strerror_)>(sym("fda_strerror"));
   abi.last_cuda_error = reinterpret_cast<decltype(abi.last_cuda_error)>(sym("fda_last_cuda_error"));
+  Py_INCREF(args[1]);
+  Py_XSETREF(operator_backward, args[1]);
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
@@ -651,7 +710,7 @@ PyMethodDef methods[] = {
     {"attention_packed", as_pycfunction(py_attention_packed), METH_FASTCALL, "the same on one packed projection"},
     {"forward", as_pycfunction(py_forward), METH_FASTCALL, "body of the forward operator"},
     {"backward", as_pycfunction(py_backward), METH_FASTCALL, "body of the backward operator"},
-    {"bind", py_bind, METH_O, "path of the kernel library"},
+    {"bind", as_pycfunction(py_bind), METH_FASTCALL, "path of the kernel library, backward through the operators"},
     {nullptr, nullptr, 0, nullptr},
 };
 

@@ -6,6 +6,7 @@ import math
 
 import pytest
 import torch
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from fast_diffusion_attention import diffusion_attn_func, diffusion_attn_varlen_func
 from fast_diffusion_attention.interface import diffusion_attn_qkvpacked_func, diffusion_attn_varlen_qkvpacked_func
@@ -152,3 +153,26 @@ def test_strided_offsets(layout):
     leaves, cu, do = _inputs(layout)
     out = _call(layout, leaves, torch.stack([cu, -cu], 1)[:, 0])
     _assert_all_equal((out.detach(),) + torch.autograd.grad(out, leaves, do), _expected(layout))
+
+
+# ------------------------------------------------------------------------------------------ who wants to see the calls
+
+
+class _DispatchLog(TorchDispatchMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+        self.seen.append(str(func))
+        return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_dispatch_mode_around_the_backward_alone(layout):
+    leaves, cu, do = _inputs(layout)
+    out = _call(layout, leaves, cu)
+    with _DispatchLog() as log:
+        grads = torch.autograd.grad(out, leaves, do)
+    assert any("_diffusion_attn_backward" in s for s in log.seen), log.seen
+    _assert_all_equal((out.detach(),) + grads, _expected(layout))

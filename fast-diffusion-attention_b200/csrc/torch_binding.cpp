@@ -351,7 +351,8 @@ bool plain_values(const Tensor& t) {
   return t.is_cuda() && t.layout() == at::kStrided && !t.unsafeGetTensorImpl()->is_python_dispatch() &&
          !t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
                                                    c10::DispatchKey::Functionalize, c10::DispatchKey::Batched,
-                                                   c10::DispatchKey::ZeroTensor}));
+                                                   c10::DispatchKey::ZeroTensor, c10::DispatchKey::Negative,
+                                                   c10::DispatchKey::Conjugate}));
 }
 
 // The Python layer's backward through the operators (interface.py `_gradients`), for calls that somebody wants to see.

@@ -155,6 +155,20 @@ def test_strided_offsets(layout):
     _assert_all_equal((out.detach(),) + torch.autograd.grad(out, leaves, do), _expected(layout))
 
 
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_lazily_negated_views(layout):
+    """A tensor whose values are negated by a flag on the view (as the imaginary part of a conjugate is)."""
+    leaves, cu, do = _inputs(layout)
+    want = _expected(layout)
+    with torch.no_grad():
+        negated = [torch._neg_view(-t).requires_grad_() for t in leaves]
+    assert negated[0].is_neg()
+    out = _call(layout, negated, cu)
+    _assert_all_equal((out.detach(),) + torch.autograd.grad(out, negated, do), want)
+    out = _call(layout, leaves, cu)
+    _assert_all_equal((out.detach(),) + torch.autograd.grad(out, leaves, torch._neg_view(-do)), want)
+
+
 # ------------------------------------------------------------------------------------------ who wants to see the calls
 
 

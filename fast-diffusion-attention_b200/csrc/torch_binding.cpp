@@ -21,6 +21,7 @@
 #include <torch/csrc/utils/object_ptr.h>
 
 #include <ATen/ATen.h>
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/core/LegacyTypeDispatch.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/record_function.h>
@@ -340,9 +341,9 @@ Tensor gradient_like(const Tensor& t) {
 }
 
 // ---- who may be passed by -----------------------------------------------------------------------------------------
-// No dispatch mode, function transform or tracer wants to see the operators.
+// No dispatch or function mode, function transform or tracer wants to see the operators.
 bool plain_context() {
-  return !c10::impl::dispatch_mode_enabled() && !torch::jit::tracer::isTracing() &&
+  return !c10::impl::dispatch_mode_enabled() && !at::impl::torch_function_mode_enabled() && !torch::jit::tracer::isTracing() &&
          !c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
 }
 

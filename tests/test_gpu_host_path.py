@@ -6,6 +6,7 @@ import math
 
 import pytest
 import torch
+from torch.overrides import TorchFunctionMode
 from torch.utils._python_dispatch import TorchDispatchMode
 
 from fast_diffusion_attention import diffusion_attn_func, diffusion_attn_varlen_func
@@ -170,6 +171,14 @@ def test_lazily_negated_views(layout):
 
 
 # ------------------------------------------------------------------------------------------ who wants to see the calls
+class _FunctionLog(TorchFunctionMode):
+    def __init__(self):
+        super().__init__()
+        self.seen = []
+
+    def __torch_function__(self, func, types, args=(), kwargs=None):
+        self.seen.append(str(func))
+        return func(*args, **(kwargs or {}))
 
 
 class _DispatchLog(TorchDispatchMode):
@@ -180,6 +189,15 @@ class _DispatchLog(TorchDispatchMode):
     def __torch_dispatch__(self, func, types, args=(), kwargs=None):
         self.seen.append(str(func))
         return func(*args, **(kwargs or {}))
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_function_mode_sees_the_operator(layout):
+    leaves, cu, do = _inputs(layout)
+    with _FunctionLog() as log:
+        out = _call(layout, leaves, cu)
+    assert any("_diffusion_attn_forward" in s for s in log.seen), log.seen
+    _assert_all_equal((out.detach(),) + torch.autograd.grad(out, leaves, do), _expected(layout))
 
 
 @pytest.mark.parametrize("layout", LAYOUTS)

@@ -33,6 +33,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <optional>
 #include <string>
 
 #include "../../include/fda.h"
@@ -63,7 +64,7 @@ void check_status(int rc) {
 struct Options {
   int64_t block_size = 0;
   int64_t max_seqlen = -1;      // -1: not given
-  double softmax_scale = NAN;   // NaN: 1 / sqrt(head dim)
+  std::optional<double> softmax_scale;   // not given: 1 / sqrt(head dim)
   double softcap = 0.0;
   bool deterministic = false;
   int64_t sm_margin = 0;
@@ -182,7 +183,7 @@ FdaTensor tensor_view(const Tensor& t, bool varlen) {
 }
 
 double scale_of(const Options& o, const Shape& s) {
-  return std::isnan(o.softmax_scale) ? 1.0 / std::sqrt(static_cast<double>(s.head_dim)) : o.softmax_scale;
+  return o.softmax_scale ? *o.softmax_scale : 1.0 / std::sqrt(static_cast<double>(s.head_dim));
 }
 
 FdaProblem problem_of(const Tensor& q, const Tensor& cu, const Shape& s, const Options& o) {
@@ -437,7 +438,6 @@ struct DiffusionAttentionBackward : public torch::autograd::Node {
       return THPObjectPtr(p);
     };
     auto integer = [](int64_t v) { return v < 0 ? none() : PyLong_FromLongLong(v); };
-    auto scale = [](double v) { return std::isnan(v) ? none() : PyFloat_FromDouble(v); };
     THPObjectPtr inputs = own(PyTuple_New(n_in));
     for (int i = 0; i < n_in; ++i) PyTuple_SET_ITEM(inputs.get(), i, own(THPVariable_Wrap(x[i])).release());
     THPObjectPtr args = own(PyTuple_New(12));
@@ -448,7 +448,7 @@ struct DiffusionAttentionBackward : public torch::autograd::Node {
     add(integer(opts.heads_q));
     add(integer(opts.max_seqlen));
     add(PyLong_FromLongLong(opts.block_size));
-    add(scale(opts.softmax_scale));
+    add(opts.softmax_scale ? PyFloat_FromDouble(*opts.softmax_scale) : none());
     add(PyFloat_FromDouble(opts.softcap));
     add(PyBool_FromLong(opts.deterministic));
     add(PyLong_FromLongLong(opts.sm_margin));
@@ -525,10 +525,12 @@ bool plain_tensor(PyObject* o, Tensor* out) {
 }
 bool optional_plain_tensor(PyObject* o, Tensor* out) { return o == Py_None || plain_tensor(o, out); }
 
-// softmax_scale None -> NaN
-bool to_scale(PyObject* o, double* out) {
-  if (o == Py_None) { *out = NAN; return true; }
-  return to_double(o, out);
+bool to_scale(PyObject* o, std::optional<double>* out) {
+  if (o == Py_None) return true;
+  double v;
+  if (!to_double(o, &v)) return false;
+  *out = v;
+  return true;
 }
 
 PyObject* pair_to_python(const std::pair<Tensor, Tensor>& r) {

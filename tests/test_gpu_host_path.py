@@ -170,6 +170,13 @@ def test_lazily_negated_views(layout):
     _assert_all_equal((out.detach(),) + torch.autograd.grad(out, leaves, torch._neg_view(-do)), want)
 
 
+def test_scale_that_is_not_a_number_reaches_the_output():
+    leaves, cu, _ = _inputs("batched", requires_grad=False)
+    for call in (lambda: diffusion_attn_func(*leaves, BS, softmax_scale=math.nan),
+                 lambda: torch.ops.fda._diffusion_attn_forward(*leaves, BS, softmax_scale=math.nan)[0]):
+        assert call().isnan().all()
+
+
 # ------------------------------------------------------------------------------------------ who wants to see the calls
 class _FunctionLog(TorchFunctionMode):
     def __init__(self):

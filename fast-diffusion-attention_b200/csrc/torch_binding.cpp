@@ -584,7 +584,7 @@ PyObject* py_attention_packed(PyObject*, PyObject* const* args, Py_ssize_t n) {
   TORCH_CHECK(n == 9, "attention_packed takes 9 arguments");
   Tensor x[3], cu, ds[3];
   Options o;
-  if (!plain_context() || !plain_tensor(args[0], &x[0]) || (args[1] != Py_None && !to_int(args[1], &o.heads_q)) ||
+  if (!plain_context() || !plain_tensor(args[0], &x[0]) || (args[1] != Py_None && (!to_int(args[1], &o.heads_q) || o.heads_q < 0)) ||
       !optional_plain_tensor(args[2], &cu) || (args[3] != Py_None && !to_int(args[3], &o.max_seqlen)) ||
       !to_int(args[4], &o.block_size) || !to_scale(args[5], &o.softmax_scale) || !to_double(args[6], &o.softcap) ||
       !to_bool(args[7], &o.deterministic) || !to_int(args[8], &o.sm_margin)) {

@@ -177,6 +177,12 @@ def test_scale_that_is_not_a_number_reaches_the_output():
         assert call().isnan().all()
 
 
+def test_packed_head_count_is_checked():
+    qkv = torch.randn(1, 64, 3, 2, 64, device=DEV, dtype=torch.bfloat16)
+    with pytest.raises(ValueError, match="num_heads_q disagrees"):
+        diffusion_attn_qkvpacked_func(qkv, 16, num_heads_q=-1)
+
+
 # ------------------------------------------------------------------------------------------ who wants to see the calls
 class _FunctionLog(TorchFunctionMode):
     def __init__(self):

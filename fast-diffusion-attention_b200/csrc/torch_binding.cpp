@@ -374,9 +374,8 @@ struct Gil {
 // One node for separate q, k, v and for one packed projection, batched or packed samples. Saves q, k, v (or qkv), out,
 // lse and cu_seqlens, the set the reference saves (interface.py:158, :189 there).
 struct DiffusionAttentionBackward : public torch::autograd::Node {
-  torch::autograd::SavedVariable in[3], out, lse;
-  Tensor cu;   // int32 offsets, no gradient
-  uint32_t cu_version = 0;
+  torch::autograd::SavedVariable in[3], out, lse, cu;   // cu: only of packed samples
+  bool varlen = false;
   int n_in = 0;
   Options opts;
 
@@ -385,33 +384,31 @@ struct DiffusionAttentionBackward : public torch::autograd::Node {
     for (auto& s : in) s.reset_data();
     out.reset_data();
     lse.reset_data();
-    cu = Tensor();
+    cu.reset_data();
   }
   torch::autograd::variable_list apply(torch::autograd::variable_list&& g) override {
     auto self = getptr();
     Tensor x[3];
     for (int i = 0; i < n_in; ++i) x[i] = in[i].unpack();
-    const Tensor o = out.unpack(self), l = lse.unpack(self);
-    TORCH_CHECK(!cu.defined() || cu._version() == cu_version,
-                "cu_seqlens has been modified by an inplace operation between the forward and the backward pass");
+    const Tensor o = out.unpack(self), l = lse.unpack(self), offsets = varlen ? cu.unpack() : Tensor();
     const Tensor dout = g[0].defined() ? g[0] : at::zeros_like(o);
     torch::autograd::variable_list r(n_in);
     // The graph was built by an eager call, but the backward may run where a mode is on, or get a gradient that is more
     // than its memory.
-    bool plain = plain_context() && plain_values(dout) && plain_values(o) && plain_values(l) && (!cu.defined() || plain_values(cu));
+    bool plain = plain_context() && plain_values(dout) && plain_values(o) && plain_values(l) && (!varlen || plain_values(offsets));
     for (int i = 0; i < n_in; ++i) plain = plain && plain_values(x[i]);
     if (!plain) {
-      by_operator(x, dout, o, l, &r);
+      by_operator(x, dout, o, l, offsets, &r);
     } else {
       at::AutoDispatchBelowADInplaceOrView below;
       if (n_in == 3) {
         for (int i = 0; i < 3; ++i) r[i] = gradient_like(x[i]);
-        backward_impl(dout, x[0], x[1], x[2], o, l, r[0], r[1], r[2], cu, opts, Tensor(), 7u, nullptr);
+        backward_impl(dout, x[0], x[1], x[2], o, l, r[0], r[1], r[2], offsets, opts, Tensor(), 7u, nullptr);
       } else {
         r[0] = empty_on(x[0].sizes(), x[0].scalar_type(), x[0]);
-        const Views v = split_packed(x[0], opts.heads_q, cu.defined());
-        const Views d = split_packed(r[0], opts.heads_q, cu.defined());
-        backward_impl(dout, v.q, v.k, v.v, o, l, d.q, d.k, d.v, cu, opts, Tensor(), 7u, nullptr);
+        const Views v = split_packed(x[0], opts.heads_q, varlen);
+        const Views d = split_packed(r[0], opts.heads_q, varlen);
+        backward_impl(dout, v.q, v.k, v.v, o, l, d.q, d.k, d.v, offsets, opts, Tensor(), 7u, nullptr);
       }
     }
     if (at::GradMode::is_enabled()) {
@@ -427,7 +424,8 @@ struct DiffusionAttentionBackward : public torch::autograd::Node {
 
   // _gradients(inputs, dout, out, lse, cu_seqlens, num_heads_q, max_seqlen, block_size, softmax_scale, softcap,
   //            deterministic, sm_margin) -> the inputs' gradients
-  void by_operator(const Tensor* x, const Tensor& dout, const Tensor& o, const Tensor& l, torch::autograd::variable_list* r) {
+  void by_operator(const Tensor* x, const Tensor& dout, const Tensor& o, const Tensor& l, const Tensor& offsets,
+                   torch::autograd::variable_list* r) {
     Gil gil;
     auto own = [](PyObject* p) {
       if (!p) {
@@ -444,7 +442,7 @@ struct DiffusionAttentionBackward : public torch::autograd::Node {
     int at = 0;
     auto add = [&](PyObject* p) { PyTuple_SET_ITEM(args.get(), at++, own(p).release()); };
     add(inputs.release());
-    for (const Tensor& t : {dout, o, l, cu}) add(THPVariable_Wrap(t));
+    for (const Tensor& t : {dout, o, l, offsets}) add(THPVariable_Wrap(t));
     add(integer(opts.heads_q));
     add(integer(opts.max_seqlen));
     add(PyLong_FromLongLong(opts.block_size));
@@ -470,11 +468,9 @@ std::pair<Tensor, Tensor> attention(const Tensor* x, int n_in, const Tensor& cu,
     torch::autograd::edge_list edges;
     for (int i = 0; i < n_in; ++i) edges.push_back(torch::autograd::impl::gradient_edge(x[i]));
     node->set_next_edges(std::move(edges));
-    for (int i = 0; i < n_in; ++i) node->in[i] = torch::autograd::SavedVariable(x[i], false);
     node->n_in = n_in;
+    node->varlen = cu.defined();
     node->opts = o;
-    node->cu = cu;
-    if (cu.defined()) node->cu_version = static_cast<uint32_t>(cu._version());
   }
   std::pair<Tensor, Tensor> r;
   {
@@ -489,8 +485,11 @@ std::pair<Tensor, Tensor> attention(const Tensor* x, int n_in, const Tensor& cu,
   if (node) {
     torch::autograd::set_history(r.first, node);
     torch::autograd::set_history(r.second, node);
+    // everything through hooks on saved tensors, in the order in which the Python node saves
+    for (int i = 0; i < n_in; ++i) node->in[i] = torch::autograd::SavedVariable(x[i], false);
     node->out = torch::autograd::SavedVariable(r.first, true);
     node->lse = torch::autograd::SavedVariable(r.second, true);
+    if (cu.defined()) node->cu = torch::autograd::SavedVariable(cu, false);
   }
   return r;
 }

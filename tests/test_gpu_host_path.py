@@ -221,3 +221,41 @@ def test_dispatch_mode_around_the_backward_alone(layout):
         grads = torch.autograd.grad(out, leaves, do)
     assert any("_diffusion_attn_backward" in s for s in log.seen), log.seen
     _assert_all_equal((out.detach(),) + grads, _expected(layout))
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_hooks_on_saved_tensors_see_all_of_them(layout):
+    """Everything that the node keeps goes through the hooks, in the order in which the Python twin saves it."""
+    leaves, cu, do = _inputs(layout)
+    packed, unpacked = [], []
+
+    def pack(t):
+        packed.append(t.dtype)
+        return t.cpu()
+
+    def unpack(t):
+        unpacked.append(t.dtype)
+        return t.to(DEV)
+
+    with torch.autograd.graph.saved_tensors_hooks(pack, unpack):
+        out = _call(layout, leaves, cu)
+    result = (out.detach(),) + torch.autograd.grad(out, leaves, do)
+    saved = [torch.bfloat16] * (len(leaves) + 1) + [torch.float32] + ([torch.int32] if cu is not None else [])
+    assert packed == saved and unpacked == saved
+    _assert_all_equal(result, _expected(layout))
+
+
+@pytest.mark.parametrize("layout", ["varlen", "varlen_qkv"])
+def test_offsets_changed_before_the_backward_are_noticed(layout):
+    leaves, cu, do = _inputs(layout)
+    out = _call(layout, leaves, cu)
+    cu.add_(0)
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        torch.autograd.grad(out, leaves, do)
+
+
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_checkpointed_region(layout):
+    leaves, cu, do = _inputs(layout)
+    out = torch.utils.checkpoint.checkpoint(lambda *x: _call(layout, x, cu), *leaves, use_reentrant=False)
+    _assert_all_equal((out.detach(),) + torch.autograd.grad(out, leaves, do), _expected(layout))

@@ -33,6 +33,7 @@
 
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <optional>
 #include <string>
 
@@ -381,6 +382,7 @@ struct DiffusionAttentionBackward : public torch::autograd::Node {
 
   std::string name() const override { return "_DiffusionAttentionBackward"; }
   void release_variables() override {
+    std::lock_guard<std::mutex> lock(mutex_);
     for (auto& s : in) s.reset_data();
     out.reset_data();
     lse.reset_data();
@@ -389,8 +391,14 @@ struct DiffusionAttentionBackward : public torch::autograd::Node {
   torch::autograd::variable_list apply(torch::autograd::variable_list&& g) override {
     auto self = getptr();
     Tensor x[3];
-    for (int i = 0; i < n_in; ++i) x[i] = in[i].unpack();
-    const Tensor o = out.unpack(self), l = lse.unpack(self), offsets = varlen ? cu.unpack() : Tensor();
+    Tensor o, l, offsets;
+    {
+      std::lock_guard<std::mutex> lock(mutex_);   // another thread may be releasing the same graph
+      for (int i = 0; i < n_in; ++i) x[i] = in[i].unpack();
+      o = out.unpack(self);
+      l = lse.unpack(self);
+      if (varlen) offsets = cu.unpack();
+    }
     const Tensor dout = g[0].defined() ? g[0] : at::zeros_like(o);
     torch::autograd::variable_list r(n_in);
     // The graph was built by an eager call, but the backward may run where a mode is on, or get a gradient that is more

@@ -3,6 +3,7 @@ every context that wants to see the calls (modes, hooks on saved tensors, compil
 operators hand back. Where nothing but the route differs, results are compared bitwise (deterministic backward)."""
 
 import math
+import threading
 
 import pytest
 import torch
@@ -259,3 +260,31 @@ def test_checkpointed_region(layout):
     leaves, cu, do = _inputs(layout)
     out = torch.utils.checkpoint.checkpoint(lambda *x: _call(layout, x, cu), *leaves, use_reentrant=False)
     _assert_all_equal((out.detach(),) + torch.autograd.grad(out, leaves, do), _expected(layout))
+
+
+def test_two_threads_over_one_graph():
+    """Each thread gets the gradients or, where the other has freed the graph before it, the error that says so."""
+    want = _expected("batched")[1:]
+    for _ in range(30):
+        leaves, cu, do = _inputs("batched")
+        out = _call("batched", leaves, cu)
+        results, start = [], threading.Barrier(2)
+
+        def run():
+            start.wait()
+            try:
+                results.append(torch.autograd.grad(out, leaves, do))
+            except RuntimeError as e:
+                results.append(str(e))
+
+        threads = [threading.Thread(target=run) for _ in range(2)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert len(results) == 2 and any(not isinstance(r, str) for r in results)
+        for r in results:
+            if isinstance(r, str):
+                assert "second time" in r
+            else:
+                _assert_all_equal(r, want)

@@ -17,6 +17,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
 #include <torch/csrc/autograd/variable.h>
+#include <torch/csrc/dynamo/compiled_autograd.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/utils/object_ptr.h>
 
@@ -427,6 +428,37 @@ struct DiffusionAttentionBackward : public torch::autograd::Node {
         t = (*stop)({t})[0];
       }
     }
+    return r;
+  }
+
+  // Compiled autograd: `apply` runs on traced stand-ins of the saved tensors, under the tracer's modes and so through the
+  // operators, whose shape functions are registered.
+  void compiled_args(torch::dynamo::autograd::CompiledNodeArgs& args) const override {
+    for (int i = 0; i < n_in; ++i) args.collect(in[i], false);
+    args.collect(out, true);
+    args.collect(lse, true);
+    if (varlen) args.collect(cu, false);
+    args.collect(varlen);
+    args.collect(n_in);
+    args.collect(opts.block_size);
+    args.collect(opts.max_seqlen);
+    args.collect(opts.softmax_scale);
+    args.collect(opts.softcap);
+    args.collect(opts.deterministic);
+    args.collect(opts.sm_margin);
+    args.collect(opts.heads_q);
+  }
+  torch::autograd::variable_list apply_with_saved(const torch::autograd::variable_list& g,
+                                                  torch::dynamo::autograd::SwapSavedVariables& saved) override {
+    auto each = [&](auto&& fn) {
+      for (int i = 0; i < n_in; ++i) fn(in[i]);
+      fn(out);
+      fn(lse);
+      if (varlen) fn(cu);
+    };
+    each([&](torch::autograd::SavedVariable& v) { saved.before(v); });
+    auto r = apply(torch::autograd::variable_list(g));
+    each([&](torch::autograd::SavedVariable& v) { saved.after(v); });
     return r;
   }
 

@@ -262,6 +262,16 @@ def test_checkpointed_region(layout):
     _assert_all_equal((out.detach(),) + torch.autograd.grad(out, leaves, do), _expected(layout))
 
 
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_backward_under_compiled_autograd(layout):
+    from torch._dynamo import compiled_autograd
+    leaves, cu, do = _inputs(layout)
+    out = _call(layout, leaves, cu)
+    with compiled_autograd._enable(torch.compile(backend="eager", fullgraph=False)):
+        out.backward(do)
+    _assert_all_equal([out.detach()] + [t.grad for t in leaves], _expected(layout))
+
+
 def test_two_threads_over_one_graph():
     """Each thread gets the gradients or, where the other has freed the graph before it, the error that says so."""
     want = _expected("batched")[1:]

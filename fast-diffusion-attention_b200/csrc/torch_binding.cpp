@@ -12,7 +12,6 @@
 // layer then takes its operators, whose bodies come back here through `forward` and `backward`.
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/function.h>
-#include <torch/csrc/autograd/functions/basic_ops.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
@@ -374,7 +373,8 @@ struct Gil {
 
 // ---- autograd node ----------------------------------------------------------------------------------------------
 // One node for separate q, k, v and for one packed projection, batched or packed samples. Saves q, k, v (or qkv), out,
-// lse and cu_seqlens, the set the reference saves (interface.py:158, :189 there).
+// lse and cu_seqlens, the set the reference saves (interface.py:158, :189 there). The gradients have no derivative of their
+// own: under create_graph they come back as constants, as from the operators.
 struct DiffusionAttentionBackward : public torch::autograd::Node {
   torch::autograd::SavedVariable in[3], out, lse, cu;   // cu: only of packed samples
   bool varlen = false;
@@ -418,14 +418,6 @@ struct DiffusionAttentionBackward : public torch::autograd::Node {
         const Views v = split_packed(x[0], opts.heads_q, varlen);
         const Views d = split_packed(r[0], opts.heads_q, varlen);
         backward_impl(dout, v.q, v.k, v.v, o, l, d.q, d.k, d.v, offsets, opts, Tensor(), 7u, nullptr);
-      }
-    }
-    if (at::GradMode::is_enabled()) {
-      // create_graph: the gradients have no formula of their own, differentiating them again must not pass silently
-      for (auto& t : r) {
-        auto stop = std::make_shared<torch::autograd::DelayedError>(
-            "Trying to backward through fda::_diffusion_attn_backward but no autograd formula was registered", 1);
-        t = (*stop)({t})[0];
       }
     }
     return r;

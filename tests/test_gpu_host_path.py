@@ -272,6 +272,22 @@ def test_backward_under_compiled_autograd(layout):
     _assert_all_equal([out.detach()] + [t.grad for t in leaves], _expected(layout))
 
 
+@pytest.mark.parametrize("layout", LAYOUTS)
+def test_gradients_are_constants_under_create_graph(layout):
+    """The backward has no derivative; with the native node and with the Python one its results do not require grad."""
+    results = []
+    for mode in (_FunctionLog(), None):
+        leaves, cu, do = _inputs(layout)
+        if mode is not None:
+            with mode:
+                out = _call(layout, leaves, cu)
+        else:
+            out = _call(layout, leaves, cu)
+        results.append(torch.autograd.grad(out, leaves, do.requires_grad_(), create_graph=True))
+        assert not any(g.requires_grad for g in results[-1])
+    _assert_all_equal(*results)
+
+
 def test_two_threads_over_one_graph():
     """Each thread gets the gradients or, where the other has freed the graph before it, the error that says so."""
     want = _expected("batched")[1:]

@@ -452,12 +452,14 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         ++n_item_b;
         for (bool last = false; alive && !last; ++g) {
           const uint32_t u = g & 1u, qs = g % Cfg::kQSlots, ds = g % Cfg::kDoSlots, ss = g % Cfg::kStatSlots;
-          // the tiles are read after P^T / dS^T (pds_full), which follow products that have read them; only dO of an item
-          // that makes dV alone has not been waited for by anybody
           if (!ptx::mbar_wait(&stat_full[ss], (g / Cfg::kStatSlots) & 1u, abort_flag, 55)) { alive = false; break; }
           last = (*reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset) & 1) != 0;
           if (!ptx::mbar_wait(&pds_full[u], (g >> 1) & 1u, abort_flag, 53)) { alive = false; break; }
-          if (Cfg::kPasses == 2 && makes_dv(idx) &&
+          // The tiles this thread's products read. Most have landed long ago, but nothing it has waited for so far says so:
+          // that the other issuer saw them land reaches this thread only through its products and the compute warps.
+          if (makes_dk(idx) &&
+              !ptx::mbar_wait(&q_full[qs], (g / Cfg::kQSlots) & 1u, abort_flag, 64)) { alive = false; break; }
+          if (makes_dv(idx) &&
               !ptx::mbar_wait(&do_full[ds], (g / Cfg::kDoSlots) & 1u, abort_flag, 59)) { alive = false; break; }
           ptx::tc_fence_after();
           const uint32_t q_off = qs * (Cfg::kSubTileBytes >> 4), do_off = ds * (Cfg::kSubTileBytes >> 4);

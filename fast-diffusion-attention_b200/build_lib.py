@@ -21,6 +21,7 @@ OBJ = os.path.join(HERE, "build")
 LIB = os.path.join(HERE, "fast_diffusion_attention", "libfda_sm100.so")
 TORCH_SRC = os.path.join(CSRC, "torch_binding.cpp")
 TORCH_EXT = os.path.join(HERE, "fast_diffusion_attention", "_fda_torch.so")
+TORCH_STAMP = os.path.join(OBJ, "_fda_torch.txt")   # what TORCH_EXT was built with
 SOURCES = ["abi.cu", "fwd_sm100.cu", "bwd_sm100.cu", "bwd_fused_sm100.cu", "selftest_sm100.cu", "varlen_list.cu"]
 
 
@@ -64,6 +65,20 @@ def _stale(target, deps):
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def _torch_stamp(command):
+    import torch
+    return " ".join([torch.__version__] + command)
+
+
+def _torch_ext_stale(command):
+    """The host path is bound to the torch it was built against, whose headers no time stamp here covers: another version,
+    another place or other flags rebuild it."""
+    if _stale(TORCH_EXT, [TORCH_SRC, os.path.join(HERE, "..", "include", "fda.h")]) or not os.path.exists(TORCH_STAMP):
+        return True
+    with open(TORCH_STAMP) as f:
+        return f.read() != _torch_stamp(command)
+
+
 def build(force=False, verbose=False):
     os.makedirs(OBJ, exist_ok=True)
     flags = ["-std=c++17", "-O3", "-gencode", "arch=compute_100a,code=sm_100a", "-Xcompiler", "-fPIC",
@@ -91,10 +106,15 @@ def build(force=False, verbose=False):
             raise RuntimeError("compilation failed: " + " ".join(cmd))
 
     links = list(jobs)
-    if force or _stale(TORCH_EXT, [TORCH_SRC, os.path.join(HERE, "..", "include", "fda.h")]):
-        jobs.append(_torch_command())
+    torch_command = _torch_command()
+    torch_stale = force or _torch_ext_stale(torch_command)
+    if torch_stale:
+        jobs.append(torch_command)
     with ThreadPoolExecutor(max_workers=int(os.environ.get("MAX_JOBS", "4"))) as ex:
         list(ex.map(run, jobs))
+    if torch_stale:
+        with open(TORCH_STAMP, "w") as f:
+            f.write(_torch_stamp(torch_command))
     if force or links or _stale(LIB, objs):
         run([_nvcc(), "-shared", "-o", LIB] + objs + ["-cudart", "static"])
     return LIB

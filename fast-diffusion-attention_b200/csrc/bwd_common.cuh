@@ -218,7 +218,7 @@ __device__ __forceinline__ KvSpans make_kv_spans(const KvItem& it, int bs) {
 // P^T / dS^T, the tensor pipe runs dV / dK of the previous sub-tile and S^T / dP^T of the next one.
 constexpr int kSub = 64;
 constexpr int kSubCols = kSub / kCmpWG;  // 16 query columns per compute warpgroup
-// with no visible row is skipped. All roles walk this sequence identically.
+
 // Number of key-tile items of a launch: known to the host for the batched layout, read from the work list otherwise.
 __device__ __forceinline__ int kv_item_count(const BwdParams& p) {
   return (p.vl.base != nullptr ? p.vl.base[0] : p.tiles_per_half * p.batch) * 2 * p.heads_k;
@@ -235,32 +235,5 @@ inline int bwd_item_bound(const BwdParams& p, int heads) {
 struct SubStep {
   int h, qh, sa, sb, cls;
 };
-
-// Calls fn(SubStep) for every non-skipped sub-step of the item, in order; stops early when fn returns false.
-template <typename Fn>
-__device__ __forceinline__ bool for_each_substep(const KvItem& it, const QueryPlan& plan, const KvSpans& spans,
-                                                 int group, Fn&& fn) {
-  for (int g = 0; g < group; ++g) {
-    for (int s = 0; s < plan.steps(); ++s) {
-      int qh, qt;
-      plan.step(s, it.kh, qh, qt);
-      const int qa = qt * kTile, qb = imin(qa + kTile, it.n);
-      if (spans.classify(qh, it.kh, qa, qb) == kTileSkip) continue;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        SubStep st;
-        st.sa = qa + half * kSub;
-        if (st.sa >= qb) continue;
-        st.sb = imin(st.sa + kSub, qb);
-        st.cls = spans.classify(qh, it.kh, st.sa, st.sb);
-        if (st.cls == kTileSkip) continue;
-        st.h = it.hk * group + g;
-        st.qh = qh;
-        if (!fn(st)) return false;
-      }
-    }
-  }
-  return true;
-}
 
 }  // namespace fda

@@ -15,8 +15,8 @@
 // accumulator in global memory: the drain warps move it from tensor memory through a small shared-memory staging
 // area and out as 4 KB bulk reductions (cp.reduce.async.bulk add.f32); `bwd_dq_convert_kernel` then scales and
 // rounds the accumulator into dQ.
-// About 30 bytes per clock leave an SM towards L2 whatever the instruction, 2200 cycles for the 64 KB of a step, so the
-// drain runs under the next step's products.
+// Some 20 bytes per clock and SM go towards L2 this way when all SMs do it (5.8 TB/s in a microbenchmark, whatever the
+// instruction), 3300 cycles for the 64 KB of a step, so the drain runs under the next step's products.
 //
 // The reference does the same five GEMMs per pair with an fp32 dQ accumulator reduced through global memory
 // (csrc/fda/mainloop_bwd_sm90_tma_gmma_ws.hpp:815-984 `bwd_step`, :605-664 `store_dq`, there with
@@ -62,11 +62,12 @@ struct FusedCfg {
 // launch.
 //   Head dim 128: two compute warpgroups of 64 columns. 512 threads start with 128 registers, and the drain warps hold a
 //     whole dQ^T (128 columns): the buffer it shares with dP^T is free 250 cycles after the product instead of after 48
-//     of its 64 KB have left for L2. A step of the long loop takes 4300 cycles instead of 5300 (backward of 4 x 8192
-//     tokens, 32/8 heads of 128, blocks of 1024: 4.25 -> 3.98 ms). What bounds it now is shared memory: operands 2300
-//     cycles at 128 bytes a clock, the staging of dQ^T 1024, dS^T 256, the loads 512, statistics 250. Vector reductions
-//     straight from the registers would save the staging, but stall the load/store unit for the compute warps (their
-//     second half took 2100 cycles instead of 1150; 4.1 ms).
+//     of its 64 KB have left for L2 (backward of 4 x 8192 tokens, 32/8 heads of 128, blocks of 1024: 4.25 -> 3.98 ms).
+//     What bounds it is not settled. The kernel's time there is 6250 cycles for each of a CTA's 1107 steps. The tensor
+//     pipe's arithmetic is 2560 of them; shared memory at 128 bytes a clock 4350 (operands 2300, the staging of dQ^T 1024,
+//     the loads 512, dS^T 256, statistics 250); without the reductions themselves, everything else as it is, 5500 remain
+//     (and 3 % less time on 8 x 4096 tokens, 16 heads, blocks of 256). Vector reductions straight from the registers
+//     would save the staging, but stall the load/store unit for the compute warps (4.1 ms).
 //   Head dim 64: dQ^T has columns of its own, and the exponentials (and tanh) weigh more: four compute warpgroups of 32
 //     columns keep the special-function unit busier than two (4 x 8192 tokens, 32 heads, score cap: 2.8 against 3.2 ms).
 template <int kHeadDim>
@@ -82,7 +83,9 @@ struct FusedRoles {
   static constexpr uint32_t kProducerRegs = 64;
   static constexpr uint32_t kDrainRegs = kCmpWG == 2 ? 160 : 64;
   static constexpr int kHold = kCmpWG == 2 ? 4 : 1;   // 32-column chunks of dQ^T that a drain warp holds at once
-  // A warp of its own works the items out ahead of the loader (head dim 64, scores capped: 2.77 ms with it, 2.72 without)
+  // A warp of its own works the items out ahead of the loader. Head dim 128: backward of 8 x 4096 tokens, 16 heads, blocks
+  // of 256, 1036 us without and 1017 with it. Head dim 64: 4 x 8192, 32 heads, scores capped, 2750 without and 2824 with
+  // it; 64 x 256 tokens, 16 heads, 155 and 148; no difference on 4 x 4096, 32/8 heads.
   static constexpr bool kGeometryWarp = kHeadDim == 128;
   static_assert(128 * (kCmpWG * kComputeRegs + kProducerRegs + kDrainRegs) <= kThreads * kLaunchRegs, "register pool");
 };
@@ -102,15 +105,16 @@ struct QStep {
 
 // What the roles need to know about an item. At head dim 128 a warp of its own takes the items, works this out (some
 // twenty integer divisions and a ticket from global memory) while the last steps of the item before are under way, and
-// leaves it beside the mailbox; where items are short that counts (backward of 8 x 4096 tokens, 16 heads of 128, blocks of
-// 256: 1050 -> 1024 us). At head dim 64 the loader does it between its loads.
+// leaves it beside the mailbox; where items are short that counts. At head dim 64 the loader does it between its loads.
 struct FusedItem {
   KvItem it;
   QueryPlan plan;
   KvSpans spans;
   int grow0;   // first row of the sample in the packed row space
 };
-constexpr int kTicketSteps = 4;   // the next item is taken when at most this many steps of the current one are to be sent
+// The next item is taken when at most this many steps of the current one are to be sent: early enough for the ticket's
+// round trip, late enough that CTAs do not reserve work. It hardly matters (same backward with 1, 4, 16: 1018, 1017, 1024).
+constexpr int kTicketSteps = 4;
 
 template <typename Fn>
 __device__ __forceinline__ bool for_each_qstep(const KvItem& it, const QueryPlan& plan, const KvSpans& spans, int group,

@@ -6,20 +6,22 @@
 // epilogue_bwd.hpp:25-441), and convert passes (flash_bwd_postprocess_kernel.h:160-264). On B200 the tensor
 // memory budget (512 columns) and the cost of a global fp32 reduction lead to a different split:
 //
-//   1. bwd_preprocess : delta = rowsum(dO * O) and LSE * log2(e), written to a padded per-(sample, head, half)
-//                       layout whose padding rows carry LSE2 = +inf (so padded query rows get P = 0).
+//   1. bwd_preprocess : delta = rowsum(dO * O) and -LSE * log2(e), written to a padded per-(sample, head, half)
+//                       layout whose padding rows carry -inf for the latter (so padded query rows get P = 0). It also
+//                       zeroes the work counters and small dQ accumulators of the kernels that follow.
 //   2. bwd_dkdv       : one CTA per (128-key tile, KV head, sample, half); K, V stay in shared memory, the
 //                       visible query tiles of every query head of the group stream through. S^T = K Q^T and
 //                       dP^T = V dO^T land in tensor memory (keys on lanes); P^T and dS^T go back to tensor
 //                       memory as 16-bit A operands of dV += P^T dO and dK += dS^T Q. GQA sums over the group
-//                       inside the CTA: no fp32 dK/dV accumulators in global memory.
+//                       inside the CTA: no fp32 dK/dV accumulators in global memory. Head dims above 128: an item makes
+//                       either dK or dV.
 //   3. bwd_dq         : forward-shaped, one CTA per 128-row query tile: S = Q K^T, dP = dO V^T, dS to tensor
 //                       memory, dQ += dS K. No cross-CTA reduction at all, so dQ needs no atomics, no fp32
 //                       accumulator, no zero-fill and no convert pass.
 //
-// Seven GEMMs per tile pair instead of five, in exchange for zero global reductions; every gradient has a
-// fixed accumulation order, so the result is bitwise reproducible whether or not `deterministic` is set.
-// Numerics kept from the reference: P = exp2(S*c - LSE2) from the saved LSE, dS = P * (dP - delta)
+// Seven GEMMs per tile pair instead of five (eight for head dims above 128), in exchange for zero global reductions; every
+// gradient has a fixed accumulation order, so the result is bitwise reproducible whether or not `deterministic` is set.
+// Numerics kept from the reference: P = exp2(S*c - LSE * log2(e)) from the saved LSE, dS = P * (dP - delta)
 // [* (1 - tanh^2) with softcap, before masking], P and dS rounded to the input dtype before the second GEMMs,
 // dK and dQ scaled by softmax_scale once at the end (mainloop_bwd...hpp:836-893, :1009).
 #include <type_traits>
@@ -152,7 +154,8 @@ struct DkdvCfg {
   static_assert((11 + 2 * kQSlots + 2 * kDoSlots + kStatSlots) * 8 + 8 <= 384, "barrier area");
 };
 
-// Sub-steps of one item: query heads of the group x visible 128-row query tiles x two 64-row halves; a half
+// One CTA per SM. A sub-step is one 64-row half of a visible 128-row query tile of one query head of the group; a half with
+// no visible row is skipped.
 template <int kHeadDim, int kStages, bool kBf16, bool kSoftcap>
 __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_constant__ BwdParams p) {
   using Cfg = DkdvCfg<kHeadDim, kStages>;
@@ -1123,9 +1126,11 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
     if (stage_mask & 1u) p.zero_tickets = p.ticket_kv;
     else FDA_CUDA_TRY(cudaMemsetAsync(p.ticket_kv, 0, kTicketInts * 4, stream));
   }
-  // An accumulator that stays in L2 with everything else is zeroed by the preprocess (one launch less: small steps are
-  // bound by launches). A large one is zero-filled right before the kernel that adds to it, which finds its end in L2
-  // (0.03 ms better on 8 samples x 4096 x 16 heads x 128, a 268 MB accumulator).
+  // An accumulator that stays in L2 with everything else is zeroed by the preprocess: one launch less, and small steps are
+  // bound by launches (16 heads of 128, blocks of 64; fill in front of the kernel / in the preprocess: 59.3 / 56.5 us of
+  // backward with 16 MB, 71.3 / 64.7 with 25 MB). A larger one is zero-filled right before the kernel that adds to it. That
+  // won 0.03 ms at 268 MB with an earlier form of the kernel; with this one it no longer does (88.7 / 83.6 us with 34 MB,
+  // 155.8 / 148.1 with 67, 328.6 / 320.3 with 134, 1088 / 1079 with 268).
   if (single_pass && (stage_mask & 3u) == 3u && p.acc_floats * 4 <= kZeroInPreprocessBytes) {
     p.zero_acc16 = p.acc_floats / 4;
   }
@@ -1184,7 +1189,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
 
 // ------------------------------------------------------------------------------------------------------------
 // Backward without a caller-provided workspace (fda_bwd_noalloc). It always runs the split backward, whose
-// scratch (delta, LSE * log2(e), the two work counters) is small; that scratch lives in this fixed array, which
+// scratch (delta, -LSE * log2(e), the two work counters) is small; that scratch lives in this fixed array, which
 // every GPU that loads the library holds until the process exits. In host code the array's name is only a
 // stand-in for the symbol: the device address is looked up once per device, with that device current, and that
 // pointer is what the kernels receive.

@@ -6,15 +6,17 @@
 // built around tcgen05:
 //
 //   * a work item is kQTiles consecutive 128-row query tiles of one half of one (sample, head); both tiles
-//     walk ONE list of 128-key tiles (clean prefix, then the noisy diagonal), so a K/V tile fetched once by TMA
-//     feeds both; a tile that one of the query tiles cannot see is skipped for that query tile only;
-//   * warp roles: kQTiles softmax warpgroups (thread = one query row), one TMA producer warp, one MMA warp;
+//     walk ONE list of key slots (clean prefix, then the noisy diagonal) in sub-steps of 64 keys, so K and V fetched
+//     once by TMA feed both; a sub-step that one of the query tiles cannot see is skipped for that query tile only;
+//   * warp roles: kQTiles softmax warpgroups (thread = one query row), one TMA producer warp, one MMA warp for each
+//     query tile;
 //   * S = Q K^T and O += P V are tcgen05.mma with fp32 accumulators in tensor memory; P is written back over
-//     S as 16-bit and consumed from tensor memory as the A operand; V is used MN-major straight from its TMA
-//     layout;
-//   * online softmax with the scale folded into one FMA + exp2, a running row maximum that is only advanced
-//     when it grows by more than 2^8 (O is rescaled in tensor memory only then), LSE in natural-log units;
-//   * only visible tiles are enumerated, only tiles crossing a block boundary (or the end of a half) get the
+//     S in the type of the inputs and consumed from tensor memory as the A operand; V is used MN-major straight from its
+//     TMA layout;
+//   * online softmax with the scale folded into one FMA + exp2, a running row maximum that (after the first 128 keys, and
+//     for 16-bit types) is only advanced when it grows by more than 2^8 (O is rescaled in tensor memory only then), LSE in
+//     natural-log units;
+//   * only visible sub-steps are enumerated, only those crossing a block boundary (or the end of a half) get the
 //     element mask;
 //   * persistent CTAs; items are ordered longest first (query tiles near the end of a half see most keys).
 //
@@ -149,8 +151,8 @@ __device__ __forceinline__ TileSpans make_tile_spans(const Item& it, int t, int 
 }
 
 // What the roles need to know about an item. The TMA warp works it out once (that is where the divisions by the
-// block size and the head counts happen) and leaves it in shared memory next to the scheduler's mailbox; the MMA
-// thread and the softmax warps copy it from there.
+// block size and the head counts happen) and leaves it in shared memory next to the scheduler's mailbox; the softmax
+// warps copy it from there. (The MMA warps need less: a word of flags beside every K slot.)
 struct ItemDesc {
   Item it;
   KeyPlan plan;
@@ -174,7 +176,7 @@ struct FwdConfig {
   static constexpr int kHalves = kSlotKeys / kSubKeys;                // sub-steps per slot
   // Two query tiles: the two softmax warpgroups need more registers than an even split of the file gives them
   // (168 per thread with the block rounded up to whole warpgroups), so the block is padded to three whole
-  // warpgroups and the third (TMA warp, MMA warp, two idle warps) hands registers to the other two.
+  // warpgroups and the third (TMA warp, two MMA warps, an idle warp) hands registers to the other two.
   static constexpr bool kRegRealloc = kQTiles == 2;
   static constexpr int kThreads = kRegRealloc ? 384 : 128 * kQTiles + 64;
   static constexpr uint32_t kSoftmaxRegs = 200, kProducerRegs = 104;
@@ -200,10 +202,10 @@ struct FwdConfig {
 // The keys advance in sub-steps of 64 and every query tile has two 64-column S buffers (kBufs), used in turn, P written
 // over the S it came from. While the softmax warps turn one buffer into P, the tensor pipe runs P V of the other and
 // then the S product that refills it, so neither waits for the other's latency. With ONE 128-column buffer per tile the
-// chain S -> softmax -> P V -> next S was serial and set the pace: 3700 cycles for two query tiles against 128 keys of
-// head dimension 128, of which the tensor pipe has 2048 and the special-function unit 2048 to do. The price is the
-// shared-memory traffic of N = 64 products (6 KB per 32 cycles of arithmetic, 48 cycles at 128 bytes per clock):
-// about 2600 cycles.
+// chain S -> softmax -> P V -> next S was serial. The price is the shared-memory traffic of N = 64 products (6 KB per 32
+// cycles of arithmetic, 48 cycles at 128 bytes per clock). On 4 x 8192 tokens, 32/8 heads of 128, blocks of 1024: 1.24 ->
+// 1.14 ms, 4400 -> 4000 cycles of kernel time for two query tiles against 128 keys, of which the tensor pipe has 2048 and
+// the special-function unit 2048 to do. What fills the rest is not settled.
 //
 // Every query tile has its own issuing warp, and that warp does next to nothing but wait and issue: the TMA warp, which
 // has time, walks the geometry and leaves one word of flags beside every K slot. (A single thread that decoded items and

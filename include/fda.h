@@ -116,7 +116,7 @@ int fda_bwd(const FdaBwdArgs* args, void* stream);
  * accumulator in the workspace; the order of those adds varies from run to run. The split form (everything
  * else, or FDA_BWD_FORCE_SPLIT) runs a dK/dV kernel and a dQ kernel with no cross-block reduction; its result
  * is bitwise reproducible. */
-#define FDA_BWD_STAGE_PREPROCESS 1u /* delta = rowsum(dO * O) and LSE * log2(e) into the workspace */
+#define FDA_BWD_STAGE_PREPROCESS 1u /* delta = rowsum(dO * O) and -LSE * log2(e) into the workspace */
 #define FDA_BWD_STAGE_MAIN 2u       /* single-pass kernel (with its accumulator zero-fill), or the dK/dV kernel */
 #define FDA_BWD_STAGE_DQ 4u         /* accumulator -> dQ conversion, or the dQ kernel */
 #define FDA_BWD_FORCE_SPLIT 8u      /* use the split form even where the single-pass form applies */

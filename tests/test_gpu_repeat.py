@@ -92,6 +92,27 @@ def test_sm_margin_changes_the_grid_not_the_result():
     assert _lib.device_status()[0] == 0
 
 
+@pytest.mark.parametrize("dtype,softcap", [(torch.bfloat16, 0.0), (torch.bfloat16, 20.0), (torch.float16, 0.0),
+                                           (torch.float8_e4m3fn, 0.0)])
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("n,bs", [(900, 64), (333, 20), (128, 1024)])
+def test_one_or_two_query_tiles_per_item_give_the_same_result(n, bs, d, dtype, softcap):
+    """A forward whose items of one 128-row query tile all find an SM takes those; with fewer SMs left to it the same call
+    takes items of two. Each query tile sees the same sub-steps in the same order either way, batched or packed."""
+    torch.manual_seed(12)
+    heads, heads_k = 4, 2
+    q, k, v = (torch.randn(1, 2 * n, h, d, device=DEV).to(dtype) for h in (heads, heads_k, heads_k))
+    cu = torch.tensor([0, 2 * n], device=DEV, dtype=torch.int32)
+    results = []
+    for margin in (0, 147):
+        results.append(diffusion_attn_func(q, k, v, bs, softcap=softcap, sm_margin=margin, return_attn_probs=True))
+        out, lse = diffusion_attn_varlen_func(q[0], k[0], v[0], cu, cu, 2 * n, 2 * n, bs, softcap=softcap, sm_margin=margin,
+                                              return_attn_probs=True)
+        results.append((out[None], lse[None]))
+    for out, lse in results[1:]:
+        assert torch.equal(out, results[0][0]) and torch.equal(lse, results[0][1])
+
+
 @pytest.mark.parametrize("heads,heads_k,d", [(32, 8, 64), (8, 8, 64), (32, 8, 128)])
 def test_no_wait_expires_over_many_backward_passes(heads, heads_k, d):
     """The roles of the single-pass backward run a step apart; where one of them can be lapped by another, a wait by

@@ -87,6 +87,7 @@ struct FusedRoles {
   // of 256, 1036 us without and 1017 with it. Head dim 64: 4 x 8192, 32 heads, scores capped, 2750 without and 2824 with
   // it; 64 x 256 tokens, 16 heads, 155 and 148; no difference on 4 x 4096, 32/8 heads.
   static constexpr bool kGeometryWarp = kHeadDim == 128;
+  static constexpr bool kPolyCap = kHeadDim == 64;   // capped scores by the polynomial where it holds: see softcap.cuh
   static_assert(128 * (kCmpWG * kComputeRegs + kProducerRegs + kDrainRegs) <= kThreads * kLaunchRegs, "register pool");
 };
 
@@ -647,8 +648,8 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
           ptx::tmem_wait_ld();
           const float4* l2v = reinterpret_cast<const float4*>(stats);
           // the fully visible tile (the common one) carries no per-element compare
-          auto first_half = [&](auto masked_tag) {
-            constexpr bool kMasked = decltype(masked_tag)::value;
+          auto first_half = [&](auto masked_tag, auto poly_tag) {
+            constexpr bool kMasked = decltype(masked_tag)::value, kPoly = decltype(poly_tag)::value;
 #pragma unroll
             for (int half = 0; half < kChunks; ++half) {
               uint32_t pk[16];
@@ -662,8 +663,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
                   float x0 = pr[c], x1 = pr[c + 1];
                   float dt0 = 1.f, dt1 = 1.f;
                   if (kSoftcap) {
-                    x0 = ptx::tanh_fast(x0 * p.softcap_pre);
-                    x1 = ptx::tanh_fast(x1 * p.softcap_pre);
+                    cap2<kPoly>(x0, x1, p.cap);
                     dt0 = 1.f - x0 * x0;
                     dt1 = 1.f - x1 * x1;
                   }
@@ -682,8 +682,15 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
               ptx::tmem_st16(s_t + 32 * half, pk);
             }
           };
-          if (masked) first_half(std::true_type{});
-          else first_half(std::false_type{});
+          using Poly = std::integral_constant<bool, kSoftcap && R::kPolyCap>;
+          const bool poly = Poly::value && cap_poly_holds<R::kCols>(pr, p.cap);
+          if (masked) {
+            if (poly) first_half(std::true_type{}, Poly{});
+            else first_half(std::true_type{}, std::false_type{});
+          } else {
+            if (poly) first_half(std::false_type{}, Poly{});
+            else first_half(std::false_type{}, std::false_type{});
+          }
           ptx::tmem_wait_st();
           ptx::tc_fence_before();
           ptx::mbar_arrive_warp(p_full);

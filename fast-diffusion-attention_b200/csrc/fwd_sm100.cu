@@ -539,6 +539,11 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       const CapPoly& cap = Cfg::kFp8 ? cap_fp8 : p.cap;
       constexpr float kThreshold = Cfg::kFp8 ? 0.f : kRescaleThreshold;
       constexpr float kPShift = Cfg::kFp8 ? 8.f : 0.f;
+      // Where O is rescaled often (fp8) or the exponentials take long (capped scores) that is done behind them, so that the
+      // last P V, which must be done first, runs under them. (e4m3, 2 x 16384 tokens, 8 heads of 256: 950 -> 897 us;
+      // cap 30, 4 x 8192 tokens, 32 heads of 64: 1257 -> 1173. Elsewhere O is rescaled about once an item and the order is worth
+      // nothing: 1310 against 1326 us on 4 x 8192 tokens, 32/8 heads of 128.)
+      constexpr bool kLateRescale = kSoftcap || Cfg::kFp8;
       float m_run = -INFINITY;  // reference maximum (unscaled scores, or tanh values with softcap)
       float l_run = 0.f;
       bool o_started = false, settled = false;   // one sub-step, two sub-steps of this tile are done
@@ -602,33 +607,38 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
         // (Settling it on 64 keys saves a rescale of O an item, 289 instead of 298 us on 8 x 4096 tokens, 16 heads of 128,
         // but the relative error of the output, over 24 drawn shapes in bf16, is 2.21e-3 instead of 2.17e-3.)
         const bool need = (m_new - m_run) * scale_log2 > (settled ? kThreshold : 0.f);
-        if (__any_sync(0xffffffffu, need)) {
-          const float factor = need ? ptx::ex2((m_run - m_new) * scale_log2) : 1.f;
-          if (o_started) {
-            // every P V of this tile so far must have updated O. In this buffer it has: S followed it through the
-            // pipe. In the others the last one may still run (an unused buffer's barrier passes at once).
+        const bool any_need = __any_sync(0xffffffffu, need);
+        float factor = 1.f;
+        auto rescale = [&]() {
+          // every P V of this tile so far must have updated O. In this buffer it has: S followed it through the
+          // pipe. In the others the last one may still run (an unused buffer's barrier passes at once).
 #pragma unroll
-            for (int b = 0; b < kBufs; ++b) {
-              if (b == buf) continue;
-              if (!ptx::mbar_wait(&pv_done[t * kBufs + b], ((s_par >> b) & 1u) ^ 1u, abort_flag, 33)) { alive = false; break; }
-            }
+          for (int b = 0; b < kBufs; ++b) {
+            if (b == buf) continue;
+            if (!ptx::mbar_wait(&pv_done[t * kBufs + b], ((s_par >> b) & 1u) ^ 1u, abort_flag, 33)) { alive = false; return; }
+          }
+          ptx::tc_fence_after();
+          // A load is answered after some 250 cycles while products run, however wide it is. fp8 rescales often, and with
+          // one query tile has the registers for 128 columns a round (2 x 16384 tokens, 8 heads of 256: 1017 -> 948 us;
+          // with two tiles 64 are slower than 32, 646 against 610 us on 4 x 8192 tokens, 16/4 heads of 128).
+          constexpr int kRound = Cfg::kFp8 && kQTiles == 1 ? 128 : 32;
+#pragma unroll
+          for (int c0 = 0; c0 < kHeadDim; c0 += kRound) {
+            uint32_t o[kRound];
+#pragma unroll
+            for (int c = 0; c < kRound; c += 32) ptx::tmem_ld32(tmem_o + c0 + c, o + c);
+            ptx::tmem_wait_ld();
+#pragma unroll
+            for (int i = 0; i < kRound; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+#pragma unroll
+            for (int c = 0; c < kRound; c += 32) ptx::tmem_st32(tmem_o + c0 + c, o + c);
+          }
+        };
+        if (any_need) {
+          if (need) factor = ptx::ex2((m_run - m_new) * scale_log2);
+          if (!kLateRescale && o_started) {
+            rescale();
             if (!alive) break;
-            ptx::tc_fence_after();
-            // A load is answered after some 250 cycles while products run, however wide it is. fp8 rescales often, and with
-            // one query tile has the registers for 128 columns a round (2 x 16384 tokens, 8 heads of 256: 1017 -> 948 us;
-            // with two tiles 64 are slower than 32, 646 against 610 us on 4 x 8192 tokens, 16/4 heads of 128).
-            constexpr int kRound = Cfg::kFp8 && kQTiles == 1 ? 128 : 32;
-#pragma unroll
-            for (int c0 = 0; c0 < kHeadDim; c0 += kRound) {
-              uint32_t o[kRound];
-#pragma unroll
-              for (int c = 0; c < kRound; c += 32) ptx::tmem_ld32(tmem_o + c0 + c, o + c);
-              ptx::tmem_wait_ld();
-#pragma unroll
-              for (int i = 0; i < kRound; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
-#pragma unroll
-              for (int c = 0; c < kRound; c += 32) ptx::tmem_st32(tmem_o + c0 + c, o + c);
-            }
           }
           l_run *= factor;
           if (need) m_run = m_new;
@@ -674,6 +684,10 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
         l_run += (sum4[0] + sum4[1]) + (sum4[2] + sum4[3]);
         if (Cfg::kPCols == 32) ptx::tmem_st32(tmem_sb, pk);
         else ptx::tmem_st16(tmem_sb, pk);
+        if (kLateRescale && any_need && o_started) {
+          rescale();
+          if (!alive) break;
+        }
         ptx::tmem_wait_st();
         ptx::tc_fence_before();
         ptx::mbar_arrive_warp(&p_full[t * kBufs + buf]);

@@ -240,6 +240,16 @@ __device__ __forceinline__ void umma_ts_f8(uint32_t d_tmem, uint32_t a_tmem, uin
       ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// 128 rows x 32 bytes from shared memory (described like a K-major MMA operand) into eight tensor-memory columns: what one
+// reduction step of an A operand takes. Later MMAs of the same thread see the copy; a copy does not wait for earlier MMAs.
+__device__ __forceinline__ void tmem_cp_128x32b_lh(uint32_t taddr, uint32_t desc_lo, uint32_t desc_hi) {
+  asm volatile(
+      "{\n\t.reg .b64 d;\n\t"
+      "mov.b64 d, {%1, %2};\n\t"
+      "tcgen05.cp.cta_group::1.128x256b [%0], d;\n\t}"
+      ::"r"(taddr), "r"(desc_lo), "r"(desc_hi)
+      : "memory");
+}
 // The mbarrier gets one arrival when every MMA this thread issued so far has completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))

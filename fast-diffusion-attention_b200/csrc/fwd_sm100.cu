@@ -181,7 +181,7 @@ struct FwdConfig {
   // (168 per thread with the block rounded up to whole warpgroups), so the block is padded to three whole
   // warpgroups and the third (TMA warp, two MMA warps, an idle warp) hands registers to the other two.
   static constexpr bool kRegRealloc = kQTiles == 2;
-  static constexpr bool kPolyCap = kQTiles == 2;   // capped scores: see softcap.cuh
+  static constexpr bool kPolyCap = kHeadDim <= 128;   // capped scores: see softcap.cuh
   static constexpr int kThreads = kRegRealloc ? 384 : 128 * kQTiles + 64;
   static constexpr uint32_t kSoftmaxRegs = 200, kProducerRegs = 104;
   // the pool is what the block got at launch, 384 threads x 168 registers: 2 * 128 * 200 + 128 * 104 = 384 * 168.

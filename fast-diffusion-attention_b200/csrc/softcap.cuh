@@ -9,8 +9,8 @@
 // under a cap of 30 by 1.1e-5 instead of 1e-7; a fifth one up to 0.75 takes registers that cost the 128-wide forward what the
 // polynomial gains it.
 //
-// Used where two warps or more of a scheduler share its special-function unit all the time: the forward with two query tiles
-// and the single-pass backward at head dimension 64. With 32 heads of 64 on 4 x 8192 tokens (cap
+// Used in the forward up to head dimension 128 (with one query tile an item, where it hardly matters, too: both give the same
+// bits) and in the single-pass backward at head dimension 64. With 32 heads of 64 on 4 x 8192 tokens (cap
 // 30) the forward went from 1325 to 1257 us and the backward kernel from 2763 to 2615, with 16 heads of 128 on 4 x 4096 tokens
 // the forward from 242 to 220.
 // Elsewhere the unit's tanh is as fast or faster (forward of 256-wide heads 98.2 against 101.2 us on 2 x 4096 tokens, 8 heads;

@@ -47,8 +47,9 @@ struct FusedCfg {
   static constexpr int kSmemBytes = kOffBar + 768;   // barriers 384, mailbox 64, item descriptions
   // tensor memory: S^T / P^T at 0, dP^T / dQ^T at 128, dK and dV behind
   static constexpr int kTmemS = 0, kTmemDP = 128, kTmemDK = 256, kTmemDV = 256 + kHeadDim;
-  // Head dimension 64 leaves 128 columns behind the accumulators: dQ^T gets them, and the next dP^T no longer waits
-  // for the drain of this step's dQ^T. At 128 all 512 columns are taken and dQ^T overwrites dP^T.
+  // Head dimension 64 leaves 128 columns behind the accumulators: dQ^T (or dQ) gets them, and the next dP^T no longer waits
+  // for the drain of this step's dQ^T. At 128 all 512 columns are taken and dQ^T overwrites dP^T. (The other use of the 128, a
+  // second S^T buffer, with dQ over dP^T: kernel time 2361 instead of 2211 us on 4 x 8192 tokens, 32 heads.)
   static constexpr bool kOwnDq = 256 + 2 * kHeadDim + 128 <= 512;
   static constexpr int kTmemDQ = kOwnDq ? 256 + 2 * kHeadDim : kTmemDP;
   static_assert(kHeadDim == 64 || kHeadDim == 128, "the single-pass backward covers head dimensions up to 128");
@@ -87,6 +88,11 @@ struct FusedRoles {
   // of 256, 1036 us without and 1017 with it. Head dim 64: 4 x 8192, 32 heads, scores capped, 2750 without and 2824 with
   // it; 64 x 256 tokens, 16 heads, 155 and 148; no difference on 4 x 4096, 32/8 heads.
   static constexpr bool kGeometryWarp = kHeadDim == 128;
+  // dQ = dS K instead of dQ^T = K^T dS^T: at head dim 64, where dQ^T has only 64 rows, so that half of an M = 128 product is
+  // thrown away and two of the four drain warps do all the work (backward of 4 x 4096 tokens, 32/8 heads, blocks of 64: 706 ->
+  // 684 us; 4 x 8192, 32 heads, blocks of 256: 2358 -> 2320). With capped scores, whose arithmetic leaves time for both, it is
+  // not faster (2616 / 2710 us on the latter shape).
+  static constexpr bool dq_rows(bool softcap) { return kHeadDim == 64 && !softcap; }
   static constexpr bool kPolyCap = kHeadDim == 64;   // capped scores by the polynomial where it holds: see softcap.cuh
   static_assert(128 * (kCmpWG * kComputeRegs + kProducerRegs + kDrainRegs) <= kThreads * kLaunchRegs, "register pool");
 };
@@ -142,12 +148,13 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
   using Cfg = FusedCfg<kHeadDim, kSlots, kDoSlots>;
   using T = TileCfg<kHeadDim>;
   using R = FusedRoles<kHeadDim>;
+  constexpr bool kDqRows = R::dq_rows(kSoftcap);
   // The tiles need 1024-byte alignment for the 128-byte swizzle. Dynamic shared memory starts at the beginning of the
   // block's window, which is aligned that far; the budget leaves no room to round the base up, so a base that is not
   // aligned is reported through the status word instead.
   extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* sK = smem;
-  uint8_t* sV = smem + T::kTileBytes;   // directly behind K: for head dim 64 it is the second panel of the M = 128
+  uint8_t* sV = smem + T::kTileBytes;   // directly behind K: for head dim 64 it may be the second panel of the M = 128
                                         // operand of dQ^T (rows 64..127 of that product are never read)
   uint8_t* sQ = smem + Cfg::kOffQ;
   uint8_t* sDo = smem + Cfg::kOffDo;
@@ -168,13 +175,13 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
   uint64_t* p_full = dp_full + 1;              // P^T written over S^T
   uint64_t* ds_full = p_full + 1;              // dS^T in shared memory, dP^T in registers
   uint64_t* s_free = ds_full + 1;              // dV has read P^T: the next S^T may overwrite it
-  uint64_t* dq_full = s_free + 1;              // dQ^T complete
-  uint64_t* dp_free = dq_full + 1;             // dQ^T is in the drain warps' registers: its columns may be overwritten
-                                               // (by the next dP^T, or by the next dQ^T where it has columns of its own)
+  uint64_t* dq_full = s_free + 1;              // dQ complete
+  uint64_t* dp_free = dq_full + 1;             // dQ is in the drain warps' registers: its columns may be overwritten
+                                               // (by the next dP^T, or by the next dQ where it has columns of its own)
   uint64_t* ds_free = dp_free + 1;             // dQ^T and dK have read dS^T: the next step may overwrite it
   uint64_t* acc_full = ds_free + 1;
   uint64_t* acc_free = acc_full + 1;
-  // [2] The step's description for the drain warps is in dq_desc[g & 1]. They do not wait for ds_full: where dQ^T has its
+  // [2] The step's description for the drain warps is in dq_desc[g & 1]. They do not wait for ds_full: where dQ has its
   // own columns, dS^T of step g + 1 can be complete before they look for step g, and a wait by parity that is one whole
   // round late waits for ever. A barrier for even and one for odd steps cannot be lapped (step g + 2 needs dp_free of g).
   uint64_t* desc_full = acc_free + 1;
@@ -257,7 +264,9 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const bool drain_rows = quad * 32 < p.head_dim;   // the quarters behind the head dimension hold nothing of dQ^T
+    // dQ^T: a lane is a value of the head dimension, the columns are the step's queries. dQ: a lane is a query, the columns are
+    // the head dimension.
+    constexpr int kDqCols = kDqRows ? kHeadDim : kTile;
     uint32_t n_item = 0, gd = 0, n_bulk = 0;
     bool alive = true;
     for (uint32_t n_sched = 0; alive; ++n_sched) {
@@ -277,12 +286,13 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
         ptx::tc_fence_after();
         // kHold chunks of 32 columns go to registers at once; when the last is there the columns are free and the adds
         // follow behind the next step's products. Blocks of 32 query rows of the accumulator are stored as
-        // [head dim / 32][8 groups of 4 queries][32 head-dim values][4 queries]: a warp's 32 x 32 piece goes through
-        // shared memory (16 bytes a thread, a quarter of the store instructions of single values) and out as ONE 4 KB bulk
-        // reduction issued by lane 0. Two staging slots per warp alternate.
-        float* dst = p.dq_acc + static_cast<size_t>(acc_row) * kHeadDim + quad * 1024;
+        // [head dim / 32][8][32][4]: 8 groups of 4 queries x 32 head-dim values (dQ^T), or 8 groups of 4 head-dim values x 32
+        // queries (dQ). Either way a warp's 32 x 32 piece goes through shared memory (16 bytes a thread, a quarter of the
+        // store instructions of single values) and out as ONE 4 KB bulk reduction issued by lane 0. Two staging slots per warp
+        // alternate.
+        float* dst = p.dq_acc + static_cast<size_t>(acc_row) * kHeadDim + quad * (kDqRows ? 32 * kHeadDim : 1024);
 #pragma unroll 1
-        for (int c0 = 0; c0 < kTile / 32; c0 += R::kHold) {
+        for (int c0 = 0; c0 < kDqCols / 32; c0 += R::kHold) {
           uint32_t a[32 * R::kHold];
 #pragma unroll
           for (int c = 0; c < R::kHold; ++c) ptx::tmem_ld32(tmem + Cfg::kTmemDQ + lane_addr + (c0 + c) * 32, a + c * 32);
@@ -291,14 +301,15 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
             __syncwarp();
           }
           ptx::tmem_wait_ld();
-          if (c0 + R::kHold == kTile / 32) {
+          if (c0 + R::kHold == kDqCols / 32) {
             ptx::tc_fence_before();
             ptx::mbar_arrive_warp(dp_free);
           }
-          if (!drain_rows) continue;
 #pragma unroll
           for (int c = 0; c < R::kHold; ++c) {
-            if ((c0 + c) * 32 < rows_left) {
+            // pieces of queries that do not exist or behind the head dimension hold nothing
+            const int col = (c0 + c) * 32;
+            if (kDqRows ? quad * 32 < rows_left && col < p.head_dim : col < rows_left && quad * 32 < p.head_dim) {
               uint8_t* stage = sStage + (quad * 2 + (n_bulk & 1u)) * Cfg::kStageChunk;
               // the bulk reduction that last read this slot (two chunks ago) must have finished reading it
               if (R::kHold > 1) {
@@ -313,7 +324,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
               ptx::fence_async_smem();
               __syncwarp();
               if (lane == 0) {
-                float* target = dst + (c0 + c) * (32 * kHeadDim);
+                float* target = dst + (c0 + c) * (kDqRows ? 1024 : 32 * kHeadDim);
                 if (target >= p.dq_acc && target + 1024 <= p.dq_acc + p.acc_floats) {
                   ptx::bulk_reduce_add_f32(target, stage, Cfg::kStageChunk);
                   ptx::bulk_commit_group();
@@ -477,7 +488,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
     // ------------------------------------------------------------------- MMA issuer 1: S^T = K Q^T, dP^T = V dO^T
     // Two threads issue the MMAs of this kernel, so that the barrier waits and commits of one overlap the MMAs of
     // the other. S^T of step g + 1 may overwrite P^T of step g once dV has read it (s_free); dP^T of step g + 1
-    // may overwrite dQ^T of step g once the drain warps hold it (dp_free) or, where dQ^T has its own columns, dP^T of
+    // may overwrite dQ^T of step g once the drain warps hold it (dp_free) or, where dQ has its own columns, dP^T of
     // step g once the compute warps hold it (ds_full).
     if (lane == 0) {
       constexpr int kFmt = kBf16 ? 1 : 0;
@@ -532,12 +543,14 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
     if (lane == 0) {
       constexpr int kFmt = kBf16 ? 1 : 0;
       const uint32_t idesc_g = ptx::make_idesc(kTile, kHeadDim, kFmt, false, true);   // A K-major, B MN-major
-      const uint32_t idesc_q = ptx::make_idesc(kTile, kTile, kFmt, true, true);       // A and B MN-major
+      // dQ^T = K^T dS^T or dQ = dS K: A and B MN-major (the reduction runs over key rows)
+      const uint32_t idesc_q = ptx::make_idesc(kTile, kDqRows ? kHeadDim : kTile, kFmt, true, true);
       constexpr uint32_t kHi = ptx::smem_desc_hi(1024);
       const uint32_t q_mn = ptx::smem_desc_lo(ptx::smem_u32(sQ), T::kPanelBytes);     // Q / dO as MN-major B: rows of
       const uint32_t do_mn = ptx::smem_desc_lo(ptx::smem_u32(sDo), T::kPanelBytes);   // queries are the reduction
-      const uint32_t kt_lo = ptx::smem_desc_lo(ptx::smem_u32(sK), T::kPanelBytes);    // K^T: key rows are the reduction
-      const uint32_t ds_mn = ptx::smem_desc_lo(ptx::smem_u32(sDs), Cfg::kDsPanelBytes);   // dS^T as B of dQ^T
+      const uint32_t k_mn = ptx::smem_desc_lo(ptx::smem_u32(sK), T::kPanelBytes);
+      const uint32_t ds_mn = ptx::smem_desc_lo(ptx::smem_u32(sDs), Cfg::kDsPanelBytes);
+      const uint32_t dq_a = kDqRows ? ds_mn : k_mn, dq_b = kDqRows ? k_mn : ds_mn;
       const uint32_t ds_k = ptx::smem_desc_lo(ptx::smem_u32(sDs), 16);                // dS^T as K-major A of dK
       uint32_t g = 0, n_item_b = 0;
       bool alive = true;
@@ -570,15 +583,15 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
           ptx::umma_commit(&do_empty[g % kDoSlots]);
           if (!ptx::mbar_wait(ds_full, g & 1u, abort_flag, 59)) { alive = false; break; }
           ptx::tc_fence_after();
-          // dQ^T before dK: its drain (tensor memory -> registers -> global adds) then runs under dK
+          // dQ before dK: its drain (tensor memory -> registers -> global adds) then runs under dK
           if (Cfg::kOwnDq) {
-            // the drain warps hold dQ^T of the previous step
+            // the drain warps hold dQ of the previous step
             if (!ptx::mbar_wait(dp_free, (g & 1u) ^ 1u, abort_flag, 68)) { alive = false; break; }
             ptx::tc_fence_after();
           }
 #pragma unroll
           for (int kk = 0; kk < kTile / 16; ++kk) {
-            ptx::umma_ss_f16_lh(tmem + Cfg::kTmemDQ, kt_lo + kk * (2048 >> 4), ds_mn + kk * (2048 >> 4), kHi, idesc_q, kk > 0);
+            ptx::umma_ss_f16_lh(tmem + Cfg::kTmemDQ, dq_a + kk * (2048 >> 4), dq_b + kk * (2048 >> 4), kHi, idesc_q, kk > 0);
           }
           ptx::umma_commit(dq_full);
           // K is read by S^T (complete for every step of this item by now) and by dQ^T: after the last dQ^T the next
@@ -741,7 +754,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
 // dQ = round(accumulator * softmax_scale). One block per 64 query rows of a (sample, head, half); stands where the
 // reference converts its accumulator (csrc/fda/flash_bwd_postprocess_kernel.h:160-264 there).
 // ------------------------------------------------------------------------------------------------------------
-template <int kHeadDim, bool kBf16>
+template <int kHeadDim, bool kBf16, bool kSoftcap>
 __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const __grid_constant__ BwdParams p) {
   const int h = blockIdx.y >> 1, half = blockIdx.y & 1;
   const int b = blockIdx.z;
@@ -751,23 +764,27 @@ __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const __grid_consta
   const int grow0 = p.cu_seqlens != nullptr ? sm.row0 : b * p.seqlen;
   const float* src =
       p.dq_acc + (static_cast<size_t>(h) * p.acc_tiles * 64 + acc_row_of(grow0, sm.n, b, half, qa)) * kHeadDim;
-  // The accumulator is read in its own order ([head dim / 32][8 groups of 4 rows][32 values][4 rows] per 32 rows, 16 bytes
-  // a lane), rounded, transposed through shared memory and written in rows. The pad of 16 bytes keeps the row reads of 16
+  // The accumulator is read in its own order (see the drain; 16 bytes a lane), rounded, transposed through shared memory and
+  // written in rows. The pad of 16 bytes keeps the row reads of 16
   // bytes aligned and the 2-byte writes of a warp (32 neighbouring values of a row) free of conflicts.
   constexpr int kRowElems = kHeadDim + 8;
   __shared__ __align__(16) uint16_t tile[64 * kRowElems];
   const float sc = p.softmax_scale;
 #pragma unroll
   for (int i = threadIdx.x; i < 16 * kHeadDim; i += 256) {
-    const int e = i % 32, q4 = (i / 32) % 8, panel = (i / 256) % (kHeadDim / 32), q32 = i / (8 * kHeadDim);
+    const int e = i % 32, g = (i / 32) % 8, panel = (i / 256) % (kHeadDim / 32), q32 = i / (8 * kHeadDim);
     if (panel * 32 >= p.head_dim) continue;
     const float4 x = reinterpret_cast<const float4*>(src)[i];
     const uint32_t w0 = ptx::pack2<kBf16>(x.x * sc, x.y * sc), w1 = ptx::pack2<kBf16>(x.z * sc, x.w * sc);
-    uint16_t* t = tile + (q32 * 32 + q4 * 4) * kRowElems + panel * 32 + e;
-    t[0] = static_cast<uint16_t>(w0);
-    t[kRowElems] = static_cast<uint16_t>(w0 >> 16);
-    t[2 * kRowElems] = static_cast<uint16_t>(w1);
-    t[3 * kRowElems] = static_cast<uint16_t>(w1 >> 16);
+    if (FusedRoles<kHeadDim>::dq_rows(kSoftcap)) {   // 4 values of row e
+      *reinterpret_cast<uint2*>(tile + (q32 * 32 + e) * kRowElems + panel * 32 + g * 4) = make_uint2(w0, w1);
+    } else {           // value e of 4 rows
+      uint16_t* t = tile + (q32 * 32 + g * 4) * kRowElems + panel * 32 + e;
+      t[0] = static_cast<uint16_t>(w0);
+      t[kRowElems] = static_cast<uint16_t>(w0 >> 16);
+      t[2 * kRowElems] = static_cast<uint16_t>(w1);
+      t[3 * kRowElems] = static_cast<uint16_t>(w1 >> 16);
+    }
   }
   __syncthreads();
   constexpr int kPieces = kHeadDim / 8;
@@ -799,7 +816,7 @@ int launch_fused_instance(const BwdParams& p, int sm_count, unsigned stages, cud
   }
   if (stages & 4u) {
     dim3 grid(p.n_pad / 64, 2 * p.heads, p.batch);
-    bwd_dq_convert_kernel<kHeadDim, kBf16><<<grid, 256, 0, stream>>>(p);
+    bwd_dq_convert_kernel<kHeadDim, kBf16, kSoftcap><<<grid, 256, 0, stream>>>(p);
     FDA_CUDA_TRY(cudaGetLastError());
   }
   return FDA_OK;

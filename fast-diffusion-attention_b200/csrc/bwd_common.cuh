@@ -57,6 +57,9 @@ struct BwdParams {
   int wide_store;      // dq/dk/dv rows allow 32-byte stores
   float scale_log2, softmax_scale;
   CapPoly cap;         // tanh of a capped score; its argument scale is softmax_scale / softcap
+  int kv_split;         // single-pass backward: parts into which a key tile's query heads are dealt (a divisor of the group)
+  float* dkv_part;      // ... their fp32 dK and dV: [2][kv_split][heads_k][acc_tiles * 64 rows][head dim]; nullptr without parts
+  int64_t part_floats;  // size of that
 };
 
 struct Sample {

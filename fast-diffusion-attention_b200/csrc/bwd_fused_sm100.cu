@@ -118,6 +118,7 @@ struct FusedItem {
   QueryPlan plan;
   KvSpans spans;
   int grow0;   // first row of the sample in the packed row space
+  int part;    // which of the kv_split parts of the group's query heads
 };
 // The next item is taken when at most this many steps of the current one are to be sent: early enough for the ticket's
 // round trip, late enough that CTAs do not reserve work. It hardly matters (same backward with 1, 4, 16: 1018, 1017, 1024).
@@ -125,8 +126,8 @@ constexpr int kTicketSteps = 4;
 
 template <typename Fn>
 __device__ __forceinline__ bool for_each_qstep(const KvItem& it, const QueryPlan& plan, const KvSpans& spans, int group,
-                                               Fn&& fn) {
-  for (int g = 0; g < group; ++g) {
+                                               int head0, int head1, Fn&& fn) {
+  for (int g = head0; g < head1; ++g) {
     for (int s = 0; s < plan.steps(); ++s) {
       QStep st;
       int qt;
@@ -136,14 +137,14 @@ __device__ __forceinline__ bool for_each_qstep(const KvItem& it, const QueryPlan
       st.cls = spans.classify(st.qh, it.kh, st.qa, qb);
       if (st.cls == kTileSkip) continue;
       st.h = it.hk * group + g;
-      st.left = (group - 1 - g) * plan.steps() + plan.steps() - 1 - s;
+      st.left = (head1 - 1 - g) * plan.steps() + plan.steps() - 1 - s;
       if (!fn(st)) return false;
     }
   }
   return true;
 }
 
-template <int kHeadDim, int kSlots, int kDoSlots, bool kBf16, bool kSoftcap>
+template <int kHeadDim, int kSlots, int kDoSlots, bool kBf16, bool kSoftcap, bool kParts>
 __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_kernel(const __grid_constant__ BwdParams p) {
   using Cfg = FusedCfg<kHeadDim, kSlots, kDoSlots>;
   using T = TileCfg<kHeadDim>;
@@ -243,15 +244,17 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
   const uint32_t tmem = *tmem_slot;
   const int bs = p.block_size;
   const int group = p.heads / p.heads_k;
-  const int total_items = kv_item_count(p);
+  const int split = kParts ? p.kv_split : 1;   // CTAs that share a key tile
+  const int total_items = kv_item_count(p) * split;
 
   auto make_item = [&](int idx, FusedItem& d) -> bool {   // false: a tile that does not exist
-    const KvItem it = decode_kv_item(p, idx);
+    const KvItem it = decode_kv_item(p, idx / split);
     if (!it.valid) return false;
     d.it = it;
     d.plan = make_query_plan(it.kh, it.k0, it.k1, it.n, bs, kTile);
     d.spans = make_kv_spans(it, bs);
     d.grow0 = p.cu_seqlens != nullptr ? it.row0 : it.b * p.seqlen;
+    d.part = idx % split;
     return true;
   };
 
@@ -272,7 +275,9 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
     for (uint32_t n_sched = 0; alive; ++n_sched) {
       const int idx = R::kGeometryWarp ? sched_peek(mbox, n_sched, abort_flag) : sched_consume<true>(mbox, n_sched, abort_flag);
       if (idx < 0 || idx >= total_items) break;
-      const KvItem it = R::kGeometryWarp ? items[n_sched & 1u].it : decode_kv_item(p, idx);
+      const KvItem it = R::kGeometryWarp ? items[n_sched & 1u].it : decode_kv_item(p, idx / split);
+      const int part = R::kGeometryWarp ? items[n_sched & 1u].part : idx % split;
+      const int grow0 = p.cu_seqlens != nullptr ? it.row0 : it.b * p.seqlen;
       if (R::kGeometryWarp) sched_release<true>(mbox, n_sched);
       else if (!it.valid) continue;
       for (bool last = false; alive && !last; ++gd) {
@@ -348,6 +353,47 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
       if (!ptx::mbar_wait(acc_full, n_item & 1, abort_flag, 62)) break;
       ++n_item;
       ptx::tc_fence_after();
+      if (kParts) {
+        // A part of the group's heads: 32 x 32 pieces of dK and dV go out as they are, in the order of the dQ accumulator's
+        // blocks ([head dim / 32][8 groups of 4 values][32 rows][4 values]); the convert kernel adds the parts up.
+        const int arow = acc_row_of(grow0, it.n, it.b, it.kh, it.k0) + quad * 32;
+#pragma unroll 1
+        for (int c = 0; c < 2 * kHeadDim / 32; ++c) {
+          uint32_t accv[32];
+          ptx::tmem_ld32(tmem + Cfg::kTmemDK + lane_addr + c * 32, accv);
+          if (lane == 0) ptx::bulk_wait_group_read<1>();
+          __syncwarp();
+          ptx::tmem_wait_ld();
+          if (c == 2 * kHeadDim / 32 - 1) {
+            ptx::tc_fence_before();
+            ptx::mbar_arrive_warp(acc_free);
+          }
+          const int is_dv = c * 32 >= kHeadDim ? 1 : 0, col = c * 32 - is_dv * kHeadDim;
+          if (rows_valid > 0 && col < p.head_dim) {
+            uint8_t* stage = sStage + (quad * 2 + (n_bulk & 1u)) * Cfg::kStageChunk;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              ptx::st_shared_v4(stage + i * 512 + lane * 16, accv[4 * i], accv[4 * i + 1], accv[4 * i + 2], accv[4 * i + 3]);
+            }
+            ptx::fence_async_smem();
+            __syncwarp();
+            if (lane == 0) {
+              const int64_t block = (static_cast<int64_t>(is_dv) * p.kv_split + part) * p.heads_k + it.hk;
+              const int64_t at = (block * p.acc_tiles * 64 + arow) * kHeadDim + col * 32;
+              if (at >= 0 && at + 1024 <= p.part_floats) {
+                ptx::bulk_store_1d(p.dkv_part + at, stage, Cfg::kStageChunk);
+                ptx::bulk_commit_group();
+              } else if (atomicCAS(&g_fda_status[0], 0, 122) == 0) {   // never expected: recorded, not performed
+                g_fda_status[1] = static_cast<int>(blockIdx.x);
+                g_fda_status[2] = arow;
+                g_fda_status[3] = c;
+              }
+            }
+            ++n_bulk;
+          }
+        }
+        continue;
+      }
       // dK and dV sit side by side in tensor memory. With the registers for it (kHold > 1) both are rounded first, in three
       // rounds of loads (a load is answered after 250 cycles and more while the products run, however wide it is), and
       // the next item's products may overwrite them while the rows are stored. (Tile copies through the staging slots
@@ -460,7 +506,8 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
         };
         QStep pend{};
         bool have = false;
-        alive = for_each_qstep(it, d.plan, d.spans, group, [&](const QStep& st) -> bool {
+        const int part_heads = group / split;
+        alive = for_each_qstep(it, d.plan, d.spans, group, d.part * part_heads, (d.part + 1) * part_heads, [&](const QStep& st) -> bool {
           if (have && !emit(pend, false)) return false;
           pend = st;
           have = true;
@@ -503,7 +550,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
       for (uint32_t n_sched = 0; alive; ++n_sched) {
         const int idx = sched_consume<false>(mbox, n_sched, abort_flag);
         if (idx < 0 || idx >= total_items) break;
-        if (!R::kGeometryWarp && !decode_kv_item(p, idx).valid) continue;
+        if (!R::kGeometryWarp && !decode_kv_item(p, idx / split).valid) continue;
         if (!ptx::mbar_wait(k_full, n_item & 1, abort_flag, 51)) break;
         bool first = true;
         for (bool last = false; alive && !last; ++g) {
@@ -557,7 +604,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
       for (uint32_t n_sched = 0; alive; ++n_sched) {
         const int idx = sched_consume<false>(mbox, n_sched, abort_flag);
         if (idx < 0 || idx >= total_items) break;
-        if (!R::kGeometryWarp && !decode_kv_item(p, idx).valid) continue;
+        if (!R::kGeometryWarp && !decode_kv_item(p, idx / split).valid) continue;
         bool acc = false;
         // the first dV / dK products of an item overwrite the accumulators: the epilogue must have read the last item's
         if (!ptx::mbar_wait(acc_free, (n_item_b & 1u) ^ 1u, abort_flag, 57)) break;
@@ -631,7 +678,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
     for (uint32_t n_sched = 0; alive; ++n_sched) {
       const int idx = R::kGeometryWarp ? sched_peek(mbox, n_sched, abort_flag) : sched_consume<true>(mbox, n_sched, abort_flag);
       if (idx < 0 || idx >= total_items) break;
-      const KvItem it = R::kGeometryWarp ? items[n_sched & 1u].it : decode_kv_item(p, idx);
+      const KvItem it = R::kGeometryWarp ? items[n_sched & 1u].it : decode_kv_item(p, idx / split);
       if (R::kGeometryWarp) sched_release<true>(mbox, n_sched);
       else if (!it.valid) continue;
       const int kj = it.k0 + row;
@@ -754,29 +801,40 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
 // dQ = round(accumulator * softmax_scale). One block per 64 query rows of a (sample, head, half); stands where the
 // reference converts its accumulator (csrc/fda/flash_bwd_postprocess_kernel.h:160-264 there).
 // ------------------------------------------------------------------------------------------------------------
-template <int kHeadDim, bool kBf16, bool kSoftcap>
+template <int kHeadDim, bool kBf16, bool kSoftcap, bool kParts>
 __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const __grid_constant__ BwdParams p) {
-  const int h = blockIdx.y >> 1, half = blockIdx.y & 1;
+  const int hh = blockIdx.y >> 1, half = blockIdx.y & 1;
   const int b = blockIdx.z;
   const Sample sm = sample_of(p, b);
   const int qa = blockIdx.x * 64;
   if (qa >= sm.n) return;
   const int grow0 = p.cu_seqlens != nullptr ? sm.row0 : b * p.seqlen;
-  const float* src =
-      p.dq_acc + (static_cast<size_t>(h) * p.acc_tiles * 64 + acc_row_of(grow0, sm.n, b, half, qa)) * kHeadDim;
+  // a query head's dQ, or (behind all of them, where the heads of a group were dealt out) a KV head's dK or dV
+  const int kv = kParts ? hh - p.heads : -1, is_dv = kv >= p.heads_k ? 1 : 0;
+  const int h = kv < 0 ? hh : kv - is_dv * p.heads_k;
+  const size_t rows = static_cast<size_t>(p.acc_tiles) * 64, row = acc_row_of(grow0, sm.n, b, half, qa);
+  const float* src = kv < 0 ? p.dq_acc + (h * rows + row) * kHeadDim
+                            : p.dkv_part + ((static_cast<size_t>(is_dv) * p.kv_split * p.heads_k + h) * rows + row) * kHeadDim;
+  const int parts = kv < 0 ? 1 : p.kv_split;
+  const bool row_lanes = FusedRoles<kHeadDim>::dq_rows(kSoftcap) || (kParts && kv >= 0);
   // The accumulator is read in its own order (see the drain; 16 bytes a lane), rounded, transposed through shared memory and
   // written in rows. The pad of 16 bytes keeps the row reads of 16
   // bytes aligned and the 2-byte writes of a warp (32 neighbouring values of a row) free of conflicts.
   constexpr int kRowElems = kHeadDim + 8;
   __shared__ __align__(16) uint16_t tile[64 * kRowElems];
-  const float sc = p.softmax_scale;
+  const float sc = kv >= 0 && is_dv ? 1.f : p.softmax_scale;
 #pragma unroll
   for (int i = threadIdx.x; i < 16 * kHeadDim; i += 256) {
     const int e = i % 32, g = (i / 32) % 8, panel = (i / 256) % (kHeadDim / 32), q32 = i / (8 * kHeadDim);
     if (panel * 32 >= p.head_dim) continue;
-    const float4 x = reinterpret_cast<const float4*>(src)[i];
+    float4 x = reinterpret_cast<const float4*>(src)[i];
+#pragma unroll 4
+    for (int part = 1; kParts && part < parts; ++part) {   // always in this order: dK and dV are the same in every run
+      const float4 y = reinterpret_cast<const float4*>(src + part * p.heads_k * rows * kHeadDim)[i];
+      x = make_float4(x.x + y.x, x.y + y.y, x.z + y.z, x.w + y.w);
+    }
     const uint32_t w0 = ptx::pack2<kBf16>(x.x * sc, x.y * sc), w1 = ptx::pack2<kBf16>(x.z * sc, x.w * sc);
-    if (FusedRoles<kHeadDim>::dq_rows(kSoftcap)) {   // 4 values of row e
+    if (row_lanes) {   // 4 values of row e
       *reinterpret_cast<uint2*>(tile + (q32 * 32 + e) * kRowElems + panel * 32 + g * 4) = make_uint2(w0, w1);
     } else {           // value e of 4 rows
       uint16_t* t = tile + (q32 * 32 + g * 4) * kRowElems + panel * 32 + e;
@@ -793,33 +851,48 @@ __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const __grid_consta
     const int qr = i / kPieces, piece = i % kPieces;
     if (qa + qr >= sm.n || piece * 8 >= p.head_dim) continue;
     const int64_t srow = static_cast<int64_t>(sm.row0) + half * sm.n + qa + qr;
-    uint16_t* dst = static_cast<uint16_t*>(p.dq) + sm.bcoord * p.dq_bs + srow * p.dq_rs + h * p.dq_hs + piece * 8;
+    uint16_t* dst = static_cast<uint16_t*>(kv < 0 ? p.dq : is_dv ? p.dv : p.dk) +
+                    sm.bcoord * (kv < 0 ? p.dq_bs : is_dv ? p.dv_bs : p.dk_bs) +
+                    srow * (kv < 0 ? p.dq_rs : is_dv ? p.dv_rs : p.dk_rs) +
+                    h * (kv < 0 ? p.dq_hs : is_dv ? p.dv_hs : p.dk_hs) + piece * 8;
     *reinterpret_cast<uint4*>(dst) = *reinterpret_cast<const uint4*>(tile + qr * kRowElems + piece * 8);
   }
 }
 
-template <int kHeadDim, int kSlots, int kDoSlots, bool kBf16, bool kSoftcap>
+template <int kHeadDim, int kSlots, int kDoSlots, bool kBf16, bool kSoftcap, bool kParts>
 int launch_fused_instance(const BwdParams& p, int sm_count, unsigned stages, cudaStream_t stream) {
   if (stages & 2u) {
     using Cfg = FusedCfg<kHeadDim, kSlots, kDoSlots>;
-    auto kernel = bwd_fused_kernel<kHeadDim, kSlots, kDoSlots, kBf16, kSoftcap>;
+    auto kernel = bwd_fused_kernel<kHeadDim, kSlots, kDoSlots, kBf16, kSoftcap, kParts>;
     static PerDeviceFlags smem_set;
     const int rc = set_dynamic_smem(kernel, Cfg::kSmemBytes, smem_set);
     if (rc) return rc;
     if (p.zero_acc16 == 0) {
       FDA_CUDA_TRY(cudaMemsetAsync(p.dq_acc, 0, static_cast<size_t>(p.heads) * p.acc_tiles * 64 * kHeadDim * 4, stream));
     }
-    const int items = bwd_item_bound(p, p.heads_k);
-    const int grid = items < sm_count ? items : sm_count;
+    const int64_t items = static_cast<int64_t>(bwd_item_bound(p, p.heads_k)) * p.kv_split;
+    const int grid = items < sm_count ? static_cast<int>(items) : sm_count;
     kernel<<<grid, FusedRoles<kHeadDim>::kThreads, Cfg::kSmemBytes, stream>>>(p);
     FDA_CUDA_TRY(cudaGetLastError());
   }
   if (stages & 4u) {
-    dim3 grid(p.n_pad / 64, 2 * p.heads, p.batch);
-    bwd_dq_convert_kernel<kHeadDim, kBf16, kSoftcap><<<grid, 256, 0, stream>>>(p);
+    dim3 grid(p.n_pad / 64, 2 * (p.heads + (p.kv_split > 1 ? 2 * p.heads_k : 0)), p.batch);
+    bwd_dq_convert_kernel<kHeadDim, kBf16, kSoftcap, kParts><<<grid, 256, 0, stream>>>(p);
     FDA_CUDA_TRY(cudaGetLastError());
   }
   return FDA_OK;
+}
+
+template <bool kParts>
+int dispatch_fused(const BwdParams& p, int d_round, bool bf16, bool softcap, int sm_count, unsigned stages,
+                   cudaStream_t stream) {
+  auto go = [&](auto bf16_tag, auto softcap_tag) {
+    constexpr bool kB = decltype(bf16_tag)::value, kC = decltype(softcap_tag)::value;
+    return d_round == 64 ? launch_fused_instance<64, 3, 3, kB, kC, kParts>(p, sm_count, stages, stream)
+                         : launch_fused_instance<128, 2, 1, kB, kC, kParts>(p, sm_count, stages, stream);
+  };
+  if (bf16) return softcap ? go(std::true_type{}, std::true_type{}) : go(std::true_type{}, std::false_type{});
+  return softcap ? go(std::false_type{}, std::true_type{}) : go(std::false_type{}, std::false_type{});
 }
 
 }  // namespace
@@ -835,19 +908,40 @@ size_t bwd_fused_acc_bytes(const FdaProblem& pr) {
   return static_cast<size_t>(pr.heads) * bwd_fused_acc_tiles(pr) * 64 * d_round * 4;
 }
 
+// Parts into which the query heads of a group are dealt. A key tile's steps are a chain, and those of the first clean tile
+// (2 x tiles x group, with tiles = n / 128) are more than a CTA's share of all steps (tiles (tiles + 2) x group for each KV
+// head and sample, over 148 CTAs) where batch x heads_k x (tiles + 2) is below 296: few tokens and few KV heads leave most of
+// the chip idle. Then as many parts as make the chain at most 1.2 times that share, as far as the group goes.
+// (Backward of 2 x 1000 tokens, 8 heads of 128 on one: 164 -> 62 us; 1 x 8192 tokens, 8/2 heads: 613 -> 233; 1 x 4096 tokens,
+// 32/8 heads: 416 -> 281, with a line at 296 that gives four parts instead of two 307; 3 x 666 tokens, 12/4 heads of 96:
+// 66 -> 55.)
+// Packed batches are judged by their longest sample and the least that the steps of all can sum up to. Chains of up to 32 steps
+// stay whole although 18 of them would gain too: the parts' sums round differently, and on small problems dK and dV of the two
+// forms of the backward are promised to be the same bits.
+int bwd_fused_kv_split(const FdaProblem& pr) {
+  const int group = pr.heads_k > 0 ? pr.heads / pr.heads_k : 1;
+  if (group <= 1 || pr.batch <= 0) return 1;
+  const double longest = (pr.seqlen / 2 + kTile - 1) / kTile;
+  if (2 * longest * group <= 32) return 1;
+  const double tiles = pr.cu_seqlens == nullptr ? longest * pr.batch : pr.total / (2.0 * kTile);
+  const double steps = pr.heads_k * (tiles * tiles / pr.batch + 2 * tiles);
+  int split = 1;
+  while (split < group && split * steps < 240 * longest) {
+    do ++split; while (group % split != 0);
+  }
+  return split;
+}
+
+size_t bwd_fused_part_bytes(const FdaProblem& pr) {
+  const int split = bwd_fused_kv_split(pr), d_round = pr.head_dim <= 64 ? 64 : 128;
+  return split == 1 ? 0 : 2 * static_cast<size_t>(split) * pr.heads_k * bwd_fused_acc_tiles(pr) * 64 * d_round * 4;
+}
+
 // stages: bit 1 = accumulator zero-fill + single-pass kernel, bit 2 = dQ convert.
 int launch_bwd_fused(const BwdParams& p, int d_round, bool bf16, bool softcap, int sm_count, unsigned stages,
                      cudaStream_t stream) {
-  if (d_round == 64) {
-    if (bf16) return softcap ? launch_fused_instance<64, 3, 3, true, true>(p, sm_count, stages, stream)
-                             : launch_fused_instance<64, 3, 3, true, false>(p, sm_count, stages, stream);
-    return softcap ? launch_fused_instance<64, 3, 3, false, true>(p, sm_count, stages, stream)
-                   : launch_fused_instance<64, 3, 3, false, false>(p, sm_count, stages, stream);
-  }
-  if (bf16) return softcap ? launch_fused_instance<128, 2, 1, true, true>(p, sm_count, stages, stream)
-                           : launch_fused_instance<128, 2, 1, true, false>(p, sm_count, stages, stream);
-  return softcap ? launch_fused_instance<128, 2, 1, false, true>(p, sm_count, stages, stream)
-                 : launch_fused_instance<128, 2, 1, false, false>(p, sm_count, stages, stream);
+  return p.kv_split > 1 ? dispatch_fused<true>(p, d_round, bf16, softcap, sm_count, stages, stream)
+                        : dispatch_fused<false>(p, d_round, bf16, softcap, sm_count, stages, stream);
 }
 
 int read_status_bwd_fused(int32_t* out4) {

@@ -1013,6 +1013,8 @@ inline int64_t round_up64(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 // bwd_fused_sm100.cu
 size_t bwd_fused_acc_bytes(const FdaProblem& pr);
 int64_t bwd_fused_acc_tiles(const FdaProblem& pr);
+int bwd_fused_kv_split(const FdaProblem& pr);
+size_t bwd_fused_part_bytes(const FdaProblem& pr);
 int launch_bwd_fused(const BwdParams& p, int d_round, bool bf16, bool softcap, int sm_count, unsigned stages,
                      cudaStream_t stream);
 
@@ -1030,10 +1032,12 @@ size_t bwd_split_workspace_bytes(const FdaProblem& pr) {
   return static_cast<size_t>(2 * one + 256) + (pr.cu_seqlens != nullptr ? varlen_list_bytes(pr.batch) : 0);
 }
 
-// The single-pass backward keeps its fp32 dQ accumulator behind that.
+// The single-pass backward keeps its fp32 dQ accumulator behind that, and behind it parts of dK and dV where it makes some.
 size_t bwd_workspace_bytes(const FdaProblem& pr) {
   size_t bytes = bwd_split_workspace_bytes(pr);
-  if (bwd_single_pass(pr)) bytes += static_cast<size_t>(round_up64(static_cast<int64_t>(bwd_fused_acc_bytes(pr)), 256));
+  if (bwd_single_pass(pr)) {
+    bytes += static_cast<size_t>(round_up64(static_cast<int64_t>(bwd_fused_acc_bytes(pr)), 256)) + bwd_fused_part_bytes(pr);
+  }
   return bytes;
 }
 
@@ -1120,6 +1124,9 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
     p.dq_acc = reinterpret_cast<float*>(static_cast<uint8_t*>(a.workspace) + bwd_split_workspace_bytes(pr));
     p.acc_tiles = static_cast<int>(bwd_fused_acc_tiles(pr));
     p.acc_floats = static_cast<int64_t>(bwd_fused_acc_bytes(pr) / 4);
+    p.kv_split = bwd_fused_kv_split(pr);
+    p.part_floats = static_cast<int64_t>(bwd_fused_part_bytes(pr) / 4);
+    if (p.kv_split > 1) p.dkv_part = p.dq_acc + round_up64(p.acc_floats, 64);
   }
   // The work counters are zeroed by whichever kernel runs before the persistent ones anyway.
   if ((stage_mask & 6u) != 0 && !varlen) {
@@ -1159,7 +1166,8 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
     // dK/dV: the noisy key tiles (the second half of the ranks) are short; dQ: the shortest eighth (fractions
     // found by measurement on the benchmark shape); few items per CTA: rank for rank over all of them
     const int per_bh = 2 * p.tiles_per_half;
-    p.n_long_kv = order_n_long(per_bh, FDA_SHORT8_KV, static_cast<long long>(per_bh) * pr.batch * pr.heads_k, sm_count);
+    const int parts = single_pass ? p.kv_split : 1;
+    p.n_long_kv = order_n_long(per_bh, FDA_SHORT8_KV, static_cast<long long>(per_bh) * pr.batch * pr.heads_k * parts, sm_count);
     p.n_long_q = order_n_long(per_bh, FDA_SHORT8_Q, static_cast<long long>(per_bh) * pr.batch * pr.heads, sm_count);
   }
   const bool bf16 = pr.dtype == FDA_BF16;

@@ -147,6 +147,12 @@ __device__ __forceinline__ void bulk_reduce_add_f32(float* gmem_dst, const void*
                "r"(smem_u32(smem_src)), "r"(bytes)
                : "memory");
 }
+// Untiled bulk copy shared -> global, under the same conditions.
+__device__ __forceinline__ void bulk_store_1d(void* gmem_dst, const void* smem_src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem_dst), "r"(smem_u32(smem_src)),
+               "r"(bytes)
+               : "memory");
+}
 // all committed groups of this thread are complete
 __device__ __forceinline__ void bulk_wait_group0() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_smem() {

@@ -1018,8 +1018,6 @@ size_t bwd_fused_part_bytes(const FdaProblem& pr);
 int launch_bwd_fused(const BwdParams& p, int d_round, bool bf16, bool softcap, int sm_count, unsigned stages,
                      cudaStream_t stream);
 
-constexpr int64_t kZeroInPreprocessBytes = 32 << 20;
-
 // The single-pass backward adds dQ partials in an order that depends on scheduling and needs head dim <= 128.
 bool bwd_single_pass(const FdaProblem& pr) { return pr.deterministic == 0 && pr.head_dim <= 128; }
 
@@ -1133,14 +1131,10 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
     if (stage_mask & 1u) p.zero_tickets = p.ticket_kv;
     else FDA_CUDA_TRY(cudaMemsetAsync(p.ticket_kv, 0, kTicketInts * 4, stream));
   }
-  // An accumulator that stays in L2 with everything else is zeroed by the preprocess: one launch less, and small steps are
-  // bound by launches (16 heads of 128, blocks of 64; fill in front of the kernel / in the preprocess: 59.3 / 56.5 us of
-  // backward with 16 MB, 71.3 / 64.7 with 25 MB). A larger one is zero-filled right before the kernel that adds to it. That
-  // won 0.03 ms at 268 MB with an earlier form of the kernel; with this one it no longer does (88.7 / 83.6 us with 34 MB,
-  // 155.8 / 148.1 with 67, 328.6 / 320.3 with 134, 1088 / 1079 with 268).
-  if (single_pass && (stage_mask & 3u) == 3u && p.acc_floats * 4 <= kZeroInPreprocessBytes) {
-    p.zero_acc16 = p.acc_floats / 4;
-  }
+  // The accumulator is zeroed by the preprocess (a stage call of the kernel alone fills it itself): one launch less, and the
+  // fill runs beside the loads of O and dO. In front of the kernel / in the preprocess, backward with 16
+  // heads of 128: 87.0 / 80.8 us (34 MB), 1163 / 1143 (268 MB); 32/8 heads of 64, 134 MB: 672 / 659.
+  if (single_pass && (stage_mask & 3u) == 3u) p.zero_acc16 = p.acc_floats / 4;
   if (varlen) {
     // the work list of the persistent kernels is built on the device (no host synchronisation); every stage call
     // rebuilds it, so stages may be launched one by one

@@ -913,11 +913,10 @@ size_t bwd_fused_acc_bytes(const FdaProblem& pr) {
 // head and sample, over 148 CTAs) where batch x heads_k x (tiles + 2) is below 296: few tokens and few KV heads leave most of
 // the chip idle. Then as many parts as make the chain at most 1.2 times that share, as far as the group goes.
 // (Backward of 2 x 1000 tokens, 8 heads of 128 on one: 164 -> 62 us; 1 x 8192 tokens, 8/2 heads: 613 -> 233; 1 x 4096 tokens,
-// 32/8 heads: 416 -> 281, with a line at 296 that gives four parts instead of two 307; 3 x 666 tokens, 12/4 heads of 96:
-// 66 -> 55.)
+// 32/8 heads: 416 -> 281, with a line at 296 that gives four parts instead of two 307.)
 // Packed batches are judged by their longest sample and the least that the steps of all can sum up to. Chains of up to 32 steps
-// stay whole although 18 of them would gain too: the parts' sums round differently, and on small problems dK and dV of the two
-// forms of the backward are promised to be the same bits.
+// stay whole although they would gain too (3 x 666 tokens, 12/4 heads of 96, 18 steps: 66 -> 55 us): the sums of parts round
+// differently, and on small problems the two forms of the backward have always given the same bits of dK and dV.
 int bwd_fused_kv_split(const FdaProblem& pr) {
   const int group = pr.heads_k > 0 ? pr.heads / pr.heads_k : 1;
   if (group <= 1 || pr.batch <= 0) return 1;

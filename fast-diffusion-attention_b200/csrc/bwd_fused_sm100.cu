@@ -1,7 +1,8 @@
 // Single-pass backward of block-diffusion attention for sm_100a: dK, dV and dQ from five GEMMs per tile pair.
 //
 // One CTA per (128-key tile, KV head, sample, half), persistent. K and V stay in shared memory; the visible
-// 128-row query tiles of every query head of the group stream through. Per (key tile, query tile) step:
+// 128-row query tiles of every query head of the group stream through (few tokens and few KV heads: of a part of the heads,
+// see bwd_fused_kv_split). Per (key tile, query tile) step:
 //   S^T  = K Q^T                        keys on tensor-memory lanes, 128 query columns
 //   P^T  = exp2(S^T c - LSE2)           compute warps; written back over S^T as 16-bit (with a score cap: of
 //                                       cap * tanh(S^T / cap), and the factor kept for dS^T is P^T (1 - tanh^2))
@@ -9,7 +10,8 @@
 //   dS^T = P^T (dP^T - delta)           compute warps; to shared memory as 16-bit, [keys][queries]
 //   dV  += P^T dO, dK += dS^T Q         accumulators in tensor memory for the whole key tile
 //   dQ^T = K^T dS^T                     head dim on lanes, 128 query columns, written over the consumed dP^T buffer
-//                                       (head dim 64 leaves room for columns of its own)
+//                                       (head dim 64 leaves room for columns of its own; without score cap it is
+//                                       dQ = dS K there, queries on lanes, 64 columns)
 // The two halves of the arithmetic hang on different products, so they overlap different MMAs: P^T is computed while
 // dP^T (and the tail of the previous step) runs, dS^T while dV runs. The partial dQ^T of a step is added into an fp32
 // accumulator in global memory: the drain warps move it from tensor memory through a small shared-memory staging
@@ -64,10 +66,10 @@ struct FusedCfg {
 //   Head dim 128: two compute warpgroups of 64 columns. 512 threads start with 128 registers, and the drain warps hold a
 //     whole dQ^T (128 columns): the buffer it shares with dP^T is free 250 cycles after the product instead of after 48
 //     of its 64 KB have left for L2 (backward of 4 x 8192 tokens, 32/8 heads of 128, blocks of 1024: 4.25 -> 3.98 ms).
-//     What bounds it is not settled. The kernel's time there is 6250 cycles for each of a CTA's 1107 steps. The tensor
-//     pipe's arithmetic is 2560 of them; shared memory at 128 bytes a clock 4350 (operands 2300, the staging of dQ^T 1024,
-//     the loads 512, dS^T 256, statistics 250); without the reductions themselves, everything else as it is, 5500 remain
-//     (and 3 % less time on 8 x 4096 tokens, 16 heads, blocks of 256). Vector reductions straight from the registers
+//     It is bound by shared memory and by power: a step takes 4450 cycles there (of a clock of 1.46 to 1.65 GHz), of which
+//     shared memory at 128 bytes a clock has 4350 (operands 2300, the staging of dQ^T 1024, the loads 512, dS^T 256,
+//     statistics 250), the tensor pipe's arithmetic 2560; without the reductions themselves it takes 11 % less time
+//     (3 % less on 8 x 4096 tokens, 16 heads, blocks of 256). Vector reductions straight from the registers
 //     would save the staging, but stall the load/store unit for the compute warps (4.1 ms).
 //   Head dim 64: dQ^T has columns of its own, and the exponentials (and tanh) weigh more: four compute warpgroups of 32
 //     columns keep the special-function unit busier than two (4 x 8192 tokens, 32 heads, score cap: 2.8 against 3.2 ms).

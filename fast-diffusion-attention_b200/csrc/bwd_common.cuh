@@ -9,7 +9,6 @@
 #include "host_util.h"
 #include "ptx.cuh"
 #include "sched.cuh"
-#include "softcap.cuh"
 #include "varlen_list.cuh"
 
 #ifndef FDA_SHORT8_KV
@@ -55,8 +54,7 @@ struct BwdParams {
   int64_t acc_floats;   // size of the accumulator
   VarlenList vl;     // packed batches: samples longest first with running 128-row tile counts (base == nullptr otherwise)
   int wide_store;      // dq/dk/dv rows allow 32-byte stores
-  float scale_log2, softmax_scale;
-  CapPoly cap;         // tanh of a capped score; its argument scale is softmax_scale / softcap
+  float scale_log2, softcap_pre, softmax_scale;
   int kv_split;         // single-pass backward: parts into which a key tile's query heads are dealt (a divisor of the group)
   float* dkv_part;      // ... their fp32 dK and dV: [2][kv_split][heads_k][acc_tiles * 64 rows][head dim]; nullptr without parts
   int64_t part_floats;  // size of that
@@ -128,20 +126,20 @@ static_assert(kCols == 32, "one 32-column tensor-memory load per operand and war
 template <int kN, bool kBf16, bool kSoftcap, bool kPerColumn, bool kMasked, bool kNeedP, bool kNeedDs = true>
 __device__ __forceinline__ void softmax_backward_cols(const uint32_t* s, const uint32_t* dp, const float* lse2_col,
                                                       const float* delta_col, float lse2_row, float delta_row,
-                                                      float scale_log2, const CapPoly& cap, int lo, int hi,
+                                                      float scale_log2, float softcap_pre, int lo, int hi,
                                                       uint32_t* pk_p, uint32_t* pk_ds) {
-  float xs[kN];
-#pragma unroll
-  for (int c = 0; c < kN; ++c) xs[c] = __uint_as_float(s[c]);
-  if (kSoftcap) cap_scores<kN>(xs, cap, false);
 #pragma unroll
   for (int c = 0; c < kN; c += 2) {
     float pv[2], dsv[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
       const int col = c + e;
-      const float x = xs[col];
-      const float dt = kSoftcap ? 1.f - x * x : 1.f;
+      float x = __uint_as_float(s[col]);
+      float dt = 1.f;
+      if (kSoftcap) {
+        x = ptx::tanh_fast(x * softcap_pre);
+        dt = 1.f - x * x;
+      }
       const float l2 = kPerColumn ? lse2_col[col] : lse2_row;
       const float dl = kPerColumn ? delta_col[col] : delta_row;
       float pr = ptx::ex2(fmaf(x, scale_log2, l2));

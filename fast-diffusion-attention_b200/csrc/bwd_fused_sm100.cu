@@ -92,10 +92,9 @@ struct FusedRoles {
   static constexpr bool kGeometryWarp = kHeadDim == 128;
   // dQ = dS K instead of dQ^T = K^T dS^T: at head dim 64, where dQ^T has only 64 rows, so that half of an M = 128 product is
   // thrown away and two of the four drain warps do all the work (backward of 4 x 4096 tokens, 32/8 heads, blocks of 64: 706 ->
-  // 684 us; 4 x 8192, 32 heads, blocks of 256: 2358 -> 2320). With capped scores, whose arithmetic leaves time for both, it is
-  // not faster (2616 / 2710 us on the latter shape).
+  // 684 us; 4 x 8192, 32 heads, blocks of 256: 2358 -> 2320). With capped scores, whose arithmetic leaves time for both, it was
+  // not faster (2710 / 2616 us on the latter shape, with a tanh cheaper than the present one).
   static constexpr bool dq_rows(bool softcap) { return kHeadDim == 64 && !softcap; }
-  static constexpr bool kPolyCap = kHeadDim == 64;   // capped scores by the polynomial where it holds: see softcap.cuh
   static_assert(128 * (kCmpWG * kComputeRegs + kProducerRegs + kDrainRegs) <= kThreads * kLaunchRegs, "register pool");
 };
 
@@ -710,8 +709,8 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
           ptx::tmem_wait_ld();
           const float4* l2v = reinterpret_cast<const float4*>(stats);
           // the fully visible tile (the common one) carries no per-element compare
-          auto first_half = [&](auto masked_tag, auto poly_tag) {
-            constexpr bool kMasked = decltype(masked_tag)::value, kPoly = decltype(poly_tag)::value;
+          auto first_half = [&](auto masked_tag) {
+            constexpr bool kMasked = decltype(masked_tag)::value;
 #pragma unroll
             for (int half = 0; half < kChunks; ++half) {
               uint32_t pk[16];
@@ -725,7 +724,8 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
                   float x0 = pr[c], x1 = pr[c + 1];
                   float dt0 = 1.f, dt1 = 1.f;
                   if (kSoftcap) {
-                    cap2<kPoly>(x0, x1, p.cap);
+                    x0 = ptx::tanh_fast(x0 * p.softcap_pre);
+                    x1 = ptx::tanh_fast(x1 * p.softcap_pre);
                     dt0 = 1.f - x0 * x0;
                     dt1 = 1.f - x1 * x1;
                   }
@@ -744,15 +744,8 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
               ptx::tmem_st16(s_t + 32 * half, pk);
             }
           };
-          using Poly = std::integral_constant<bool, kSoftcap && R::kPolyCap>;
-          const bool poly = Poly::value && cap_poly_holds<R::kCols>(pr, p.cap);
-          if (masked) {
-            if (poly) first_half(std::true_type{}, Poly{});
-            else first_half(std::true_type{}, std::false_type{});
-          } else {
-            if (poly) first_half(std::false_type{}, Poly{});
-            else first_half(std::false_type{}, std::false_type{});
-          }
+          if (masked) first_half(std::true_type{});
+          else first_half(std::false_type{});
           ptx::tmem_wait_st();
           ptx::tc_fence_before();
           ptx::mbar_arrive_warp(p_full);

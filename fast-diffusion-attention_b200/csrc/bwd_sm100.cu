@@ -547,10 +547,10 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
           ptx::tmem_wait_ld();
           if (masked) {
             softmax_backward_cols<kSubCols, kBf16, kSoftcap, true, true, kP, kDs>(sv, dpv, l2r, dlr, 0.f, 0.f, p.scale_log2,
-                                                                                  p.cap, lo, hi, pk_p, pk_ds);
+                                                                                  p.softcap_pre, lo, hi, pk_p, pk_ds);
           } else {
             softmax_backward_cols<kSubCols, kBf16, kSoftcap, true, false, kP, kDs>(sv, dpv, l2r, dlr, 0.f, 0.f, p.scale_log2,
-                                                                                   p.cap, 0, 0, pk_p, pk_ds);
+                                                                                   p.softcap_pre, 0, 0, pk_p, pk_ds);
           }
           // a warp overwrites only columns it has itself already loaded: its packed P^T / dS^T pieces go to the
           // start of its own kSubCols columns
@@ -922,10 +922,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
         uint32_t pk_ds[kKc / 2];
         if (cls == kTileMasked) {
           softmax_backward_cols<kKc, kBf16, kSoftcap, false, true, false>(sv, dpv, nullptr, nullptr, cur.lse2, cur.delta,
-                                                                          p.scale_log2, p.cap, lo, hi, nullptr, pk_ds);
+                                                                          p.scale_log2, p.softcap_pre, lo, hi, nullptr, pk_ds);
         } else {
           softmax_backward_cols<kKc, kBf16, kSoftcap, false, false, false>(sv, dpv, nullptr, nullptr, cur.lse2, cur.delta,
-                                                                           p.scale_log2, p.cap, 0, 0, nullptr, pk_ds);
+                                                                           p.scale_log2, p.softcap_pre, 0, 0, nullptr, pk_ds);
         }
         if (!ptx::mbar_wait(ds_free, (cnt & 1) ^ 1, abort_flag, 92)) { alive = false; break; }
         ++cnt;
@@ -1150,9 +1150,10 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   p.softmax_scale = pr.softmax_scale;
   if (softcap) {
     p.scale_log2 = pr.softcap * kLog2e;
-    p.cap = make_cap_poly(pr.softmax_scale / pr.softcap);
+    p.softcap_pre = pr.softmax_scale / pr.softcap;
   } else {
     p.scale_log2 = pr.softmax_scale * kLog2e;
+    p.softcap_pre = 0.f;
   }
   int sm_count = info.sm_count - (pr.sm_margin > 0 ? pr.sm_margin : 0);
   if (sm_count < 1) sm_count = 1;

@@ -23,13 +23,10 @@
 // Numerics contract kept from the reference: fp32 accumulation, softcap applied before the mask
 // (mainloop_fwd...hpp:679-683), P rounded to the input dtype before P V (:782), row sums accumulated in fp32
 // from the unrounded P, LSE = max * scale + ln(sum) (softmax.h:137-154).
-#include <type_traits>
-
 #include "geometry.h"
 #include "host_util.h"
 #include "ptx.cuh"
 #include "sched.cuh"
-#include "softcap.cuh"
 #include "varlen_list.cuh"
 
 
@@ -69,7 +66,7 @@ struct FwdParams {
   const float* v_descale;
   int64_t descale_bs[3], descale_hs[3];
   float scale_log2;    // exponent scale: softmax_scale*log2(e), or softcap*log2(e) with softcapping
-  CapPoly cap;         // tanh of a capped score; its argument scale is softmax_scale / softcap
+  float softcap_pre;   // softmax_scale / softcap (tanh argument scale)
   float lse_scale;     // natural-log scale of the row maximum: softmax_scale, or softcap
 };
 
@@ -181,7 +178,6 @@ struct FwdConfig {
   // (168 per thread with the block rounded up to whole warpgroups), so the block is padded to three whole
   // warpgroups and the third (TMA warp, two MMA warps, an idle warp) hands registers to the other two.
   static constexpr bool kRegRealloc = kQTiles == 2;
-  static constexpr bool kPolyCap = kHeadDim <= 128;   // capped scores: see softcap.cuh
   static constexpr int kThreads = kRegRealloc ? 384 : 128 * kQTiles + 64;
   static constexpr uint32_t kSoftmaxRegs = 200, kProducerRegs = 104;
   // the pool is what the block got at launch, 384 threads x 168 registers: 2 * 128 * 200 + 128 * 104 = 384 * 168.
@@ -539,15 +535,14 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       const int blk1 = imin(blk0 + bs, it.n);
       // FP8: the per-(sample, KV head) descales of q and k fold into the score scale, the descale of v into the
       // final normalisation (the reference does the same, flash_fwd_kernel_sm90.h:299-305, mainloop_fwd...:818-822)
-      float scale_log2 = p.scale_log2, lse_scale = p.lse_scale, out_scale = 1.f;
-      CapPoly cap_fp8{};
+      float scale_log2 = p.scale_log2, softcap_pre = p.softcap_pre, lse_scale = p.lse_scale, out_scale = 1.f;
       if (Cfg::kFp8) {
         float qk = 1.f;
         if (p.q_descale != nullptr) qk *= p.q_descale[it.b * p.descale_bs[0] + it.hk * p.descale_hs[0]];
         if (p.k_descale != nullptr) qk *= p.k_descale[it.b * p.descale_bs[1] + it.hk * p.descale_hs[1]];
         if (p.v_descale != nullptr) out_scale = p.v_descale[it.b * p.descale_bs[2] + it.hk * p.descale_hs[2]];
         if (kSoftcap) {
-          cap_fp8 = make_cap_poly(p.cap.pre * qk);
+          softcap_pre *= qk;
         } else {
           scale_log2 *= qk;
           lse_scale *= qk;
@@ -559,7 +554,6 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       // 557 instead of 610 us on 4 x 8192 tokens, 16/4 heads of 128, but would round the probability that matters most,
       // by up to 6 %, and the relative error of the output rises from 1.97e-2 to 2.06e-2.) 16-bit P may run up to 2^8
       // above 1 before the maximum is advanced.
-      const CapPoly& cap = Cfg::kFp8 ? cap_fp8 : p.cap;
       constexpr float kThreshold = Cfg::kFp8 ? 0.f : kRescaleThreshold;
       constexpr float kPShift = Cfg::kFp8 ? 8.f : 0.f;
       // Where O is rescaled often (fp8) or the exponentials take long (capped scores) that is done behind them, so that the
@@ -588,13 +582,9 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
           for (int c = 0; c < kSubKeys / 32; ++c) ptx::tmem_ld32(tmem_sb + c * 32, w + c * 32);
           ptx::tmem_wait_ld();
         }
-        // Capped scores: a fully visible sub-step keeps the raw ones where the polynomial holds (tanh rises with the score,
-        // so the maximum may be taken of those) and caps them between the exponentials below; a masked one caps them here.
-        bool capped_late = false;
         if (kSoftcap) {
-          const bool poly = Cfg::kPolyCap && cap_poly_holds<kSubKeys>(v, cap);
-          capped_late = poly && cls != kTileMasked;
-          if (!capped_late) cap_scores<kSubKeys>(v, cap, poly);
+#pragma unroll
+          for (int c = 0; c < kSubKeys; ++c) v[c] = ptx::tanh_fast(v[c] * softcap_pre);
         }
         if (cls == kTileMasked) {
           int lo, hi;
@@ -618,12 +608,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
 #pragma unroll
           for (int i = 0; i < 8; ++i) mx[i] = ptx::max3(mx[i], v[c + 2 * i], v[c + 2 * i + 1]);
         }
-        float m_tile = fmaxf(ptx::max3(mx[0], mx[1], mx[2]), ptx::max3(ptx::max3(mx[3], mx[4], mx[5]), mx[6], mx[7]));
-        if (kSoftcap && capped_late) {
-          float t0, t1;
-          cap_poly2(t0, t1, m_tile, m_tile, cap);
-          m_tile *= t0;
-        }
+        const float m_tile = fmaxf(ptx::max3(mx[0], mx[1], mx[2]), ptx::max3(ptx::max3(mx[3], mx[4], mx[5]), mx[6], mx[7]));
         const float m_new = fmaxf(m_run, m_tile);
         // Advance the reference maximum only when it grew by more than the threshold. In the first two sub-steps at every
         // increase: the largest of the first 128 scores then has P = 1 exactly, and few rows have a larger one after that.
@@ -673,10 +658,6 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
         if (Cfg::kFp8) {
 #pragma unroll
           for (int c = 0; c < kSubKeys; c += 4) {
-            if (kSoftcap && capped_late) {
-              cap2<true>(v[c], v[c + 1], cap);
-              cap2<true>(v[c + 2], v[c + 3], cap);
-            }
             const float p0 = ptx::ex2(fmaf(v[c], scale_log2, neg_m));
             const float p1 = ptx::ex2(fmaf(v[c + 1], scale_log2, neg_m));
             const float p2 = ptx::ex2(fmaf(v[c + 2], scale_log2, neg_m));
@@ -687,20 +668,15 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
         } else {
           // two elements per FMA and per ADD: the sums run as four pairs of partial sums
           float sumb[4] = {0.f, 0.f, 0.f, 0.f};
-          auto exponentials = [&](auto late_tag) {
 #pragma unroll
-            for (int c = 0; c < kSubKeys; c += 2) {
-              float y0, y1;
-              if (decltype(late_tag)::value) cap2<true>(v[c], v[c + 1], cap);
-              ptx::fma2(y0, y1, v[c], v[c + 1], scale_log2, scale_log2, neg_m, neg_m);
-              const float p0 = ptx::ex2(y0);
-              const float p1 = ptx::ex2(y1);
-              ptx::add2(sum4[(c / 2) & 3], sumb[(c / 2) & 3], sum4[(c / 2) & 3], sumb[(c / 2) & 3], p0, p1);
-              pk[c / 2] = ptx::pack2<kType == 0>(p0, p1);
-            }
-          };
-          if (kSoftcap && capped_late) exponentials(std::integral_constant<bool, kSoftcap>{});
-          else exponentials(std::false_type{});
+          for (int c = 0; c < kSubKeys; c += 2) {
+            float y0, y1;
+            ptx::fma2(y0, y1, v[c], v[c + 1], scale_log2, scale_log2, neg_m, neg_m);
+            const float p0 = ptx::ex2(y0);
+            const float p1 = ptx::ex2(y1);
+            ptx::add2(sum4[(c / 2) & 3], sumb[(c / 2) & 3], sum4[(c / 2) & 3], sumb[(c / 2) & 3], p0, p1);
+            pk[c / 2] = ptx::pack2<kType == 0>(p0, p1);
+          }
 #pragma unroll
           for (int i = 0; i < 4; ++i) sum4[i] += sumb[i];
         }
@@ -915,10 +891,11 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
   const bool softcap = pr.softcap > 0.f;
   if (softcap) {
     p.scale_log2 = pr.softcap * kLog2e;
-    p.cap = make_cap_poly(pr.softmax_scale / pr.softcap);
+    p.softcap_pre = pr.softmax_scale / pr.softcap;
     p.lse_scale = pr.softcap;
   } else {
     p.scale_log2 = pr.softmax_scale * kLog2e;
+    p.softcap_pre = 0.f;
     p.lse_scale = pr.softmax_scale;
   }
   if (p.total_items <= 0) return FDA_OK;

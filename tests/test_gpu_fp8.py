@@ -50,6 +50,30 @@ def test_forward_fp8(batch, n, bs, varlen, use_descale, heads, heads_k, d):
     assert diff.mean().abs().item() <= 0.1 * diff.abs().mean().item() + 1e-5
 
 
+@pytest.mark.parametrize("d", [64, 128, 256])
+@pytest.mark.parametrize("quantised", [False, True])
+@pytest.mark.parametrize("gain", [0.5, 3.0])
+@pytest.mark.parametrize("batch,n,bs", [(2, 600, 24), (1, 130, 256)])
+def test_forward_fp8_capped(batch, n, bs, gain, quantised, d):
+    """With a score cap: inputs as they are, and scaled by their largest magnitude over 448, where scale / cap times the
+    descales is some 1e-7."""
+    torch.manual_seed(n + d)
+    cap, scale = 5.0, gain * d ** -0.5
+    x = [torch.randn(batch, 2 * n, h, d, device=DEV) for h in (6, 2, 2)]
+    descales = [t.unflatten(2, (2, -1)).abs().amax(dim=(1, 3, 4)) / 448 if quantised else torch.ones(batch, 2, device=DEV) for t in x]
+    q8, k8, v8 = ((t / s.repeat_interleave(t.shape[2] // 2, dim=1)[:, None, :, None]).to(E4M3) for t, s in zip(x, descales))
+    kw = dict(zip(("q_descale", "k_descale", "v_descale"), descales if quantised else [None] * 3))
+    out, lse = diffusion_attn_func(q8, k8, v8, bs, softmax_scale=scale, softcap=cap, return_attn_probs=True, **kw)
+    assert _lib.device_status()[0] == 0
+    # the truth keeps the descales in fp32 (applied to the e4m3 values, which bf16 holds exactly)
+    up = [t.float() * s.repeat_interleave(t.shape[2] // 2, dim=1)[:, None, :, None] for t, s in zip((q8, k8, v8), descales)]
+    truth, lse_t = orc.forward(*up, bs, softmax_scale=scale, softcap=cap)
+    plain, _ = orc.forward(*(t.to(torch.bfloat16) for t in (q8, k8, v8)), bs, softmax_scale=scale, softcap=cap,
+                           compute_dtype=torch.bfloat16, p_dtype=E4M3, **kw)
+    assert_within_2x("out", out, truth, plain)
+    assert (lse - lse_t).abs().max().item() <= cap * 2.0 ** -11 + 1e-4
+
+
 def test_fp8_backward_is_rejected():
     q8 = torch.randn(1, 64, 2, 64, device=DEV).to(E4M3).requires_grad_()
     out = diffusion_attn_func(q8, q8.detach(), q8.detach(), 4)

@@ -903,32 +903,56 @@ size_t bwd_fused_acc_bytes(const FdaProblem& pr) {
   return static_cast<size_t>(pr.heads) * bwd_fused_acc_tiles(pr) * 64 * d_round * 4;
 }
 
-// Parts into which the query heads of a group are dealt. A key tile's steps are a chain, and those of the first clean tile
-// (2 x tiles x group, with tiles = n / 128) are more than a CTA's share of all steps (tiles (tiles + 2) x group for each KV
-// head and sample, over 148 CTAs) where batch x heads_k x (tiles + 2) is below 296: few tokens and few KV heads leave most of
-// the chip idle. Then as many parts as make the chain at most 1.2 times that share, as far as the group goes.
+namespace {
+
+constexpr int64_t kMaxPartBytes = 128ll << 20;
+
+// fp32 dK and dV of `split` parts, in the accumulator's layout
+int64_t part_bytes(const FdaProblem& pr, int split) {
+  const int d_round = pr.head_dim <= 64 ? 64 : 128;
+  return 2ll * split * pr.heads_k * bwd_fused_acc_tiles(pr) * 64 * d_round * 4;
+}
+
+}  // namespace
+
+// Parts into which the query heads of a group are dealt. A key tile's steps are a chain, and those of the longest sample's first
+// clean tile (2 x tiles x group, with tiles = n / 128) are more than a CTA's share of all steps (tiles (tiles + 2) x group for
+// each KV head and sample, over 148 CTAs) where few tokens and few KV heads leave most of the chip idle. Then as many parts as
+// make the chain at most 1.23 times that share, as far as the group goes.
 // (Backward of 2 x 1000 tokens, 8 heads of 128 on one: 164 -> 62 us; 1 x 8192 tokens, 8/2 heads: 613 -> 233; 1 x 4096 tokens,
-// 32/8 heads: 416 -> 281, with a line at 296 that gives four parts instead of two 307.)
-// Packed batches are judged by their longest sample and the least that the steps of all can sum up to. Chains of up to 32 steps
-// stay whole although they would gain too (3 x 666 tokens, 12/4 heads of 96, 18 steps: 66 -> 55 us): the sums of parts round
-// differently, and on small problems the two forms of the backward have always given the same bits of dK and dV.
+// 32/8 heads: 416 -> 281, with a chain of at most the share itself, which takes four parts instead of two, 307.)
+// Lengths of packed samples are on the device. What is known of them here, the longest (or a bound of it) and their sum, bounds
+// their steps from below: one sample as long as that, the rest equal. Samples of one length count like a batch of them.
+// All samples are dealt alike, so one long sample among many short ones would need much memory: no more than kMaxPartBytes, of
+// which the cases above take up to a half.
+// Chains of up to 32 steps stay whole although they would gain too (3 x 666 tokens, 12/4 heads of 96, 18 steps: 66 -> 55 us): the
+// sums of parts round differently, and on small problems the two forms of the backward give the same bits of dK and dV.
+// sm_margin does not count: it changes no result.
 int bwd_fused_kv_split(const FdaProblem& pr) {
+  constexpr double kLine = 240;   // 2 x 148 / 1.23
   const int group = pr.heads_k > 0 ? pr.heads / pr.heads_k : 1;
   if (group <= 1 || pr.batch <= 0) return 1;
-  const double longest = (pr.seqlen / 2 + kTile - 1) / kTile;
+  double longest = (pr.seqlen / 2 + kTile - 1) / kTile, all = longest * pr.batch, squares = longest * all;   // in tiles
+  if (pr.cu_seqlens != nullptr && pr.total != static_cast<int64_t>(pr.batch) * pr.seqlen) {
+    all = pr.total / (2.0 * kTile);
+    if (longest > all) longest = all;
+    squares = longest * longest + (pr.batch > 1 ? (all - longest) * (all - longest) / (pr.batch - 1) : 0);
+  }
   if (2 * longest * group <= 32) return 1;
-  const double tiles = pr.cu_seqlens == nullptr ? longest * pr.batch : pr.total / (2.0 * kTile);
-  const double steps = pr.heads_k * (tiles * tiles / pr.batch + 2 * tiles);
+  const double steps = pr.heads_k * (squares + 2 * all);   // of one query head of each group
   int split = 1;
-  while (split < group && split * steps < 240 * longest) {
-    do ++split; while (group % split != 0);
+  while (split * steps < kLine * longest) {
+    int next = split + 1;
+    while (next < group && group % next != 0) ++next;
+    if (next > group || part_bytes(pr, next) > kMaxPartBytes) break;
+    split = next;
   }
   return split;
 }
 
 size_t bwd_fused_part_bytes(const FdaProblem& pr) {
-  const int split = bwd_fused_kv_split(pr), d_round = pr.head_dim <= 64 ? 64 : 128;
-  return split == 1 ? 0 : 2 * static_cast<size_t>(split) * pr.heads_k * bwd_fused_acc_tiles(pr) * 64 * d_round * 4;
+  const int split = bwd_fused_kv_split(pr);
+  return split == 1 ? 0 : static_cast<size_t>(part_bytes(pr, split));
 }
 
 // stages: bit 1 = accumulator zero-fill + single-pass kernel, bit 2 = dQ convert.

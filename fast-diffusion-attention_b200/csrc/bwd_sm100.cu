@@ -1018,6 +1018,8 @@ size_t bwd_fused_part_bytes(const FdaProblem& pr);
 int launch_bwd_fused(const BwdParams& p, int d_round, bool bf16, bool softcap, int sm_count, unsigned stages,
                      cudaStream_t stream);
 
+constexpr int64_t kSmallAccBytes = 32 << 20;
+
 // The single-pass backward adds dQ partials in an order that depends on scheduling and needs head dim <= 128.
 bool bwd_single_pass(const FdaProblem& pr) { return pr.deterministic == 0 && pr.head_dim <= 128; }
 
@@ -1134,7 +1136,14 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   // The accumulator is zeroed by the preprocess (a stage call of the kernel alone fills it itself): one launch less, and the
   // fill runs beside the loads of O and dO. In front of the kernel / in the preprocess, backward with 16
   // heads of 128: 87.0 / 80.8 us (34 MB), 1163 / 1143 (268 MB); 32/8 heads of 64, 134 MB: 672 / 659.
-  if (single_pass && (stage_mask & 3u) == 3u) p.zero_acc16 = p.acc_floats / 4;
+  // Not where packed samples are much shorter than max_seqlen: most blocks of the preprocess then have nothing but padding to
+  // write, and the stores are dear there. 32 samples of 1024 tokens, 32/8 heads of 128 (in front / in the preprocess): 1116 / 1114 us
+  // with max_seqlen as it is, 1161 / 1168 with three times that, 1225 / 1256 with four, 1474 / 1537 with eight. (Small
+  // accumulators are always filled there: the launch counts for more.)
+  const int64_t padded_rows = static_cast<int64_t>(pr.batch) * 2 * p.n_pad, acc_rows = static_cast<int64_t>(p.acc_tiles) * 64;
+  if (single_pass && (stage_mask & 3u) == 3u && (padded_rows <= 3 * acc_rows || p.acc_floats * 4 <= kSmallAccBytes)) {
+    p.zero_acc16 = p.acc_floats / 4;
+  }
   if (varlen) {
     // the work list of the persistent kernels is built on the device (no host synchronisation); every stage call
     // rebuilds it, so stages may be launched one by one

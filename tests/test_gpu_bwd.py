@@ -177,3 +177,22 @@ def test_backward_many_short_items(bs, d):
     cu = torch.tensor([0] + list(torch.tensor([2 * x for x in ns]).cumsum(0)), device=DEV, dtype=torch.int32)
     q, k, v = (torch.randn(2 * sum(ns), h, d, device=DEV, dtype=torch.bfloat16) for h in (4, 2, 2))
     check_backward(q, k, v, bs, cu=cu)
+
+
+@pytest.mark.parametrize("n,max_n", [(512, 512), (512, 1500), (500, 1600), (512, 5000)])
+def test_backward_loose_max_seqlen(n, max_n):
+    """max_seqlen may be any upper bound. The dQ accumulator (67 MB here) is zeroed by the preprocess up to a padding of three
+    times the rows and by a fill of its own beyond; twice in a row, so that the second call finds the first one's sums."""
+    torch.manual_seed(n + max_n)
+    batch, heads, d, bs = 8, 16, 128, 64
+    q, k, v, g = (torch.randn(batch, 2 * n, heads, d, device=DEV, dtype=torch.bfloat16) for _ in range(4))
+    leaves = [x.requires_grad_() for x in (q, k, v)]
+    want = torch.autograd.grad(diffusion_attn_func(*leaves, bs), leaves, g)
+    cu = torch.arange(0, batch * 2 * n + 1, 2 * n, device=DEV, dtype=torch.int32)
+    flat = [x.detach().flatten(0, 1).requires_grad_() for x in (q, k, v)]
+    for _ in range(2):
+        out = diffusion_attn_varlen_func(*flat, cu, cu, 2 * max_n, 2 * max_n, bs)
+        got = torch.autograd.grad(out, flat, g.flatten(0, 1))
+        for name, a, b in zip(("dq", "dk", "dv"), got, want):
+            assert_same_gradients(name, a.unflatten(0, (batch, -1)), b, exact=name != "dq")
+    assert _lib.device_status()[0] == 0

@@ -854,6 +854,10 @@ __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const __grid_consta
   }
 }
 
+// A row of the convert kernel's grid is one half of a query head's dQ or, with parts, of a KV head's dK or dV.
+int convert_rows(int heads, int heads_k, bool parts) { return 2 * (heads + (parts ? 2 * heads_k : 0)); }
+constexpr int kMaxGridY = 65535;
+
 template <int kHeadDim, int kSlots, int kDoSlots, bool kBf16, bool kSoftcap, bool kParts>
 int launch_fused_instance(const BwdParams& p, int sm_count, unsigned stages, cudaStream_t stream) {
   if (stages & 2u) {
@@ -871,7 +875,7 @@ int launch_fused_instance(const BwdParams& p, int sm_count, unsigned stages, cud
     FDA_CUDA_TRY(cudaGetLastError());
   }
   if (stages & 4u) {
-    dim3 grid(p.n_pad / 64, 2 * (p.heads + (p.kv_split > 1 ? 2 * p.heads_k : 0)), p.batch);
+    dim3 grid(p.n_pad / 64, convert_rows(p.heads, p.heads_k, p.kv_split > 1), p.batch);
     bwd_dq_convert_kernel<kHeadDim, kBf16, kSoftcap, kParts><<<grid, 256, 0, stream>>>(p);
     FDA_CUDA_TRY(cudaGetLastError());
   }
@@ -927,6 +931,7 @@ int64_t part_bytes(const FdaProblem& pr, int split) {
 // which the cases above take up to a half.
 // Chains of up to 32 steps stay whole although they would gain too (3 x 666 tokens, 12/4 heads of 96, 18 steps: 66 -> 55 us): the
 // sums of parts round differently, and on small problems the two forms of the backward give the same bits of dK and dV.
+// They stay whole, too, where the convert kernel's grid has no rows left for dK and dV (more than 32700 heads or so).
 // sm_margin does not count: it changes no result.
 int bwd_fused_kv_split(const FdaProblem& pr) {
   constexpr double kLine = 240;   // 2 x 148 / 1.23
@@ -938,7 +943,7 @@ int bwd_fused_kv_split(const FdaProblem& pr) {
     if (longest > all) longest = all;
     squares = longest * longest + (pr.batch > 1 ? (all - longest) * (all - longest) / (pr.batch - 1) : 0);
   }
-  if (2 * longest * group <= 32) return 1;
+  if (2 * longest * group <= 32 || convert_rows(pr.heads, pr.heads_k, true) > kMaxGridY) return 1;
   const double steps = pr.heads_k * (squares + 2 * all);   // of one query head of each group
   int split = 1;
   while (split * steps < kLine * longest) {

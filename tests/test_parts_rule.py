@@ -72,3 +72,11 @@ def test_parts_stay_small():
 def test_packed_samples_of_one_length_are_dealt_like_a_batch(n, batch):
     for heads, heads_k in [(8, 1), (8, 2), (32, 8), (12, 4), (31, 1)]:
         assert parts(2 * n, heads, heads_k, 128, batch=batch)[0] == parts(heads=heads, heads_k=heads_k, d=128, **_packed([n] * batch))[0]
+
+
+def test_the_convert_grid_holds_every_head():
+    """dQ of each head and, with parts, dK and dV of each KV head are (half, head) rows of one grid, 65535 at most: a call that
+    the rest of the backward takes must not fail there."""
+    for heads, heads_k in [(32766, 6), (32767, 7), (32767, 1), (32760, 8), (16000, 1)]:
+        n, _ = parts(512, heads, heads_k, 64, batch=1)
+        assert n == 1 or 2 * (heads + 2 * heads_k) <= 65535, (heads, heads_k, n)

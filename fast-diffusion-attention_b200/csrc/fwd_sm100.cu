@@ -556,11 +556,12 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       // above 1 before the maximum is advanced.
       constexpr float kThreshold = Cfg::kFp8 ? 0.f : kRescaleThreshold;
       constexpr float kPShift = Cfg::kFp8 ? 8.f : 0.f;
-      // Where O is rescaled often (fp8) or the exponentials take long (capped scores) that is done behind them, so that the
-      // last P V, which must be done first, runs under them. (e4m3, 2 x 16384 tokens, 8 heads of 256: 950 -> 897 us;
-      // cap 30, 4 x 8192 tokens, 32 heads of 64: 1257 -> 1173. Elsewhere O is rescaled about once an item and the order is worth
-      // nothing: 1310 against 1326 us on 4 x 8192 tokens, 32/8 heads of 128.)
-      constexpr bool kLateRescale = kSoftcap || Cfg::kFp8;
+      // fp8 rescales O often. That is done behind the exponentials, so that the last P V, which must be done first, runs under
+      // them (2 x 16384 tokens, 8 heads of 256: 950 -> 897 us; 4 x 8192 tokens, 16/4 heads of 64, 128, 256: 607, 616, 1044 -> 596, 604,
+      // 997). 16-bit P rescales O about once an item and gains nothing (1310 against 1326 us on 4 x 8192 tokens, 32/8 heads of 128).
+      // Capped scores rescale less: there it is worth it with one query tile only (4 x 8192 tokens, 16/4 heads of 256
+      // 1316 -> 1296; of 64 and 128, two tiles, 846 and 852 -> 864 and 871; 16-bit 1328 -> 1339 with 32 heads of 64).
+      constexpr bool kLateRescale = Cfg::kFp8 && (!kSoftcap || kHeadDim == 256);
       float m_run = -INFINITY;  // reference maximum (unscaled scores, or tanh values with softcap)
       float l_run = 0.f;
       bool o_started = false, settled = false;   // one sub-step, two sub-steps of this tile are done

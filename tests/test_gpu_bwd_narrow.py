@@ -1,6 +1,6 @@
-"""Single-pass backward at head dimensions up to 64: dQ is made with a query on every lane, S^T is a step ahead in a buffer of
-its own. Sizes where that can go wrong: one step, two, three (the buffers, the ring of Q); quarters of a step without queries;
-head dimensions that end inside or before the second 32 columns; several heads of a group; ends of samples."""
+"""Single-pass backward at head dimensions up to 64: dQ is made with a query on every lane, in tensor-memory columns of its own.
+Sizes where that can go wrong: one step, two, three (the ring of Q); quarters of a step without queries; head dimensions that end
+inside or before the second 32 columns; several heads of a group; ends of samples."""
 
 import pytest
 import torch

@@ -1,6 +1,8 @@
 """Single-pass backward where the query heads of a group are dealt out to several CTAs and their dK and dV added up afterwards:
-few tokens, few KV heads, more than 32 steps a key tile. Groups with and without small divisors, head dimensions that do not fill a piece, ends of halves
-inside a piece of 32 rows, packed batches with empty samples, strided outputs; dk and dv are the same in every run."""
+few tokens, few KV heads, more than 32 steps a key tile (the smallest shapes here, with smaller groups, are just below that and
+stay whole). One head a part and several, groups with and without small divisors, head dimensions that do not fill a piece,
+ends of halves inside a piece of 32 rows, packed batches with empty samples, strided outputs; dk and dv are the same in every
+run."""
 
 import pytest
 import torch
@@ -9,6 +11,7 @@ from fast_diffusion_attention import diffusion_attn_func
 from fast_diffusion_attention.interface import diffusion_attn_varlen_qkvpacked_func
 from oracle import diffusion_oracle as orc
 from test_gpu_bwd import check_backward
+from test_parts_rule import parts
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -25,6 +28,27 @@ def test_parts_of_a_group(batch, n, bs, heads, heads_k, d):
     runs = [torch.autograd.grad(diffusion_attn_func(*leaves, bs), leaves, torch.ones_like(q)) for _ in range(3)]
     for run in runs[1:]:
         assert torch.equal(run[1], runs[0][1]) and torch.equal(run[2], runs[0][2])
+
+
+@pytest.mark.parametrize("d", [128, 64, 96])
+@pytest.mark.parametrize("layout", ["batched", "packed"])
+@pytest.mark.parametrize("heads,heads_k,batch,n,bs,n_parts", [
+    (64, 8, 4, 300, 24, 2),      # four heads a part
+    (24, 4, 3, 700, 64, 3),      # two
+    (32, 2, 3, 1000, 300, 4),    # four
+    (24, 4, 6, 400, 1024, 2),    # three
+])
+def test_parts_of_several_heads(heads, heads_k, batch, n, bs, n_parts, layout, d):
+    lead = (batch, 2 * n) if layout == "batched" else (2 * batch * n,)
+    cu = None if layout == "batched" else torch.arange(0, 2 * batch * n + 1, 2 * n, device=DEV, dtype=torch.int32)
+    assert parts(2 * n, heads, heads_k, d, batch=batch, total=None if cu is None else 2 * batch * n)[0] == n_parts
+    torch.manual_seed(n)
+    q, k, v = (torch.randn(*lead, h, d, device=DEV, dtype=torch.bfloat16) for h in (heads, heads_k, heads_k))
+    first = check_backward(q, k, v, bs, cu=cu)
+    torch.manual_seed(n)
+    q, k, v = (torch.randn(*lead, h, d, device=DEV, dtype=torch.bfloat16) for h in (heads, heads_k, heads_k))
+    again = check_backward(q, k, v, bs, cu=cu)
+    assert torch.equal(again[1], first[1]) and torch.equal(again[2], first[2])
 
 
 @pytest.mark.parametrize("d", [128, 64])

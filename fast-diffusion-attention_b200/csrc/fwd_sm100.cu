@@ -160,7 +160,7 @@ struct ItemDesc {
 };
 
 // kType: 0 bf16, 1 fp16, 2 fp8 e4m3 (forward only; the output is bf16)
-template <int kHeadDim, int kQTiles, int kType, bool kSoftcap>
+template <int kHeadDim, int kQTiles, int kType, bool kSoftcap, bool kQInTmem>
 struct FwdConfig {
   static constexpr bool kFp8 = kType == 2;
   static constexpr int kElemBytes = kFp8 ? 1 : 2;
@@ -196,10 +196,10 @@ struct FwdConfig {
   // tensor memory: S of query tile t, buffer b at (t * kBufs + b) * 64 (P over its first columns), O behind
   static constexpr int kTmemO = kQTiles * kBufs * kSubKeys;
   static_assert(kTmemO + kQTiles * kHeadDim <= 512, "tensor memory budget");
-  // ... and, for head dim 256, Q behind that. The S product then fetches only K from shared memory (16 instead of
-  // 48 cycles a reduction step of 32 bytes): 1225 -> 1154 us on 2 x 16384 tokens, 8 heads, e4m3 916 -> 903. Head dim 64, where
+  // ... and, for head dim 256, Q behind that (see launch_fwd). The S product then fetches only K from shared memory (16 instead
+  // of 48 cycles a reduction step of 32 bytes): 1225 -> 1154 us on 2 x 16384 tokens, 8 heads, e4m3 916 -> 903. Head dim 64, where
   // columns are left too, gains nothing (256 / 254 us on 4 x 4096 tokens, 32/8 heads; 806 / 830 on 4 x 8192, 32 heads).
-  static constexpr bool kTmemHasQ = kHeadDim == 256;
+  static constexpr bool kTmemHasQ = kQInTmem;
   static constexpr int kTmemQ = kTmemO + kQTiles * kHeadDim;
   static_assert(!kTmemHasQ || (kQTiles == 1 && kTmemQ + kHeadDim * kElemBytes / 4 <= 512), "tensor memory budget");
   static constexpr int kPCols = kSubKeys * kElemBytes / 4;            // tensor-memory columns of the packed P
@@ -219,9 +219,9 @@ struct FwdConfig {
 // part in waits and loop control, one elected lane issues, which keeps descriptors and counters in uniform registers.)
 constexpr uint32_t kInfoFirst = 16, kInfoLast = 32, kInfoHalf1 = 64, kInfoStop = 128, kInfoTile0 = 256;  // bit 2 t + h: tile t sees half h
 
-template <int kHeadDim, int kQTiles, int kType, bool kSoftcap>
+template <int kHeadDim, int kQTiles, int kType, bool kSoftcap, bool kQInTmem>
 __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fwd_kernel(const __grid_constant__ FwdParams p) {
-  using Cfg = FwdConfig<kHeadDim, kQTiles, kType, kSoftcap>;
+  using Cfg = FwdConfig<kHeadDim, kQTiles, kType, kSoftcap, kQInTmem>;
   constexpr int kStages = 2 * Cfg::kPairs;         // slot 2 i: K of pair i, slot 2 i + 1: its V
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -777,10 +777,10 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
   if (warp == Cfg::kLoadWarp) ptx::tmem_dealloc(tmem, 512);
 }
 
-template <int kHeadDim, int kQTiles, int kType, bool kSoftcap>
+template <int kHeadDim, int kQTiles, int kType, bool kSoftcap, bool kQInTmem>
 int launch_fwd_instance(const FwdParams& p, int grid, cudaStream_t stream) {
-  using Cfg = FwdConfig<kHeadDim, kQTiles, kType, kSoftcap>;
-  auto kernel = fwd_kernel<kHeadDim, kQTiles, kType, kSoftcap>;
+  using Cfg = FwdConfig<kHeadDim, kQTiles, kType, kSoftcap, kQInTmem>;
+  auto kernel = fwd_kernel<kHeadDim, kQTiles, kType, kSoftcap, kQInTmem>;
   static PerDeviceFlags smem_set;
   const int rc = set_dynamic_smem(kernel, Cfg::kSmemBytes, smem_set);
   if (rc) return rc;
@@ -789,20 +789,20 @@ int launch_fwd_instance(const FwdParams& p, int grid, cudaStream_t stream) {
   return FDA_OK;
 }
 
-template <int kHeadDim, int kQTiles>
+template <int kHeadDim, int kQTiles, bool kQInTmem = false>
 int dispatch_fwd(const FwdParams& p, int grid, bool bf16, bool softcap, cudaStream_t stream) {
   if (bf16) {
-    return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 0, true>(p, grid, stream)
-                   : launch_fwd_instance<kHeadDim, kQTiles, 0, false>(p, grid, stream);
+    return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 0, true, kQInTmem>(p, grid, stream)
+                   : launch_fwd_instance<kHeadDim, kQTiles, 0, false, kQInTmem>(p, grid, stream);
   }
-  return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 1, true>(p, grid, stream)
-                 : launch_fwd_instance<kHeadDim, kQTiles, 1, false>(p, grid, stream);
+  return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 1, true, kQInTmem>(p, grid, stream)
+                 : launch_fwd_instance<kHeadDim, kQTiles, 1, false, kQInTmem>(p, grid, stream);
 }
 
-template <int kHeadDim, int kQTiles>
+template <int kHeadDim, int kQTiles, bool kQInTmem = false>
 int dispatch_fwd_fp8(const FwdParams& p, int grid, bool softcap, cudaStream_t stream) {
-  return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 2, true>(p, grid, stream)
-                 : launch_fwd_instance<kHeadDim, kQTiles, 2, false>(p, grid, stream);
+  return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 2, true, kQInTmem>(p, grid, stream)
+                 : launch_fwd_instance<kHeadDim, kQTiles, 2, false, kQInTmem>(p, grid, stream);
 }
 
 }  // namespace
@@ -921,10 +921,18 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
   }
   const bool bf16 = pr.dtype == FDA_BF16;
   if (fp8) {
-    if (d_round == 256) return dispatch_fwd_fp8<256, 1>(p, grid, softcap, stream);
+    if (d_round == 256) return dispatch_fwd_fp8<256, 1, true>(p, grid, softcap, stream);
     return q_tiles == 2 ? dispatch_fwd_fp8<128, 2>(p, grid, softcap, stream) : dispatch_fwd_fp8<128, 1>(p, grid, softcap, stream);
   }
-  if (d_round == 256) return dispatch_fwd<256, 1>(p, grid, bf16, softcap, stream);
+  if (d_round == 256) {
+    // Q goes to tensor memory once an item, which short items do not earn back. Q in shared / in tensor memory, us, 16/8 heads of
+    // 256, 65536 tokens, blocks of 16, 256 and 1024, by the tokens of a half: 64 779 / 780, 506 / 513, 504 / 511; 192 674 / 678,
+    // 529 / 552, 531 / 554; 320 689 / 690, 596 / 617, 636 / 657; 512 652 / 650, 599 / 611, 712 / 707; 640 694 / 690, 644 / 650, 838 / 834;
+    // 1024 860 / 883, 892 / 852, 1336 / 1327; 4096 2607 / 2507, 2561 / 2437, 2988 / 2829. e4m3, with half the bytes, is within 1.5 %
+    // either way on short ones.
+    if (max_n < 640) return dispatch_fwd<256, 1>(p, grid, bf16, softcap, stream);
+    return dispatch_fwd<256, 1, true>(p, grid, bf16, softcap, stream);
+  }
   if (d_round == 128) {
     return q_tiles == 2 ? dispatch_fwd<128, 2>(p, grid, bf16, softcap, stream) : dispatch_fwd<128, 1>(p, grid, bf16, softcap, stream);
   }

@@ -927,10 +927,11 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
   if (d_round == 256) {
     // Q goes to tensor memory once an item, which short items do not earn back. Q in shared / in tensor memory, us, 16/8 heads of
     // 256, 65536 tokens, blocks of 16, 256 and 1024, by the tokens of a half: 64 779 / 780, 506 / 513, 504 / 511; 192 674 / 678,
-    // 529 / 552, 531 / 554; 320 689 / 690, 596 / 617, 636 / 657; 512 652 / 650, 599 / 611, 712 / 707; 640 694 / 690, 644 / 650, 838 / 834;
+    // 529 / 552, 531 / 554; 320 689 / 690, 596 / 617, 636 / 657; 512 652 / 650, 599 / 611, 712 / 707; 640 694 / 690, 644 / 650, 838 / 834 (one
+    // sample of 624, 16 heads, blocks of 9, with its gradients 130.5 / 129.3);
     // 1024 860 / 883, 892 / 852, 1336 / 1327; 4096 2607 / 2507, 2561 / 2437, 2988 / 2829. e4m3, with half the bytes, is within 1.5 %
     // either way on short ones.
-    if (max_n < 640) return dispatch_fwd<256, 1>(p, grid, bf16, softcap, stream);
+    if (max_n <= 512) return dispatch_fwd<256, 1>(p, grid, bf16, softcap, stream);
     return dispatch_fwd<256, 1, true>(p, grid, bf16, softcap, stream);
   }
   if (d_round == 128) {

@@ -508,7 +508,8 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
         QStep pend{};
         bool have = false;
         const int part_heads = group / split;
-        alive = for_each_qstep(it, d.plan, d.spans, group, d.part * part_heads, (d.part + 1) * part_heads, [&](const QStep& st) -> bool {
+        const int head0 = d.part * part_heads;
+        alive = for_each_qstep(it, d.plan, d.spans, group, head0, head0 + part_heads, [&](const QStep& st) -> bool {
           if (have && !emit(pend, false)) return false;
           pend = st;
           have = true;
@@ -909,7 +910,7 @@ size_t bwd_fused_acc_bytes(const FdaProblem& pr) {
 
 namespace {
 
-constexpr int64_t kMaxPartBytes = 128ll << 20;
+constexpr int64_t kMaxPartBytes = 512ll << 20, kMaxPartBytesMixed = 256ll << 20;
 
 // fp32 dK and dV of `split` parts, in the accumulator's layout
 int64_t part_bytes(const FdaProblem& pr, int split) {
@@ -927,8 +928,8 @@ int64_t part_bytes(const FdaProblem& pr, int split) {
 // 32/8 heads: 416 -> 281, with a chain of at most the share itself, which takes four parts instead of two, 307.)
 // Lengths of packed samples are on the device. What is known of them here, the longest (or a bound of it) and their sum, bounds
 // their steps from below: one sample as long as that, the rest equal. Samples of one length count like a batch of them.
-// All samples are dealt alike, so one long sample among many short ones would need much memory: no more than kMaxPartBytes, of
-// which the cases above take up to a half.
+// All samples are dealt alike, so one long sample among many short ones would need much memory: parts of samples of unlike lengths
+// take kMaxPartBytesMixed at most, others kMaxPartBytes (4 x 6000 tokens, 14/2 heads of 128 need 337 MiB: 1260 -> 995 us).
 // Chains of up to 32 steps stay whole although they would gain too (3 x 666 tokens, 12/4 heads of 96, 18 steps: 66 -> 55 us): the
 // sums of parts round differently, and on small problems the two forms of the backward give the same bits of dK and dV.
 // They stay whole, too, where the convert kernel's grid has no rows left for dK and dV (more than 32700 heads or so).
@@ -938,7 +939,8 @@ int bwd_fused_kv_split(const FdaProblem& pr) {
   const int group = pr.heads_k > 0 ? pr.heads / pr.heads_k : 1;
   if (group <= 1 || pr.batch <= 0) return 1;
   double longest = (pr.seqlen / 2 + kTile - 1) / kTile, all = longest * pr.batch, squares = longest * all;   // in tiles
-  if (pr.cu_seqlens != nullptr && pr.total != static_cast<int64_t>(pr.batch) * pr.seqlen) {
+  const bool one_length = pr.cu_seqlens == nullptr || pr.total == static_cast<int64_t>(pr.batch) * pr.seqlen;
+  if (!one_length) {
     all = pr.total / (2.0 * kTile);
     if (longest > all) longest = all;
     squares = longest * longest + (pr.batch > 1 ? (all - longest) * (all - longest) / (pr.batch - 1) : 0);
@@ -949,7 +951,7 @@ int bwd_fused_kv_split(const FdaProblem& pr) {
   while (split * steps < kLine * longest) {
     int next = split + 1;
     while (next < group && group % next != 0) ++next;
-    if (next > group || part_bytes(pr, next) > kMaxPartBytes) break;
+    if (next > group || part_bytes(pr, next) > (one_length ? kMaxPartBytes : kMaxPartBytesMixed)) break;
     split = next;
   }
   return split;

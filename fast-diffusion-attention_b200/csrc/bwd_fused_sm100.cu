@@ -930,12 +930,15 @@ int64_t part_bytes(const FdaProblem& pr, int split) {
 // their steps from below: one sample as long as that, the rest equal. Samples of one length count like a batch of them.
 // All samples are dealt alike, so one long sample among many short ones would need much memory: parts of samples of unlike lengths
 // take kMaxPartBytesMixed at most, others kMaxPartBytes (4 x 6000 tokens, 14/2 heads of 128 need 337 MiB: 1260 -> 995 us).
+// Where a block is half of the longest sample or more, that chain is shorter and the others are more like it, so that whole chains
+// fill the chip better than the sums above say. Parts then have to save at least 12 of its steps (8 x 1280 tokens, 8/2 heads of 128,
+// blocks of 512: 121 us whole, 143 in parts; 4 x 2000 tokens, 12/4 heads, one block each 202 and 229).
 // Chains of up to 32 steps stay whole although they would gain too (3 x 666 tokens, 12/4 heads of 96, 18 steps: 66 -> 55 us): the
 // sums of parts round differently, and on small problems the two forms of the backward give the same bits of dK and dV.
 // They stay whole, too, where the convert kernel's grid has no rows left for dK and dV (more than 32700 heads or so).
 // sm_margin does not count: it changes no result.
 int bwd_fused_kv_split(const FdaProblem& pr) {
-  constexpr double kLine = 240;   // 2 x 148 / 1.23
+  constexpr double kCtas = 148, kLine = 240;   // 2 x 148 / 1.23
   const int group = pr.heads_k > 0 ? pr.heads / pr.heads_k : 1;
   if (group <= 1 || pr.batch <= 0) return 1;
   double longest = (pr.seqlen / 2 + kTile - 1) / kTile, all = longest * pr.batch, squares = longest * all;   // in tiles
@@ -953,6 +956,12 @@ int bwd_fused_kv_split(const FdaProblem& pr) {
     while (next < group && group % next != 0) ++next;
     if (next > group || part_bytes(pr, next) > (one_length ? kMaxPartBytes : kMaxPartBytesMixed)) break;
     split = next;
+  }
+  const double block = pr.block_size >= pr.seqlen / 2 || pr.block_size / kTile > longest ? longest : pr.block_size / kTile;
+  if (2 * block >= longest) {
+    const double whole = (2 * longest - block) * group;
+    const double share = (steps + pr.heads_k * (one_length ? all : longest) * (block > 2 ? block - 2 : 0)) * group / kCtas;
+    if (whole - (share > whole / split ? share : whole / split) < 12) return 1;
   }
   return split;
 }

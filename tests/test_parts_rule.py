@@ -53,6 +53,39 @@ def test_batches_with_enough_work_stay_whole(heads, heads_k, d, ns, max_n):
     assert parts(heads=heads, heads_k=heads_k, d=d, **_packed(ns, max_n)) == (1, 0)
 
 
+def _whole_without_parts(n, batch, bs, heads_k):
+    """(steps of the longest chain, of all chains) of one query head a group, counted tile pair by tile pair."""
+    tiles, chains = -(-n // 128), []
+    span = [(128 * t, min(128 * t + 128, n)) for t in range(tiles)]
+    for k0, k1 in span:
+        first, last = k0 // bs, (k1 - 1) // bs
+        noisy = sum(q0 // bs <= last and (q1 - 1) // bs >= first for q0, q1 in span)
+        clean = sum((q1 - 1) // bs >= first for q0, q1 in span)
+        cross = sum((q1 - 1) // bs > first for q0, q1 in span)
+        chains += [noisy, clean + cross]
+    return max(chains), sum(chains) * heads_k * batch
+
+
+@pytest.mark.parametrize("bs", [1, 32, 128, 200, 256, 512, 1000, 4096])
+def test_the_rule_follows_the_steps(bs):
+    """Parts where the longest chain is well above a CTA's share of all steps, none where it is well below, and with blocks of half
+    a sample or more only where they save a number of steps."""
+    for n in (300, 1000, 1500, 2048, 4096):
+        for batch in (1, 2, 4, 8):
+            for heads, heads_k in [(8, 2), (32, 8), (12, 4), (8, 1), (32, 1), (14, 2)]:
+                group, tiles = heads // heads_k, -(-n // 128)
+                chain, steps = _whole_without_parts(n, batch, bs, heads_k)
+                got, nbytes = parts(2 * n, heads, heads_k, 64, batch=batch, bs=bs)
+                case = (n, batch, heads, heads_k, chain, steps, got)
+                if 2 * bs >= n:
+                    assert got == 1 or (chain - steps / 148) * group >= 10, case   # the host's count is off by a tile's edges
+                elif bs <= 128:
+                    if steps < 0.8 * 120 * chain and 2 * tiles * group > 32 and group < 30:
+                        assert got > 1, case
+                    if steps > 1.25 * 120 * chain:
+                        assert got == 1, case
+
+
 def test_parts_stay_small():
     rng = random.Random(0)
     seen = set()

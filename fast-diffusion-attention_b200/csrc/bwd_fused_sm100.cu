@@ -16,7 +16,7 @@
 // dP^T (and the tail of the previous step) runs, dS^T while dV runs. The partial dQ^T of a step is added into an fp32
 // accumulator in global memory: the drain warps move it from tensor memory through a small shared-memory staging
 // area and out as 4 KB bulk reductions (cp.reduce.async.bulk add.f32); `bwd_dq_convert_kernel` then scales and
-// rounds the accumulator into dQ.
+// rounds the accumulator into dQ (and, where there are parts, adds up those of dK and dV).
 // Some 20 bytes per clock and SM go towards L2 this way when all SMs do it (5.8 TB/s in a microbenchmark, whatever the
 // instruction), 3300 cycles for the 64 KB of a step, so the drain runs under the next step's products.
 //
@@ -794,8 +794,9 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
 }
 
 // ------------------------------------------------------------------------------------------------------------
-// dQ = round(accumulator * softmax_scale). One block per 64 query rows of a (sample, head, half); stands where the
-// reference converts its accumulator (csrc/fda/flash_bwd_postprocess_kernel.h:160-264 there).
+// dQ = round(accumulator * softmax_scale) and, where the heads of a group were dealt out, dK and dV = rounded sums of the parts
+// (dK scaled too). One block per 64 rows of a (sample, query or KV head, half); stands where the reference converts its
+// accumulator (csrc/fda/flash_bwd_postprocess_kernel.h:160-264 there).
 // ------------------------------------------------------------------------------------------------------------
 template <int kHeadDim, bool kBf16, bool kSoftcap, bool kParts>
 __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const __grid_constant__ BwdParams p) {

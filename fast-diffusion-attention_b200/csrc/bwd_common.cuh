@@ -122,7 +122,9 @@ static_assert(kCols == 32, "one 32-column tensor-memory load per operand and war
 
 // P and dS of kN columns for one thread. `s`/`dp` hold the raw accumulators; the results are packed 16-bit.
 // lse2 (negated) / delta are per column (kPerColumn, read from shared memory) or per thread. kMasked is a template
-// parameter so that the common fully-visible tile carries no per-element compare/select at all.
+// parameter so that the common fully-visible tile carries no per-element compare/select at all. Two elements per instruction
+// wherever there is one (backward and forward of 1 x 8192 tokens, 8 heads of 256: 850 -> 834 us; the single-pass form likewise,
+// 2 x 8192 tokens, 32 heads of 64, capped: 2028 -> 1984).
 template <int kN, bool kBf16, bool kSoftcap, bool kPerColumn, bool kMasked, bool kNeedP, bool kNeedDs = true>
 __device__ __forceinline__ void softmax_backward_cols(const uint32_t* s, const uint32_t* dp, const float* lse2_col,
                                                       const float* delta_col, float lse2_row, float delta_row,
@@ -130,31 +132,31 @@ __device__ __forceinline__ void softmax_backward_cols(const uint32_t* s, const u
                                                       uint32_t* pk_p, uint32_t* pk_ds) {
 #pragma unroll
   for (int c = 0; c < kN; c += 2) {
-    float pv[2], dsv[2];
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int col = c + e;
-      float x = __uint_as_float(s[col]);
-      float dt = 1.f;
-      if (kSoftcap) {
-        x = ptx::tanh_fast(x * softcap_pre);
-        dt = 1.f - x * x;
-      }
-      const float l2 = kPerColumn ? lse2_col[col] : lse2_row;
-      const float dl = kPerColumn ? delta_col[col] : delta_row;
-      float pr = ptx::ex2(fmaf(x, scale_log2, l2));
+    float x0 = __uint_as_float(s[c]), x1 = __uint_as_float(s[c + 1]);
+    if (kSoftcap) {
+      ptx::mul2(x0, x1, x0, x1, softcap_pre, softcap_pre);
+      x0 = ptx::tanh_fast(x0);
+      x1 = ptx::tanh_fast(x1);
+    }
+    const float l0 = kPerColumn ? lse2_col[c] : lse2_row, l1 = kPerColumn ? lse2_col[c + 1] : lse2_row;
+    float y0, y1;
+    ptx::fma2(y0, y1, x0, x1, scale_log2, scale_log2, l0, l1);
+    float p0 = ptx::ex2(y0), p1 = ptx::ex2(y1);
+    float d0 = p0, d1 = p1;
+    if (kNeedDs) {
       // the derivative of the cap goes onto P first: the single-pass backward computes P (1 - tanh^2) in the first
       // half of its arithmetic and meets dP only in the second, and both forms round alike
-      float d = kNeedDs ? (kSoftcap ? pr * dt : pr) * (__uint_as_float(dp[col]) - dl) : 0.f;
-      if (kMasked && (col < lo || col >= hi)) {
-        pr = 0.f;
-        d = 0.f;
-      }
-      pv[e] = pr;
-      dsv[e] = d;
+      if (kSoftcap) ptx::mul2(d0, d1, d0, d1, 1.f - x0 * x0, 1.f - x1 * x1);
+      const float e0 = kPerColumn ? delta_col[c] : delta_row, e1 = kPerColumn ? delta_col[c + 1] : delta_row;
+      float t0, t1;
+      // dP - delta: there is no packed subtraction, the FMA with -1 rounds once like one
+      ptx::fma2(t0, t1, e0, e1, -1.f, -1.f, __uint_as_float(dp[c]), __uint_as_float(dp[c + 1]));
+      ptx::mul2(d0, d1, d0, d1, t0, t1);
     }
-    if (kNeedP) pk_p[c / 2] = ptx::pack2<kBf16>(pv[0], pv[1]);
-    if (kNeedDs) pk_ds[c / 2] = ptx::pack2<kBf16>(dsv[0], dsv[1]);
+    if (kMasked && (c < lo || c >= hi)) { p0 = 0.f; d0 = 0.f; }
+    if (kMasked && (c + 1 < lo || c + 1 >= hi)) { p1 = 0.f; d1 = 0.f; }
+    if (kNeedP) pk_p[c / 2] = ptx::pack2<kBf16>(p0, p1);
+    if (kNeedDs) pk_ds[c / 2] = ptx::pack2<kBf16>(d0, d1);
   }
 }
 

@@ -725,8 +725,9 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
                   float x0 = pr[c], x1 = pr[c + 1];
                   float dt0 = 1.f, dt1 = 1.f;
                   if (kSoftcap) {
-                    x0 = ptx::tanh_fast(x0 * p.softcap_pre);
-                    x1 = ptx::tanh_fast(x1 * p.softcap_pre);
+                    ptx::mul2(x0, x1, x0, x1, p.softcap_pre, p.softcap_pre);
+                    x0 = ptx::tanh_fast(x0);
+                    x1 = ptx::tanh_fast(x1);
                     dt0 = 1.f - x0 * x0;
                     dt1 = 1.f - x1 * x1;
                   }
@@ -736,8 +737,9 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
                   if (kMasked && (c < lo || c >= hi)) v0 = 0.f;
                   if (kMasked && (c + 1 < lo || c + 1 >= hi)) v1 = 0.f;
                   pk[2 * i + j / 2] = ptx::pack2<kBf16>(v0, v1);
-                  pr[c] = kSoftcap ? v0 * dt0 : v0;
-                  pr[c + 1] = kSoftcap ? v1 * dt1 : v1;
+                  if (kSoftcap) ptx::mul2(v0, v1, v0, v1, dt0, dt1);
+                  pr[c] = v0;
+                  pr[c + 1] = v1;
                 }
               }
               // a warp overwrites only columns it has itself already loaded: the 16-bit P^T of 32 queries goes to the

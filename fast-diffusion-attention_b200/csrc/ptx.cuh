@@ -440,6 +440,12 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+// bits 0 .. x - 1 of a word (none for x <= 0, all for x >= 32): element masks, a predicate a bit
+__device__ __forceinline__ uint32_t bits_below(int x) {
+  uint32_t r;
+  asm("shl.b32 %0, 1, %1;" : "=r"(r) : "r"(max(x, 0)));   // shifts of 32 and more give 0
+  return r - 1;
+}
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));

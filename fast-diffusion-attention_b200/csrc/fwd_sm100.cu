@@ -23,6 +23,8 @@
 // Numerics contract kept from the reference: fp32 accumulation, softcap applied before the mask
 // (mainloop_fwd...hpp:679-683), P rounded to the input dtype before P V (:782), row sums accumulated in fp32
 // from the unrounded P, LSE = max * scale + ln(sum) (softmax.h:137-154).
+#include <type_traits>
+
 #include "geometry.h"
 #include "host_util.h"
 #include "ptx.cuh"
@@ -202,6 +204,12 @@ struct FwdConfig {
   static constexpr bool kTmemHasQ = kQInTmem;
   static constexpr int kTmemQ = kTmemO + kQTiles * kHeadDim;
   static_assert(!kTmemHasQ || (kQTiles == 1 && kTmemQ + kHeadDim * kElemBytes / 4 <= 512), "tensor memory budget");
+  // The loop over fully visible sub-steps takes two of them, one a buffer, where that is not too much code: head dim 64 (4 x 8192
+  // tokens, 32 heads: 768 / 753 us; capped 1284 / 1253) and e4m3 (2 x 16384 tokens, 8 heads of 256: 813 / 788; 4 x 8192, 16/4
+  // heads of 128: 531 / 519); 16-bit at 128 loses by it (1 x 16384, 32/8 heads 884 / 913), at 256 too (1081 / 1101).
+  // 16-bit heads of 256, which wait for K and V, get one loop for all (two loops 1 % slower).
+  static constexpr bool kFullLoop = kHeadDim < 256 || kFp8;
+  static constexpr bool kUnrollFull = kHeadDim == 64 || kFp8;
   static constexpr int kPCols = kSubKeys * kElemBytes / 4;            // tensor-memory columns of the packed P
 };
 
@@ -565,14 +573,21 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       float m_run = -INFINITY;  // reference maximum (unscaled scores, or tanh values with softcap)
       float l_run = 0.f;
       bool o_started = false, settled = false;   // one sub-step, two sub-steps of this tile are done
-      int buf = 0;
-      for (int u = 0; u < subs && alive; ++u, buf = buf + 1 == kBufs ? 0 : buf + 1) {
-        int kh, kt;
-        plan.step(u / Cfg::kHalves, kh, kt);
-        const int k0 = kt * Cfg::kSlotKeys + (u % Cfg::kHalves) * kSubKeys;
-        const int cls = spans.classify(kh, k0);
-        if (cls == kTileSkip) continue;
-        if (!ptx::mbar_wait(&s_full[t * kBufs + buf], (s_par >> buf) & 1u, abort_flag, 31)) { alive = false; break; }
+      // The clean keys come first, and the first n_full sub-steps of them this tile sees in full: they have a loop of their own
+      // without classification and mask (1 x 16384 tokens, 32/8 heads of 128: 919 -> 884 us; 4 x 8192, 32 heads of 64: 792 -> 768;
+      // e4m3, 2 x 16384, 8 heads of 256: 850 -> 813).
+      const int n_full = Cfg::kFullLoop ? imin(spans.half[1].hi_first / kSubKeys, plan.n_clean * Cfg::kHalves) : 0;
+      auto sub_step = [&](auto full_tag, int u, const int buf) {
+        constexpr bool kFull = decltype(full_tag)::value;
+        int kh = 1, k0 = 0, cls = kTileFull;
+        if (!kFull) {
+          int kt;
+          plan.step(u / Cfg::kHalves, kh, kt);
+          k0 = kt * Cfg::kSlotKeys + (u % Cfg::kHalves) * kSubKeys;
+          cls = spans.classify(kh, k0);
+          if (cls == kTileSkip) return;
+        }
+        if (!ptx::mbar_wait(&s_full[t * kBufs + buf], (s_par >> buf) & 1u, abort_flag, 31)) { alive = false; return; }
         s_par ^= 1u << buf;
         ptx::tc_fence_after();
         const uint32_t tmem_sb = tmem_s + buf * kSubKeys;
@@ -591,7 +606,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
             v[c + 1] = ptx::tanh_fast(v[c + 1]);
           }
         }
-        if (cls == kTileMasked) {
+        if (!kFull && cls == kTileMasked) {
           int lo, hi;
           if (it.qh == 1) { lo = 0; hi = blk1; }
           else if (kh == 1) { lo = 0; hi = blk0; }
@@ -658,7 +673,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
           if (need) factor = ptx::ex2((m_run - m_new) * scale_log2);
           if (!kLateRescale && o_started) {
             rescale();
-            if (!alive) break;
+            if (!alive) return;
           }
           l_run *= factor;
           if (need) m_run = m_new;
@@ -696,14 +711,27 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
         else ptx::tmem_st16(tmem_sb, pk);
         if (kLateRescale && any_need && o_started) {
           rescale();
-          if (!alive) break;
+          if (!alive) return;
         }
         ptx::tmem_wait_st();
         ptx::tc_fence_before();
         ptx::mbar_arrive_warp(&p_full[t * kBufs + buf]);
         settled = o_started;
         o_started = true;
+      };
+      int u = 0;
+      if (Cfg::kUnrollFull) {
+#pragma unroll 1
+        for (; u + 2 <= n_full && alive; u += 2) {
+          sub_step(std::true_type{}, u, 0);
+          if (alive) sub_step(std::true_type{}, u + 1, 1);
+        }
+      } else {
+#pragma unroll 1
+        for (; u < n_full && alive; ++u) sub_step(std::true_type{}, u, u & 1);
       }
+#pragma unroll 1
+      for (; u < subs && alive; ++u) sub_step(std::false_type{}, u, u & 1);
       if (!alive) break;
       // ---- epilogue: O / l -> global, LSE
       if (!ptx::mbar_wait(&o_full[t], cnt_o & 1, abort_flag, 32)) { alive = false; break; }

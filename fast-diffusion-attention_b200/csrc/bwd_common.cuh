@@ -130,6 +130,8 @@ __device__ __forceinline__ void softmax_backward_cols(const uint32_t* s, const u
                                                       const float* delta_col, float lse2_row, float delta_row,
                                                       float scale_log2, float softcap_pre, int lo, int hi,
                                                       uint32_t* pk_p, uint32_t* pk_ds) {
+  static_assert(kN <= 32, "a word of visible columns");
+  const uint32_t seen = kMasked ? ptx::bits_below(hi) & ~ptx::bits_below(lo) : 0u;
 #pragma unroll
   for (int c = 0; c < kN; c += 2) {
     float x0 = __uint_as_float(s[c]), x1 = __uint_as_float(s[c + 1]);
@@ -153,8 +155,8 @@ __device__ __forceinline__ void softmax_backward_cols(const uint32_t* s, const u
       ptx::fma2(t0, t1, e0, e1, -1.f, -1.f, __uint_as_float(dp[c]), __uint_as_float(dp[c + 1]));
       ptx::mul2(d0, d1, d0, d1, t0, t1);
     }
-    if (kMasked && (c < lo || c >= hi)) { p0 = 0.f; d0 = 0.f; }
-    if (kMasked && (c + 1 < lo || c + 1 >= hi)) { p1 = 0.f; d1 = 0.f; }
+    if (kMasked && !(seen & (1u << c))) { p0 = 0.f; d0 = 0.f; }
+    if (kMasked && !(seen & (2u << c))) { p1 = 0.f; d1 = 0.f; }
     if (kNeedP) pk_p[c / 2] = ptx::pack2<kBf16>(p0, p1);
     if (kNeedDs) pk_ds[c / 2] = ptx::pack2<kBf16>(d0, d1);
   }

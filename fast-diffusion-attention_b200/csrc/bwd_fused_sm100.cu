@@ -715,6 +715,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
 #pragma unroll
             for (int half = 0; half < kChunks; ++half) {
               uint32_t pk[16];
+              const uint32_t seen = kMasked ? ptx::bits_below(hi - 32 * half) & ~ptx::bits_below(lo - 32 * half) : 0u;
 #pragma unroll
               for (int i = 0; i < 8; ++i) {
                 const float4 nl2 = l2v[8 * half + i];
@@ -734,8 +735,8 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
                   float y0, y1;
                   ptx::fma2(y0, y1, x0, x1, p.scale_log2, p.scale_log2, nl2a[j], nl2a[j + 1]);
                   float v0 = ptx::ex2(y0), v1 = ptx::ex2(y1);
-                  if (kMasked && (c < lo || c >= hi)) v0 = 0.f;
-                  if (kMasked && (c + 1 < lo || c + 1 >= hi)) v1 = 0.f;
+                  if (kMasked && !(seen & (1u << (4 * i + j)))) v0 = 0.f;
+                  if (kMasked && !(seen & (2u << (4 * i + j)))) v1 = 0.f;
                   pk[2 * i + j / 2] = ptx::pack2<kBf16>(v0, v1);
                   if (kSoftcap) ptx::mul2(v0, v1, v0, v1, dt0, dt1);
                   pr[c] = v0;

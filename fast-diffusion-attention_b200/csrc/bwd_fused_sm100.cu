@@ -535,11 +535,14 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
     }
   } else if (warp == R::kMmaWarp) {
     // ------------------------------------------------------------------- MMA issuer 1: S^T = K Q^T, dP^T = V dO^T
-    // Two threads issue the MMAs of this kernel, so that the barrier waits and commits of one overlap the MMAs of
-    // the other. S^T of step g + 1 may overwrite P^T of step g once dV has read it (s_free); dP^T of step g + 1
+    // Two warps issue the MMAs of this kernel, so that the barrier waits and commits of one overlap the MMAs of
+    // the other. The whole warp takes part in waits and loop control and one elected lane issues, which keeps descriptors and
+    // counters in uniform registers (with a single thread in the loop every MMA moved them there first: step of packed samples
+    // with blocks of 4, 32/8 heads of 128, 3790 -> 3630 us; 1 x 8192 tokens, 32/8 heads, 1325 -> 1252; 2 x 8192, 32 heads of 64,
+    // capped, 1957 -> 1820). S^T of step g + 1 may overwrite P^T of step g once dV has read it (s_free); dP^T of step g + 1
     // may overwrite dQ^T of step g once the drain warps hold it (dp_free) or, where dQ has its own columns, dP^T of
     // step g once the compute warps hold it (ds_full).
-    if (lane == 0) {
+    {
       constexpr int kFmt = kBf16 ? 1 : 0;
       const uint32_t idesc_s = ptx::make_idesc(kTile, kTile, kFmt, false, false);
       constexpr uint32_t kHi = ptx::smem_desc_hi(1024);
@@ -550,7 +553,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
       uint32_t n_item = 0, g = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = sched_consume<false>(mbox, n_sched, abort_flag);
+        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
         if (idx < 0 || idx >= total_items) break;
         if (!R::kGeometryWarp && !decode_kv_item(p, idx / split).valid) continue;
         if (!ptx::mbar_wait(k_full, n_item & 1, abort_flag, 51)) break;
@@ -559,37 +562,41 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
           const uint32_t slot = g % kSlots, spar = (g / kSlots) & 1u;
           const uint32_t t_off = slot * (T::kTileBytes >> 4);
           if (!ptx::mbar_wait(&q_full[slot], spar, abort_flag, 52)) { alive = false; break; }
-          last = (hdr[4 * slot] & 1) != 0;
+          last = (__shfl_sync(0xffffffffu, hdr[4 * slot], 0) & 1) != 0;
           if (!ptx::mbar_wait(s_free, (g & 1u) ^ 1u, abort_flag, 54)) { alive = false; break; }
           ptx::tc_fence_after();
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kHeadDim / 16; ++kk) {
-            const uint32_t off = ((kk / 4) * T::kPanelBytes + (kk % 4) * 32) >> 4;
-            ptx::umma_ss_f16_lh(tmem + Cfg::kTmemS, k_lo + off, q_lo + t_off + off, kHi, idesc_s, kk > 0);
+            for (int kk = 0; kk < kHeadDim / 16; ++kk) {
+              const uint32_t off = ((kk / 4) * T::kPanelBytes + (kk % 4) * 32) >> 4;
+              ptx::umma_ss_f16_lh(tmem + Cfg::kTmemS, k_lo + off, q_lo + t_off + off, kHi, idesc_s, kk > 0);
+            }
+            ptx::umma_commit(s_full);
           }
-          ptx::umma_commit(s_full);
           const uint32_t dslot = g % kDoSlots;
           if (!ptx::mbar_wait(&do_full[dslot], (g / kDoSlots) & 1u, abort_flag, 56)) { alive = false; break; }
           if (first && !ptx::mbar_wait(v_full, n_item & 1, abort_flag, 69)) { alive = false; break; }
           first = false;
           if (!ptx::mbar_wait(Cfg::kOwnDq ? ds_full : dp_free, (g & 1u) ^ 1u, abort_flag, 58)) { alive = false; break; }
           ptx::tc_fence_after();
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kHeadDim / 16; ++kk) {
-            const uint32_t off = ((kk / 4) * T::kPanelBytes + (kk % 4) * 32) >> 4;
-            ptx::umma_ss_f16_lh(tmem + Cfg::kTmemDP, v_lo + off, do_lo + dslot * (T::kTileBytes >> 4) + off, kHi, idesc_s,
-                                kk > 0);
+            for (int kk = 0; kk < kHeadDim / 16; ++kk) {
+              const uint32_t off = ((kk / 4) * T::kPanelBytes + (kk % 4) * 32) >> 4;
+              ptx::umma_ss_f16_lh(tmem + Cfg::kTmemDP, v_lo + off, do_lo + dslot * (T::kTileBytes >> 4) + off, kHi, idesc_s,
+                                  kk > 0);
+            }
+            ptx::umma_commit(dp_full);
+            ptx::umma_commit(&do_empty[dslot]);
+            if (last) ptx::umma_commit(v_empty);
           }
-          ptx::umma_commit(dp_full);
-          ptx::umma_commit(&do_empty[dslot]);
-          if (last) ptx::umma_commit(v_empty);
         }
         ++n_item;
       }
     }
   } else if (warp == R::kMmaWarp + 1) {
     // -------------------------------------------------- MMA issuer 2: dV += P^T dO, dQ^T = K^T dS^T, dK += dS^T Q
-    if (lane == 0) {
+    {
       constexpr int kFmt = kBf16 ? 1 : 0;
       const uint32_t idesc_g = ptx::make_idesc(kTile, kHeadDim, kFmt, false, true);   // A K-major, B MN-major
       // dQ^T = K^T dS^T or dQ = dS K: A and B MN-major (the reduction runs over key rows)
@@ -604,7 +611,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
       uint32_t g = 0, n_item_b = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = sched_consume<false>(mbox, n_sched, abort_flag);
+        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
         if (idx < 0 || idx >= total_items) break;
         if (!R::kGeometryWarp && !decode_kv_item(p, idx / split).valid) continue;
         bool acc = false;
@@ -615,21 +622,23 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
           const uint32_t slot = g % kSlots, spar = (g / kSlots) & 1u;
           const uint32_t t_off = slot * (T::kTileBytes >> 4);
           if (!ptx::mbar_wait(&q_full[slot], spar, abort_flag, 55)) { alive = false; break; }
-          last = (hdr[4 * slot] & 1) != 0;
+          last = (__shfl_sync(0xffffffffu, hdr[4 * slot], 0) & 1) != 0;
           if (!ptx::mbar_wait(p_full, g & 1u, abort_flag, 53)) { alive = false; break; }
           // dO usually landed long ago (dP^T of this step reads it too), but nothing this thread has waited for so far
           // says so
           if (!ptx::mbar_wait(&do_full[g % kDoSlots], (g / kDoSlots) & 1u, abort_flag, 67)) { alive = false; break; }
           ptx::tc_fence_after();
           // dV += P^T dO: P^T of the 16 queries of reduction step kk sits at column 32 (kk / 2) + 8 (kk % 2)
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kTile / 16; ++kk) {
-            ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS + 32 * (kk / 2) + 8 * (kk % 2),
-                                do_mn + (g % kDoSlots) * (T::kTileBytes >> 4) + kk * (2048 >> 4), kHi, idesc_g,
-                                (acc || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < kTile / 16; ++kk) {
+              ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDV, tmem + Cfg::kTmemS + 32 * (kk / 2) + 8 * (kk % 2),
+                                  do_mn + (g % kDoSlots) * (T::kTileBytes >> 4) + kk * (2048 >> 4), kHi, idesc_g,
+                                  (acc || kk > 0) ? 1u : 0u);
+            }
+            ptx::umma_commit(s_free);
+            ptx::umma_commit(&do_empty[g % kDoSlots]);
           }
-          ptx::umma_commit(s_free);
-          ptx::umma_commit(&do_empty[g % kDoSlots]);
           if (!ptx::mbar_wait(ds_full, g & 1u, abort_flag, 59)) { alive = false; break; }
           ptx::tc_fence_after();
           // dQ before dK: its drain (tensor memory -> registers -> global adds) then runs under dK
@@ -638,26 +647,28 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
             if (!ptx::mbar_wait(dp_free, (g & 1u) ^ 1u, abort_flag, 68)) { alive = false; break; }
             ptx::tc_fence_after();
           }
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kTile / 16; ++kk) {
-            ptx::umma_ss_f16_lh(tmem + Cfg::kTmemDQ, dq_a + kk * (2048 >> 4), dq_b + kk * (2048 >> 4), kHi, idesc_q, kk > 0);
-          }
-          ptx::umma_commit(dq_full);
-          // K is read by S^T (complete for every step of this item by now) and by dQ^T: after the last dQ^T the next
-          // item's K may load. (The rows of dQ^T that come from V at head dim 64, where V may be changing by then, are
-          // the ones nobody reads.)
-          if (last) ptx::umma_commit(k_empty);
+            for (int kk = 0; kk < kTile / 16; ++kk) {
+              ptx::umma_ss_f16_lh(tmem + Cfg::kTmemDQ, dq_a + kk * (2048 >> 4), dq_b + kk * (2048 >> 4), kHi, idesc_q, kk > 0);
+            }
+            ptx::umma_commit(dq_full);
+            // K is read by S^T (complete for every step of this item by now) and by dQ^T: after the last dQ^T the next
+            // item's K may load. (The rows of dQ^T that come from V at head dim 64, where V may be changing by then, are
+            // the ones nobody reads.)
+            if (last) ptx::umma_commit(k_empty);
 #pragma unroll
-          for (int kk = 0; kk < kTile / 16; ++kk) {
-            ptx::umma_ss_f16_lh(tmem + Cfg::kTmemDK, ds_k + (((kk / 4) * Cfg::kDsPanelBytes + (kk % 4) * 32) >> 4),
-                                q_mn + t_off + kk * (2048 >> 4), kHi, idesc_g, (acc || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < kTile / 16; ++kk) {
+              ptx::umma_ss_f16_lh(tmem + Cfg::kTmemDK, ds_k + (((kk / 4) * Cfg::kDsPanelBytes + (kk % 4) * 32) >> 4),
+                                  q_mn + t_off + kk * (2048 >> 4), kHi, idesc_g, (acc || kk > 0) ? 1u : 0u);
+            }
+            ptx::umma_commit(&q_empty[slot]);
+            ptx::umma_commit(ds_free);
           }
           acc = true;
-          ptx::umma_commit(&q_empty[slot]);
-          ptx::umma_commit(ds_free);
         }
         if (!alive) break;
-        ptx::umma_commit(acc_full);
+        if (ptx::elect_one()) ptx::umma_commit(acc_full);
       }
     }
   }

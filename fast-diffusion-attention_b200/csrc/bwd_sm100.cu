@@ -372,11 +372,14 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
     }
   } else if (warp == kMmaWarpB) {
     // ------------------------------------------------------------------- MMA issuer 1: S^T = K Q^T, dP^T = V dO^T
-    // Two threads issue the MMAs of this kernel. The tensor pipe's queue is short, so whatever else an issuing
-    // thread does (barrier waits, commits) leaves the pipe idle; with two issuers one's bookkeeping overlaps the
+    // Two warps issue the MMAs of this kernel, one elected lane of them: with the whole warp in waits and loop control the
+    // descriptors and counters stay in uniform registers (a single thread in the loop moved them there for every MMA; both
+    // kernels of this file, step of 2 x 8192 tokens, 8 heads of 256, 1810 -> 1705 us, of 4 x 4096 tokens, 32/8 heads of 128,
+    // deterministic, 1925 -> 1790). The tensor pipe's queue is short, so whatever else an issuing warp does (barrier waits,
+    // commits) leaves the pipe idle; with two issuers one's bookkeeping overlaps the
     // other's MMAs. Their only mutual dependency is the S^T / dP^T buffer: sub-step g may overwrite buffer g & 1
     // once dV / dK of sub-step g - 2 have read it (buf_free).
-    if (lane == 0) {
+    {
       constexpr int kFmt = kBf16 ? 1 : 0;
       const uint32_t idesc_s = ptx::make_idesc(kTile, kSub, kFmt, false, false);
       constexpr uint32_t kHi = ptx::smem_desc_hi(1024);
@@ -387,7 +390,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       uint32_t n_item = 0, g = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = sched_consume<false>(mbox, n_sched, abort_flag);
+        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
         if (idx < 0 || idx >= total_items) break;
         const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
         if (!it.valid) continue;
@@ -395,7 +398,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         for (bool last = false; alive && !last; ++g) {
           const uint32_t u = g & 1u, qs = g % Cfg::kQSlots, ds = g % Cfg::kDoSlots, ss = g % Cfg::kStatSlots;
           if (!ptx::mbar_wait(&stat_full[ss], (g / Cfg::kStatSlots) & 1u, abort_flag, 52)) { alive = false; break; }
-          last = (*reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset) & 1) != 0;
+          last = (__shfl_sync(0xffffffffu, *reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset), 0) & 1) != 0;
           if (!ptx::mbar_wait(&q_full[qs], (g / Cfg::kQSlots) & 1u, abort_flag, 56)) { alive = false; break; }
           if (!ptx::mbar_wait(&buf_free[u], ((g >> 1) & 1u) ^ 1u, abort_flag, 54)) { alive = false; break; }
           if (Cfg::kPasses == 1 &&
@@ -408,35 +411,41 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
             ptx::umma_ss_f16_lh(tmem + u * 128 + d_off, a_lo + a_off, b_lo + b_off, kHi, idesc_s, kk > 0);
           };
           if (Cfg::kPasses == 1) {
+            if (ptx::elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kHeadDim / 16; ++kk) {
-              product(kk, 0, k_lo, q_lo + q_off);
-              product(kk, 64, v_lo, do_lo + do_off);
+              for (int kk = 0; kk < kHeadDim / 16; ++kk) {
+                product(kk, 0, k_lo, q_lo + q_off);
+                product(kk, 64, v_lo, do_lo + do_off);
+              }
             }
           } else {
+            if (ptx::elect_one()) {
 #pragma unroll
-            for (int kk = 0; kk < kHeadDim / 16; ++kk) product(kk, 0, k_lo, q_lo + q_off);
+              for (int kk = 0; kk < kHeadDim / 16; ++kk) product(kk, 0, k_lo, q_lo + q_off);
+            }
             if (makes_dk(idx)) {
               if (!ptx::mbar_wait(&do_full[ds], (g / Cfg::kDoSlots) & 1u, abort_flag, 58)) { alive = false; break; }
               ptx::tc_fence_after();
+              if (ptx::elect_one()) {
 #pragma unroll
-              for (int kk = 0; kk < kHeadDim / 16; ++kk) product(kk, 64, v_lo, do_lo + do_off);
-              ptx::umma_commit(&do_empty[ds]);   // dK does not read dO
+                for (int kk = 0; kk < kHeadDim / 16; ++kk) product(kk, 64, v_lo, do_lo + do_off);
+                ptx::umma_commit(&do_empty[ds]);   // dK does not read dO
+              }
             } else {
-              ptx::umma_commit(&q_empty[qs]);    // dV does not read Q
+              if (ptx::elect_one()) ptx::umma_commit(&q_empty[qs]);    // dV does not read Q
             }
           }
-          ptx::umma_commit(&sdp_full[u]);
+          if (ptx::elect_one()) ptx::umma_commit(&sdp_full[u]);
         }
         // K and V are read by these products only: the next item's tiles may load while the last dV / dK products
         // and the epilogue of this item still run
-        if (alive) ptx::umma_commit(kv_empty);
+        if (alive && ptx::elect_one()) ptx::umma_commit(kv_empty);
         ++n_item;
       }
     }
   } else if (warp == kMmaWarpB + 1) {
     // ------------------------------------------------------------------- MMA issuer 2: dV += P^T dO, dK += dS^T Q
-    if (lane == 0) {
+    {
       constexpr int kFmt = kBf16 ? 1 : 0;
       const uint32_t idesc_g = ptx::make_idesc(kTile, kHeadDim, kFmt, false, true);
       constexpr uint32_t kHi = ptx::smem_desc_hi(1024);
@@ -445,7 +454,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       uint32_t g = 0, n_item_b = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = sched_consume<false>(mbox, n_sched, abort_flag);
+        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
         if (idx < 0 || idx >= total_items) break;
         const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
         if (!it.valid) continue;
@@ -456,7 +465,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         for (bool last = false; alive && !last; ++g) {
           const uint32_t u = g & 1u, qs = g % Cfg::kQSlots, ds = g % Cfg::kDoSlots, ss = g % Cfg::kStatSlots;
           if (!ptx::mbar_wait(&stat_full[ss], (g / Cfg::kStatSlots) & 1u, abort_flag, 55)) { alive = false; break; }
-          last = (*reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset) & 1) != 0;
+          last = (__shfl_sync(0xffffffffu, *reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset), 0) & 1) != 0;
           if (!ptx::mbar_wait(&pds_full[u], (g >> 1) & 1u, abort_flag, 53)) { alive = false; break; }
           // The tiles this thread's products read. Most have landed long ago, but nothing it has waited for so far says so:
           // that the other issuer saw them land reaches this thread only through its products and the compute warps.
@@ -467,23 +476,25 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
           ptx::tc_fence_after();
           const uint32_t q_off = qs * (Cfg::kSubTileBytes >> 4), do_off = ds * (Cfg::kSubTileBytes >> 4);
           const uint32_t st_t = tmem + u * 128, dpt_t = tmem + u * 128 + 64;
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kSub / 16; ++kk) {
-            const uint32_t on = (acc || kk > 0) ? 1u : 0u;
-            if (makes_dv(idx)) {
-              ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDV, st_t + kk * kSubCols, do_mn + do_off + kk * (2048 >> 4), kHi, idesc_g, on);
+            for (int kk = 0; kk < kSub / 16; ++kk) {
+              const uint32_t on = (acc || kk > 0) ? 1u : 0u;
+              if (makes_dv(idx)) {
+                ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDV, st_t + kk * kSubCols, do_mn + do_off + kk * (2048 >> 4), kHi, idesc_g, on);
+              }
+              if (makes_dk(idx)) {
+                ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDK, dpt_t + kk * kSubCols, q_mn + q_off + kk * (2048 >> 4), kHi, idesc_g, on);
+              }
             }
-            if (makes_dk(idx)) {
-              ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDK, dpt_t + kk * kSubCols, q_mn + q_off + kk * (2048 >> 4), kHi, idesc_g, on);
-            }
+            ptx::umma_commit(&buf_free[u]);
+            if (makes_dk(idx)) ptx::umma_commit(&q_empty[qs]);
+            if (makes_dv(idx)) ptx::umma_commit(&do_empty[ds]);
           }
           acc = true;
-          ptx::umma_commit(&buf_free[u]);
-          if (makes_dk(idx)) ptx::umma_commit(&q_empty[qs]);
-          if (makes_dv(idx)) ptx::umma_commit(&do_empty[ds]);
         }
         if (!alive) break;
-        ptx::umma_commit(acc_full);
+        if (ptx::elect_one()) ptx::umma_commit(acc_full);
       }
     }
   }
@@ -753,10 +764,10 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
     }
   } else if (warp == kMmaWarpB) {
     // ------------------------------------------------------------------ MMA issuer 1: S = Q K^T and dP = dO V^T
-    // As in the dK/dV kernel two threads issue MMAs, so that the barrier waits of one overlap the MMAs of the
+    // As in the dK/dV kernel two warps issue MMAs, so that the barrier waits of one overlap the MMAs of the
     // other. They share nothing but the compute warps between them: S / dP of step j + 1 may start as soon as the
     // compute warps have S / dP of step j in registers, whatever the state of dQ.
-    if (lane == 0) {
+    {
       constexpr int kFmt = kBf16 ? 1 : 0;
       const uint32_t idesc_s = ptx::make_idesc(kTile, Cfg::kKeys, kFmt, false, false);
       constexpr uint32_t kHi = ptx::smem_desc_hi(1024);
@@ -766,7 +777,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
       uint32_t n_item = 0, step = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = sched_consume<false>(mbox, n_sched, abort_flag);
+        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
         if (idx < 0 || idx >= total_items) break;
         const QItem it = decode_q_item(p, idx);
         if (!it.valid) continue;
@@ -786,26 +797,28 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
           if (!ptx::mbar_wait(&kv_full[vs], Cfg::v_parity(step), abort_flag, 84)) { alive = false; break; }
           if (!ptx::mbar_wait(sdp_free, (step & 1) ^ 1, abort_flag, 82)) { alive = false; break; }
           ptx::tc_fence_after();
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kHeadDim / 16; ++kk) {
-            const uint32_t a_off = ((kk / 4) * T::kPanelBytes + (kk % 4) * 32) >> 4;
-            const uint32_t b_off = ((kk / 4) * Cfg::kKvPanelBytes + (kk % 4) * 32) >> 4;
-            ptx::umma_ss_f16_lh(tmem + Cfg::kTmemS, q_lo + a_off, kv_lo_k + ks * (Cfg::kKvTileBytes >> 4) + b_off, kHi,
-                                idesc_s, kk > 0);
-            ptx::umma_ss_f16_lh(tmem + Cfg::kTmemDP, do_lo + a_off, kv_lo_k + vs * (Cfg::kKvTileBytes >> 4) + b_off, kHi,
-                                idesc_s, kk > 0);
+            for (int kk = 0; kk < kHeadDim / 16; ++kk) {
+              const uint32_t a_off = ((kk / 4) * T::kPanelBytes + (kk % 4) * 32) >> 4;
+              const uint32_t b_off = ((kk / 4) * Cfg::kKvPanelBytes + (kk % 4) * 32) >> 4;
+              ptx::umma_ss_f16_lh(tmem + Cfg::kTmemS, q_lo + a_off, kv_lo_k + ks * (Cfg::kKvTileBytes >> 4) + b_off, kHi,
+                                  idesc_s, kk > 0);
+              ptx::umma_ss_f16_lh(tmem + Cfg::kTmemDP, do_lo + a_off, kv_lo_k + vs * (Cfg::kKvTileBytes >> 4) + b_off, kHi,
+                                  idesc_s, kk > 0);
+            }
+            ptx::umma_commit(sdp_full);
+            ptx::umma_commit(&kv_empty[vs]);  // V tile no longer needed
           }
-          ptx::umma_commit(sdp_full);
-          ptx::umma_commit(&kv_empty[vs]);  // V tile no longer needed
         }
         // Q and dO are read by these products only: the tiles of the next item may load while the last dQ
         // product and the epilogue of this one still run
-        if (alive) ptx::umma_commit(q_empty);
+        if (alive && ptx::elect_one()) ptx::umma_commit(q_empty);
       }
     }
   } else if (warp == kMmaWarpB + 1) {
     // ------------------------------------------------------------------------------ MMA issuer 2: dQ += dS K
-    if (lane == 0) {
+    {
       constexpr int kFmt = kBf16 ? 1 : 0;
       const uint32_t idesc_g = ptx::make_idesc(kTile, kHeadDim, kFmt, false, true);
       constexpr uint32_t kHi = ptx::smem_desc_hi(1024);
@@ -813,7 +826,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
       uint32_t step = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = sched_consume<false>(mbox, n_sched, abort_flag);
+        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
         if (idx < 0 || idx >= total_items) break;
         const QItem it = decode_q_item(p, idx);
         if (!it.valid) continue;
@@ -832,17 +845,19 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
           if (!ptx::mbar_wait(ds_full, step & 1, abort_flag, 85)) { alive = false; break; }
           ptx::tc_fence_after();
           // dQ += dS K: the packed dS pieces of the compute warpgroups lie side by side, 8 columns per 16 keys
+          if (ptx::elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < Cfg::kKeys / 16; ++kk) {
-            ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDQ, tmem + Cfg::kTmemDS + kk * 8,
-                                kv_lo_mn + ks * (Cfg::kKvTileBytes >> 4) + kk * (2048 >> 4), kHi, idesc_g,
-                                (j > 0 || kk > 0) ? 1u : 0u);
+            for (int kk = 0; kk < Cfg::kKeys / 16; ++kk) {
+              ptx::umma_ts_f16_lh(tmem + Cfg::kTmemDQ, tmem + Cfg::kTmemDS + kk * 8,
+                                  kv_lo_mn + ks * (Cfg::kKvTileBytes >> 4) + kk * (2048 >> 4), kHi, idesc_g,
+                                  (j > 0 || kk > 0) ? 1u : 0u);
+            }
+            ptx::umma_commit(&kv_empty[ks]);
+            ptx::umma_commit(ds_free);
           }
-          ptx::umma_commit(&kv_empty[ks]);
-          ptx::umma_commit(ds_free);
         }
         if (!alive) break;
-        ptx::umma_commit(dq_full);
+        if (ptx::elect_one()) ptx::umma_commit(dq_full);
       }
     }
   }

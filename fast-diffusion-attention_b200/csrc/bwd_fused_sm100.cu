@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
   FusedItem* items = reinterpret_cast<FusedItem*>(reinterpret_cast<uint8_t*>(bars) + 448);   // [2], like the mailbox
   static_assert(sizeof(SchedMailbox) <= 64 && 2 * sizeof(FusedItem) <= 320, "mailbox and item descriptions");
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   if ((ptx::smem_u32(smem) & 1023u) != 0) {
     if (threadIdx.x == 0 && atomicCAS(&g_fda_status[0], 0, 120) == 0) {
       g_fda_status[1] = static_cast<int>(blockIdx.x);
@@ -242,7 +242,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int group = p.heads / p.heads_k;
   const int split = kParts ? p.kv_split : 1;   // CTAs that share a key tile
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
       uint32_t n_item = 0, g = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
+        const int idx = ptx::uniform(sched_consume<true>(mbox, n_sched, abort_flag));
         if (idx < 0 || idx >= total_items) break;
         if (!R::kGeometryWarp && !decode_kv_item(p, idx / split).valid) continue;
         if (!ptx::mbar_wait(k_full, n_item & 1, abort_flag, 51)) break;
@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
           const uint32_t slot = g % kSlots, spar = (g / kSlots) & 1u;
           const uint32_t t_off = slot * (T::kTileBytes >> 4);
           if (!ptx::mbar_wait(&q_full[slot], spar, abort_flag, 52)) { alive = false; break; }
-          last = (__shfl_sync(0xffffffffu, hdr[4 * slot], 0) & 1) != 0;
+          last = (ptx::uniform(hdr[4 * slot]) & 1) != 0;
           if (!ptx::mbar_wait(s_free, (g & 1u) ^ 1u, abort_flag, 54)) { alive = false; break; }
           ptx::tc_fence_after();
           if (ptx::elect_one()) {
@@ -611,7 +611,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
       uint32_t g = 0, n_item_b = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
+        const int idx = ptx::uniform(sched_consume<true>(mbox, n_sched, abort_flag));
         if (idx < 0 || idx >= total_items) break;
         if (!R::kGeometryWarp && !decode_kv_item(p, idx / split).valid) continue;
         bool acc = false;
@@ -622,7 +622,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
           const uint32_t slot = g % kSlots, spar = (g / kSlots) & 1u;
           const uint32_t t_off = slot * (T::kTileBytes >> 4);
           if (!ptx::mbar_wait(&q_full[slot], spar, abort_flag, 55)) { alive = false; break; }
-          last = (__shfl_sync(0xffffffffu, hdr[4 * slot], 0) & 1) != 0;
+          last = (ptx::uniform(hdr[4 * slot]) & 1) != 0;
           if (!ptx::mbar_wait(p_full, g & 1u, abort_flag, 53)) { alive = false; break; }
           // dO usually landed long ago (dP^T of this step reads it too), but nothing this thread has waited for so far
           // says so

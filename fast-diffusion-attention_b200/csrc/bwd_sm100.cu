@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   SchedMailbox* mbox = reinterpret_cast<SchedMailbox*>(reinterpret_cast<uint8_t*>(bars) + 384);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   if ((ptx::smem_u32(smem) & 1023u) != 0) {
     if (threadIdx.x == 0 && atomicCAS(&g_fda_status[0], 0, 120) == 0) {
       g_fda_status[1] = static_cast<int>(blockIdx.x);
@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int group = p.heads / p.heads_k;
   const int total_items = kv_item_count(p) * Cfg::kPasses;
@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       uint32_t n_item = 0, g = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
+        const int idx = ptx::uniform(sched_consume<true>(mbox, n_sched, abort_flag));
         if (idx < 0 || idx >= total_items) break;
         const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
         if (!it.valid) continue;
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         for (bool last = false; alive && !last; ++g) {
           const uint32_t u = g & 1u, qs = g % Cfg::kQSlots, ds = g % Cfg::kDoSlots, ss = g % Cfg::kStatSlots;
           if (!ptx::mbar_wait(&stat_full[ss], (g / Cfg::kStatSlots) & 1u, abort_flag, 52)) { alive = false; break; }
-          last = (__shfl_sync(0xffffffffu, *reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset), 0) & 1) != 0;
+          last = (ptx::uniform(*reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset)) & 1) != 0;
           if (!ptx::mbar_wait(&q_full[qs], (g / Cfg::kQSlots) & 1u, abort_flag, 56)) { alive = false; break; }
           if (!ptx::mbar_wait(&buf_free[u], ((g >> 1) & 1u) ^ 1u, abort_flag, 54)) { alive = false; break; }
           if (Cfg::kPasses == 1 &&
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       uint32_t g = 0, n_item_b = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
+        const int idx = ptx::uniform(sched_consume<true>(mbox, n_sched, abort_flag));
         if (idx < 0 || idx >= total_items) break;
         const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
         if (!it.valid) continue;
@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         for (bool last = false; alive && !last; ++g) {
           const uint32_t u = g & 1u, qs = g % Cfg::kQSlots, ds = g % Cfg::kDoSlots, ss = g % Cfg::kStatSlots;
           if (!ptx::mbar_wait(&stat_full[ss], (g / Cfg::kStatSlots) & 1u, abort_flag, 55)) { alive = false; break; }
-          last = (__shfl_sync(0xffffffffu, *reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset), 0) & 1) != 0;
+          last = (ptx::uniform(*reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset)) & 1) != 0;
           if (!ptx::mbar_wait(&pds_full[u], (g >> 1) & 1u, abort_flag, 53)) { alive = false; break; }
           // The tiles this thread's products read. Most have landed long ago, but nothing it has waited for so far says so:
           // that the other issuer saw them land reaches this thread only through its products and the compute warps.
@@ -687,7 +687,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   SchedMailbox* mbox = reinterpret_cast<SchedMailbox*>(reinterpret_cast<uint8_t*>(bars) + 256);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = ptx::uniform(static_cast<int>(threadIdx.x >> 5)), lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     *abort_flag = 0;
     sched_init(mbox, 4 * kCmpWG + 2);
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int total_items = (p.vl.base != nullptr ? p.vl.base[0] : p.tiles_per_half * p.batch) * 2 * p.heads;
 
@@ -777,7 +777,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
       uint32_t n_item = 0, step = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
+        const int idx = ptx::uniform(sched_consume<true>(mbox, n_sched, abort_flag));
         if (idx < 0 || idx >= total_items) break;
         const QItem it = decode_q_item(p, idx);
         if (!it.valid) continue;
@@ -826,7 +826,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
       uint32_t step = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = __shfl_sync(0xffffffffu, sched_consume<true>(mbox, n_sched, abort_flag), 0);
+        const int idx = ptx::uniform(sched_consume<true>(mbox, n_sched, abort_flag));
         if (idx < 0 || idx >= total_items) break;
         const QItem it = decode_q_item(p, idx);
         if (!it.valid) continue;

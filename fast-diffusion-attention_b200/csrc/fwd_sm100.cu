@@ -253,7 +253,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
   ItemDesc* desc = reinterpret_cast<ItemDesc*>(reinterpret_cast<uint8_t*>(bars) + 512);  // two slots
   static_assert(Cfg::kMmaWarp + kQTiles <= Cfg::kThreads / 32 && sizeof(SchedMailbox) <= 192 && 2 * sizeof(ItemDesc) <= 512, "mailbox and item descriptions");
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = ptx::uniform(static_cast<int>(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
   const int total_items = p.vl.base != nullptr ? p.vl.base[0] * 2 * p.heads : p.total_items;
 
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
 
   // The register counts are set inside the role branches: after a point where the branches meet again the
@@ -391,7 +391,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
     constexpr uint32_t kIdescS = ptx::make_idesc(kBlockM, kSubKeys, kFmt, false, false);
     constexpr uint32_t kIdescO = ptx::make_idesc(kBlockM, kHeadDim, kFmt, false, true);
     constexpr uint32_t kDescHi = ptx::smem_desc_hi(1024);
-    const int t = __shfl_sync(0xffffffffu, warp, 0) - Cfg::kMmaWarp;
+    const int t = warp - Cfg::kMmaWarp;
     // descriptor low words of slot 0; a slot adds its bytes / 16, a k-step a constant
     const uint32_t q_lo = ptx::smem_desc_lo(ptx::smem_u32(sQ), 16) + t * (Cfg::kTileBytes >> 4);
     const uint32_t k_lo0 = ptx::smem_desc_lo(ptx::smem_u32(sKV), 16);
@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
 
     while (alive) {
       if (!ptx::mbar_wait(&kv_full[2 * pair], par, abort_flag, 22)) break;
-      const uint32_t info = __shfl_sync(0xffffffffu, slot_info[pair], 0);
+      const uint32_t info = ptx::uniform(slot_info[pair]);
       if (info & kInfoStop) break;
       if (info & kInfoFirst) {
         if (!ptx::mbar_wait(q_full, q_par, abort_flag, 21)) break;
@@ -515,12 +515,19 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
   } else {
     // ------------------------------------------------------------------------------------ softmax + epilogue
     if (Cfg::kRegRealloc) ptx::reg_acquire_to<Cfg::kSoftmaxRegs>();
-    const int t = warp >> 2;                       // query tile of this warpgroup
-    const int quad = warp & 3;                     // tensor-memory lane quadrant of this warp
+    // Loop bounds and addresses in uniform registers: one query tile and e4m3 (2 x 16384 tokens, 8 heads of 256, e4m3: 788 -> 765
+    // us; 32 x 512, 16/8 heads of 256, 138 -> 133). With two tiles of 16 bits they are better where the compiler puts them from a
+    // plain warp number (4 x 8192 tokens, 32 heads of 64: 771 / 744 us; 1 x 16384, 32/8 heads of 128 872 / 862).
+    constexpr bool kUniform = Cfg::kFp8 || kQTiles == 1;
+    auto uni = [](auto x) { return kUniform ? ptx::uniform(x) : x; };
+    const int own_warp = uni(static_cast<int>(threadIdx.x >> 5));
+    const uint32_t tmem_own = uni(*reinterpret_cast<volatile uint32_t*>(tmem_slot));
+    const int t = own_warp >> 2;                   // query tile of this warpgroup
+    const int quad = own_warp & 3;                     // tensor-memory lane quadrant of this warp
     const int row = quad * 32 + lane;              // row inside the tile
     const uint32_t lane_addr = static_cast<uint32_t>(quad * 32) << 16;
-    const uint32_t tmem_s = tmem + t * kBufs * kSubKeys + lane_addr;
-    const uint32_t tmem_o = tmem + Cfg::kTmemO + t * kHeadDim + lane_addr;
+    const uint32_t tmem_s = tmem_own + t * kBufs * kSubKeys + lane_addr;
+    const uint32_t tmem_o = tmem_own + Cfg::kTmemO + t * kHeadDim + lane_addr;
     uint32_t s_par = 0;   // bit b: parity of the next S in buffer b
     uint32_t cnt_o = 0;
     bool alive = true;
@@ -535,7 +542,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       if (!it.valid) continue;
       const int ta = it.qa + t * kBlockM;
       if (ta >= it.qb) continue;
-      const int subs = plan.steps() * Cfg::kHalves;
+      const int subs = uni(plan.steps() * Cfg::kHalves);
       const int r = ta + row;                      // position in the half
       const bool row_valid = r < it.n;
       const int r_eff = row_valid ? r : it.n - 1;
@@ -576,7 +583,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       // The clean keys come first, and the first n_full sub-steps of them this tile sees in full: they have a loop of their own
       // without classification and mask (1 x 16384 tokens, 32/8 heads of 128: 919 -> 884 us; 4 x 8192, 32 heads of 64: 792 -> 768;
       // e4m3, 2 x 16384, 8 heads of 256: 850 -> 813).
-      const int n_full = Cfg::kFullLoop ? imin(spans.half[1].hi_first / kSubKeys, plan.n_clean * Cfg::kHalves) : 0;
+      const int n_full = Cfg::kFullLoop ? uni(imin(spans.half[1].hi_first / kSubKeys, plan.n_clean * Cfg::kHalves)) : 0;
       auto sub_step = [&](auto full_tag, int u, const int buf) {
         constexpr bool kFull = decltype(full_tag)::value;
         int kh = 1, k0 = 0, cls = kTileFull;

@@ -33,6 +33,11 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// The value of lane 0, for values that are the same in every lane: what is computed from the result (loop control, barrier and
+// tensor-memory addresses) can then stay in uniform registers.
+__device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
+__device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
+
 // ---- mbarrier -------------------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

@@ -98,14 +98,6 @@ struct FusedRoles {
   static_assert(128 * (kCmpWG * kComputeRegs + kProducerRegs + kDrainRegs) <= kThreads * kLaunchRegs, "register pool");
 };
 
-// Rows of the dQ accumulator come in blocks of 64. Every half of every sample starts at its own block: the
-// "+ 2 b + qh" gives each of the 2 * batch halves one block of slack, so rounding the start down never lets two
-// halves share a block. Returns the first accumulator row of query row `qa` (a multiple of 64) of half `qh` of a
-// sample whose first row in the packed row space is `grow0`.
-__device__ __forceinline__ int acc_row_of(int grow0, int n, int b, int qh, int qa) {
-  return ((grow0 + qh * n) / 64 + 2 * b + qh) * 64 + qa;
-}
-
 // One step of an item: a visible 128-row query tile of one query head. At most `left` steps follow it.
 struct QStep {
   int h, qh, qa, cls, left;
@@ -919,7 +911,7 @@ int64_t bwd_fused_acc_tiles(const FdaProblem& pr) {
 }
 
 size_t bwd_fused_acc_bytes(const FdaProblem& pr) {
-  const int d_round = pr.head_dim <= 64 ? 64 : 128;
+  const int d_round = pr.head_dim <= 64 ? 64 : pr.head_dim <= 128 ? 128 : 256;
   return static_cast<size_t>(pr.heads) * bwd_fused_acc_tiles(pr) * 64 * d_round * 4;
 }
 
@@ -934,6 +926,45 @@ int64_t part_bytes(const FdaProblem& pr, int split) {
 }
 
 }  // namespace
+
+namespace {
+
+// What the host knows of the samples, in tiles: the longest, their sum, the sum of their squares (bounded from below where packed
+// samples are not all as long as max_seqlen says: one sample as long as that, the rest equal). Returns whether they are.
+bool known_tiles(const FdaProblem& pr, double& longest, double& all, double& squares) {
+  longest = (pr.seqlen / 2 + kTile - 1) / kTile;
+  all = longest * pr.batch;
+  squares = longest * all;
+  const bool one_length = pr.cu_seqlens == nullptr || pr.total == static_cast<int64_t>(pr.batch) * pr.seqlen;
+  if (!one_length) {
+    all = pr.total / (2.0 * kTile);
+    if (longest > all) longest = all;
+    squares = longest * longest + (pr.batch > 1 ? (all - longest) * (all - longest) / (pr.batch - 1) : 0);
+  }
+  return one_length;
+}
+
+// The longest chain, 2 x longest steps of a query head, is at most 1.23 times a CTA's share of all steps where these are at least
+// kLine x longest (kLine = 2 x 148 / 1.23).
+constexpr double kLine = 240;
+
+}  // namespace
+
+// Whether heads wider than 128 take bwd_wide_kernel and the dV kernel instead of the split form's three passes. Its key tiles are
+// chains over all query heads of a group (the dQ kernel has an item for each head and query tile), so the longest must not be more
+// than a CTA's share, as above; and short items pay for the copy of V and the wait for the last dQ^T. Backward, split / this, us, heads
+// of 256, blocks of 16 and 512: 16 x 1000 tokens, 8 heads 320 / 365 and 403 / 427; 12 x 1536 432 / 448 and 497 / 480; 8 x 2000
+// 449 / 415 and 530 / 457, 16/8 heads 812 / 848 and 994 / 953; 5 x 3000, 8 heads 541 / 466 and 606 / 510, 16/8 1004 / 948 and
+// 1179 / 1050, 16/4 1095 / 1008 and 1169 / 1069; 2 x 8192, 8 heads 1202 / 964 and 1257 / 1029. Longest chain above the share: 4 x
+// 4096, 8/1 heads 1058 / 1690; 1 x 8192, 16/4 1374 / 2219.
+bool bwd_wide_pays(const FdaProblem& pr) {
+  constexpr int kTokens = 1400;   // of a half, of the longest sample and on average
+  if (pr.heads_k <= 0 || pr.batch <= 0 || pr.seqlen / 2 < kTokens || pr.total / 2 < static_cast<int64_t>(pr.batch) * kTokens) return false;
+  if (convert_rows(pr.heads, pr.heads_k, false) > kMaxGridY) return false;
+  double longest, all, squares;
+  known_tiles(pr, longest, all, squares);
+  return pr.heads_k * (squares + 2 * all) >= kLine * longest;
+}
 
 // Parts into which the query heads of a group are dealt. A key tile's steps are a chain, and those of the longest sample's first
 // clean tile (2 x tiles x group, with tiles = n / 128) are more than a CTA's share of all steps (tiles (tiles + 2) x group for
@@ -953,16 +984,11 @@ int64_t part_bytes(const FdaProblem& pr, int split) {
 // They stay whole, too, where the convert kernel's grid has no rows left for dK and dV (more than 32700 heads or so).
 // sm_margin does not count: it changes no result.
 int bwd_fused_kv_split(const FdaProblem& pr) {
-  constexpr double kCtas = 148, kLine = 240;   // 2 x 148 / 1.23
+  constexpr double kCtas = 148;
   const int group = pr.heads_k > 0 ? pr.heads / pr.heads_k : 1;
   if (group <= 1 || pr.batch <= 0) return 1;
-  double longest = (pr.seqlen / 2 + kTile - 1) / kTile, all = longest * pr.batch, squares = longest * all;   // in tiles
-  const bool one_length = pr.cu_seqlens == nullptr || pr.total == static_cast<int64_t>(pr.batch) * pr.seqlen;
-  if (!one_length) {
-    all = pr.total / (2.0 * kTile);
-    if (longest > all) longest = all;
-    squares = longest * longest + (pr.batch > 1 ? (all - longest) * (all - longest) / (pr.batch - 1) : 0);
-  }
+  double longest, all, squares;
+  const bool one_length = known_tiles(pr, longest, all, squares);
   if (2 * longest * group <= 32 || convert_rows(pr.heads, pr.heads_k, true) > kMaxGridY) return 1;
   const double steps = pr.heads_k * (squares + 2 * all);   // of one query head of each group
   int split = 1;
@@ -991,6 +1017,15 @@ int launch_bwd_fused(const BwdParams& p, int d_round, bool bf16, bool softcap, i
                      cudaStream_t stream) {
   return p.kv_split > 1 ? dispatch_fused<true>(p, d_round, bf16, softcap, sm_count, stages, stream)
                         : dispatch_fused<false>(p, d_round, bf16, softcap, sm_count, stages, stream);
+}
+
+// The convert kernel of head dims above 128 (bwd_wide_sm100.cu).
+int launch_wide_convert(const BwdParams& p, bool bf16, cudaStream_t stream) {
+  dim3 grid(p.n_pad / 64, convert_rows(p.heads, p.heads_k, false), p.batch);
+  if (bf16) bwd_dq_convert_kernel<256, true, false, false><<<grid, 256, 0, stream>>>(p);
+  else bwd_dq_convert_kernel<256, false, false, false><<<grid, 256, 0, stream>>>(p);
+  FDA_CUDA_TRY(cudaGetLastError());
+  return FDA_OK;
 }
 
 int read_status_bwd_fused(int32_t* out4) {

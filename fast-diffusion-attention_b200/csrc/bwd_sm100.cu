@@ -124,7 +124,8 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
 // 2. dK / dV
 // ------------------------------------------------------------------------------------------------------------
 
-template <int kHeadDim, int kStages>
+// kDvOnly (head dims above 128): dV items only, dK is made with dQ (bwd_wide_sm100.cu).
+template <int kHeadDim, int kStages, bool kDvOnly>
 struct DkdvCfg {
   using T = TileCfg<kHeadDim>;
   static constexpr int kSubTileBytes = kSub * kHeadDim * 2;     // Q or dO sub-tile
@@ -136,17 +137,21 @@ struct DkdvCfg {
   // both instead takes S^T and dP^T twice, six products for five. (Backward of 2 x 16384 tokens, 8 heads of 256, blocks of
   // 256: 7.34 -> 4.97 ms with the rings below.)
   static constexpr int kPasses = kHeadDim > 128 ? 2 : 1;
+  static constexpr int kItems = kDvOnly ? 1 : kPasses;   // a key tile
+  static_assert(!kDvOnly || kPasses == 2, "head dims above 128");
   static constexpr int kTmemDK = 256, kTmemDV = kPasses == 2 ? 256 : 256 + kHeadDim;
   static_assert(kTmemDV + kHeadDim <= 512, "tensor memory budget");
   // Rings of Q and dO sub-tiles of their own. With 128 KB of K and V there is room for three of 32 KB: two for Q, one for
   // dO, so that the next sub-step's tiles load while this one's are in use (one slot for both left the pipe waiting for
   // every load).
-  static constexpr int kQSlots = kPasses == 2 ? 2 : kStages, kDoSlots = kPasses == 2 ? 1 : kStages;
+  // Without dK nobody reads V, and dO gets three slots: with one, a dV product waited for the load
+  // behind the last (2 x 16384 tokens, 8 heads of 256: 1346 -> 934 us for dV).
+  static constexpr int kQSlots = kPasses == 2 ? 2 : kStages, kDoSlots = kDvOnly ? 3 : kPasses == 2 ? 1 : kStages;
   // lse2[64], delta[64] and the header of a sub-step. The slot of step x is written when Q of step x - 2 is done with,
   // which for dV means S^T of x - 2 complete, so that step x - 4 is the last that every role has certainly left.
   static constexpr int kStatSlots = kPasses == 2 ? 4 : kStages;
   static constexpr int kHeaderOffset = 2 * kSub * 4, kStatBytes = kHeaderOffset + 32;
-  static constexpr int kOffQ = 2 * T::kTileBytes, kOffDo = kOffQ + kQSlots * kSubTileBytes;
+  static constexpr int kOffQ = (kDvOnly ? 1 : 2) * T::kTileBytes, kOffDo = kOffQ + kQSlots * kSubTileBytes;
   static constexpr int kOffStat = kOffDo + kDoSlots * kSubTileBytes;
   static constexpr int kOffBar = kOffStat + kStatSlots * kStatBytes;
   static constexpr int kSmemBytes = kOffBar + 512;
@@ -156,9 +161,9 @@ struct DkdvCfg {
 
 // One CTA per SM. A sub-step is one 64-row half of a visible 128-row query tile of one query head of the group; a half with
 // no visible row is skipped.
-template <int kHeadDim, int kStages, bool kBf16, bool kSoftcap>
+template <int kHeadDim, int kStages, bool kBf16, bool kSoftcap, bool kDvOnly>
 __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_constant__ BwdParams p) {
-  using Cfg = DkdvCfg<kHeadDim, kStages>;
+  using Cfg = DkdvCfg<kHeadDim, kStages, kDvOnly>;
   using T = TileCfg<kHeadDim>;
   // The tiles need 1024-byte alignment for the 128-byte swizzle. Dynamic shared memory starts at the beginning of the
   // block's window, which is aligned that far; head dimension 256 leaves no room to round the base up, so a base that is
@@ -229,35 +234,10 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
   const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int group = p.heads / p.heads_k;
-  const int total_items = kv_item_count(p) * Cfg::kPasses;
+  const int total_items = kv_item_count(p) * Cfg::kItems;
   // what the item with this index makes
-  auto makes_dk = [](int idx) { return Cfg::kPasses == 1 || (idx & 1) == 0; };
-  auto makes_dv = [](int idx) { return Cfg::kPasses == 1 || (idx & 1) == 1; };
-
-  // Calls fn(SubStep) for every non-skipped sub-step of the item, in order; stops early when fn returns false.
-  auto for_each_substep = [&](const KvItem& it, const QueryPlan& plan, const KvSpans& spans, auto&& fn) -> bool {
-    for (int g = 0; g < group; ++g) {
-      for (int s = 0; s < plan.steps(); ++s) {
-        int qh, qt;
-        plan.step(s, it.kh, qh, qt);
-        const int qa = qt * kTile, qb = imin(qa + kTile, it.n);
-        if (spans.classify(qh, it.kh, qa, qb) == kTileSkip) continue;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          SubStep st;
-          st.sa = qa + half * kSub;
-          if (st.sa >= qb) continue;
-          st.sb = imin(st.sa + kSub, qb);
-          st.cls = spans.classify(qh, it.kh, st.sa, st.sb);
-          if (st.cls == kTileSkip) continue;
-          st.h = it.hk * group + g;
-          st.qh = qh;
-          if (!fn(st)) return false;
-        }
-      }
-    }
-    return true;
-  };
+  auto makes_dk = [](int idx) { return !kDvOnly && (Cfg::kPasses == 1 || (idx & 1) == 0); };
+  auto makes_dv = [](int idx) { return kDvOnly || Cfg::kPasses == 1 || (idx & 1) == 1; };
 
   // Whole warpgroups: four of compute warps, one of the TMA warp, the two MMA warps and an idle warp. The fifth
   // hands registers to the other four. The counts are set inside the role branches, so that the compiler never
@@ -274,7 +254,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
     for (uint32_t n_sched = 0;; ++n_sched) {
       const int idx = sched_consume<true>(mbox, n_sched, abort_flag);
       if (idx < 0 || idx >= total_items) break;
-      const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
+      const KvItem it = decode_kv_item(p, idx / Cfg::kItems);
       if (!it.valid) continue;
       const int kj = it.k0 + row;
       const int rows_valid = imax(0, imin(32, it.n - (it.k0 + quad * 32)));  // of this warp's 32 key rows
@@ -316,7 +296,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       for (uint32_t n_sched = 0; alive; ++n_sched) {
         const int idx = sched_produce(mbox, n_sched, p.ticket_kv, abort_flag);
         if (idx < 0 || idx >= total_items) break;
-        const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
+        const KvItem it = decode_kv_item(p, idx / Cfg::kItems);
         if (!it.valid) continue;
         const QueryPlan plan = make_query_plan(it.kh, it.k0, it.k1, it.n, bs, kTile);
         const KvSpans spans = make_kv_spans(it, bs);
@@ -358,7 +338,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         };
         SubStep pend{};
         bool have = false;
-        alive = for_each_substep(it, plan, spans, [&](const SubStep& st) -> bool {
+        alive = for_each_substep(it, plan, spans, group, [&](const SubStep& st) -> bool {
           if (have && !emit(pend, false)) return false;
           pend = st;
           have = true;
@@ -392,7 +372,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       for (uint32_t n_sched = 0; alive; ++n_sched) {
         const int idx = ptx::uniform(sched_consume<true>(mbox, n_sched, abort_flag));
         if (idx < 0 || idx >= total_items) break;
-        const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
+        const KvItem it = decode_kv_item(p, idx / Cfg::kItems);
         if (!it.valid) continue;
         if (!ptx::mbar_wait(kv_full, n_item & 1, abort_flag, 51)) break;
         for (bool last = false; alive && !last; ++g) {
@@ -456,7 +436,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       for (uint32_t n_sched = 0; alive; ++n_sched) {
         const int idx = ptx::uniform(sched_consume<true>(mbox, n_sched, abort_flag));
         if (idx < 0 || idx >= total_items) break;
-        const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
+        const KvItem it = decode_kv_item(p, idx / Cfg::kItems);
         if (!it.valid) continue;
         bool acc = false;
         // the first products of an item overwrite the accumulators: the epilogue warps must have read the last item's
@@ -510,7 +490,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
     for (uint32_t n_sched = 0; alive; ++n_sched) {
       const int idx = sched_consume<true>(mbox, n_sched, abort_flag);
       if (idx < 0 || idx >= total_items) break;
-      const KvItem it = decode_kv_item(p, idx / Cfg::kPasses);
+      const KvItem it = decode_kv_item(p, idx / Cfg::kItems);
       if (!it.valid) continue;
       const int kj = it.k0 + row;
       // queries that see this thread's key: same-half tiles and (clean keys only) noisy tiles of later blocks
@@ -984,20 +964,20 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
   if (warp == kLoadWarpB) ptx::tmem_dealloc(tmem, 512);
 }
 
-template <int kHeadDim, int kStagesKv, int kStagesQ, bool kBf16, bool kSoftcap>
+template <int kHeadDim, int kStagesKv, int kStagesQ, bool kBf16, bool kSoftcap, bool kDvOnly>
 int launch_bwd_instance(const BwdParams& p, int sm_count, unsigned stages, cudaStream_t stream) {
   if (stages & 2u) {
-    using Cfg = DkdvCfg<kHeadDim, kStagesKv>;
-    auto kernel = bwd_dkdv_kernel<kHeadDim, kStagesKv, kBf16, kSoftcap>;
+    using Cfg = DkdvCfg<kHeadDim, kStagesKv, kDvOnly>;
+    auto kernel = bwd_dkdv_kernel<kHeadDim, kStagesKv, kBf16, kSoftcap, kDvOnly>;
     static PerDeviceFlags smem_set;
     int rc = set_dynamic_smem(kernel, Cfg::kSmemBytes, smem_set);
     if (rc) return rc;
-    const int items = bwd_item_bound(p, p.heads_k) * Cfg::kPasses;
+    const int items = bwd_item_bound(p, p.heads_k) * Cfg::kItems;
     const int grid = items < sm_count ? items : sm_count;
     kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(p);
     FDA_CUDA_TRY(cudaGetLastError());
   }
-  if (stages & 4u) {
+  if (!kDvOnly && (stages & 4u)) {
     using Cfg = DqCfg<kHeadDim, kStagesQ>;
     auto kernel = bwd_dq_kernel<kHeadDim, kStagesQ, kBf16, kSoftcap>;
     static PerDeviceFlags smem_set;
@@ -1011,21 +991,25 @@ int launch_bwd_instance(const BwdParams& p, int sm_count, unsigned stages, cudaS
   return FDA_OK;
 }
 
-template <int kHeadDim, int kStagesKv, int kStagesQ>
+template <int kHeadDim, int kStagesKv, int kStagesQ, bool kDvOnly = false>
 int dispatch_bwd(const BwdParams& p, int sm_count, bool bf16, bool softcap, unsigned stages, cudaStream_t stream) {
   if (bf16) {
-    return softcap ? launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, true, true>(p, sm_count, stages, stream)
-                   : launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, true, false>(p, sm_count, stages, stream);
+    return softcap ? launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, true, true, kDvOnly>(p, sm_count, stages, stream)
+                   : launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, true, false, kDvOnly>(p, sm_count, stages, stream);
   }
-  return softcap ? launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, false, true>(p, sm_count, stages, stream)
-                 : launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, false, false>(p, sm_count, stages, stream);
+  return softcap ? launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, false, true, kDvOnly>(p, sm_count, stages, stream)
+                 : launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, false, false, kDvOnly>(p, sm_count, stages, stream);
 }
 
 inline int64_t round_up64(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
 }  // namespace
 
+// bwd_wide_sm100.cu
+int launch_bwd_wide(const BwdParams& p, bool bf16, bool softcap, int sm_count, cudaStream_t stream);
 // bwd_fused_sm100.cu
+bool bwd_wide_pays(const FdaProblem& pr);
+int launch_wide_convert(const BwdParams& p, bool bf16, cudaStream_t stream);
 size_t bwd_fused_acc_bytes(const FdaProblem& pr);
 int64_t bwd_fused_acc_tiles(const FdaProblem& pr);
 int bwd_fused_kv_split(const FdaProblem& pr);
@@ -1037,6 +1021,9 @@ constexpr int64_t kSmallAccBytes = 32 << 20;
 
 // The single-pass backward adds dQ partials in an order that depends on scheduling and needs head dim <= 128.
 bool bwd_single_pass(const FdaProblem& pr) { return pr.deterministic == 0 && pr.head_dim <= 128; }
+
+// Head dims above 128: dK and dQ in one kernel, dV in another (bwd_wide_sm100.cu). dQ's partials are added in such an order too.
+bool bwd_wide(const FdaProblem& pr) { return pr.deterministic == 0 && pr.head_dim > 128 && bwd_wide_pays(pr); }
 
 // Scratch of the split backward: delta_pad then lse2_pad, each batch * heads * 2 * n_pad floats (256-byte aligned
 // pieces), then 256 bytes of work counters.
@@ -1050,6 +1037,7 @@ size_t bwd_split_workspace_bytes(const FdaProblem& pr) {
 // The single-pass backward keeps its fp32 dQ accumulator behind that, and behind it parts of dK and dV where it makes some.
 size_t bwd_workspace_bytes(const FdaProblem& pr) {
   size_t bytes = bwd_split_workspace_bytes(pr);
+  if (bwd_wide(pr)) bytes += bwd_fused_acc_bytes(pr);
   if (bwd_single_pass(pr)) {
     bytes += static_cast<size_t>(round_up64(static_cast<int64_t>(bwd_fused_acc_bytes(pr)), 256)) + bwd_fused_part_bytes(pr);
   }
@@ -1072,6 +1060,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   BwdParams p;
   memset(&p, 0, sizeof(p));
   const bool single_pass = bwd_single_pass(pr) && (stage_mask & FDA_BWD_FORCE_SPLIT) == 0;
+  const bool wide = bwd_wide(pr) && (stage_mask & FDA_BWD_FORCE_SPLIT) == 0;
   auto encode = [&](CUtensorMap* map, const FdaTensor& t, int heads, int box_rows) {
     return encode_tile_map(map, t.ptr, 2, false, fp16, d, rows, heads, tma_batch, t.row_stride, t.head_stride,
                            t.batch_stride, 64, box_rows);
@@ -1084,7 +1073,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   if (!single_pass && ((rc = encode(&p.tm_q64, a.q, pr.heads, kSub)) || (rc = encode(&p.tm_do64, a.dout, pr.heads, kSub)))) {
     return rc;
   }
-  if (!single_pass && d > 128 && ((rc = encode(&p.tm_k64, a.k, pr.heads_k, 64)) || (rc = encode(&p.tm_v64, a.v, pr.heads_k, 64)))) {
+  if (!single_pass && !wide && d > 128 && ((rc = encode(&p.tm_k64, a.k, pr.heads_k, 64)) || (rc = encode(&p.tm_v64, a.v, pr.heads_k, 64)))) {
     return rc;
   }
   // the preprocess and the epilogues use 16-byte vector accesses on rows of out / dout / dq / dk / dv
@@ -1134,11 +1123,13 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   p.lse2_pad = reinterpret_cast<float*>(static_cast<uint8_t*>(a.workspace) + one);
   p.ticket_kv = reinterpret_cast<int*>(static_cast<uint8_t*>(a.workspace) + 2 * one);
   p.ticket_q = p.ticket_kv + 32;
-  if (single_pass) {
+  if (single_pass || wide) {
     if (a.workspace_bytes < bwd_workspace_bytes(pr)) return FDA_ERR_WORKSPACE;
     p.dq_acc = reinterpret_cast<float*>(static_cast<uint8_t*>(a.workspace) + bwd_split_workspace_bytes(pr));
     p.acc_tiles = static_cast<int>(bwd_fused_acc_tiles(pr));
     p.acc_floats = static_cast<int64_t>(bwd_fused_acc_bytes(pr) / 4);
+  }
+  if (single_pass) {
     p.kv_split = bwd_fused_kv_split(pr);
     p.part_floats = static_cast<int64_t>(bwd_fused_part_bytes(pr) / 4);
     if (p.kv_split > 1) p.dkv_part = p.dq_acc + round_up64(p.acc_floats, 64);
@@ -1156,7 +1147,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   // with max_seqlen as it is, 1161 / 1168 with three times that, 1225 / 1256 with four, 1474 / 1537 with eight. (Small
   // accumulators are always filled there: the launch counts for more.)
   const int64_t padded_rows = static_cast<int64_t>(pr.batch) * 2 * p.n_pad, acc_rows = static_cast<int64_t>(p.acc_tiles) * 64;
-  if (single_pass && (stage_mask & 3u) == 3u && (padded_rows <= 3 * acc_rows || p.acc_floats * 4 <= kSmallAccBytes)) {
+  if ((single_pass || wide) && (stage_mask & 3u) == 3u && (padded_rows <= 3 * acc_rows || p.acc_floats * 4 <= kSmallAccBytes)) {
     p.zero_acc16 = p.acc_floats / 4;
   }
   if (varlen) {
@@ -1185,7 +1176,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
     // dK/dV: the noisy key tiles (the second half of the ranks) are short; dQ: the shortest eighth (fractions
     // found by measurement on the benchmark shape); few items per CTA: rank for rank over all of them
     const int per_bh = 2 * p.tiles_per_half;
-    const int parts = single_pass ? p.kv_split : 1;
+    const int parts = single_pass ? p.kv_split : 1;   // (nor does bwd_wide_kernel deal out a group's heads)
     p.n_long_kv = order_n_long(per_bh, FDA_SHORT8_KV, static_cast<long long>(per_bh) * pr.batch * pr.heads_k * parts, sm_count);
     p.n_long_q = order_n_long(per_bh, FDA_SHORT8_Q, static_cast<long long>(per_bh) * pr.batch * pr.heads, sm_count);
   }
@@ -1207,6 +1198,16 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
     FDA_CUDA_TRY(cudaGetLastError());
   }
   if (single_pass) return launch_bwd_fused(p, d_round, bf16, softcap, sm_count, stage_mask, stream);
+  if (wide) {
+    if (stage_mask & 2u) {
+      if (p.zero_acc16 == 0) FDA_CUDA_TRY(cudaMemsetAsync(p.dq_acc, 0, static_cast<size_t>(p.acc_floats) * 4, stream));
+      if ((rc = dispatch_bwd<256, 1, 3, true>(p, sm_count, bf16, softcap, 2u, stream)) ||
+          (rc = launch_bwd_wide(p, bf16, softcap, sm_count, stream))) {
+        return rc;
+      }
+    }
+    return stage_mask & 4u ? launch_wide_convert(p, bf16, stream) : FDA_OK;
+  }
   if (d_round == 64) return dispatch_bwd<64, 6, 7>(p, sm_count, bf16, softcap, stage_mask, stream);
   if (d_round == 128) return dispatch_bwd<128, 4, 5>(p, sm_count, bf16, softcap, stage_mask, stream);
   return dispatch_bwd<256, 1, 3>(p, sm_count, bf16, softcap, stage_mask, stream);

@@ -950,6 +950,15 @@ constexpr double kLine = 240;
 
 }  // namespace
 
+// Samples of that many tokens a half, the longest and on average, and no chain of a key tile's steps over all heads of a group longer
+// than 1.23 times a CTA's share.
+bool bwd_chains_fit(const FdaProblem& pr, int tokens) {
+  if (pr.heads_k <= 0 || pr.batch <= 0 || pr.seqlen / 2 < tokens || pr.total / 2 < static_cast<int64_t>(pr.batch) * tokens) return false;
+  double longest, all, squares;
+  known_tiles(pr, longest, all, squares);
+  return pr.heads_k * (squares + 2 * all) >= kLine * longest;
+}
+
 // Whether heads wider than 128 take bwd_wide_kernel and the dV kernel instead of the split form's three passes. Its key tiles are
 // chains over all query heads of a group (the dQ kernel has an item for each head and query tile), so the longest must not be more
 // than a CTA's share, as above; and short items pay for the copy of V and the wait for the last dQ^T. Backward, split / this, us, heads
@@ -958,12 +967,7 @@ constexpr double kLine = 240;
 // 1179 / 1050, 16/4 1095 / 1008 and 1169 / 1069; 2 x 8192, 8 heads 1202 / 964 and 1257 / 1029. Longest chain above the share: 4 x
 // 4096, 8/1 heads 1058 / 1690; 1 x 8192, 16/4 1374 / 2219.
 bool bwd_wide_pays(const FdaProblem& pr) {
-  constexpr int kTokens = 1400;   // of a half, of the longest sample and on average
-  if (pr.heads_k <= 0 || pr.batch <= 0 || pr.seqlen / 2 < kTokens || pr.total / 2 < static_cast<int64_t>(pr.batch) * kTokens) return false;
-  if (convert_rows(pr.heads, pr.heads_k, false) > kMaxGridY) return false;
-  double longest, all, squares;
-  known_tiles(pr, longest, all, squares);
-  return pr.heads_k * (squares + 2 * all) >= kLine * longest;
+  return convert_rows(pr.heads, pr.heads_k, false) <= kMaxGridY && bwd_chains_fit(pr, 1400);
 }
 
 // Parts into which the query heads of a group are dealt. A key tile's steps are a chain, and those of the longest sample's first

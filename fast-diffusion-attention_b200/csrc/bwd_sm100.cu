@@ -124,8 +124,8 @@ __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_consta
 // 2. dK / dV
 // ------------------------------------------------------------------------------------------------------------
 
-// kDvOnly (head dims above 128): dV items only, dK is made with dQ (bwd_wide_sm100.cu).
-template <int kHeadDim, int kStages, bool kDvOnly>
+// kMakes: bit 0 dK, bit 1 dV (one without the other: head dims above 128).
+template <int kHeadDim, int kStages, int kMakes>
 struct DkdvCfg {
   using T = TileCfg<kHeadDim>;
   static constexpr int kSubTileBytes = kSub * kHeadDim * 2;     // Q or dO sub-tile
@@ -137,8 +137,9 @@ struct DkdvCfg {
   // both instead takes S^T and dP^T twice, six products for five. (Backward of 2 x 16384 tokens, 8 heads of 256, blocks of
   // 256: 7.34 -> 4.97 ms with the rings below.)
   static constexpr int kPasses = kHeadDim > 128 ? 2 : 1;
-  static constexpr int kItems = kDvOnly ? 1 : kPasses;   // a key tile
-  static_assert(!kDvOnly || kPasses == 2, "head dims above 128");
+  static constexpr int kItems = kMakes == 3 ? kPasses : 1;   // a key tile
+  static constexpr bool kDvOnly = kMakes == 2;
+  static_assert(kMakes == 3 || kPasses == 2, "head dims above 128");
   static constexpr int kTmemDK = 256, kTmemDV = kPasses == 2 ? 256 : 256 + kHeadDim;
   static_assert(kTmemDV + kHeadDim <= 512, "tensor memory budget");
   // Rings of Q and dO sub-tiles of their own. With 128 KB of K and V there is room for three of 32 KB: two for Q, one for
@@ -161,9 +162,9 @@ struct DkdvCfg {
 
 // One CTA per SM. A sub-step is one 64-row half of a visible 128-row query tile of one query head of the group; a half with
 // no visible row is skipped.
-template <int kHeadDim, int kStages, bool kBf16, bool kSoftcap, bool kDvOnly>
+template <int kHeadDim, int kStages, bool kBf16, bool kSoftcap, int kMakes>
 __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_constant__ BwdParams p) {
-  using Cfg = DkdvCfg<kHeadDim, kStages, kDvOnly>;
+  using Cfg = DkdvCfg<kHeadDim, kStages, kMakes>;
   using T = TileCfg<kHeadDim>;
   // The tiles need 1024-byte alignment for the 128-byte swizzle. Dynamic shared memory starts at the beginning of the
   // block's window, which is aligned that far; head dimension 256 leaves no room to round the base up, so a base that is
@@ -236,8 +237,8 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
   const int group = p.heads / p.heads_k;
   const int total_items = kv_item_count(p) * Cfg::kItems;
   // what the item with this index makes
-  auto makes_dk = [](int idx) { return !kDvOnly && (Cfg::kPasses == 1 || (idx & 1) == 0); };
-  auto makes_dv = [](int idx) { return kDvOnly || Cfg::kPasses == 1 || (idx & 1) == 1; };
+  auto makes_dk = [](int idx) { return kMakes == 3 ? Cfg::kPasses == 1 || (idx & 1) == 0 : kMakes == 1; };
+  auto makes_dv = [](int idx) { return kMakes == 3 ? Cfg::kPasses == 1 || (idx & 1) == 1 : kMakes == 2; };
 
   // Whole warpgroups: four of compute warps, one of the TMA warp, the two MMA warps and an idle warp. The fifth
   // hands registers to the other four. The counts are set inside the role branches, so that the compiler never
@@ -964,18 +965,39 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
   if (warp == kLoadWarpB) ptx::tmem_dealloc(tmem, 512);
 }
 
+template <int kHeadDim, int kStages, bool kBf16, bool kSoftcap, int kMakes>
+int launch_dkdv(const BwdParams& p, int sm_count, cudaStream_t stream) {
+  using Cfg = DkdvCfg<kHeadDim, kStages, kMakes>;
+  auto kernel = bwd_dkdv_kernel<kHeadDim, kStages, kBf16, kSoftcap, kMakes>;
+  static PerDeviceFlags smem_set;
+  const int rc = set_dynamic_smem(kernel, Cfg::kSmemBytes, smem_set);
+  if (rc) return rc;
+  const int items = bwd_item_bound(p, p.heads_k) * Cfg::kItems;
+  const int grid = items < sm_count ? items : sm_count;
+  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(p);
+  FDA_CUDA_TRY(cudaGetLastError());
+  return FDA_OK;
+}
+
 template <int kHeadDim, int kStagesKv, int kStagesQ, bool kBf16, bool kSoftcap, bool kDvOnly>
 int launch_bwd_instance(const BwdParams& p, int sm_count, unsigned stages, cudaStream_t stream) {
   if (stages & 2u) {
-    using Cfg = DkdvCfg<kHeadDim, kStagesKv, kDvOnly>;
-    auto kernel = bwd_dkdv_kernel<kHeadDim, kStagesKv, kBf16, kSoftcap, kDvOnly>;
-    static PerDeviceFlags smem_set;
-    int rc = set_dynamic_smem(kernel, Cfg::kSmemBytes, smem_set);
+    int rc;
+    if constexpr (kHeadDim > 128) {
+      if (kDvOnly || p.apart) {
+        rc = launch_dkdv<kHeadDim, kStagesKv, kBf16, kSoftcap, 2>(p, sm_count, stream);
+        if (rc == FDA_OK && !kDvOnly) {
+          BwdParams q = p;
+          q.ticket_kv = p.ticket_kv + 16;   // a counter of its own
+          rc = launch_dkdv<kHeadDim, kStagesKv, kBf16, kSoftcap, 1>(q, sm_count, stream);
+        }
+      } else {
+        rc = launch_dkdv<kHeadDim, kStagesKv, kBf16, kSoftcap, 3>(p, sm_count, stream);
+      }
+    } else {
+      rc = launch_dkdv<kHeadDim, kStagesKv, kBf16, kSoftcap, 3>(p, sm_count, stream);
+    }
     if (rc) return rc;
-    const int items = bwd_item_bound(p, p.heads_k) * Cfg::kItems;
-    const int grid = items < sm_count ? items : sm_count;
-    kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(p);
-    FDA_CUDA_TRY(cudaGetLastError());
   }
   if (!kDvOnly && (stages & 4u)) {
     using Cfg = DqCfg<kHeadDim, kStagesQ>;
@@ -1008,6 +1030,7 @@ inline int64_t round_up64(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 // bwd_wide_sm100.cu
 int launch_bwd_wide(const BwdParams& p, bool bf16, bool softcap, int sm_count, cudaStream_t stream);
 // bwd_fused_sm100.cu
+bool bwd_chains_fit(const FdaProblem& pr, int tokens);
 bool bwd_wide_pays(const FdaProblem& pr);
 int launch_wide_convert(const BwdParams& p, bool bf16, cudaStream_t stream);
 size_t bwd_fused_acc_bytes(const FdaProblem& pr);
@@ -1060,6 +1083,12 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   BwdParams p;
   memset(&p, 0, sizeof(p));
   const bool single_pass = bwd_single_pass(pr) && (stage_mask & FDA_BWD_FORCE_SPLIT) == 0;
+  // Heads wider than 128, split form: dV items in a launch of their own have three dO slots, at the price of a second tail and of
+  // items that cannot fill each other's gaps. Backward, together / apart, us, heads of 256: 16 x 2000 tokens, 8 heads, blocks of 16
+  // 820 / 789, 16/8 heads, blocks of 512 1844 / 1721; deterministic, 4 x 4096, 8 heads 679 / 641, 1 x 16384 2173 / 2000. Short
+  // ones and those whose longest chain is more than a CTA's share stay together (32 x 512 tokens 246 / 264; 1 x 16384, 8/2 heads
+  // 2360 / 3140).
+  p.apart = d > 128 && bwd_chains_fit(pr, 700) ? 1 : 0;
   const bool wide = bwd_wide(pr) && (stage_mask & FDA_BWD_FORCE_SPLIT) == 0;
   auto encode = [&](CUtensorMap* map, const FdaTensor& t, int heads, int box_rows) {
     return encode_tile_map(map, t.ptr, 2, false, fp16, d, rows, heads, tma_batch, t.row_stride, t.head_stride,

@@ -189,7 +189,13 @@ struct FwdConfig {
   static constexpr int kMmaWarp = 4 * kQTiles + 1;                    // one issuing warp per query tile
   // epilogue staging: per query tile one [128 rows][64 columns] 16-bit tile, stored to out as a whole
   static constexpr int kStageOBytes = kBlockM * 128;
-  static constexpr int kFixedBytes = kQTiles * (kTileBytes + kStageOBytes) + 1024 /*alignment slack*/ +
+  // 16-bit Q on its way to tensor memory comes through the ring: a pair of slots holds it, and the ring has a
+  // pair more. With two pairs the loads' latency set the pace (nothing but loads took 894 of 1090 us on 2 x 16384 tokens, 8 heads: now
+  // 890; packed samples of 517 to 4095 tokens a half, 8 heads of 192, 438 -> 342; 51 x 640 tokens, 16/8 heads 602 -> 546, 256 x 384
+  // 529 -> 445, which read Q from shared memory before).
+  static constexpr bool kQInRing = kQInTmem && !kFp8;
+  static_assert(!kQInRing || kTileBytes == 2 * kSlotBytes, "a pair of slots holds a query tile");
+  static constexpr int kFixedBytes = kQTiles * ((kQInRing ? 0 : kTileBytes) + kStageOBytes) + 1024 /*alignment slack*/ +
                                      1024 /*barriers, mailbox, item descriptions*/;
   static constexpr int kFit = (232448 - kFixedBytes) / (2 * kSlotBytes);
   static constexpr int kPairs = kFit < 4 ? kFit : 4;                  // the ring holds pairs of a K and a V slot
@@ -198,7 +204,7 @@ struct FwdConfig {
   // tensor memory: S of query tile t, buffer b at (t * kBufs + b) * 64 (P over its first columns), O behind
   static constexpr int kTmemO = kQTiles * kBufs * kSubKeys;
   static_assert(kTmemO + kQTiles * kHeadDim <= 512, "tensor memory budget");
-  // ... and, for head dim 256, Q behind that (see launch_fwd). The S product then fetches only K from shared memory (16 instead
+  // ... and, for head dim 256, Q behind that. The S product then fetches only K from shared memory (16 instead
   // of 48 cycles a reduction step of 32 bytes): 1225 -> 1154 us on 2 x 16384 tokens, 8 heads, e4m3 916 -> 903. Head dim 64, where
   // columns are left too, gains nothing (256 / 254 us on 4 x 4096 tokens, 32/8 heads; 806 / 830 on 4 x 8192, 32 heads).
   static constexpr bool kTmemHasQ = kQInTmem;
@@ -225,7 +231,7 @@ struct FwdConfig {
 // has time, walks the geometry and leaves one word of flags beside every K slot. (A single thread that decoded items and
 // classified tiles between the products spent 1200 cycles a round on that while the pipe ran dry; the whole warp takes
 // part in waits and loop control, one elected lane issues, which keeps descriptors and counters in uniform registers.)
-constexpr uint32_t kInfoFirst = 16, kInfoLast = 32, kInfoHalf1 = 64, kInfoStop = 128, kInfoTile0 = 256;  // bit 2 t + h: tile t sees half h
+constexpr uint32_t kInfoFirst = 16, kInfoLast = 32, kInfoHalf1 = 64, kInfoStop = 128, kInfoTile0 = 256, kInfoQ = 1024;  // bit 2 t + h: tile t sees half h
 
 template <int kHeadDim, int kQTiles, int kType, bool kSoftcap, bool kQInTmem>
 __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fwd_kernel(const __grid_constant__ FwdParams p) {
@@ -234,7 +240,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* sQ = smem;
-  uint8_t* sKV = smem + kQTiles * Cfg::kTileBytes;
+  uint8_t* sKV = smem + (Cfg::kQInRing ? 0 : kQTiles * Cfg::kTileBytes);
   uint8_t* sStageO = sKV + kStages * Cfg::kSlotBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(sStageO + kQTiles * Cfg::kStageOBytes);
   uint64_t* q_full = bars;                         // 1
@@ -339,6 +345,21 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
           for (int t = 0; t < kQTiles; ++t) bits |= spans[t].classify(kh, k0) != kTileSkip ? 1u << (2 * t + sub) : 0u;
           return bits;
         };
+        if (Cfg::kQInRing) {
+          // the item's Q, half of it in each slot of a pair
+          for (int which = 0; which < 2; ++which) {
+            const uint32_t slot = 2 * pair + which;
+            if (!ptx::mbar_wait(&kv_empty[slot], empty_par, abort_flag, 12)) { alive = false; break; }
+            if (which == 0) slot_info[pair] = kInfoQ;
+            ptx::mbar_expect_tx(&kv_full[slot], Cfg::kSlotBytes);
+#pragma unroll
+            for (int c = 0; c < Cfg::kPanels / 2; ++c) {
+              ptx::tma_load_4d(sKV + slot * Cfg::kSlotBytes + c * kQPanelBytes, &p.tm_q, &kv_full[slot],
+                               (which * (Cfg::kPanels / 2) + c) * Cfg::kPanelElems, q_row, it.h, it.bcoord);
+            }
+          }
+          if (++pair == Cfg::kPairs) { pair = 0; empty_par ^= 1; }
+        }
         for (int s = 0; s < tiles && alive; ++s) {
           int kh, kt;
           plan.step(s, kh, kt);
@@ -364,7 +385,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
               ptx::tma_load_4d(dst + c * Cfg::kSlotPanelBytes, tm, &kv_full[slot], c * Cfg::kPanelElems, k_row, it.hk,
                                it.bcoord);
             }
-            if (s == 0 && which == 0) {
+            if (!Cfg::kQInRing && s == 0 && which == 0) {
               // Q after the first K slot: the first MMA needs both, the previous item may still own Q.
               if (!ptx::mbar_wait(q_empty, (n_item & 1) ^ 1, abort_flag, 12)) { alive = false; break; }
               ptx::mbar_expect_tx(q_full, ntiles * Cfg::kTileBytes);
@@ -445,7 +466,24 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       if (!ptx::mbar_wait(&kv_full[2 * pair], par, abort_flag, 22)) break;
       const uint32_t info = ptx::uniform(slot_info[pair]);
       if (info & kInfoStop) break;
-      if (info & kInfoFirst) {
+      if (Cfg::kQInRing && (info & kInfoQ)) {
+        // Every S product of the last item is complete: this warp has waited for the P of each.
+        if (!ptx::mbar_wait(&kv_full[2 * pair + 1], par, abort_flag, 21)) break;
+        ptx::tc_fence_after();
+        if (ptx::elect_one()) {
+          const uint32_t lo = k_lo0 + 2 * pair * (Cfg::kSlotBytes >> 4);
+#pragma unroll
+          for (int kk = 0; kk < kHeadDim / Cfg::kStepElems; ++kk) {
+            ptx::tmem_cp_128x32b_lh(tmem_q + kk * 8, lo + (((kk / 4) * kQPanelBytes + (kk % 4) * 32) >> 4), kDescHi);
+          }
+          ptx::umma_commit(&kv_empty[2 * pair]);
+          ptx::umma_commit(&kv_empty[2 * pair + 1]);
+        }
+        if (++pair == Cfg::kPairs) { pair = 0; par ^= 1; }
+        o_acc = false;
+        continue;
+      }
+      if (!Cfg::kQInRing && (info & kInfoFirst)) {
         if (!ptx::mbar_wait(q_full, q_par, abort_flag, 21)) break;
         q_par ^= 1;
         o_acc = false;
@@ -970,13 +1008,6 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
     return q_tiles == 2 ? dispatch_fwd_fp8<128, 2>(p, grid, softcap, stream) : dispatch_fwd_fp8<128, 1>(p, grid, softcap, stream);
   }
   if (d_round == 256) {
-    // Q goes to tensor memory once an item, which short items do not earn back. Q in shared / in tensor memory, us, 16/8 heads of
-    // 256, 65536 tokens, blocks of 16, 256 and 1024, by the tokens of a half: 64 779 / 780, 506 / 513, 504 / 511; 192 674 / 678,
-    // 529 / 552, 531 / 554; 320 689 / 690, 596 / 617, 636 / 657; 512 652 / 650, 599 / 611, 712 / 707; 640 694 / 690, 644 / 650, 838 / 834 (one
-    // sample of 624, 16 heads, blocks of 9, with its gradients 130.5 / 129.3);
-    // 1024 860 / 883, 892 / 852, 1336 / 1327; 4096 2607 / 2507, 2561 / 2437, 2988 / 2829. e4m3, with half the bytes, is within 1.5 %
-    // either way on short ones.
-    if (max_n <= 512) return dispatch_fwd<256, 1>(p, grid, bf16, softcap, stream);
     return dispatch_fwd<256, 1, true>(p, grid, bf16, softcap, stream);
   }
   if (d_round == 128) {

@@ -66,8 +66,8 @@ struct FusedCfg {
 //   Head dim 128: two compute warpgroups of 64 columns. 512 threads start with 128 registers, and the drain warps hold a
 //     whole dQ^T (128 columns): the buffer it shares with dP^T is free 250 cycles after the product instead of after 48
 //     of its 64 KB have left for L2 (backward of 4 x 8192 tokens, 32/8 heads of 128, blocks of 1024: 4.25 -> 3.98 ms).
-//     It is bound by shared memory and by power: a step takes 4450 cycles there (of a clock of 1.46 to 1.65 GHz), of which
-//     shared memory at 128 bytes a clock has 4350 (operands 2300, the staging of dQ^T 1024, the loads 512, dS^T 256,
+//     It is bound by shared memory and by power: a step takes 4260 cycles there (of a clock of 1.46 to 1.65 GHz), of which
+//     shared memory at 128 bytes a clock has some 4300 (operands 2300, the staging of dQ^T 1024, the loads 512, dS^T 256,
 //     statistics 250), the tensor pipe's arithmetic 2560; without the reductions themselves it takes 11 % less time
 //     (3 % less on 8 x 4096 tokens, 16 heads, blocks of 256). Vector reductions straight from the registers
 //     would save the staging, but stall the load/store unit for the compute warps (4.1 ms).

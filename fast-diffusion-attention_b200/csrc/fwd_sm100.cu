@@ -224,8 +224,11 @@ struct FwdConfig {
 // then the S product that refills it, so neither waits for the other's latency. With ONE 128-column buffer per tile the
 // chain S -> softmax -> P V -> next S was serial. The price is the shared-memory traffic of N = 64 products (6 KB per 32
 // cycles of arithmetic, 48 cycles at 128 bytes per clock). On 4 x 8192 tokens, 32/8 heads of 128, blocks of 1024: 1.24 ->
-// 1.14 ms, 4400 -> 4000 cycles of kernel time for two query tiles against 128 keys, of which the tensor pipe has 2048 and
-// the special-function unit 2048 to do. What fills the rest is not settled.
+// 1.14 ms, 4400 -> 4000 cycles of kernel time for two query tiles against 128 keys, of which the tensor pipe has 2300 (that mix
+// of products measured alone) and the special-function unit 2048 to do. The rest is the softmax warps' own chain of a sub-step: wait,
+// load (some 300 cycles), maximum, vote, pack, store, hand over. Without exponentials and products the kernel still takes half its
+// time, and what shortens that chain by instructions helps. (Loads ahead, turns at the exponentials and more warps a tile do not:
+// each adds hand-overs, 3-40 % slower.)
 //
 // Every query tile has its own issuing warp, and that warp does next to nothing but wait and issue: the TMA warp, which
 // has time, walks the geometry and leaves one word of flags beside every K slot. (A single thread that decoded items and

@@ -54,6 +54,7 @@ struct BwdParams {
   int64_t acc_floats;   // size of the accumulator
   VarlenList vl;     // packed batches: samples longest first with running 128-row tile counts (base == nullptr otherwise)
   int wide_store;      // dq/dk/dv rows allow 32-byte stores
+  int overlap;         // host: overlapped_launches
   float scale_log2, softcap_pre, softmax_scale;
   int apart;            // split backward, head dims above 128: dV items in a launch of their own
   int kv_split;         // single-pass backward: parts into which a key tile's query heads are dealt (a divisor of the group)

@@ -234,6 +234,8 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
+  ptx::wait_for_stream();
+  ptx::let_next_start();
   const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int group = p.heads / p.heads_k;
@@ -806,6 +808,8 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
 // ------------------------------------------------------------------------------------------------------------
 template <int kHeadDim, bool kBf16, bool kSoftcap, bool kParts>
 __global__ void __launch_bounds__(256) bwd_dq_convert_kernel(const __grid_constant__ BwdParams p) {
+  ptx::wait_for_stream();
+  ptx::let_next_start();
   const int hh = blockIdx.y >> 1, half = blockIdx.y & 1;
   const int b = blockIdx.z;
   const Sample sm = sample_of(p, b);
@@ -879,13 +883,11 @@ int launch_fused_instance(const BwdParams& p, int sm_count, unsigned stages, cud
     }
     const int64_t items = static_cast<int64_t>(bwd_item_bound(p, p.heads_k)) * p.kv_split;
     const int grid = items < sm_count ? static_cast<int>(items) : sm_count;
-    kernel<<<grid, FusedRoles<kHeadDim>::kThreads, Cfg::kSmemBytes, stream>>>(p);
-    FDA_CUDA_TRY(cudaGetLastError());
+    if (const int launched = launch_kernel(p.overlap != 0, kernel, grid, FusedRoles<kHeadDim>::kThreads, Cfg::kSmemBytes, stream, p)) return launched;
   }
   if (stages & 4u) {
     dim3 grid(p.n_pad / 64, convert_rows(p.heads, p.heads_k, p.kv_split > 1), p.batch);
-    bwd_dq_convert_kernel<kHeadDim, kBf16, kSoftcap, kParts><<<grid, 256, 0, stream>>>(p);
-    FDA_CUDA_TRY(cudaGetLastError());
+    if (const int launched = launch_kernel(p.overlap != 0, bwd_dq_convert_kernel<kHeadDim, kBf16, kSoftcap, kParts>, grid, 256, 0, stream, p)) return launched;
   }
   return FDA_OK;
 }
@@ -1026,10 +1028,8 @@ int launch_bwd_fused(const BwdParams& p, int d_round, bool bf16, bool softcap, i
 // The convert kernel of head dims above 128 (bwd_wide_sm100.cu).
 int launch_wide_convert(const BwdParams& p, bool bf16, cudaStream_t stream) {
   dim3 grid(p.n_pad / 64, convert_rows(p.heads, p.heads_k, false), p.batch);
-  if (bf16) bwd_dq_convert_kernel<256, true, false, false><<<grid, 256, 0, stream>>>(p);
-  else bwd_dq_convert_kernel<256, false, false, false><<<grid, 256, 0, stream>>>(p);
-  FDA_CUDA_TRY(cudaGetLastError());
-  return FDA_OK;
+  return launch_kernel(p.overlap != 0, bf16 ? bwd_dq_convert_kernel<256, true, false, false> : bwd_dq_convert_kernel<256, false, false, false>, grid, 256, 0,
+                           stream, p);
 }
 
 int read_status_bwd_fused(int32_t* out4) {

@@ -40,6 +40,8 @@ constexpr int kPreUnroll = 2;
 
 template <bool kBf16, int kLanes>
 __global__ void __launch_bounds__(256) bwd_preprocess_kernel(const __grid_constant__ BwdParams p) {
+  ptx::wait_for_stream();
+  ptx::let_next_start();
   constexpr int kRowsPerWarp = 32 / kLanes;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int sub = lane / kLanes, l = lane % kLanes;
@@ -232,6 +234,8 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
+  ptx::wait_for_stream();
+  ptx::let_next_start();
   const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int group = p.heads / p.heads_k;
@@ -692,6 +696,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
+  ptx::wait_for_stream();
+  ptx::let_next_start();
   const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int total_items = (p.vl.base != nullptr ? p.vl.base[0] : p.tiles_per_half * p.batch) * 2 * p.heads;
@@ -974,8 +980,7 @@ int launch_dkdv(const BwdParams& p, int sm_count, cudaStream_t stream) {
   if (rc) return rc;
   const int items = bwd_item_bound(p, p.heads_k) * Cfg::kItems;
   const int grid = items < sm_count ? items : sm_count;
-  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(p);
-  FDA_CUDA_TRY(cudaGetLastError());
+  if (const int launched = launch_kernel(p.overlap != 0, kernel, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, p)) return launched;
   return FDA_OK;
 }
 
@@ -1007,8 +1012,7 @@ int launch_bwd_instance(const BwdParams& p, int sm_count, unsigned stages, cudaS
     if (rc) return rc;
     const int items = bwd_item_bound(p, p.heads);
     const int grid = items < sm_count ? items : sm_count;
-    kernel<<<grid, kBwdThreads, Cfg::kSmemBytes, stream>>>(p);
-    FDA_CUDA_TRY(cudaGetLastError());
+    if (const int launched = launch_kernel(p.overlap != 0, kernel, grid, kBwdThreads, Cfg::kSmemBytes, stream, p)) return launched;
   }
   return FDA_OK;
 }
@@ -1143,6 +1147,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   p.total = pr.total;
   p.heads = pr.heads;
   p.heads_k = pr.heads_k;
+  p.overlap = overlapped_launches(pr) ? 1 : 0;
   p.head_dim = d;
   p.block_size = pr.block_size;
   p.n_pad = static_cast<int>(round_up64(pr.seqlen / 2 > 0 ? pr.seqlen / 2 : 1, kTile));
@@ -1184,7 +1189,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
     // rebuilds it, so stages may be launched one by one
     int* list = reinterpret_cast<int*>(static_cast<uint8_t*>(a.workspace) + 2 * one + 256);
     if (stage_mask & 6u) {
-      rc = launch_varlen_prepare(pr.cu_seqlens, pr.batch, kTile, list, p.ticket_kv, stream);
+      rc = launch_varlen_prepare(pr.cu_seqlens, pr.batch, kTile, list, p.ticket_kv, stream, p.overlap != 0);
       if (rc) return rc;
     }
     p.vl.base = list;
@@ -1215,16 +1220,12 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
     const int lanes = d <= 64 ? 8 : (d <= 128 ? 16 : 32);
     const int rows_per_block = 8 * (32 / lanes) * kPreUnroll;
     dim3 grid((p.n_pad + rows_per_block - 1) / rows_per_block, 2 * pr.heads, pr.batch);
-    if (bf16) {
-      if (lanes == 8) bwd_preprocess_kernel<true, 8><<<grid, 256, 0, stream>>>(p);
-      else if (lanes == 16) bwd_preprocess_kernel<true, 16><<<grid, 256, 0, stream>>>(p);
-      else bwd_preprocess_kernel<true, 32><<<grid, 256, 0, stream>>>(p);
-    } else {
-      if (lanes == 8) bwd_preprocess_kernel<false, 8><<<grid, 256, 0, stream>>>(p);
-      else if (lanes == 16) bwd_preprocess_kernel<false, 16><<<grid, 256, 0, stream>>>(p);
-      else bwd_preprocess_kernel<false, 32><<<grid, 256, 0, stream>>>(p);
-    }
-    FDA_CUDA_TRY(cudaGetLastError());
+    auto pre = [&](auto bf16_tag) {
+      constexpr bool kB = decltype(bf16_tag)::value;
+      return lanes == 8 ? bwd_preprocess_kernel<kB, 8> : lanes == 16 ? bwd_preprocess_kernel<kB, 16> : bwd_preprocess_kernel<kB, 32>;
+    };
+    rc = launch_kernel(p.overlap != 0, bf16 ? pre(std::true_type{}) : pre(std::false_type{}), grid, 256, 0, stream, p);
+    if (rc) return rc;
   }
   if (single_pass) return launch_bwd_fused(p, d_round, bf16, softcap, sm_count, stage_mask, stream);
   if (wide) {

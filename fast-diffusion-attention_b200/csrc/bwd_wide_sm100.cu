@@ -111,6 +111,8 @@ __global__ void __launch_bounds__(WideCfg::kThreads, 1) bwd_wide_kernel(const __
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
+  ptx::wait_for_stream();
+  ptx::let_next_start();
   const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int group = p.heads / p.heads_k;
@@ -486,8 +488,7 @@ int launch_wide_instance(const BwdParams& p, int sm_count, cudaStream_t stream) 
   const int rc = set_dynamic_smem(kernel, WideCfg::kSmemBytes, smem_set);
   if (rc) return rc;
   const int items = bwd_item_bound(p, p.heads_k);
-  kernel<<<items < sm_count ? items : sm_count, WideCfg::kThreads, WideCfg::kSmemBytes, stream>>>(p);
-  FDA_CUDA_TRY(cudaGetLastError());
+  if (const int launched = launch_kernel(p.overlap != 0, kernel, items < sm_count ? items : sm_count, WideCfg::kThreads, WideCfg::kSmemBytes, stream, p)) return launched;
   return FDA_OK;
 }
 

@@ -63,6 +63,7 @@ struct FwdParams {
   VarlenList vl;       // packed batches: samples longest first with running item counts (base == nullptr otherwise)
   int* ticket;         // global work counter, zeroed before the launch
   int wide_store;      // rows of out allow 32-byte stores
+  int overlap;         // host: overlapped_launches
   const float* q_descale;  // FP8 only: (batch, heads_k) factors, element strides below; nullptr = 1
   const float* k_descale;
   const float* v_descale;
@@ -264,7 +265,6 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
 
   const int warp = ptx::uniform(static_cast<int>(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
-  const int total_items = p.vl.base != nullptr ? p.vl.base[0] * 2 * p.heads : p.total_items;
 
   if (threadIdx.x == 0) {
     *abort_flag = 0;
@@ -295,8 +295,11 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
+  ptx::wait_for_stream();
+  ptx::let_next_start();
   const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
+  const int total_items = p.vl.base != nullptr ? p.vl.base[0] * 2 * p.heads : p.total_items;
 
   // The register counts are set inside the role branches: after a point where the branches meet again the
   // compiler would have to assume the smaller count for everything.
@@ -870,8 +873,7 @@ int launch_fwd_instance(const FwdParams& p, int grid, cudaStream_t stream) {
   static PerDeviceFlags smem_set;
   const int rc = set_dynamic_smem(kernel, Cfg::kSmemBytes, smem_set);
   if (rc) return rc;
-  kernel<<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(p);
-  FDA_CUDA_TRY(cudaGetLastError());
+  if (const int launched = launch_kernel(p.overlap != 0, kernel, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, p)) return launched;
   return FDA_OK;
 }
 
@@ -970,6 +972,7 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
   p.total = pr.total;
   p.heads = pr.heads;
   p.heads_k = pr.heads_k;
+  p.overlap = overlapped_launches(pr) ? 1 : 0;
   p.head_dim = d;
   p.block_size = pr.block_size;
   const int max_n = pr.seqlen / 2;
@@ -994,7 +997,7 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
     // the work list is built on the device from cu_seqlens (no host synchronisation): the host only knows an upper
     // bound of the number of items, blocks beyond the real number find no work and leave
     int* list = reinterpret_cast<int*>(static_cast<uint8_t*>(a.workspace) + 256);
-    const int rc = launch_varlen_prepare(pr.cu_seqlens, pr.batch, q_tiles * kBlockM, list, p.ticket, stream);
+    const int rc = launch_varlen_prepare(pr.cu_seqlens, pr.batch, q_tiles * kBlockM, list, p.ticket, stream, p.overlap != 0);
     if (rc) return rc;
     p.vl.base = list;
     p.vl.batch = pr.batch;

@@ -111,6 +111,34 @@ int set_dynamic_smem(Kernel kernel, int bytes, PerDeviceFlags& flags) {
   return FDA_OK;
 }
 
+// Launches a kernel; with `overlap` its blocks may start, up to ptx::wait_for_stream, while the last blocks of the kernel ahead in the
+// stream are still running (if that is one of ours and has called ptx::let_next_start; behind anything else it starts as usual): the
+// launch, the set-up of barriers and the allocation of tensor memory come off the path.
+template <typename... Params, typename... Args>
+int launch_kernel(bool overlap, void (*kernel)(Params...), dim3 grid, int threads, int smem_bytes, cudaStream_t stream,
+                  const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  FDA_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, args...));
+  return FDA_OK;
+}
+
+// Where launches overlap: on little work, where they are a good part of the time (step of 2 x 512 tokens, 4 heads of 64, 33.1 -> 26.4
+// us; 3 x 666, 12/4 heads of 96, 100 -> 94; 1 x 2048, 4 heads of 256, 129 -> 120; forward of 1 x 1024, 16 heads of 128, 16.6 -> 14.3). At
+// twice the line, 16 x 512 tokens, 16/4 heads of 128, there is nothing left of it (150 / 152), and long kernels get slower (2 x 8192, 8
+// heads of 256, 1340 -> 1445: blocks land on other SMs, in the order in which these become free).
+inline bool overlapped_launches(const FdaProblem& pr) {
+  return static_cast<int64_t>(pr.total) * pr.heads * pr.head_dim <= (1 << 23);
+}
+
 struct DeviceInfo {
   int device = -1;
   int sm_count = 0;

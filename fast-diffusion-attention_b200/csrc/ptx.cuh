@@ -38,6 +38,13 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 __device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
 
+// ---- overlapped launches (see launch_kernel) -------------------------------------------------------------
+// Everything that reads or writes global memory comes behind this: it returns when the kernels ahead in the stream are complete
+// and what they wrote is visible. Every block executes it, so that a kernel is never complete before those ahead of it.
+__device__ __forceinline__ void wait_for_stream() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The next kernel's blocks may start their prologue as this one's leave.
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- mbarrier -------------------------------------------------------------------------------------------
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");

@@ -2,11 +2,14 @@
 #include "varlen_list.cuh"
 
 #include "host_util.h"
+#include "ptx.cuh"
 
 namespace fda {
 
 __global__ void __launch_bounds__(256) varlen_prepare_kernel(const int32_t* __restrict__ cu_seqlens, int batch,
                                                              int unit_rows, int* out, int* tickets) {
+  ptx::wait_for_stream();
+  ptx::let_next_start();
   if (threadIdx.x < kTicketInts) tickets[threadIdx.x] = 0;
   int* order = out + 1;
   int* cum = out + 1 + batch;
@@ -35,10 +38,9 @@ __global__ void __launch_bounds__(256) varlen_prepare_kernel(const int32_t* __re
   }
 }
 
-int launch_varlen_prepare(const int32_t* cu_seqlens, int batch, int unit_rows, int* out, int* tickets, void* stream) {
-  varlen_prepare_kernel<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(cu_seqlens, batch, unit_rows, out, tickets);
-  FDA_CUDA_TRY(cudaGetLastError());
-  return FDA_OK;
+int launch_varlen_prepare(const int32_t* cu_seqlens, int batch, int unit_rows, int* out, int* tickets, void* stream,
+                          bool overlap) {
+  return launch_kernel(overlap, varlen_prepare_kernel, 1, 256, 0, static_cast<cudaStream_t>(stream), cu_seqlens, batch, unit_rows, out, tickets);
 }
 
 }  // namespace fda

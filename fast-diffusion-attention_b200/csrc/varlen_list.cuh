@@ -51,6 +51,7 @@ constexpr int kTicketInts = 64;
 __global__ void varlen_prepare_kernel(const int32_t* __restrict__ cu_seqlens, int batch, int unit_rows, int* out,
                                       int* tickets);
 
-int launch_varlen_prepare(const int32_t* cu_seqlens, int batch, int unit_rows, int* out, int* tickets, void* stream);
+int launch_varlen_prepare(const int32_t* cu_seqlens, int batch, int unit_rows, int* out, int* tickets, void* stream,
+                          bool overlap);
 
 }  // namespace fda

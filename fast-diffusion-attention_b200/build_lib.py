@@ -22,7 +22,7 @@ LIB = os.path.join(HERE, "fast_diffusion_attention", "libfda_sm100.so")
 TORCH_SRC = os.path.join(CSRC, "torch_binding.cpp")
 TORCH_EXT = os.path.join(HERE, "fast_diffusion_attention", "_fda_torch.so")
 TORCH_STAMP = os.path.join(OBJ, "_fda_torch.txt")   # what TORCH_EXT was built with
-SOURCES = ["abi.cu", "fwd_sm100.cu", "bwd_sm100.cu", "bwd_fused_sm100.cu", "bwd_wide_sm100.cu", "selftest_sm100.cu", "varlen_list.cu"]
+SOURCES = ["abi.cu", "fwd_sm100.cu", "bwd_sm100.cu", "bwd_fused_sm100.cu", "selftest_sm100.cu", "varlen_list.cu"]
 
 
 def _nvcc():

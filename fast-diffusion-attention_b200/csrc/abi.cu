@@ -115,7 +115,7 @@ int fda_device_status(int32_t* out4) {
   int32_t tmp[4];
   out4[0] = out4[1] = out4[2] = out4[3] = 0;
   int (*readers[])(int32_t*) = {fda::read_status_fwd, fda::read_status_bwd, fda::read_status_bwd_fused,
-                                 fda::read_status_bwd_wide, fda::read_status_selftest};
+                                 fda::read_status_selftest};
   for (auto reader : readers) {
     int rc = reader(tmp);
     if (rc) return rc;

@@ -241,43 +241,8 @@ inline int bwd_item_bound(const BwdParams& p, int heads) {
   return bound > (1 << 30) ? (1 << 30) : static_cast<int>(bound);
 }
 
-// Rows of the dQ accumulator come in blocks of 64. Every half of every sample starts at its own block: the
-// "+ 2 b + qh" gives each of the 2 * batch halves one block of slack, so rounding the start down never lets two
-// halves share a block. Returns the first accumulator row of query row `qa` (a multiple of 64) of half `qh` of a
-// sample whose first row in the packed row space is `grow0`.
-__device__ __forceinline__ int acc_row_of(int grow0, int n, int b, int qh, int qa) {
-  return ((grow0 + qh * n) / 64 + 2 * b + qh) * 64 + qa;
-}
-
 struct SubStep {
   int h, qh, sa, sb, cls;
 };
-
-// Calls fn(SubStep) for every non-skipped sub-step of the item, in order; stops early when fn returns false. A sub-step is one
-// 64-row half of a visible 128-row query tile of one query head of the group; a half with no visible row is skipped.
-template <typename Fn>
-__device__ __forceinline__ bool for_each_substep(const KvItem& it, const QueryPlan& plan, const KvSpans& spans, int group, Fn&& fn) {
-  for (int g = 0; g < group; ++g) {
-    for (int s = 0; s < plan.steps(); ++s) {
-      int qh, qt;
-      plan.step(s, it.kh, qh, qt);
-      const int qa = qt * kTile, qb = imin(qa + kTile, it.n);
-      if (spans.classify(qh, it.kh, qa, qb) == kTileSkip) continue;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        SubStep st;
-        st.sa = qa + half * kSub;
-        if (st.sa >= qb) continue;
-        st.sb = imin(st.sa + kSub, qb);
-        st.cls = spans.classify(qh, it.kh, st.sa, st.sb);
-        if (st.cls == kTileSkip) continue;
-        st.h = it.hk * group + g;
-        st.qh = qh;
-        if (!fn(st)) return false;
-      }
-    }
-  }
-  return true;
-}
 
 }  // namespace fda

@@ -98,6 +98,14 @@ struct FusedRoles {
   static_assert(128 * (kCmpWG * kComputeRegs + kProducerRegs + kDrainRegs) <= kThreads * kLaunchRegs, "register pool");
 };
 
+// Rows of the dQ accumulator come in blocks of 64. Every half of every sample starts at its own block: the
+// "+ 2 b + qh" gives each of the 2 * batch halves one block of slack, so rounding the start down never lets two
+// halves share a block. Returns the first accumulator row of query row `qa` (a multiple of 64) of half `qh` of a
+// sample whose first row in the packed row space is `grow0`.
+__device__ __forceinline__ int acc_row_of(int grow0, int n, int b, int qh, int qa) {
+  return ((grow0 + qh * n) / 64 + 2 * b + qh) * 64 + qa;
+}
+
 // One step of an item: a visible 128-row query tile of one query head. At most `left` steps follow it.
 struct QStep {
   int h, qh, qa, cls, left;
@@ -913,7 +921,7 @@ int64_t bwd_fused_acc_tiles(const FdaProblem& pr) {
 }
 
 size_t bwd_fused_acc_bytes(const FdaProblem& pr) {
-  const int d_round = pr.head_dim <= 64 ? 64 : pr.head_dim <= 128 ? 128 : 256;
+  const int d_round = pr.head_dim <= 64 ? 64 : 128;
   return static_cast<size_t>(pr.heads) * bwd_fused_acc_tiles(pr) * 64 * d_round * 4;
 }
 
@@ -959,17 +967,6 @@ bool bwd_chains_fit(const FdaProblem& pr, int tokens) {
   double longest, all, squares;
   known_tiles(pr, longest, all, squares);
   return pr.heads_k * (squares + 2 * all) >= kLine * longest;
-}
-
-// Whether heads wider than 128 take bwd_wide_kernel and the dV kernel instead of the split form's three passes. Its key tiles are
-// chains over all query heads of a group (the dQ kernel has an item for each head and query tile), so the longest must not be more
-// than a CTA's share, as above; and short items pay for the copy of V and the wait for the last dQ^T. Backward, split / this, us, heads
-// of 256, blocks of 16 and 512: 16 x 1000 tokens, 8 heads 320 / 365 and 403 / 427; 12 x 1536 432 / 448 and 497 / 480; 8 x 2000
-// 449 / 415 and 530 / 457, 16/8 heads 812 / 848 and 994 / 953; 5 x 3000, 8 heads 541 / 466 and 606 / 510, 16/8 1004 / 948 and
-// 1179 / 1050, 16/4 1095 / 1008 and 1169 / 1069; 2 x 8192, 8 heads 1202 / 964 and 1257 / 1029. Longest chain above the share: 4 x
-// 4096, 8/1 heads 1058 / 1690; 1 x 8192, 16/4 1374 / 2219.
-bool bwd_wide_pays(const FdaProblem& pr) {
-  return convert_rows(pr.heads, pr.heads_k, false) <= kMaxGridY && bwd_chains_fit(pr, 1400);
 }
 
 // Parts into which the query heads of a group are dealt. A key tile's steps are a chain, and those of the longest sample's first
@@ -1023,13 +1020,6 @@ int launch_bwd_fused(const BwdParams& p, int d_round, bool bf16, bool softcap, i
                      cudaStream_t stream) {
   return p.kv_split > 1 ? dispatch_fused<true>(p, d_round, bf16, softcap, sm_count, stages, stream)
                         : dispatch_fused<false>(p, d_round, bf16, softcap, sm_count, stages, stream);
-}
-
-// The convert kernel of head dims above 128 (bwd_wide_sm100.cu).
-int launch_wide_convert(const BwdParams& p, bool bf16, cudaStream_t stream) {
-  dim3 grid(p.n_pad / 64, convert_rows(p.heads, p.heads_k, false), p.batch);
-  return launch_kernel(p.overlap != 0, bf16 ? bwd_dq_convert_kernel<256, true, false, false> : bwd_dq_convert_kernel<256, false, false, false>, grid, 256, 0,
-                           stream, p);
 }
 
 int read_status_bwd_fused(int32_t* out4) {

@@ -162,6 +162,33 @@ struct DkdvCfg {
   static_assert((11 + 2 * kQSlots + 2 * kDoSlots + kStatSlots) * 8 + 8 <= 384, "barrier area");
 };
 
+// Calls fn(SubStep) for every non-skipped sub-step of the item, in order; stops early when fn returns false. A sub-step is one
+// 64-row half of a visible 128-row query tile of one query head of the group; a half with no visible row is skipped.
+template <typename Fn>
+__device__ __forceinline__ bool for_each_substep(const KvItem& it, const QueryPlan& plan, const KvSpans& spans, int group, Fn&& fn) {
+  for (int g = 0; g < group; ++g) {
+    for (int s = 0; s < plan.steps(); ++s) {
+      int qh, qt;
+      plan.step(s, it.kh, qh, qt);
+      const int qa = qt * kTile, qb = imin(qa + kTile, it.n);
+      if (spans.classify(qh, it.kh, qa, qb) == kTileSkip) continue;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        SubStep st;
+        st.sa = qa + half * kSub;
+        if (st.sa >= qb) continue;
+        st.sb = imin(st.sa + kSub, qb);
+        st.cls = spans.classify(qh, it.kh, st.sa, st.sb);
+        if (st.cls == kTileSkip) continue;
+        st.h = it.hk * group + g;
+        st.qh = qh;
+        if (!fn(st)) return false;
+      }
+    }
+  }
+  return true;
+}
+
 // One CTA per SM. A sub-step is one 64-row half of a visible 128-row query tile of one query head of the group; a half with
 // no visible row is skipped.
 template <int kHeadDim, int kStages, bool kBf16, bool kSoftcap, int kMakes>
@@ -984,14 +1011,14 @@ int launch_dkdv(const BwdParams& p, int sm_count, cudaStream_t stream) {
   return FDA_OK;
 }
 
-template <int kHeadDim, int kStagesKv, int kStagesQ, bool kBf16, bool kSoftcap, bool kDvOnly>
+template <int kHeadDim, int kStagesKv, int kStagesQ, bool kBf16, bool kSoftcap>
 int launch_bwd_instance(const BwdParams& p, int sm_count, unsigned stages, cudaStream_t stream) {
   if (stages & 2u) {
     int rc;
     if constexpr (kHeadDim > 128) {
-      if (kDvOnly || p.apart) {
+      if (p.apart) {
         rc = launch_dkdv<kHeadDim, kStagesKv, kBf16, kSoftcap, 2>(p, sm_count, stream);
-        if (rc == FDA_OK && !kDvOnly) {
+        if (rc == FDA_OK) {
           BwdParams q = p;
           q.ticket_kv = p.ticket_kv + 16;   // a counter of its own
           rc = launch_dkdv<kHeadDim, kStagesKv, kBf16, kSoftcap, 1>(q, sm_count, stream);
@@ -1004,7 +1031,7 @@ int launch_bwd_instance(const BwdParams& p, int sm_count, unsigned stages, cudaS
     }
     if (rc) return rc;
   }
-  if (!kDvOnly && (stages & 4u)) {
+  if (stages & 4u) {
     using Cfg = DqCfg<kHeadDim, kStagesQ>;
     auto kernel = bwd_dq_kernel<kHeadDim, kStagesQ, kBf16, kSoftcap>;
     static PerDeviceFlags smem_set;
@@ -1017,26 +1044,22 @@ int launch_bwd_instance(const BwdParams& p, int sm_count, unsigned stages, cudaS
   return FDA_OK;
 }
 
-template <int kHeadDim, int kStagesKv, int kStagesQ, bool kDvOnly = false>
+template <int kHeadDim, int kStagesKv, int kStagesQ>
 int dispatch_bwd(const BwdParams& p, int sm_count, bool bf16, bool softcap, unsigned stages, cudaStream_t stream) {
   if (bf16) {
-    return softcap ? launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, true, true, kDvOnly>(p, sm_count, stages, stream)
-                   : launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, true, false, kDvOnly>(p, sm_count, stages, stream);
+    return softcap ? launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, true, true>(p, sm_count, stages, stream)
+                   : launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, true, false>(p, sm_count, stages, stream);
   }
-  return softcap ? launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, false, true, kDvOnly>(p, sm_count, stages, stream)
-                 : launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, false, false, kDvOnly>(p, sm_count, stages, stream);
+  return softcap ? launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, false, true>(p, sm_count, stages, stream)
+                 : launch_bwd_instance<kHeadDim, kStagesKv, kStagesQ, false, false>(p, sm_count, stages, stream);
 }
 
 inline int64_t round_up64(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
 
 }  // namespace
 
-// bwd_wide_sm100.cu
-int launch_bwd_wide(const BwdParams& p, bool bf16, bool softcap, int sm_count, cudaStream_t stream);
 // bwd_fused_sm100.cu
 bool bwd_chains_fit(const FdaProblem& pr, int tokens);
-bool bwd_wide_pays(const FdaProblem& pr);
-int launch_wide_convert(const BwdParams& p, bool bf16, cudaStream_t stream);
 size_t bwd_fused_acc_bytes(const FdaProblem& pr);
 int64_t bwd_fused_acc_tiles(const FdaProblem& pr);
 int bwd_fused_kv_split(const FdaProblem& pr);
@@ -1048,9 +1071,6 @@ constexpr int64_t kSmallAccBytes = 32 << 20;
 
 // The single-pass backward adds dQ partials in an order that depends on scheduling and needs head dim <= 128.
 bool bwd_single_pass(const FdaProblem& pr) { return pr.deterministic == 0 && pr.head_dim <= 128; }
-
-// Head dims above 128: dK and dQ in one kernel, dV in another (bwd_wide_sm100.cu). dQ's partials are added in such an order too.
-bool bwd_wide(const FdaProblem& pr) { return pr.deterministic == 0 && pr.head_dim > 128 && bwd_wide_pays(pr); }
 
 // Scratch of the split backward: delta_pad then lse2_pad, each batch * heads * 2 * n_pad floats (256-byte aligned
 // pieces), then 256 bytes of work counters.
@@ -1064,7 +1084,6 @@ size_t bwd_split_workspace_bytes(const FdaProblem& pr) {
 // The single-pass backward keeps its fp32 dQ accumulator behind that, and behind it parts of dK and dV where it makes some.
 size_t bwd_workspace_bytes(const FdaProblem& pr) {
   size_t bytes = bwd_split_workspace_bytes(pr);
-  if (bwd_wide(pr)) bytes += bwd_fused_acc_bytes(pr);
   if (bwd_single_pass(pr)) {
     bytes += static_cast<size_t>(round_up64(static_cast<int64_t>(bwd_fused_acc_bytes(pr)), 256)) + bwd_fused_part_bytes(pr);
   }
@@ -1093,7 +1112,6 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   // ones and those whose longest chain is more than a CTA's share stay together (32 x 512 tokens 246 / 264; 1 x 16384, 8/2 heads
   // 2360 / 3140).
   p.apart = d > 128 && bwd_chains_fit(pr, 700) ? 1 : 0;
-  const bool wide = bwd_wide(pr) && (stage_mask & FDA_BWD_FORCE_SPLIT) == 0;
   auto encode = [&](CUtensorMap* map, const FdaTensor& t, int heads, int box_rows) {
     return encode_tile_map(map, t.ptr, 2, false, fp16, d, rows, heads, tma_batch, t.row_stride, t.head_stride,
                            t.batch_stride, 64, box_rows);
@@ -1106,7 +1124,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   if (!single_pass && ((rc = encode(&p.tm_q64, a.q, pr.heads, kSub)) || (rc = encode(&p.tm_do64, a.dout, pr.heads, kSub)))) {
     return rc;
   }
-  if (!single_pass && !wide && d > 128 && ((rc = encode(&p.tm_k64, a.k, pr.heads_k, 64)) || (rc = encode(&p.tm_v64, a.v, pr.heads_k, 64)))) {
+  if (!single_pass && d > 128 && ((rc = encode(&p.tm_k64, a.k, pr.heads_k, 64)) || (rc = encode(&p.tm_v64, a.v, pr.heads_k, 64)))) {
     return rc;
   }
   // the preprocess and the epilogues use 16-byte vector accesses on rows of out / dout / dq / dk / dv
@@ -1157,13 +1175,11 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   p.lse2_pad = reinterpret_cast<float*>(static_cast<uint8_t*>(a.workspace) + one);
   p.ticket_kv = reinterpret_cast<int*>(static_cast<uint8_t*>(a.workspace) + 2 * one);
   p.ticket_q = p.ticket_kv + 32;
-  if (single_pass || wide) {
+  if (single_pass) {
     if (a.workspace_bytes < bwd_workspace_bytes(pr)) return FDA_ERR_WORKSPACE;
     p.dq_acc = reinterpret_cast<float*>(static_cast<uint8_t*>(a.workspace) + bwd_split_workspace_bytes(pr));
     p.acc_tiles = static_cast<int>(bwd_fused_acc_tiles(pr));
     p.acc_floats = static_cast<int64_t>(bwd_fused_acc_bytes(pr) / 4);
-  }
-  if (single_pass) {
     p.kv_split = bwd_fused_kv_split(pr);
     p.part_floats = static_cast<int64_t>(bwd_fused_part_bytes(pr) / 4);
     if (p.kv_split > 1) p.dkv_part = p.dq_acc + round_up64(p.acc_floats, 64);
@@ -1181,7 +1197,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   // with max_seqlen as it is, 1161 / 1168 with three times that, 1225 / 1256 with four, 1474 / 1537 with eight. (Small
   // accumulators are always filled there: the launch counts for more.)
   const int64_t padded_rows = static_cast<int64_t>(pr.batch) * 2 * p.n_pad, acc_rows = static_cast<int64_t>(p.acc_tiles) * 64;
-  if ((single_pass || wide) && (stage_mask & 3u) == 3u && (padded_rows <= 3 * acc_rows || p.acc_floats * 4 <= kSmallAccBytes)) {
+  if (single_pass && (stage_mask & 3u) == 3u && (padded_rows <= 3 * acc_rows || p.acc_floats * 4 <= kSmallAccBytes)) {
     p.zero_acc16 = p.acc_floats / 4;
   }
   if (varlen) {
@@ -1210,7 +1226,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
     // dK/dV: the noisy key tiles (the second half of the ranks) are short; dQ: the shortest eighth (fractions
     // found by measurement on the benchmark shape); few items per CTA: rank for rank over all of them
     const int per_bh = 2 * p.tiles_per_half;
-    const int parts = single_pass ? p.kv_split : 1;   // (nor does bwd_wide_kernel deal out a group's heads)
+    const int parts = single_pass ? p.kv_split : 1;
     p.n_long_kv = order_n_long(per_bh, FDA_SHORT8_KV, static_cast<long long>(per_bh) * pr.batch * pr.heads_k * parts, sm_count);
     p.n_long_q = order_n_long(per_bh, FDA_SHORT8_Q, static_cast<long long>(per_bh) * pr.batch * pr.heads, sm_count);
   }
@@ -1228,16 +1244,6 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
     if (rc) return rc;
   }
   if (single_pass) return launch_bwd_fused(p, d_round, bf16, softcap, sm_count, stage_mask, stream);
-  if (wide) {
-    if (stage_mask & 2u) {
-      if (p.zero_acc16 == 0) FDA_CUDA_TRY(cudaMemsetAsync(p.dq_acc, 0, static_cast<size_t>(p.acc_floats) * 4, stream));
-      if ((rc = dispatch_bwd<256, 1, 3, true>(p, sm_count, bf16, softcap, 2u, stream)) ||
-          (rc = launch_bwd_wide(p, bf16, softcap, sm_count, stream))) {
-        return rc;
-      }
-    }
-    return stage_mask & 4u ? launch_wide_convert(p, bf16, stream) : FDA_OK;
-  }
   if (d_round == 64) return dispatch_bwd<64, 6, 7>(p, sm_count, bf16, softcap, stage_mask, stream);
   if (d_round == 128) return dispatch_bwd<128, 4, 5>(p, sm_count, bf16, softcap, stage_mask, stream);
   return dispatch_bwd<256, 1, 3>(p, sm_count, bf16, softcap, stage_mask, stream);

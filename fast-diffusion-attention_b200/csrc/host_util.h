@@ -172,7 +172,6 @@ int launch_selftest_wait(long long limit_cycles, cudaStream_t stream);
 int read_status_fwd(int32_t* out4);
 int read_status_bwd(int32_t* out4);
 int read_status_bwd_fused(int32_t* out4);
-int read_status_bwd_wide(int32_t* out4);
 int read_status_selftest(int32_t* out4);
 
 }  // namespace fda

@@ -113,13 +113,11 @@ int fda_bwd(const FdaBwdArgs* args, void* stream);
  * stages as separate launches (csrc/fda/flash_bwd_launch_template.h:47-239).
  * The backward has two forms. The single-pass form (deterministic == 0 and head_dim <= 128) computes dK, dV and
  * the partial dQ of every (key tile, query tile) pair in one kernel and adds the partials into an fp32
- * accumulator in the workspace; the order of those adds varies from run to run. With deterministic == 0 and
- * head_dim > 128, samples of 1400 tokens a half and more take a kernel for dV and one for dK and the partial dQ, which
- * are added up likewise, where that keeps all SMs busy. The split form (everything
+ * accumulator in the workspace; the order of those adds varies from run to run. The split form (everything
  * else, or FDA_BWD_FORCE_SPLIT) runs a dK/dV kernel and a dQ kernel with no cross-block reduction; its result
  * is bitwise reproducible. */
 #define FDA_BWD_STAGE_PREPROCESS 1u /* delta = rowsum(dO * O) and -LSE * log2(e) into the workspace */
-#define FDA_BWD_STAGE_MAIN 2u       /* single-pass kernel (with its accumulator zero-fill), the two kernels, or the dK/dV kernel */
+#define FDA_BWD_STAGE_MAIN 2u       /* single-pass kernel (with its accumulator zero-fill), or the dK/dV kernel */
 #define FDA_BWD_STAGE_DQ 4u         /* accumulator -> dQ conversion, or the dQ kernel */
 #define FDA_BWD_FORCE_SPLIT 8u      /* use the split form even where the single-pass form applies */
 int fda_bwd_stages(const FdaBwdArgs* args, unsigned stage_mask, void* stream);

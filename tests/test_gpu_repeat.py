@@ -32,6 +32,8 @@ def _step(q, k, v, do, bs, cu=None, max_len=None, **kw):
     (8, 2, 128, 96, 1100, 3),       # grouped heads, masked tiles, partial last tile
     (6, 6, 64, 32, 1500, 4),
     (4, 4, 256, 128, 1024, 2),
+    (10, 10, 256, 64, 1500, 2),     # wide heads, samples long and heads many enough for dK and dV items in launches of their own
+    (20, 10, 136, 96, 2100, 2),
 ])
 def test_bitwise_stable_over_repetitions(heads, heads_k, d, bs, n, batch, deterministic):
     torch.manual_seed(7)

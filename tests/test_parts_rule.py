@@ -34,6 +34,14 @@ def _packed(ns, max_n=None):
     return dict(seqlen=2 * (max_n or max(ns)), batch=len(ns), total=2 * sum(ns))
 
 
+@pytest.mark.parametrize("d", [136, 192, 256])
+def test_wide_heads_need_no_accumulator(d):
+    """Above head dim 128 the default backward is the deterministic one: the same bits in every run, and the same workspace."""
+    for kw in (dict(seqlen=16384, heads=8, heads_k=8, batch=2), dict(seqlen=2800, heads=20, heads_k=10, batch=2),
+               dict(heads=32, heads_k=8, **_packed([4095, 1203, 2750, 3391, 1876, 2049]))):
+        assert _bytes(d=d, **kw) == _bytes(d=d, deterministic=1, **kw)
+
+
 def test_few_tokens_and_few_heads_are_dealt_out():
     assert parts(2000, 8, 1, 128, batch=1)[0] == 8
     assert parts(8192, 8, 2, 128, batch=1)[0] == 4

@@ -8,6 +8,7 @@ namespace fda {
 
 size_t bwd_workspace_bytes(const FdaProblem& p);  // bwd_sm100.cu
 size_t fwd_workspace_bytes(const FdaProblem& p);  // fwd_sm100.cu
+bool forward_full_loop(const FdaProblem& p);      // fwd_sm100.cu
 
 namespace {
 
@@ -176,6 +177,11 @@ int fda_geom_item_order(int idx, int per_group, int n_groups, int short8, int ct
   *out_group = group;
   *out_rank = rank;
   return 0;
+}
+
+unsigned fda_launch_choices(const FdaProblem* p) {
+  if (!p || fda::check_problem(*p, false) != FDA_OK) return 0;
+  return fda::forward_full_loop(*p) ? FDA_CHOICE_FORWARD_FULL_LOOP : 0u;
 }
 
 int fda_selftest_wait(long long limit_cycles, void* stream) {

@@ -214,8 +214,6 @@ struct FwdConfig {
   // The loop over fully visible sub-steps takes two of them, one a buffer, where that is not too much code: head dim 64 (4 x 8192
   // tokens, 32 heads: 768 / 753 us; capped 1284 / 1253) and e4m3 (2 x 16384 tokens, 8 heads of 256: 813 / 788; 4 x 8192, 16/4
   // heads of 128: 531 / 519); 16-bit at 128 loses by it (1 x 16384, 32/8 heads 884 / 913), at 256 too (1081 / 1101).
-  // 16-bit heads of 256, which wait for K and V, get one loop for all (two loops 1 % slower).
-  static constexpr bool kFullLoop = kHeadDim < 256 || kFp8;
   static constexpr bool kUnrollFull = kHeadDim == 64 || kFp8;
   static constexpr int kPCols = kSubKeys * kElemBytes / 4;            // tensor-memory columns of the packed P
 };
@@ -237,7 +235,8 @@ struct FwdConfig {
 // part in waits and loop control, one elected lane issues, which keeps descriptors and counters in uniform registers.)
 constexpr uint32_t kInfoFirst = 16, kInfoLast = 32, kInfoHalf1 = 64, kInfoStop = 128, kInfoTile0 = 256, kInfoQ = 1024;  // bit 2 t + h: tile t sees half h
 
-template <int kHeadDim, int kQTiles, int kType, bool kSoftcap, bool kQInTmem>
+// kFullLoop: fully visible sub-steps have a loop of their own (see forward_full_loop).
+template <int kHeadDim, int kQTiles, int kType, bool kSoftcap, bool kQInTmem, bool kFullLoop>
 __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fwd_kernel(const __grid_constant__ FwdParams p) {
   using Cfg = FwdConfig<kHeadDim, kQTiles, kType, kSoftcap, kQInTmem>;
   constexpr int kStages = 2 * Cfg::kPairs;         // slot 2 i: K of pair i, slot 2 i + 1: its V
@@ -624,10 +623,9 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       float m_run = -INFINITY;  // reference maximum (unscaled scores, or tanh values with softcap)
       float l_run = 0.f;
       bool o_started = false, settled = false;   // one sub-step, two sub-steps of this tile are done
-      // The clean keys come first, and the first n_full sub-steps of them this tile sees in full: they have a loop of their own
-      // without classification and mask (1 x 16384 tokens, 32/8 heads of 128: 919 -> 884 us; 4 x 8192, 32 heads of 64: 792 -> 768;
-      // e4m3, 2 x 16384, 8 heads of 256: 850 -> 813).
-      const int n_full = Cfg::kFullLoop ? uni(imin(spans.half[1].hi_first / kSubKeys, plan.n_clean * Cfg::kHalves)) : 0;
+      // The clean keys come first, and the first n_full sub-steps of them this tile sees in full: with long samples they have a loop
+      // of their own without classification and mask.
+      const int n_full = kFullLoop ? uni(imin(spans.half[1].hi_first / kSubKeys, plan.n_clean * Cfg::kHalves)) : 0;
       auto sub_step = [&](auto full_tag, int u, const int buf) {
         constexpr bool kFull = decltype(full_tag)::value;
         int kh = 1, k0 = 0, cls = kTileFull;
@@ -866,10 +864,10 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
   if (warp == Cfg::kLoadWarp) ptx::tmem_dealloc(tmem, 512);
 }
 
-template <int kHeadDim, int kQTiles, int kType, bool kSoftcap, bool kQInTmem>
+template <int kHeadDim, int kQTiles, int kType, bool kSoftcap, bool kQInTmem, bool kFullLoop>
 int launch_fwd_instance(const FwdParams& p, int grid, cudaStream_t stream) {
   using Cfg = FwdConfig<kHeadDim, kQTiles, kType, kSoftcap, kQInTmem>;
-  auto kernel = fwd_kernel<kHeadDim, kQTiles, kType, kSoftcap, kQInTmem>;
+  auto kernel = fwd_kernel<kHeadDim, kQTiles, kType, kSoftcap, kQInTmem, kFullLoop>;
   static PerDeviceFlags smem_set;
   const int rc = set_dynamic_smem(kernel, Cfg::kSmemBytes, smem_set);
   if (rc) return rc;
@@ -877,20 +875,23 @@ int launch_fwd_instance(const FwdParams& p, int grid, cudaStream_t stream) {
   return FDA_OK;
 }
 
-template <int kHeadDim, int kQTiles, bool kQInTmem = false>
-int dispatch_fwd(const FwdParams& p, int grid, bool bf16, bool softcap, cudaStream_t stream) {
-  if (bf16) {
-    return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 0, true, kQInTmem>(p, grid, stream)
-                   : launch_fwd_instance<kHeadDim, kQTiles, 0, false, kQInTmem>(p, grid, stream);
+template <int kHeadDim, int kQTiles, int kType, bool kQInTmem>
+int dispatch_fwd(const FwdParams& p, int grid, bool softcap, bool full_loop, cudaStream_t stream) {
+  // who has the loop over fully visible sub-steps: see forward_full_loop
+  constexpr bool kHas = kHeadDim <= 128 || kType == 2;
+  constexpr bool kHasCapped = kHas && !(kHeadDim == 128 && kType != 2);
+  if (softcap) {
+    return kHasCapped && full_loop ? launch_fwd_instance<kHeadDim, kQTiles, kType, true, kQInTmem, kHasCapped>(p, grid, stream)
+                                   : launch_fwd_instance<kHeadDim, kQTiles, kType, true, kQInTmem, false>(p, grid, stream);
   }
-  return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 1, true, kQInTmem>(p, grid, stream)
-                 : launch_fwd_instance<kHeadDim, kQTiles, 1, false, kQInTmem>(p, grid, stream);
+  return kHas && full_loop ? launch_fwd_instance<kHeadDim, kQTiles, kType, false, kQInTmem, kHas>(p, grid, stream)
+                           : launch_fwd_instance<kHeadDim, kQTiles, kType, false, kQInTmem, false>(p, grid, stream);
 }
 
 template <int kHeadDim, int kQTiles, bool kQInTmem = false>
-int dispatch_fwd_fp8(const FwdParams& p, int grid, bool softcap, cudaStream_t stream) {
-  return softcap ? launch_fwd_instance<kHeadDim, kQTiles, 2, true, kQInTmem>(p, grid, stream)
-                 : launch_fwd_instance<kHeadDim, kQTiles, 2, false, kQInTmem>(p, grid, stream);
+int dispatch_fwd16(const FwdParams& p, int grid, bool bf16, bool softcap, bool full_loop, cudaStream_t stream) {
+  return bf16 ? dispatch_fwd<kHeadDim, kQTiles, 0, kQInTmem>(p, grid, softcap, full_loop, stream)
+              : dispatch_fwd<kHeadDim, kQTiles, 1, kQInTmem>(p, grid, softcap, full_loop, stream);
 }
 
 }  // namespace
@@ -898,6 +899,32 @@ int dispatch_fwd_fp8(const FwdParams& p, int grid, bool softcap, cudaStream_t st
 size_t fwd_workspace_bytes(const FdaProblem& pr) {
   // scheduler words, and for packed batches the work list
   return 256 + (pr.cu_seqlens != nullptr ? varlen_list_bytes(pr.batch) : 0);
+}
+
+// Whether fully visible sub-steps get a loop of their own. It saves their classification and mask, and makes a second and a
+// third copy of a long body. Where CTAs take many items of few sub-steps each, or of few that the loop takes (noisy rows of large
+// blocks see no clean key in full), the warps run from one copy into another and wait for instructions. One loop / two, us, d = 64, d =
+// 128, e4m3, e4m3 of 256 (16/8 heads, blocks of 64):
+//   32 x 1024 tokens  111 / 142  138 / 160  135 / 188  238 / 277      4 x 6000   257 / 252  313 / 311  327 / 323  550 / 538
+//   8 x 3000          157 / 164  183 / 190  197 / 219  332 / 355      3 x 8192   322 / 313  395 / 391  413 / 398  692 / 663
+//   8 x 4096          248 / 252  302 / 301  314 / 331  535 / 550      1 x 16384  383 / 370  489 / 481  491 / 468  826 / 782
+// 3 x 8192 in blocks of 1024: 349 / 349, 466 / 451, 474 / 450, 802 / 768; in one block: 558 / 580, 737 / 760, 747 / 737, 1223 / 1223.
+// Capped, 3 x 8192: 499 / 492, 525 / 526 (so not there), 605 / 577, 898 / 846. With at most eight items a CTA the loop loses nothing from
+// 2000 tokens on (blocks of 16): 1 x 2000, 8 heads 20.0 / 18.7, 20.7 / 20.7, 22.7 / 22.2, 26.8 / 25.0; 1 x 3000, 16 heads 35.7 / 33.1,
+// 39.1 / 38.6, 43.3 / 40.8, 55.9 / 55.4; 1 x 6000, 3 heads 38.8 / 35.2, 41.2 / 40.7, 46.8 / 43.3, 49.7 / 49.9; 1 x 4096, 16 heads in
+// one block 69.1 / 69.9, 78.8 / 79.7, 88.7 / 88.0, 141 / 137. 16-bit heads of 256, which wait for K and V, get one loop for all (1 %
+// the other way).
+bool forward_full_loop(const FdaProblem& pr) {
+  if (pr.batch <= 0) return false;
+  const int64_t tokens = pr.total / (2 * static_cast<int64_t>(pr.batch));   // of a half, on average
+  const bool fp8 = pr.dtype == FDA_E4M3;
+  if (!fp8 && (pr.head_dim > 128 || (pr.head_dim > 64 && pr.softcap > 0.f))) return false;
+  const int item_rows = pr.head_dim > 128 ? kBlockM : 2 * kBlockM;
+  const int64_t items = (tokens + item_rows - 1) / item_rows * 2 * pr.heads * pr.batch;
+  const bool few = items <= 8 * 148;
+  if (fp8) return tokens >= (few ? 1000 : 3000);
+  if (pr.head_dim <= 64) return tokens >= (few ? 1000 : 4096) && (few ? 2 : 4) * static_cast<int64_t>(pr.block_size) <= tokens;
+  return tokens >= (few ? 2048 : 4096) && 4 * static_cast<int64_t>(pr.block_size) <= tokens;
 }
 
 int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
@@ -1009,17 +1036,19 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
     FDA_CUDA_TRY(cudaMemsetAsync(p.ticket, 0, kTicketInts * 4, stream));
   }
   const bool bf16 = pr.dtype == FDA_BF16;
+  const bool full_loop = forward_full_loop(pr);
   if (fp8) {
-    if (d_round == 256) return dispatch_fwd_fp8<256, 1, true>(p, grid, softcap, stream);
-    return q_tiles == 2 ? dispatch_fwd_fp8<128, 2>(p, grid, softcap, stream) : dispatch_fwd_fp8<128, 1>(p, grid, softcap, stream);
+    if (d_round == 256) return dispatch_fwd<256, 1, 2, true>(p, grid, softcap, full_loop, stream);
+    return q_tiles == 2 ? dispatch_fwd<128, 2, 2, false>(p, grid, softcap, full_loop, stream)
+                        : dispatch_fwd<128, 1, 2, false>(p, grid, softcap, full_loop, stream);
   }
-  if (d_round == 256) {
-    return dispatch_fwd<256, 1, true>(p, grid, bf16, softcap, stream);
-  }
+  if (d_round == 256) return dispatch_fwd16<256, 1, true>(p, grid, bf16, softcap, full_loop, stream);
   if (d_round == 128) {
-    return q_tiles == 2 ? dispatch_fwd<128, 2>(p, grid, bf16, softcap, stream) : dispatch_fwd<128, 1>(p, grid, bf16, softcap, stream);
+    return q_tiles == 2 ? dispatch_fwd16<128, 2>(p, grid, bf16, softcap, full_loop, stream)
+                        : dispatch_fwd16<128, 1>(p, grid, bf16, softcap, full_loop, stream);
   }
-  return q_tiles == 2 ? dispatch_fwd<64, 2>(p, grid, bf16, softcap, stream) : dispatch_fwd<64, 1>(p, grid, bf16, softcap, stream);
+  return q_tiles == 2 ? dispatch_fwd16<64, 2>(p, grid, bf16, softcap, full_loop, stream)
+                      : dispatch_fwd16<64, 1>(p, grid, bf16, softcap, full_loop, stream);
 }
 
 int read_status_fwd(int32_t* out4) {

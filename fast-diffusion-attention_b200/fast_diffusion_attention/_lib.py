@@ -15,6 +15,9 @@ LIB_PATH = os.environ.get("FDA_LIBRARY") or os.path.join(_HERE, "libfda_sm100.so
 
 FDA_BF16, FDA_FP16, FDA_E4M3 = 0, 1, 2
 
+# bits of fda_launch_choices
+FDA_CHOICE_FORWARD_FULL_LOOP = 1
+
 FDA_OK = 0
 FDA_ERR_DEVICE_WAIT = 14
 FDA_ERR_SCRATCH_LIMIT = 15
@@ -50,7 +53,8 @@ class FdaBwdArgs(C.Structure):
 EXPORTS = [
     "fda_fwd_workspace_bytes", "fda_bwd_workspace_bytes", "fda_fwd", "fda_bwd", "fda_bwd_stages", "fda_bwd_noalloc", "fda_strerror",
     "fda_last_cuda_error", "fda_device_status", "fda_version", "fda_geom_key_plan", "fda_geom_query_plan",
-    "fda_geom_classify", "fda_geom_item_order", "fda_selftest_umma", "fda_selftest_wait",
+    "fda_geom_classify", "fda_geom_item_order", "fda_launch_choices",
+    "fda_selftest_umma", "fda_selftest_wait",
 ]
 
 _lib = None
@@ -92,6 +96,8 @@ def load():
     lib.fda_geom_classify.argtypes = [C.c_int] * 10
     lib.fda_geom_item_order.restype = C.c_int
     lib.fda_geom_item_order.argtypes = [C.c_int] * 5 + [C.POINTER(C.c_int32), C.POINTER(C.c_int32)]
+    lib.fda_launch_choices.restype = C.c_uint
+    lib.fda_launch_choices.argtypes = [C.POINTER(FdaProblem)]
     lib.fda_selftest_umma.restype = C.c_int
     lib.fda_selftest_umma.argtypes = [C.c_int, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_void_p]
     lib.fda_selftest_wait.restype = C.c_int

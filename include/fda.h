@@ -172,6 +172,11 @@ int fda_geom_classify(int qh, int kh, int qa, int qb, int k0, int bn, int n, int
  * reference (its schedulers are tile_scheduler.hpp:51-482 there). */
 int fda_geom_item_order(int idx, int per_group, int n_groups, int short8, int ctas, int32_t* out_group, int32_t* out_rank);
 
+/* ---- host-only probe of the launchers' rules (no GPU needed); used by their unit tests ------------------ */
+/* Which forms of the kernels a problem takes, as a sum of the bits below; 0 for a problem that fda_fwd refuses. */
+#define FDA_CHOICE_FORWARD_FULL_LOOP 1u /* forward: fully visible sub-steps in a loop of their own */
+unsigned fda_launch_choices(const FdaProblem* p);
+
 /* ---- tensor-core self test (GPU): C[128 x n] = A[128 x k] * B with the operand layouts the kernels use ---- */
 /* mode 0: A, B both K-major from shared memory; mode 1: A from tensor memory, B MN-major from shared memory;
  * mode 2: A and B both MN-major from shared memory (the dQ^T product of the single-pass backward).

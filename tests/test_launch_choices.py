@@ -1,0 +1,60 @@
+"""Which forms of the kernels a call takes, by the launchers' own rules (no GPU needed), and, on the GPU, that forms chosen for speed
+alone give the same bits."""
+
+import ctypes as C
+
+import pytest
+import torch
+
+from fast_diffusion_attention import _lib, diffusion_attn_varlen_func
+
+
+def _choices(seqlen, heads, heads_k, d, bs=64, *, batch=1, total=None, dtype=_lib.FDA_BF16, softcap=0.0, sm_margin=0, deterministic=0):
+    packed = total is not None
+    p = _lib.FdaProblem(dtype, batch, seqlen, total if packed else batch * seqlen, heads, heads_k, d, bs, 0.1, softcap, sm_margin,
+                        deterministic, C.c_void_p(256) if packed else None)
+    return _lib.load().fda_launch_choices(C.byref(p))
+
+
+@pytest.mark.parametrize("dtype,d,softcap,line,few", [(_lib.FDA_BF16, 64, 0.0, 4096, 1000), (_lib.FDA_FP16, 96, 0.0, 4096, 2048),
+                                                      (_lib.FDA_BF16, 64, 30.0, 4096, 1000), (_lib.FDA_E4M3, 64, 0.0, 3000, 1000),
+                                                      (_lib.FDA_E4M3, 256, 30.0, 3000, 1000)])
+def test_only_long_samples_have_a_loop_for_full_sub_steps(dtype, d, softcap, line, few):
+    def takes(n, bs=64, heads=16, **kw):
+        return bool(_choices(2 * n, heads, heads, d, bs, dtype=dtype, softcap=softcap, **kw) & _lib.FDA_CHOICE_FORWARD_FULL_LOOP)
+
+    assert takes(line, batch=4) and takes(line, batch=16) and takes(8192, bs=2048, batch=4)
+    for n in (64, 256, 512, 1024, 1500, 2048, line - 1):
+        assert not takes(n, batch=128)
+    assert takes(few, heads=2) and not takes(few - 1, heads=2) and not takes(512, heads=1)   # few items a CTA
+    assert not takes(8192, batch=41, total=2 * (8192 + 40 * 300))     # one long sample among short ones
+    assert not takes(32768, batch=64, total=2 * 64 * 512)             # max_seqlen is an upper bound
+    assert takes(8192, bs=8192, batch=4) == (dtype == _lib.FDA_E4M3)  # noisy rows of one block see no clean key
+
+
+def test_who_has_no_such_loop():
+    for kw in (dict(d=256), dict(d=136), dict(d=128, softcap=30.0), dict(d=72, softcap=30.0)):
+        assert not _choices(16384, 16, 8, **kw) & _lib.FDA_CHOICE_FORWARD_FULL_LOOP
+    assert _choices(16384, 16, 8, d=60) == 0   # refused
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,bs", [(4096, 1), (4097, 64), (4100, 300), (4159, 1024)])
+@pytest.mark.parametrize("dtype,d,softcap", [(torch.bfloat16, 64, 0.0), (torch.float16, 128, 0.0), (torch.bfloat16, 64, 20.0),
+                                             (torch.float8_e4m3fn, 128, 0.0), (torch.float8_e4m3fn, 256, 20.0)])
+def test_both_loops_give_the_same_bits(n, bs, dtype, d, softcap):
+    """A sample alone, and in front of short ones that take the mean length below the line."""
+    torch.manual_seed(n)
+    q, k, v = (torch.randn(2 * n + 512, h, d, device="cuda").to(dtype) for h in (4, 2, 2))
+    code = {torch.bfloat16: _lib.FDA_BF16, torch.float16: _lib.FDA_FP16}.get(dtype, _lib.FDA_E4M3)
+    outs = []
+    for ns in ([n], [n] + [32] * 8):
+        total = 2 * sum(ns)
+        assert bool(_choices(2 * n, 4, 2, d, bs, batch=len(ns), total=total, dtype=code, softcap=softcap) & 1) == (len(ns) == 1)
+        cu = torch.tensor([0] + ns, device="cuda").cumsum(0).int() * 2
+        out, lse = diffusion_attn_varlen_func(q[:total], k[:total], v[:total], cu, cu, 2 * n, 2 * n, bs, softcap=softcap,
+                                              return_attn_probs=True)
+        outs.append((out[:2 * n], lse[:, :2 * n]))
+    torch.cuda.synchronize()
+    assert _lib.device_status()[0] == 0
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])

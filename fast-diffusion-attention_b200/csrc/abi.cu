@@ -181,7 +181,8 @@ int fda_geom_item_order(int idx, int per_group, int n_groups, int short8, int ct
 
 unsigned fda_launch_choices(const FdaProblem* p) {
   if (!p || fda::check_problem(*p, false) != FDA_OK) return 0;
-  return fda::forward_full_loop(*p) ? FDA_CHOICE_FORWARD_FULL_LOOP : 0u;
+  return (fda::forward_full_loop(*p) ? FDA_CHOICE_FORWARD_FULL_LOOP : 0u) |
+         (fda::overlapped_launches(*p) ? FDA_CHOICE_FORWARD_OVERLAP | FDA_CHOICE_BACKWARD_OVERLAP : 0u);
 }
 
 int fda_selftest_wait(long long limit_cycles, void* stream) {

@@ -55,6 +55,7 @@ struct BwdParams {
   VarlenList vl;     // packed batches: samples longest first with running 128-row tile counts (base == nullptr otherwise)
   int wide_store;      // dq/dk/dv rows allow 32-byte stores
   int overlap;         // host: overlapped_launches
+  int next_early;      // the next kernel may start early: no SMs are kept free
   float scale_log2, softcap_pre, softmax_scale;
   int apart;            // split backward, head dims above 128: dV items in a launch of their own
   int kv_split;         // single-pass backward: parts into which a key tile's query heads are dealt (a divisor of the group)

@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
   __syncthreads();
   ptx::tc_fence_after();
   ptx::wait_for_stream();
-  ptx::let_next_start();
+  if (p.next_early) ptx::let_next_start();
   const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int group = p.heads / p.heads_k;

@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
   __syncthreads();
   ptx::tc_fence_after();
   ptx::wait_for_stream();
-  ptx::let_next_start();
+  if (p.next_early) ptx::let_next_start();
   const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int group = p.heads / p.heads_k;
@@ -724,7 +724,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
   __syncthreads();
   ptx::tc_fence_after();
   ptx::wait_for_stream();
-  ptx::let_next_start();
+  if (p.next_early) ptx::let_next_start();
   const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int total_items = (p.vl.base != nullptr ? p.vl.base[0] : p.tiles_per_half * p.batch) * 2 * p.heads;
@@ -1166,6 +1166,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   p.heads = pr.heads;
   p.heads_k = pr.heads_k;
   p.overlap = overlapped_launches(pr) ? 1 : 0;
+  p.next_early = pr.sm_margin <= 0 ? 1 : 0;
   p.head_dim = d;
   p.block_size = pr.block_size;
   p.n_pad = static_cast<int>(round_up64(pr.seqlen / 2 > 0 ? pr.seqlen / 2 : 1, kTile));

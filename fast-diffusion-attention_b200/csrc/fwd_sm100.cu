@@ -64,6 +64,7 @@ struct FwdParams {
   int* ticket;         // global work counter, zeroed before the launch
   int wide_store;      // rows of out allow 32-byte stores
   int overlap;         // host: overlapped_launches
+  int next_early;      // the next kernel may start early: no SMs are kept free
   const float* q_descale;  // FP8 only: (batch, heads_k) factors, element strides below; nullptr = 1
   const float* k_descale;
   const float* v_descale;
@@ -295,7 +296,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
   __syncthreads();
   ptx::tc_fence_after();
   ptx::wait_for_stream();
-  ptx::let_next_start();
+  if (p.next_early) ptx::let_next_start();
   const uint32_t tmem = ptx::uniform(*tmem_slot);
   const int bs = p.block_size;
   const int total_items = p.vl.base != nullptr ? p.vl.base[0] * 2 * p.heads : p.total_items;
@@ -1000,6 +1001,7 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
   p.heads = pr.heads;
   p.heads_k = pr.heads_k;
   p.overlap = overlapped_launches(pr) ? 1 : 0;
+  p.next_early = pr.sm_margin <= 0 ? 1 : 0;
   p.head_dim = d;
   p.block_size = pr.block_size;
   const int max_n = pr.seqlen / 2;

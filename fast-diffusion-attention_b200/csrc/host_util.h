@@ -135,7 +135,10 @@ int launch_kernel(bool overlap, void (*kernel)(Params...), dim3 grid, int thread
 // us; 3 x 666, 12/4 heads of 96, 100 -> 94; 1 x 2048, 4 heads of 256, 129 -> 120; forward of 1 x 1024, 16 heads of 128, 16.6 -> 14.3). At
 // twice the line, 16 x 512 tokens, 16/4 heads of 128, there is nothing left of it (150 / 152), and long kernels get slower (2 x 8192, 8
 // heads of 256, 1340 -> 1445: blocks land on other SMs, in the order in which these become free).
+// Nor with sm_margin: blocks that start early go first to the SMs that the caller wants free, and hold all tensor memory there while they
+// wait. (For the same reason the kernels of such a call do not let the next one start: next_early.)
 inline bool overlapped_launches(const FdaProblem& pr) {
+  if (pr.sm_margin > 0) return false;
   return static_cast<int64_t>(pr.total) * pr.heads * pr.head_dim <= (1 << 23);
 }
 

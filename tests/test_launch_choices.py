@@ -38,6 +38,20 @@ def test_who_has_no_such_loop():
     assert _choices(16384, 16, 8, d=60) == 0   # refused
 
 
+def _overlaps(*args, **kw):
+    """(forward, backward)"""
+    c = _choices(*args, **kw)
+    return bool(c & _lib.FDA_CHOICE_FORWARD_OVERLAP), bool(c & _lib.FDA_CHOICE_BACKWARD_OVERLAP)
+
+
+def test_small_calls_overlap_and_leave_the_sms_free_that_the_caller_wants():
+    for kw in (dict(seqlen=512, heads=4, heads_k=4, d=64, batch=2), dict(seqlen=1400, heads=16, heads_k=4, d=128),
+               dict(seqlen=2048, heads=8, heads_k=8, d=256, deterministic=1), dict(seqlen=600, heads=8, heads_k=2, d=96, batch=5, total=1900)):
+        assert _overlaps(**kw) == (True, True)
+        assert _overlaps(sm_margin=1, **kw) == _overlaps(sm_margin=140, **kw) == (False, False)
+    assert _overlaps(seqlen=8192, heads=16, heads_k=16, d=128) == (False, False)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,bs", [(4096, 1), (4097, 64), (4100, 300), (4159, 1024)])
 @pytest.mark.parametrize("dtype,d,softcap", [(torch.bfloat16, 64, 0.0), (torch.float16, 128, 0.0), (torch.bfloat16, 64, 20.0),

@@ -9,6 +9,8 @@ namespace fda {
 size_t bwd_workspace_bytes(const FdaProblem& p);  // bwd_sm100.cu
 size_t fwd_workspace_bytes(const FdaProblem& p);  // fwd_sm100.cu
 bool forward_full_loop(const FdaProblem& p);      // fwd_sm100.cu
+bool bwd_single_pass(const FdaProblem& p);        // bwd_sm100.cu
+bool bwd_overlaps(const FdaProblem& p, bool single_pass);
 
 namespace {
 
@@ -182,7 +184,8 @@ int fda_geom_item_order(int idx, int per_group, int n_groups, int short8, int ct
 unsigned fda_launch_choices(const FdaProblem* p) {
   if (!p || fda::check_problem(*p, false) != FDA_OK) return 0;
   return (fda::forward_full_loop(*p) ? FDA_CHOICE_FORWARD_FULL_LOOP : 0u) |
-         (fda::overlapped_launches(*p) ? FDA_CHOICE_FORWARD_OVERLAP | FDA_CHOICE_BACKWARD_OVERLAP : 0u);
+         (fda::overlapped_launches(*p, 0) ? FDA_CHOICE_FORWARD_OVERLAP : 0u) |
+         (fda::bwd_overlaps(*p, fda::bwd_single_pass(*p)) ? FDA_CHOICE_BACKWARD_OVERLAP : 0u);
 }
 
 int fda_selftest_wait(long long limit_cycles, void* stream) {

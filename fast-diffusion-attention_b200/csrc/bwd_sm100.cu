@@ -1072,6 +1072,17 @@ constexpr int64_t kSmallAccBytes = 32 << 20;
 // The single-pass backward adds dQ partials in an order that depends on scheduling and needs head dim <= 128.
 bool bwd_single_pass(const FdaProblem& pr) { return pr.deterministic == 0 && pr.head_dim <= 128; }
 
+// The items that count for overlapped_launches, by what the host knows of the lengths.
+bool bwd_overlaps(const FdaProblem& pr, bool single_pass) {
+  int64_t items = 0;
+  if (single_pass && pr.head_dim > 64) {
+    const int64_t tiles = pr.cu_seqlens == nullptr ? (pr.seqlen / 2 + kTile - 1) / kTile * static_cast<int64_t>(pr.batch)
+                                                   : pr.total / (2 * kTile) + pr.batch;
+    items = tiles * 2 * pr.heads_k * bwd_fused_kv_split(pr);
+  }
+  return overlapped_launches(pr, items);
+}
+
 // Scratch of the split backward: delta_pad then lse2_pad, each batch * heads * 2 * n_pad floats (256-byte aligned
 // pieces), then 256 bytes of work counters.
 size_t bwd_split_workspace_bytes(const FdaProblem& pr) {
@@ -1165,7 +1176,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   p.total = pr.total;
   p.heads = pr.heads;
   p.heads_k = pr.heads_k;
-  p.overlap = overlapped_launches(pr) ? 1 : 0;
+  p.overlap = bwd_overlaps(pr, single_pass) ? 1 : 0;
   p.next_early = pr.sm_margin <= 0 ? 1 : 0;
   p.head_dim = d;
   p.block_size = pr.block_size;

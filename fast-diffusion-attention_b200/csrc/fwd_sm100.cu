@@ -1000,7 +1000,7 @@ int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {
   p.total = pr.total;
   p.heads = pr.heads;
   p.heads_k = pr.heads_k;
-  p.overlap = overlapped_launches(pr) ? 1 : 0;
+  p.overlap = overlapped_launches(pr, 0) ? 1 : 0;
   p.next_early = pr.sm_margin <= 0 ? 1 : 0;
   p.head_dim = d;
   p.block_size = pr.block_size;

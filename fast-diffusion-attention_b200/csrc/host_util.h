@@ -131,15 +131,23 @@ int launch_kernel(bool overlap, void (*kernel)(Params...), dim3 grid, int thread
   return FDA_OK;
 }
 
-// Where launches overlap: on little work, where they are a good part of the time (step of 2 x 512 tokens, 4 heads of 64, 33.1 -> 26.4
-// us; 3 x 666, 12/4 heads of 96, 100 -> 94; 1 x 2048, 4 heads of 256, 129 -> 120; forward of 1 x 1024, 16 heads of 128, 16.6 -> 14.3). At
-// twice the line, 16 x 512 tokens, 16/4 heads of 128, there is nothing left of it (150 / 152), and long kernels get slower (2 x 8192, 8
-// heads of 256, 1340 -> 1445: blocks land on other SMs, in the order in which these become free).
+// Where launches overlap: on little data and little work, where launches are a good part of the time. In one stream with nothing
+// else between them (step of 2 x 512 tokens, 4 heads of 64, 33.1 -> 26.4 us; 3 x 666, 12/4 heads of 96, 100 -> 94; 1 x 2048, 4 heads of
+// 256, 129 -> 120; forward of 1 x 1024, 16 heads of 128, 16.6 -> 14.3) a call overlaps the one before it, too. With another library's
+// kernel in between only the kernels of a call overlap each other: steps 1-5 % (1 x 1400 tokens, 16/4 heads of 128, 83.2 -> 80.1 us),
+// a forward of one kernel nothing. At twice the data, 16 x 512 tokens, 16/4 heads of 128, there is nothing left of it (150 / 152).
+// Beyond 2^36 = rows x length x heads x head dim nothing either (step of 1 x 16384 tokens, 8 heads of 64, 570 / 572; 1 x 32768, 2 heads of
+// 128, deterministic, 1088 / 1105; 1 x 8192, 4 heads of 256 400 / 398).
+// `items` is the number of items of a single-pass backward at head dims 65 to 128, else 0. With more than two a CTA that kernel gets
+// slower: its blocks land on other SMs, in the order in which these become free. 256 items: 1 x 3000 tokens, 8 heads of 128, 111 / 103; 1 x
+// 8192, 4 heads 234 / 228; 16 x 500, 8/2 heads 135 / 135. 384: 1 x 3000, 16 heads 122 / 130; 1 x 6000, 8/2 heads 207 / 224. 512: 4 x 1024, 16
+// heads 103 / 105; 1 x 8192, 8/2 heads 285 / 302; 1 x 16384, 4 heads 470 / 481. Head dim 64, 512 items: 602 / 605.
 // Nor with sm_margin: blocks that start early go first to the SMs that the caller wants free, and hold all tensor memory there while they
 // wait. (For the same reason the kernels of such a call do not let the next one start: next_early.)
-inline bool overlapped_launches(const FdaProblem& pr) {
-  if (pr.sm_margin > 0) return false;
-  return static_cast<int64_t>(pr.total) * pr.heads * pr.head_dim <= (1 << 23);
+inline bool overlapped_launches(const FdaProblem& pr, int64_t items) {
+  if (pr.sm_margin > 0 || items > 2 * 148) return false;
+  const int64_t q = static_cast<int64_t>(pr.total) * pr.heads * pr.head_dim;
+  return q <= (1 << 23) && q * (pr.seqlen < pr.total ? pr.seqlen : pr.total) <= (int64_t{1} << 36);
 }
 
 struct DeviceInfo {

@@ -176,7 +176,7 @@ int fda_geom_item_order(int idx, int per_group, int n_groups, int short8, int ct
 /* Which forms of the kernels a problem takes, as a sum of the bits below; 0 for a problem that fda_fwd refuses. */
 #define FDA_CHOICE_FORWARD_FULL_LOOP 1u /* forward: fully visible sub-steps in a loop of their own */
 #define FDA_CHOICE_FORWARD_OVERLAP 2u   /* forward: kernels may start before the ones ahead in the stream end */
-#define FDA_CHOICE_BACKWARD_OVERLAP 4u  /* backward: likewise */
+#define FDA_CHOICE_BACKWARD_OVERLAP 4u  /* backward (fda_bwd): likewise */
 unsigned fda_launch_choices(const FdaProblem* p);
 
 /* ---- tensor-core self test (GPU): C[128 x n] = A[128 x k] * B with the operand layouts the kernels use ---- */

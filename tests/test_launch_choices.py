@@ -52,6 +52,20 @@ def test_small_calls_overlap_and_leave_the_sms_free_that_the_caller_wants():
     assert _overlaps(seqlen=8192, heads=16, heads_k=16, d=128) == (False, False)
 
 
+def test_long_samples_do_not_overlap():
+    """Few rows and heads are little data, but not little work. The single-pass backward of head dims 65 to 128 overlaps with at
+    most two items a CTA (a part of a group is an item)."""
+    for n, h, hk, d, b, want in ((1500, 8, 8, 128, 1, True), (2048, 8, 8, 96, 1, True), (4096, 4, 4, 128, 1, True), (1500, 8, 2, 128, 1, True),
+                                 (1500, 16, 16, 128, 1, False), (512, 16, 16, 128, 4, False), (3000, 8, 2, 96, 1, False),
+                                 (4096, 8, 2, 128, 1, False), (8192, 4, 4, 128, 1, False), (2048, 16, 4, 128, 1, False)):
+        assert _overlaps(2 * n, h, hk, d, batch=b)[1] is want, (n, h, hk, d, b)
+    assert _overlaps(4096, 16, 16, 128, deterministic=1) == _overlaps(8192, 16, 16, 64) == _overlaps(8192, 4, 4, 256) == (True, True)
+    for d, h in ((64, 8), (128, 4), (256, 2)):
+        for deterministic in (0, 1):
+            assert _overlaps(16384, h, h, d, deterministic=deterministic) == (False, False)
+    assert _overlaps(1 << 20, 4, 4, 64, batch=2, total=1024) == (True, True)      # max_seqlen is an upper bound
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("n,bs", [(4096, 1), (4097, 64), (4100, 300), (4159, 1024)])
 @pytest.mark.parametrize("dtype,d,softcap", [(torch.bfloat16, 64, 0.0), (torch.float16, 128, 0.0), (torch.bfloat16, 64, 20.0),

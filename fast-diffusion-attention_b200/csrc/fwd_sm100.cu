@@ -911,7 +911,8 @@ size_t fwd_workspace_bytes(const FdaProblem& pr) {
 //   8 x 4096          248 / 252  302 / 301  314 / 331  535 / 550      1 x 16384  383 / 370  489 / 481  491 / 468  826 / 782
 // 3 x 8192 in blocks of 1024: 349 / 349, 466 / 451, 474 / 450, 802 / 768; in one block: 558 / 580, 737 / 760, 747 / 737, 1223 / 1223.
 // Capped, 3 x 8192: 499 / 492, 525 / 526 (so not there), 605 / 577, 898 / 846. With at most eight items a CTA the loop loses nothing from
-// 2000 tokens on (blocks of 16): 1 x 2000, 8 heads 20.0 / 18.7, 20.7 / 20.7, 22.7 / 22.2, 26.8 / 25.0; 1 x 3000, 16 heads 35.7 / 33.1,
+// 600 tokens a half on (blocks of 16): 16 x 512, 16 heads 20.6 / 20.6, 23.3 / 23.5, 21.0 / 22.7, 33.1 / 33.6; 1 x 1400, 16/4 heads 17.2 /
+// 16.7, 19.3 / 18.8, 20.3 / 19.5, 22.7 / 23.5; 4 x 1400 35.1 / 34.8, 40.6 / 39.7, 39.4 / 39.1, 63.5 / 62.4; 1 x 3000, 16 heads 35.7 / 33.1,
 // 39.1 / 38.6, 43.3 / 40.8, 55.9 / 55.4; 1 x 6000, 3 heads 38.8 / 35.2, 41.2 / 40.7, 46.8 / 43.3, 49.7 / 49.9; 1 x 4096, 16 heads in
 // one block 69.1 / 69.9, 78.8 / 79.7, 88.7 / 88.0, 141 / 137. 16-bit heads of 256, which wait for K and V, get one loop for all (1 %
 // the other way).
@@ -923,9 +924,8 @@ bool forward_full_loop(const FdaProblem& pr) {
   const int item_rows = pr.head_dim > 128 ? kBlockM : 2 * kBlockM;
   const int64_t items = (tokens + item_rows - 1) / item_rows * 2 * pr.heads * pr.batch;
   const bool few = items <= 8 * 148;
-  if (fp8) return tokens >= (few ? 1000 : 3000);
-  if (pr.head_dim <= 64) return tokens >= (few ? 1000 : 4096) && (few ? 2 : 4) * static_cast<int64_t>(pr.block_size) <= tokens;
-  return tokens >= (few ? 2048 : 4096) && 4 * static_cast<int64_t>(pr.block_size) <= tokens;
+  if (tokens < (few ? 600 : fp8 ? 3000 : 4096)) return false;
+  return fp8 || (few && pr.head_dim <= 64 ? 2 : 4) * static_cast<int64_t>(pr.block_size) <= tokens;
 }
 
 int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {

@@ -16,17 +16,17 @@ def _choices(seqlen, heads, heads_k, d, bs=64, *, batch=1, total=None, dtype=_li
     return _lib.load().fda_launch_choices(C.byref(p))
 
 
-@pytest.mark.parametrize("dtype,d,softcap,line,few", [(_lib.FDA_BF16, 64, 0.0, 4096, 1000), (_lib.FDA_FP16, 96, 0.0, 4096, 2048),
-                                                      (_lib.FDA_BF16, 64, 30.0, 4096, 1000), (_lib.FDA_E4M3, 64, 0.0, 3000, 1000),
-                                                      (_lib.FDA_E4M3, 256, 30.0, 3000, 1000)])
-def test_only_long_samples_have_a_loop_for_full_sub_steps(dtype, d, softcap, line, few):
+@pytest.mark.parametrize("dtype,d,softcap,line", [(_lib.FDA_BF16, 64, 0.0, 4096), (_lib.FDA_FP16, 96, 0.0, 4096),
+                                                      (_lib.FDA_BF16, 64, 30.0, 4096), (_lib.FDA_E4M3, 64, 0.0, 3000),
+                                                      (_lib.FDA_E4M3, 256, 30.0, 3000)])
+def test_only_long_samples_have_a_loop_for_full_sub_steps(dtype, d, softcap, line):
     def takes(n, bs=64, heads=16, **kw):
         return bool(_choices(2 * n, heads, heads, d, bs, dtype=dtype, softcap=softcap, **kw) & _lib.FDA_CHOICE_FORWARD_FULL_LOOP)
 
     assert takes(line, batch=4) and takes(line, batch=16) and takes(8192, bs=2048, batch=4)
     for n in (64, 256, 512, 1024, 1500, 2048, line - 1):
         assert not takes(n, batch=128)
-    assert takes(few, heads=2) and not takes(few - 1, heads=2) and not takes(512, heads=1)   # few items a CTA
+    assert takes(600, heads=2) and not takes(599, heads=2) and not takes(512, heads=1)   # few items a CTA
     assert not takes(8192, batch=41, total=2 * (8192 + 40 * 300))     # one long sample among short ones
     assert not takes(32768, batch=64, total=2 * 64 * 512)             # max_seqlen is an upper bound
     assert takes(8192, bs=8192, batch=4) == (dtype == _lib.FDA_E4M3)  # noisy rows of one block see no clean key
@@ -67,7 +67,7 @@ def test_long_samples_do_not_overlap():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("n,bs", [(4096, 1), (4097, 64), (4100, 300), (4159, 1024)])
+@pytest.mark.parametrize("n,bs", [(601, 16), (777, 150), (4096, 1), (4097, 64), (4100, 300), (4159, 1024)])
 @pytest.mark.parametrize("dtype,d,softcap", [(torch.bfloat16, 64, 0.0), (torch.float16, 128, 0.0), (torch.bfloat16, 64, 20.0),
                                              (torch.float8_e4m3fn, 128, 0.0), (torch.float8_e4m3fn, 256, 20.0)])
 def test_both_loops_give_the_same_bits(n, bs, dtype, d, softcap):

@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
     uint32_t n_item = 0, gd = 0, n_bulk = 0;
     bool alive = true;
     for (uint32_t n_sched = 0; alive; ++n_sched) {
-      const int idx = R::kGeometryWarp ? sched_peek(mbox, n_sched, abort_flag) : sched_consume<true>(mbox, n_sched, abort_flag);
+      const int idx = R::kGeometryWarp ? sched_peek<true>(mbox, n_sched, abort_flag) : sched_consume<true>(mbox, n_sched, abort_flag);
       if (idx < 0 || idx >= total_items) break;
       const KvItem it = R::kGeometryWarp ? items[n_sched & 1u].it : decode_kv_item(p, idx / split);
       const int part = R::kGeometryWarp ? items[n_sched & 1u].part : idx % split;
@@ -285,12 +285,12 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
       else if (!it.valid) continue;
       for (bool last = false; alive && !last; ++gd) {
         const uint32_t par = gd & 1u;
-        if (!ptx::mbar_wait(&desc_full[par], (gd >> 1) & 1u, abort_flag, 63)) { alive = false; break; }
+        if (!ptx::mbar_wait_warp(&desc_full[par], (gd >> 1) & 1u, abort_flag, 63)) { alive = false; break; }
         const int flags = dq_desc[2 * par];
         const int acc_row = dq_desc[2 * par + 1];
         last = (flags & 1) != 0;
         const int rows_left = flags >> 8;   // query rows of this tile that exist (1..128)
-        if (!ptx::mbar_wait(dq_full, par, abort_flag, 64)) { alive = false; break; }
+        if (!ptx::mbar_wait_warp(dq_full, par, abort_flag, 64)) { alive = false; break; }
         ptx::tc_fence_after();
         // kHold chunks of 32 columns go to registers at once; when the last is there the columns are free and the adds
         // follow behind the next step's products. Blocks of 32 query rows of the accumulator are stored as
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
       const int64_t srow = static_cast<int64_t>(it.row0) + it.kh * it.n + kj;
       uint16_t* dk_row = static_cast<uint16_t*>(p.dk) + it.bcoord * p.dk_bs + srow * p.dk_rs + it.hk * p.dk_hs;
       uint16_t* dv_row = static_cast<uint16_t*>(p.dv) + it.bcoord * p.dv_bs + srow * p.dv_rs + it.hk * p.dv_hs;
-      if (!ptx::mbar_wait(acc_full, n_item & 1, abort_flag, 62)) break;
+      if (!ptx::mbar_wait_warp(acc_full, n_item & 1, abort_flag, 62)) break;
       ++n_item;
       ptx::tc_fence_after();
       if (kParts) {
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
       uint32_t n_item = 0, gc = 0;
       bool alive = true;
       for (uint32_t n_sched = 0; alive; ++n_sched) {
-        const int idx = R::kGeometryWarp ? sched_peek(mbox, n_sched, abort_flag)
+        const int idx = R::kGeometryWarp ? sched_peek<false>(mbox, n_sched, abort_flag)
                                          : sched_produce(mbox, n_sched, p.ticket_kv, abort_flag);
         if (idx < 0 || idx >= total_items) break;
         FusedItem d;
@@ -558,14 +558,14 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
         const int idx = ptx::uniform(sched_consume<true>(mbox, n_sched, abort_flag));
         if (idx < 0 || idx >= total_items) break;
         if (!R::kGeometryWarp && !decode_kv_item(p, idx / split).valid) continue;
-        if (!ptx::mbar_wait(k_full, n_item & 1, abort_flag, 51)) break;
+        if (!ptx::mbar_wait_warp(k_full, n_item & 1, abort_flag, 51)) break;
         bool first = true;
         for (bool last = false; alive && !last; ++g) {
           const uint32_t slot = g % kSlots, spar = (g / kSlots) & 1u;
           const uint32_t t_off = slot * (T::kTileBytes >> 4);
-          if (!ptx::mbar_wait(&q_full[slot], spar, abort_flag, 52)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&q_full[slot], spar, abort_flag, 52)) { alive = false; break; }
           last = (ptx::uniform(hdr[4 * slot]) & 1) != 0;
-          if (!ptx::mbar_wait(s_free, (g & 1u) ^ 1u, abort_flag, 54)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(s_free, (g & 1u) ^ 1u, abort_flag, 54)) { alive = false; break; }
           ptx::tc_fence_after();
           if (ptx::elect_one()) {
 #pragma unroll
@@ -576,10 +576,10 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
             ptx::umma_commit(s_full);
           }
           const uint32_t dslot = g % kDoSlots;
-          if (!ptx::mbar_wait(&do_full[dslot], (g / kDoSlots) & 1u, abort_flag, 56)) { alive = false; break; }
-          if (first && !ptx::mbar_wait(v_full, n_item & 1, abort_flag, 69)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&do_full[dslot], (g / kDoSlots) & 1u, abort_flag, 56)) { alive = false; break; }
+          if (first && !ptx::mbar_wait_warp(v_full, n_item & 1, abort_flag, 69)) { alive = false; break; }
           first = false;
-          if (!ptx::mbar_wait(Cfg::kOwnDq ? ds_full : dp_free, (g & 1u) ^ 1u, abort_flag, 58)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(Cfg::kOwnDq ? ds_full : dp_free, (g & 1u) ^ 1u, abort_flag, 58)) { alive = false; break; }
           ptx::tc_fence_after();
           if (ptx::elect_one()) {
 #pragma unroll
@@ -618,17 +618,17 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
         if (!R::kGeometryWarp && !decode_kv_item(p, idx / split).valid) continue;
         bool acc = false;
         // the first dV / dK products of an item overwrite the accumulators: the epilogue must have read the last item's
-        if (!ptx::mbar_wait(acc_free, (n_item_b & 1u) ^ 1u, abort_flag, 57)) break;
+        if (!ptx::mbar_wait_warp(acc_free, (n_item_b & 1u) ^ 1u, abort_flag, 57)) break;
         ++n_item_b;
         for (bool last = false; alive && !last; ++g) {
           const uint32_t slot = g % kSlots, spar = (g / kSlots) & 1u;
           const uint32_t t_off = slot * (T::kTileBytes >> 4);
-          if (!ptx::mbar_wait(&q_full[slot], spar, abort_flag, 55)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&q_full[slot], spar, abort_flag, 55)) { alive = false; break; }
           last = (ptx::uniform(hdr[4 * slot]) & 1) != 0;
-          if (!ptx::mbar_wait(p_full, g & 1u, abort_flag, 53)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(p_full, g & 1u, abort_flag, 53)) { alive = false; break; }
           // dO usually landed long ago (dP^T of this step reads it too), but nothing this thread has waited for so far
           // says so
-          if (!ptx::mbar_wait(&do_full[g % kDoSlots], (g / kDoSlots) & 1u, abort_flag, 67)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&do_full[g % kDoSlots], (g / kDoSlots) & 1u, abort_flag, 67)) { alive = false; break; }
           ptx::tc_fence_after();
           // dV += P^T dO: P^T of the 16 queries of reduction step kk sits at column 32 (kk / 2) + 8 (kk % 2)
           if (ptx::elect_one()) {
@@ -641,12 +641,12 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
             ptx::umma_commit(s_free);
             ptx::umma_commit(&do_empty[g % kDoSlots]);
           }
-          if (!ptx::mbar_wait(ds_full, g & 1u, abort_flag, 59)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(ds_full, g & 1u, abort_flag, 59)) { alive = false; break; }
           ptx::tc_fence_after();
           // dQ before dK: its drain (tensor memory -> registers -> global adds) then runs under dK
           if (Cfg::kOwnDq) {
             // the drain warps hold dQ of the previous step
-            if (!ptx::mbar_wait(dp_free, (g & 1u) ^ 1u, abort_flag, 68)) { alive = false; break; }
+            if (!ptx::mbar_wait_warp(dp_free, (g & 1u) ^ 1u, abort_flag, 68)) { alive = false; break; }
             ptx::tc_fence_after();
           }
           if (ptx::elect_one()) {
@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
     uint32_t gc = 0;
     bool alive = true;
     for (uint32_t n_sched = 0; alive; ++n_sched) {
-      const int idx = R::kGeometryWarp ? sched_peek(mbox, n_sched, abort_flag) : sched_consume<true>(mbox, n_sched, abort_flag);
+      const int idx = R::kGeometryWarp ? sched_peek<true>(mbox, n_sched, abort_flag) : sched_consume<true>(mbox, n_sched, abort_flag);
       if (idx < 0 || idx >= total_items) break;
       const KvItem it = R::kGeometryWarp ? items[n_sched & 1u].it : decode_kv_item(p, idx / split);
       if (R::kGeometryWarp) sched_release<true>(mbox, n_sched);
@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
         const uint32_t slot = gc % kSlots, par = gc & 1u;
         const float* stats = reinterpret_cast<const float*>(sStat + slot * Cfg::kStatBytes) + wg * R::kCols;
         // the Q barrier orders the header and the bulk copies of lse2 / delta before our reads
-        if (!ptx::mbar_wait(&q_full[slot], (gc / kSlots) & 1u, abort_flag, 60)) { alive = false; break; }
+        if (!ptx::mbar_wait_warp(&q_full[slot], (gc / kSlots) & 1u, abort_flag, 60)) { alive = false; break; }
         const int hdr0 = hdr[4 * slot], hdr1 = hdr[4 * slot + 1], hdr2 = hdr[4 * slot + 2];
         last = (hdr0 & 1) != 0;
         const bool masked = (hdr0 & 2) != 0;
@@ -716,7 +716,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
           // First half, once S^T is complete: P^T (16-bit, back to tensor memory for dV) and, kept in registers, the
           // factor of the second half: P, or with the score cap P (1 - tanh^2).
           float pr[R::kCols];
-          if (!ptx::mbar_wait(s_full, par, abort_flag, 61)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(s_full, par, abort_flag, 61)) { alive = false; break; }
           ptx::tc_fence_after();
 #pragma unroll
           for (int half = 0; half < kChunks; ++half) ptx::tmem_ld32(s_t + 32 * half, reinterpret_cast<uint32_t*>(pr) + 32 * half);
@@ -766,9 +766,9 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
           ptx::tmem_wait_st();
           ptx::tc_fence_before();
           ptx::mbar_arrive_warp(p_full);
-          if (!ptx::mbar_wait(dp_full, par, abort_flag, 65)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(dp_full, par, abort_flag, 65)) { alive = false; break; }
           // dQ^T and dK of the previous step have read the dS^T tile (long ago in the steady state)
-          if (!ptx::mbar_wait(ds_free, par ^ 1u, abort_flag, 66)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(ds_free, par ^ 1u, abort_flag, 66)) { alive = false; break; }
           ptx::tc_fence_after();
           const float4* dlv = reinterpret_cast<const float4*>(stats + kTile);
           uint32_t dpv[R::kCols];

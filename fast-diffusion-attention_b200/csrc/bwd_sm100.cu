@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       const int64_t srow = static_cast<int64_t>(it.row0) + it.kh * it.n + kj;
       uint16_t* dk_row = static_cast<uint16_t*>(p.dk) + it.bcoord * p.dk_bs + srow * p.dk_rs + it.hk * p.dk_hs;
       uint16_t* dv_row = static_cast<uint16_t*>(p.dv) + it.bcoord * p.dv_bs + srow * p.dv_rs + it.hk * p.dv_hs;
-      if (!ptx::mbar_wait(acc_full, n_item & 1, abort_flag, 62)) break;
+      if (!ptx::mbar_wait_warp(acc_full, n_item & 1, abort_flag, 62)) break;
       ++n_item;
       ptx::tc_fence_after();
       // dK and dV sit side by side in tensor memory (or the item makes one of them): chunks of 32 columns
@@ -406,15 +406,15 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         if (idx < 0 || idx >= total_items) break;
         const KvItem it = decode_kv_item(p, idx / Cfg::kItems);
         if (!it.valid) continue;
-        if (!ptx::mbar_wait(kv_full, n_item & 1, abort_flag, 51)) break;
+        if (!ptx::mbar_wait_warp(kv_full, n_item & 1, abort_flag, 51)) break;
         for (bool last = false; alive && !last; ++g) {
           const uint32_t u = g & 1u, qs = g % Cfg::kQSlots, ds = g % Cfg::kDoSlots, ss = g % Cfg::kStatSlots;
-          if (!ptx::mbar_wait(&stat_full[ss], (g / Cfg::kStatSlots) & 1u, abort_flag, 52)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&stat_full[ss], (g / Cfg::kStatSlots) & 1u, abort_flag, 52)) { alive = false; break; }
           last = (ptx::uniform(*reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset)) & 1) != 0;
-          if (!ptx::mbar_wait(&q_full[qs], (g / Cfg::kQSlots) & 1u, abort_flag, 56)) { alive = false; break; }
-          if (!ptx::mbar_wait(&buf_free[u], ((g >> 1) & 1u) ^ 1u, abort_flag, 54)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&q_full[qs], (g / Cfg::kQSlots) & 1u, abort_flag, 56)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&buf_free[u], ((g >> 1) & 1u) ^ 1u, abort_flag, 54)) { alive = false; break; }
           if (Cfg::kPasses == 1 &&
-              !ptx::mbar_wait(&do_full[ds], (g / Cfg::kDoSlots) & 1u, abort_flag, 58)) { alive = false; break; }
+              !ptx::mbar_wait_warp(&do_full[ds], (g / Cfg::kDoSlots) & 1u, abort_flag, 58)) { alive = false; break; }
           ptx::tc_fence_after();
           const uint32_t q_off = qs * (Cfg::kSubTileBytes >> 4), do_off = ds * (Cfg::kSubTileBytes >> 4);
           auto product = [&](int kk, uint32_t d_off, uint32_t a_lo, uint32_t b_lo) {
@@ -436,7 +436,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
               for (int kk = 0; kk < kHeadDim / 16; ++kk) product(kk, 0, k_lo, q_lo + q_off);
             }
             if (makes_dk(idx)) {
-              if (!ptx::mbar_wait(&do_full[ds], (g / Cfg::kDoSlots) & 1u, abort_flag, 58)) { alive = false; break; }
+              if (!ptx::mbar_wait_warp(&do_full[ds], (g / Cfg::kDoSlots) & 1u, abort_flag, 58)) { alive = false; break; }
               ptx::tc_fence_after();
               if (ptx::elect_one()) {
 #pragma unroll
@@ -472,19 +472,19 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         if (!it.valid) continue;
         bool acc = false;
         // the first products of an item overwrite the accumulators: the epilogue warps must have read the last item's
-        if (!ptx::mbar_wait(acc_free, (n_item_b & 1u) ^ 1u, abort_flag, 57)) break;
+        if (!ptx::mbar_wait_warp(acc_free, (n_item_b & 1u) ^ 1u, abort_flag, 57)) break;
         ++n_item_b;
         for (bool last = false; alive && !last; ++g) {
           const uint32_t u = g & 1u, qs = g % Cfg::kQSlots, ds = g % Cfg::kDoSlots, ss = g % Cfg::kStatSlots;
-          if (!ptx::mbar_wait(&stat_full[ss], (g / Cfg::kStatSlots) & 1u, abort_flag, 55)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&stat_full[ss], (g / Cfg::kStatSlots) & 1u, abort_flag, 55)) { alive = false; break; }
           last = (ptx::uniform(*reinterpret_cast<const volatile int*>(sStat + ss * Cfg::kStatBytes + Cfg::kHeaderOffset)) & 1) != 0;
-          if (!ptx::mbar_wait(&pds_full[u], (g >> 1) & 1u, abort_flag, 53)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&pds_full[u], (g >> 1) & 1u, abort_flag, 53)) { alive = false; break; }
           // The tiles this thread's products read. Most have landed long ago, but nothing it has waited for so far says so:
           // that the other issuer saw them land reaches this thread only through its products and the compute warps.
           if (makes_dk(idx) &&
-              !ptx::mbar_wait(&q_full[qs], (g / Cfg::kQSlots) & 1u, abort_flag, 64)) { alive = false; break; }
+              !ptx::mbar_wait_warp(&q_full[qs], (g / Cfg::kQSlots) & 1u, abort_flag, 64)) { alive = false; break; }
           if (makes_dv(idx) &&
-              !ptx::mbar_wait(&do_full[ds], (g / Cfg::kDoSlots) & 1u, abort_flag, 59)) { alive = false; break; }
+              !ptx::mbar_wait_warp(&do_full[ds], (g / Cfg::kDoSlots) & 1u, abort_flag, 59)) { alive = false; break; }
           ptx::tc_fence_after();
           const uint32_t q_off = qs * (Cfg::kSubTileBytes >> 4), do_off = ds * (Cfg::kSubTileBytes >> 4);
           const uint32_t st_t = tmem + u * 128, dpt_t = tmem + u * 128 + 64;
@@ -534,7 +534,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
         const uint8_t* stage_base = sStat + ss * Cfg::kStatBytes;
         const float* stats = reinterpret_cast<const float*>(stage_base);
         // orders the header and the bulk copies of lse2 / delta before our reads
-        if (!ptx::mbar_wait(&stat_full[ss], (gc / Cfg::kStatSlots) & 1u, abort_flag, 60)) { alive = false; break; }
+        if (!ptx::mbar_wait_warp(&stat_full[ss], (gc / Cfg::kStatSlots) & 1u, abort_flag, 60)) { alive = false; break; }
         int2 hdr;
         hdr.x = reinterpret_cast<const volatile int*>(stage_base + Cfg::kHeaderOffset)[0];
         hdr.y = reinterpret_cast<const volatile int*>(stage_base + Cfg::kHeaderOffset)[1];
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
             dlr[4 * i] = b.x; dlr[4 * i + 1] = b.y; dlr[4 * i + 2] = b.z; dlr[4 * i + 3] = b.w;
           }
         }
-        if (!ptx::mbar_wait(&sdp_full[u], (gc >> 1) & 1u, abort_flag, 61)) { alive = false; break; }
+        if (!ptx::mbar_wait_warp(&sdp_full[u], (gc >> 1) & 1u, abort_flag, 61)) { alive = false; break; }
         ++gc;
         ptx::tc_fence_after();
         const uint32_t st_t = tmem + u * 128 + lane_addr + wg * kSubCols;
@@ -803,13 +803,13 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
           plan.step(s, kh, kt);
           active += spans.classify(kh, kt * Cfg::kKeys, Cfg::kKeys) != kTileSkip;
         }
-        if (!ptx::mbar_wait(q_full, n_item & 1, abort_flag, 81)) break;
+        if (!ptx::mbar_wait_warp(q_full, n_item & 1, abort_flag, 81)) break;
         ++n_item;
         for (int j = 0; j < active; ++j, ++step) {
           const uint32_t ks = Cfg::k_slot(step), vs = Cfg::v_slot(step);
-          if (!ptx::mbar_wait(&kv_full[ks], Cfg::k_parity(step), abort_flag, 83)) { alive = false; break; }
-          if (!ptx::mbar_wait(&kv_full[vs], Cfg::v_parity(step), abort_flag, 84)) { alive = false; break; }
-          if (!ptx::mbar_wait(sdp_free, (step & 1) ^ 1, abort_flag, 82)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&kv_full[ks], Cfg::k_parity(step), abort_flag, 83)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&kv_full[vs], Cfg::v_parity(step), abort_flag, 84)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(sdp_free, (step & 1) ^ 1, abort_flag, 82)) { alive = false; break; }
           ptx::tc_fence_after();
           if (ptx::elect_one()) {
 #pragma unroll
@@ -855,8 +855,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
         for (int j = 0; j < active; ++j, ++step) {
           const uint32_t ks = Cfg::k_slot(step);
           // the K tile arrived long ago (S of this step used it); this wait only orders our reads after the copy
-          if (!ptx::mbar_wait(&kv_full[ks], Cfg::k_parity(step), abort_flag, 86)) { alive = false; break; }
-          if (!ptx::mbar_wait(ds_full, step & 1, abort_flag, 85)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&kv_full[ks], Cfg::k_parity(step), abort_flag, 86)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(ds_full, step & 1, abort_flag, 85)) { alive = false; break; }
           ptx::tc_fence_after();
           // dQ += dS K: the packed dS pieces of the compute warpgroups lie side by side, 8 columns per 16 keys
           if (ptx::elect_one()) {
@@ -899,6 +899,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
       for (;;) {
         const int idx = sched_consume<true>(mbox, n_sched, abort_flag);
         ++n_sched;
+        if (idx < 0) alive = false;   // no wait may follow one that was abandoned
         if (idx < 0 || idx >= total_items) return false;
         const QItem it = decode_q_item(p, idx);
         if (!it.valid) continue;
@@ -935,7 +936,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
           lo -= kt * Cfg::kKeys + wg * kKc;
           hi -= kt * Cfg::kKeys + wg * kKc;
         }
-        if (!ptx::mbar_wait(sdp_full, cnt & 1, abort_flag, 91)) { alive = false; break; }
+        if (!ptx::mbar_wait_warp(sdp_full, cnt & 1, abort_flag, 91)) { alive = false; break; }
         ptx::tc_fence_after();
         uint32_t sv[kKc], dpv[kKc];
         if (kKc == 32) {
@@ -956,7 +957,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
           softmax_backward_cols<kKc, kBf16, kSoftcap, false, false, false>(sv, dpv, nullptr, nullptr, cur.lse2, cur.delta,
                                                                            p.scale_log2, p.softcap_pre, 0, 0, nullptr, pk_ds);
         }
-        if (!ptx::mbar_wait(ds_free, (cnt & 1) ^ 1, abort_flag, 92)) { alive = false; break; }
+        if (!ptx::mbar_wait_warp(ds_free, (cnt & 1) ^ 1, abort_flag, 92)) { alive = false; break; }
         ++cnt;
         ptx::tc_fence_after();
         if (kKc == 32) ptx::tmem_st16(tmem + Cfg::kTmemDS + lane_addr + wg * (kKc / 2), pk_ds);
@@ -967,7 +968,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) bwd_dq_kernel(const __grid_con
       }
       if (!alive) return false;
       const bool have_next = fetch(nxt);
-      if (!ptx::mbar_wait(dq_full, n_item & 1, abort_flag, 93)) { alive = false; return false; }
+      if (!alive) return false;
+      if (!ptx::mbar_wait_warp(dq_full, n_item & 1, abort_flag, 93)) { alive = false; return false; }
       ++n_item;
       ptx::tc_fence_after();
       constexpr int kChunks = kHeadDim / 32;  // 32-column chunks, dealt round-robin to the warpgroups

@@ -441,10 +441,10 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       if (!owed[h]) return;
       const uint32_t slot = 2 * v_pair[h] + 1;
       if (Cfg::kHalves == 1 || h == 0) {
-        if (!ptx::mbar_wait(&kv_full[slot], v_par[h], abort_flag, 23)) { alive = false; return; }
+        if (!ptx::mbar_wait_warp(&kv_full[slot], v_par[h], abort_flag, 23)) { alive = false; return; }
       }
       if (pend[h]) {
-        if (!ptx::mbar_wait(&p_full_t[h], p_par[h], abort_flag, 24)) { alive = false; return; }
+        if (!ptx::mbar_wait_warp(&p_full_t[h], p_par[h], abort_flag, 24)) { alive = false; return; }
         p_par[h] ^= 1;
         ptx::tc_fence_after();
         const uint32_t b_lo = v_lo0 + slot * (Cfg::kSlotBytes >> 4) + (Cfg::kHalves == 2 ? h * ((kSubKeys * 128) >> 4) : 0);
@@ -469,12 +469,12 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
     };
 
     while (alive) {
-      if (!ptx::mbar_wait(&kv_full[2 * pair], par, abort_flag, 22)) break;
+      if (!ptx::mbar_wait_warp(&kv_full[2 * pair], par, abort_flag, 22)) break;
       const uint32_t info = ptx::uniform(slot_info[pair]);
       if (info & kInfoStop) break;
       if (Cfg::kQInRing && (info & kInfoQ)) {
         // Every S product of the last item is complete: this warp has waited for the P of each.
-        if (!ptx::mbar_wait(&kv_full[2 * pair + 1], par, abort_flag, 21)) break;
+        if (!ptx::mbar_wait_warp(&kv_full[2 * pair + 1], par, abort_flag, 21)) break;
         ptx::tc_fence_after();
         if (ptx::elect_one()) {
           const uint32_t lo = k_lo0 + 2 * pair * (Cfg::kSlotBytes >> 4);
@@ -490,7 +490,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
         continue;
       }
       if (!Cfg::kQInRing && (info & kInfoFirst)) {
-        if (!ptx::mbar_wait(q_full, q_par, abort_flag, 21)) break;
+        if (!ptx::mbar_wait_warp(q_full, q_par, abort_flag, 21)) break;
         q_par ^= 1;
         o_acc = false;
         if (Cfg::kTmemHasQ) {
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
         if (!alive) break;
         if (Cfg::kHalves == 1 && h == 1) {
           if (!(info & kInfoHalf1)) break;
-          if (!ptx::mbar_wait(&kv_full[2 * pair], par, abort_flag, 22)) { alive = false; break; }
+          if (!ptx::mbar_wait_warp(&kv_full[2 * pair], par, abort_flag, 22)) { alive = false; break; }
         }
         const bool vis = (info >> (2 * t + h)) & 1u;
         const uint32_t slot = 2 * pair;
@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
     bool alive = true;
     uint8_t* stage_o = sStageO + t * Cfg::kStageOBytes;
     for (uint32_t n_sched = 0; alive; ++n_sched) {
-      const int idx = sched_peek(mbox, n_sched, abort_flag);
+      const int idx = sched_peek<true>(mbox, n_sched, abort_flag);
       if (idx < 0 || idx >= total_items) break;
       const Item it = desc[n_sched & 1u].it;
       const TileSpans spans = desc[n_sched & 1u].spans[t];
@@ -637,7 +637,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
           cls = spans.classify(kh, k0);
           if (cls == kTileSkip) return;
         }
-        if (!ptx::mbar_wait(&s_full[t * kBufs + buf], (s_par >> buf) & 1u, abort_flag, 31)) { alive = false; return; }
+        if (!ptx::mbar_wait_warp(&s_full[t * kBufs + buf], (s_par >> buf) & 1u, abort_flag, 31)) { alive = false; return; }
         s_par ^= 1u << buf;
         ptx::tc_fence_after();
         const uint32_t tmem_sb = tmem_s + buf * kSubKeys;
@@ -700,7 +700,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
 #pragma unroll
           for (int b = 0; b < kBufs; ++b) {
             if (b == buf) continue;
-            if (!ptx::mbar_wait(&pv_done[t * kBufs + b], ((s_par >> b) & 1u) ^ 1u, abort_flag, 33)) { alive = false; return; }
+            if (!ptx::mbar_wait_warp(&pv_done[t * kBufs + b], ((s_par >> b) & 1u) ^ 1u, abort_flag, 33)) { alive = false; return; }
           }
           ptx::tc_fence_after();
           // A load is answered after some 250 cycles while products run, however wide it is. fp8 rescales often, and with
@@ -784,7 +784,7 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
       for (; u < subs && alive; ++u) sub_step(std::false_type{}, u, u & 1);
       if (!alive) break;
       // ---- epilogue: O / l -> global, LSE
-      if (!ptx::mbar_wait(&o_full[t], cnt_o & 1, abort_flag, 32)) { alive = false; break; }
+      if (!ptx::mbar_wait_warp(&o_full[t], cnt_o & 1, abort_flag, 32)) { alive = false; break; }
       ++cnt_o;
       ptx::tc_fence_after();
       const float inv_l = out_scale / l_run;

@@ -81,9 +81,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait. `abort_flag` lives in shared memory; once any thread of the CTA gives up, every later wait
-// returns at once so the CTA can drain, free its tensor memory and exit. Returns false when aborted.
+// Bounded wait of one thread. `abort_flag` lives in shared memory; once any thread of the CTA gives up, every later wait that would
+// have to wait returns at once so the CTA can drain, free its tensor memory and exit. Returns false when aborted.
 constexpr long long kWaitLimitCycles = 4000000000LL;  // about two seconds at the boost clock
+
+__device__ __forceinline__ void note_expired_wait(uint32_t parity, volatile int* abort_flag, int code) {
+  if (atomicCAS(&g_fda_status[0], 0, code) == 0) {
+    g_fda_status[1] = static_cast<int>(blockIdx.x);
+    g_fda_status[2] = static_cast<int>(threadIdx.x);
+    g_fda_status[3] = static_cast<int>(parity);
+  }
+  *abort_flag = code;
+}
 
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code,
                                           long long limit_cycles = kWaitLimitCycles) {
@@ -95,15 +104,37 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     if ((++spins & 127u) == 0) {
       if (*abort_flag) return false;
       if (clock64() - t0 > limit_cycles) {
-        *abort_flag = code;
-        if (atomicCAS(&g_fda_status[0], 0, code) == 0) {
-          g_fda_status[1] = static_cast<int>(blockIdx.x);
-          g_fda_status[2] = static_cast<int>(threadIdx.x);
-          g_fda_status[3] = static_cast<int>(parity);
-        }
+        note_expired_wait(parity, abort_flag, code);
         return false;
       }
     }
+  }
+  return true;
+}
+
+// Whether a warp gives up a wait, with one answer for all its lanes. Behind a wait come operations that every lane has to take part in
+// (elections, shuffles, tensor-memory loads, the block's last barrier): were some lanes to see the phase complete and others only the
+// abort flag, each would wait for lanes that have left, without a bound. So a warp gives up as a whole, all its lanes here at once. While
+// lanes are missing they have seen the phase complete, and so will the others: the phase after it needs this warp's arrival. (Lanes that
+// run apart for another limit, with none through, leave one by one, which is all of them.)
+// Out of line: the dozens of waits of a kernel are then short, and its warps wait for instructions less (steps of 1 x 2000 to 4 x 4096
+// tokens 1-3 % faster than with all of it in line, forwards between 2 % and -1 %). A vote on every wait would do it as well, but costs
+// 1-2 % of a step and up to 7 % of a forward.
+static __device__ __noinline__ bool warp_gives_up(uint32_t parity, volatile int* abort_flag, int code, long long waited) {
+  if ((*abort_flag != 0 || waited > kWaitLimitCycles) && (__activemask() == 0xffffffffu || waited > 2 * kWaitLimitCycles)) {
+    note_expired_wait(parity, abort_flag, code);
+    return true;
+  }
+  return false;
+}
+
+// mbar_wait for a whole warp: all its lanes get the same answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int code) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const long long t0 = clock64();
+  uint32_t spins = 0;
+  while (!mbar_try_wait(bar, parity)) {
+    if ((++spins & 127u) == 0 && warp_gives_up(parity, abort_flag, code, clock64() - t0)) return false;
   }
   return true;
 }

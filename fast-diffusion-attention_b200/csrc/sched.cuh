@@ -63,9 +63,12 @@ __device__ __forceinline__ int sched_produce(SchedMailbox* m, uint32_t it, int* 
 // read the item's description; sched_release hands the slot back. kWholeWarp: called by every lane of a consumer
 // warp, lane 0 makes the arrival for the warp after all lanes are done with the slot. Otherwise: called by a
 // single thread that makes its own arrival.
+template <bool kWholeWarp>
 __device__ __forceinline__ int sched_peek(SchedMailbox* m, uint32_t it, volatile int* abort_flag) {
-  const uint32_t slot = it & 1u;
-  if (!ptx::mbar_wait(&m->full[slot], (it >> 1) & 1u, abort_flag, 6)) return -1;
+  const uint32_t slot = it & 1u, parity = (it >> 1) & 1u;
+  if (!(kWholeWarp ? ptx::mbar_wait_warp(&m->full[slot], parity, abort_flag, 6) : ptx::mbar_wait(&m->full[slot], parity, abort_flag, 6))) {
+    return -1;
+  }
   return m->idx[slot];
 }
 template <bool kWholeWarp>
@@ -80,7 +83,7 @@ __device__ __forceinline__ void sched_release(SchedMailbox* m, uint32_t it) {
 }
 template <bool kWholeWarp>
 __device__ __forceinline__ int sched_consume(SchedMailbox* m, uint32_t it, volatile int* abort_flag) {
-  const int v = sched_peek(m, it, abort_flag);
+  const int v = sched_peek<kWholeWarp>(m, it, abort_flag);
   if (v >= 0) sched_release<kWholeWarp>(m, it);
   return v;
 }

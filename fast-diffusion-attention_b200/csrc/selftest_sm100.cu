@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(128, 1) selftest_umma_kernel(const __grid_cons
     }
     ptx::umma_commit(&bar_mma);
   }
-  ptx::mbar_wait(&bar_mma, 0, &abort_flag, 102);
+  ptx::mbar_wait_warp(&bar_mma, 0, &abort_flag, 102);
   ptx::tc_fence_after();
   {
     const int row = warp * 32 + lane;
@@ -137,17 +137,22 @@ __global__ void __launch_bounds__(128, 1) selftest_umma_kernel(const __grid_cons
 
 // A wait that nobody ends: one block allocates tensor memory the way the attention kernels do, one thread waits on a
 // barrier no one arrives at with a SHORT limit, the others see the abort flag in their own wait, and everybody takes
-// the kernels' exit path (drain, free the tensor memory, return). Exercises ptx::mbar_wait's give-up branch, which
-// in the attention kernels is two seconds away.
+// the kernels' exit path (drain, free the tensor memory, return). Exercises the give-up branches of ptx::mbar_wait and
+// ptx::mbar_wait_warp, which in the attention kernels are two seconds away. All of warp 1 waits on that barrier and has to give up
+// as a whole (code 112 otherwise); half of warp 2 waits on one that completes after the flag is up, the other half on one that is complete from the
+// start, and all of it has to see that (code 113).
 __global__ void __launch_bounds__(128, 1) selftest_wait_kernel(long long limit_cycles) {
-  __shared__ uint64_t never;
+  __shared__ uint64_t never, complete, late;
   __shared__ uint32_t tmem_base_s;
   __shared__ int abort_flag;
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     abort_flag = 0;
     ptx::mbar_init(&never, 1);
+    ptx::mbar_init(&complete, 1);
+    ptx::mbar_init(&late, 1);
     ptx::fence_mbar_init();
+    ptx::mbar_arrive(&complete);
   }
   if (warp == 0) {
     ptx::tmem_alloc(&tmem_base_s, 512);
@@ -159,10 +164,18 @@ __global__ void __launch_bounds__(128, 1) selftest_wait_kernel(long long limit_c
   const uint32_t tmem = tmem_base_s;
   // thread 0 gives up after limit_cycles and raises the flag; the others wait with the production limit and leave
   // as soon as they see the flag
-  const bool ok = ptx::mbar_wait(&never, 0, &abort_flag, 110, threadIdx.x == 0 ? limit_cycles : ptx::kWaitLimitCycles);
-  (void)ok;
+  int wrong = 0;
+  if (warp == 1) {
+    if (__any_sync(0xffffffffu, ptx::mbar_wait_warp(&never, 0, &abort_flag, 111))) wrong = 112;
+  } else if (warp == 2) {
+    if (!__all_sync(0xffffffffu, ptx::mbar_wait_warp((threadIdx.x & 1) ? &late : &complete, 0, &abort_flag, 111))) wrong = 113;
+  } else {
+    ptx::mbar_wait(&never, 0, &abort_flag, 110, threadIdx.x == 0 ? limit_cycles : ptx::kWaitLimitCycles);
+    if (threadIdx.x == 96) ptx::mbar_arrive(&late);
+  }
   ptx::tc_fence_before();
   __syncthreads();
+  if (wrong != 0) g_fda_status[0] = wrong;
   if (warp == 0) ptx::tmem_dealloc(tmem, 512);
 }
 

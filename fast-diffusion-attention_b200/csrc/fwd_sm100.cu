@@ -214,7 +214,7 @@ struct FwdConfig {
   static_assert(!kTmemHasQ || (kQTiles == 1 && kTmemQ + kHeadDim * kElemBytes / 4 <= 512), "tensor memory budget");
   // The loop over fully visible sub-steps takes two of them, one a buffer, where that is not too much code: head dim 64 (4 x 8192
   // tokens, 32 heads: 768 / 753 us; capped 1284 / 1253) and e4m3 (2 x 16384 tokens, 8 heads of 256: 813 / 788; 4 x 8192, 16/4
-  // heads of 128: 531 / 519); 16-bit at 128 loses by it (1 x 16384, 32/8 heads 884 / 913), at 256 too (1081 / 1101).
+  // heads of 128: 531 / 519).
   static constexpr bool kUnrollFull = kHeadDim == 64 || kFp8;
   static constexpr int kPCols = kSubKeys * kElemBytes / 4;            // tensor-memory columns of the packed P
 };
@@ -878,15 +878,13 @@ int launch_fwd_instance(const FwdParams& p, int grid, cudaStream_t stream) {
 
 template <int kHeadDim, int kQTiles, int kType, bool kQInTmem>
 int dispatch_fwd(const FwdParams& p, int grid, bool softcap, bool full_loop, cudaStream_t stream) {
-  // who has the loop over fully visible sub-steps: see forward_full_loop
-  constexpr bool kHas = kHeadDim <= 128 || kType == 2;
-  constexpr bool kHasCapped = kHas && !(kHeadDim == 128 && kType != 2);
-  if (softcap) {
-    return kHasCapped && full_loop ? launch_fwd_instance<kHeadDim, kQTiles, kType, true, kQInTmem, kHasCapped>(p, grid, stream)
-                                   : launch_fwd_instance<kHeadDim, kQTiles, kType, true, kQInTmem, false>(p, grid, stream);
+  constexpr bool kHas = kHeadDim == 64 || kType == 2;   // the loop over fully visible sub-steps: see forward_full_loop
+  if (kHas && full_loop) {
+    return softcap ? launch_fwd_instance<kHeadDim, kQTiles, kType, true, kQInTmem, kHas>(p, grid, stream)
+                   : launch_fwd_instance<kHeadDim, kQTiles, kType, false, kQInTmem, kHas>(p, grid, stream);
   }
-  return kHas && full_loop ? launch_fwd_instance<kHeadDim, kQTiles, kType, false, kQInTmem, kHas>(p, grid, stream)
-                           : launch_fwd_instance<kHeadDim, kQTiles, kType, false, kQInTmem, false>(p, grid, stream);
+  return softcap ? launch_fwd_instance<kHeadDim, kQTiles, kType, true, kQInTmem, false>(p, grid, stream)
+                 : launch_fwd_instance<kHeadDim, kQTiles, kType, false, kQInTmem, false>(p, grid, stream);
 }
 
 template <int kHeadDim, int kQTiles, bool kQInTmem = false>
@@ -902,30 +900,29 @@ size_t fwd_workspace_bytes(const FdaProblem& pr) {
   return 256 + (pr.cu_seqlens != nullptr ? varlen_list_bytes(pr.batch) : 0);
 }
 
-// Whether fully visible sub-steps get a loop of their own. It saves their classification and mask, and makes a second and a
-// third copy of a long body. Where CTAs take many items of few sub-steps each, or of few that the loop takes (noisy rows of large
-// blocks see no clean key in full), the warps run from one copy into another and wait for instructions. One loop / two, us, d = 64, d =
-// 128, e4m3, e4m3 of 256 (16/8 heads, blocks of 64):
-//   32 x 1024 tokens  111 / 142  138 / 160  135 / 188  238 / 277      4 x 6000   257 / 252  313 / 311  327 / 323  550 / 538
-//   8 x 3000          157 / 164  183 / 190  197 / 219  332 / 355      3 x 8192   322 / 313  395 / 391  413 / 398  692 / 663
-//   8 x 4096          248 / 252  302 / 301  314 / 331  535 / 550      1 x 16384  383 / 370  489 / 481  491 / 468  826 / 782
-// 3 x 8192 in blocks of 1024: 349 / 349, 466 / 451, 474 / 450, 802 / 768; in one block: 558 / 580, 737 / 760, 747 / 737, 1223 / 1223.
-// Capped, 3 x 8192: 499 / 492, 525 / 526 (so not there), 605 / 577, 898 / 846. With at most eight items a CTA the loop loses nothing from
-// 600 tokens a half on (blocks of 16): 16 x 512, 16 heads 20.6 / 20.6, 23.3 / 23.5, 21.0 / 22.7, 33.1 / 33.6; 1 x 1400, 16/4 heads 17.2 /
-// 16.7, 19.3 / 18.8, 20.3 / 19.5, 22.7 / 23.5; 4 x 1400 35.1 / 34.8, 40.6 / 39.7, 39.4 / 39.1, 63.5 / 62.4; 1 x 3000, 16 heads 35.7 / 33.1,
-// 39.1 / 38.6, 43.3 / 40.8, 55.9 / 55.4; 1 x 6000, 3 heads 38.8 / 35.2, 41.2 / 40.7, 46.8 / 43.3, 49.7 / 49.9; 1 x 4096, 16 heads in
-// one block 69.1 / 69.9, 78.8 / 79.7, 88.7 / 88.0, 141 / 137. 16-bit heads of 256, which wait for K and V, get one loop for all (1 %
-// the other way).
+// Whether fully visible sub-steps get a loop of their own. It saves their classification and mask, and makes a second and a third
+// copy of a long body. Where CTAs take many items of few sub-steps each, or of few that the loop takes (noisy rows of large blocks
+// see no clean key in full), the warps run from one copy into another and wait for instructions. One loop / two, us, d = 64, e4m3, e4m3 of
+// 256 (16/8 heads, blocks of 64):
+//   32 x 1024 tokens  111 / 142  135 / 188  238 / 277      4 x 6000   257 / 252  327 / 323  550 / 538
+//   8 x 3000          157 / 164  197 / 219  332 / 355      3 x 8192   323 / 303  409 / 384  688 / 642
+//   8 x 4096          248 / 252  314 / 331  535 / 550      1 x 16384  388 / 362  487 / 454  823 / 754
+// 3 x 8192 in blocks of 1024: 355 / 345, 470 / 440, 798 / 746; in one block: 558 / 580, 744 / 723, 1216 / 1181. Capped, 3 x 8192: 501 /
+// 486, 600 / 565, 892 / 828. With at most eight items a CTA the loop loses nothing from 600 tokens a half on (blocks of 16): 16 x 512, 16
+// heads 20.6 / 20.6, 21.0 / 22.7, 33.1 / 33.6; 1 x 1400, 16/4 heads 17.2 / 16.7, 20.3 / 19.5, 22.7 / 23.5; 4 x 1400 35.1 / 34.8, 39.4 /
+// 39.1, 63.5 / 62.4; 1 x 3000, 16 heads 35.7 / 33.1, 43.3 / 40.8, 55.9 / 55.4; 1 x 6000, 3 heads 38.8 / 35.2, 46.8 / 43.3, 49.7 / 49.9; 1 x
+// 4096, 16 heads in one block 69.1 / 69.9, 88.7 / 88.0, 141 / 137.
+// 16-bit heads of 128 have one loop (1 x 16384, 32/8 heads, blocks of 64, 256 and 1024 941 / 963, 953 / 984, 1033 / 1063; 3 x 8192, 16/8, blocks
+// of 1024 427 / 448), and those of 256, which wait for K and V (1 % the other way).
 bool forward_full_loop(const FdaProblem& pr) {
-  if (pr.batch <= 0) return false;
-  const int64_t tokens = pr.total / (2 * static_cast<int64_t>(pr.batch));   // of a half, on average
   const bool fp8 = pr.dtype == FDA_E4M3;
-  if (!fp8 && (pr.head_dim > 128 || (pr.head_dim > 64 && pr.softcap > 0.f))) return false;
+  if (pr.batch <= 0 || (!fp8 && pr.head_dim > 64)) return false;
+  const int64_t tokens = pr.total / (2 * static_cast<int64_t>(pr.batch));   // of a half, on average
   const int item_rows = pr.head_dim > 128 ? kBlockM : 2 * kBlockM;
   const int64_t items = (tokens + item_rows - 1) / item_rows * 2 * pr.heads * pr.batch;
   const bool few = items <= 8 * 148;
   if (tokens < (few ? 600 : fp8 ? 3000 : 4096)) return false;
-  return fp8 || (few && pr.head_dim <= 64 ? 2 : 4) * static_cast<int64_t>(pr.block_size) <= tokens;
+  return fp8 || (few ? 2 : 4) * static_cast<int64_t>(pr.block_size) <= tokens;
 }
 
 int launch_fwd(const FdaFwdArgs& a, cudaStream_t stream) {

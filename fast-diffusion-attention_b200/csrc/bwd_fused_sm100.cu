@@ -203,6 +203,7 @@ __global__ void __launch_bounds__(FusedRoles<kHeadDim>::kThreads, 1) bwd_fused_k
       g_fda_status[2] = 0;
       g_fda_status[3] = static_cast<int>(ptx::smem_u32(smem) & 1023u);
     }
+    ptx::wait_for_stream();
     return;
   }
   if (threadIdx.x == 0) {

@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(kDkdvThreads, 1) bwd_dkdv_kernel(const __grid_
       g_fda_status[2] = 0;
       g_fda_status[3] = static_cast<int>(ptx::smem_u32(smem) & 1023u);
     }
+    ptx::wait_for_stream();
     return;
   }
   if (threadIdx.x == 0) {

@@ -2,6 +2,7 @@
 alone give the same bits."""
 
 import ctypes as C
+import os
 
 import pytest
 import torch
@@ -86,3 +87,18 @@ def test_both_loops_give_the_same_bits(n, bs, dtype, d, softcap):
     torch.cuda.synchronize()
     assert _lib.device_status()[0] == 0
     assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
+def test_no_block_ends_before_it_has_waited_for_the_stream():
+    """A kernel that may start early must not be complete before those ahead of it: the next one waits for this one only. So no kernel
+    (the self tests launch in plain order) returns ahead of ptx::wait_for_stream."""
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(_lib.__file__))), "csrc")
+    kernels = 0
+    for name in os.listdir(csrc):
+        if name.endswith(".cu") and not name.startswith("selftest"):
+            for body in open(os.path.join(csrc, name)).read().split("__global__ void")[1:]:
+                if "{" in body.split(";")[0]:   # a definition
+                    head, found, _ = body.partition("ptx::wait_for_stream();")
+                    assert found and "return;" not in head, (name, body[:120])
+                    kernels += 1
+    assert kernels == 7

@@ -11,6 +11,7 @@ size_t fwd_workspace_bytes(const FdaProblem& p);  // fwd_sm100.cu
 bool forward_full_loop(const FdaProblem& p);      // fwd_sm100.cu
 bool bwd_single_pass(const FdaProblem& p);        // bwd_sm100.cu
 bool bwd_overlaps(const FdaProblem& p, bool single_pass);
+bool bwd_dv_apart(const FdaProblem& p);
 
 namespace {
 
@@ -185,7 +186,8 @@ unsigned fda_launch_choices(const FdaProblem* p) {
   if (!p || fda::check_problem(*p, false) != FDA_OK) return 0;
   return (fda::forward_full_loop(*p) ? FDA_CHOICE_FORWARD_FULL_LOOP : 0u) |
          (fda::overlapped_launches(*p, 0) ? FDA_CHOICE_FORWARD_OVERLAP : 0u) |
-         (fda::bwd_overlaps(*p, fda::bwd_single_pass(*p)) ? FDA_CHOICE_BACKWARD_OVERLAP : 0u);
+         (fda::bwd_overlaps(*p, fda::bwd_single_pass(*p)) ? FDA_CHOICE_BACKWARD_OVERLAP : 0u) |
+         (fda::bwd_dv_apart(*p) ? FDA_CHOICE_DV_APART : 0u);
 }
 
 int fda_selftest_wait(long long limit_cycles, void* stream) {

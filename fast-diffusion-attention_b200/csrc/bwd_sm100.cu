@@ -1075,6 +1075,12 @@ constexpr int64_t kSmallAccBytes = 32 << 20;
 // The single-pass backward adds dQ partials in an order that depends on scheduling and needs head dim <= 128.
 bool bwd_single_pass(const FdaProblem& pr) { return pr.deterministic == 0 && pr.head_dim <= 128; }
 
+// Heads wider than 128, split form: dV items in a launch of their own have three dO slots, at the price of a second tail and of items
+// that cannot fill each other's gaps. Backward, together / apart, us, heads of 256: 16 x 2000 tokens, 8 heads, blocks of 16 820 / 789,
+// 16/8 heads, blocks of 512 1844 / 1721; 4 x 4096, 8 heads 679 / 641, 1 x 16384 2173 / 2000. Short ones and those whose longest
+// chain is more than a CTA's share stay together (32 x 512 tokens 246 / 264; 1 x 16384, 8/2 heads 2360 / 3140).
+bool bwd_dv_apart(const FdaProblem& pr) { return pr.head_dim > 128 && bwd_chains_fit(pr, 700); }
+
 // The items that count for overlapped_launches, by what the host knows of the lengths.
 bool bwd_overlaps(const FdaProblem& pr, bool single_pass) {
   int64_t items = 0;
@@ -1120,12 +1126,7 @@ int launch_bwd(const FdaBwdArgs& a, cudaStream_t stream, unsigned stage_mask) {
   BwdParams p;
   memset(&p, 0, sizeof(p));
   const bool single_pass = bwd_single_pass(pr) && (stage_mask & FDA_BWD_FORCE_SPLIT) == 0;
-  // Heads wider than 128, split form: dV items in a launch of their own have three dO slots, at the price of a second tail and of
-  // items that cannot fill each other's gaps. Backward, together / apart, us, heads of 256: 16 x 2000 tokens, 8 heads, blocks of 16
-  // 820 / 789, 16/8 heads, blocks of 512 1844 / 1721; deterministic, 4 x 4096, 8 heads 679 / 641, 1 x 16384 2173 / 2000. Short
-  // ones and those whose longest chain is more than a CTA's share stay together (32 x 512 tokens 246 / 264; 1 x 16384, 8/2 heads
-  // 2360 / 3140).
-  p.apart = d > 128 && bwd_chains_fit(pr, 700) ? 1 : 0;
+  p.apart = bwd_dv_apart(pr) ? 1 : 0;
   auto encode = [&](CUtensorMap* map, const FdaTensor& t, int heads, int box_rows) {
     return encode_tile_map(map, t.ptr, 2, false, fp16, d, rows, heads, tma_batch, t.row_stride, t.head_stride,
                            t.batch_stride, 64, box_rows);

@@ -19,6 +19,7 @@ FDA_BF16, FDA_FP16, FDA_E4M3 = 0, 1, 2
 FDA_CHOICE_FORWARD_FULL_LOOP = 1
 FDA_CHOICE_FORWARD_OVERLAP = 2
 FDA_CHOICE_BACKWARD_OVERLAP = 4
+FDA_CHOICE_DV_APART = 8
 
 FDA_OK = 0
 FDA_ERR_DEVICE_WAIT = 14

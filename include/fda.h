@@ -177,6 +177,7 @@ int fda_geom_item_order(int idx, int per_group, int n_groups, int short8, int ct
 #define FDA_CHOICE_FORWARD_FULL_LOOP 1u /* forward: fully visible sub-steps in a loop of their own */
 #define FDA_CHOICE_FORWARD_OVERLAP 2u   /* forward: kernels may start before the ones ahead in the stream end */
 #define FDA_CHOICE_BACKWARD_OVERLAP 4u  /* backward (fda_bwd): likewise */
+#define FDA_CHOICE_DV_APART 8u          /* split backward: dV in a launch of its own */
 unsigned fda_launch_choices(const FdaProblem* p);
 
 /* ---- tensor-core self test (GPU): C[128 x n] = A[128 x k] * B with the operand layouts the kernels use ---- */

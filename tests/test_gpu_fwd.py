@@ -185,8 +185,8 @@ def test_forward_into_a_strided_output_and_refusal_of_misaligned_ones():
 @pytest.mark.parametrize("d", [136, 256])
 @pytest.mark.parametrize("n,bs", [(1, 1), (130, 7), (400, 64), (512, 1024)])
 def test_wide_heads_short_and_long_samples_alike(n, bs, d, softcap, dtype):
-    """Head dimensions above 128: above 512 tokens a half (by max_seqlen, which may be an upper bound) Q is read from tensor
-    memory instead of shared memory. The results are the same bits."""
+    """Head dimensions above 128: Q goes through a pair of K/V slots into tensor memory, whatever the lengths, and a max_seqlen that is an
+    upper bound changes no bits."""
     torch.manual_seed(n + d)
     cu = torch.tensor([0, 2 * n, 4 * n], device=DEV, dtype=torch.int32)
     q, k, v = (torch.randn(4 * n, h, d, device=DEV, dtype=dtype) for h in (4, 2, 2))

@@ -150,7 +150,7 @@ def test_first_call_of_a_new_thread():
     assert len(got) == 1 and torch.equal(got[0], want)
 
 
-@pytest.mark.parametrize("heads,heads_k,d,deterministic", [(8, 2, 256, False), (8, 2, 128, True)])
+@pytest.mark.parametrize("heads,heads_k,d,deterministic", [(8, 2, 256, False), (10, 10, 256, False), (8, 2, 128, True)])
 def test_no_wait_expires_over_many_split_backward_passes(heads, heads_k, d, deterministic):
     torch.manual_seed(12)
     n = 1500

@@ -892,11 +892,12 @@ int launch_fused_instance(const BwdParams& p, int sm_count, unsigned stages, cud
     }
     const int64_t items = static_cast<int64_t>(bwd_item_bound(p, p.heads_k)) * p.kv_split;
     const int grid = items < sm_count ? static_cast<int>(items) : sm_count;
-    if (const int launched = launch_kernel(p.overlap != 0, kernel, grid, FusedRoles<kHeadDim>::kThreads, Cfg::kSmemBytes, stream, p)) return launched;
+    const int launched = launch_kernel(p.overlap != 0, kernel, grid, FusedRoles<kHeadDim>::kThreads, Cfg::kSmemBytes, stream, p);
+    if (launched) return launched;
   }
   if (stages & 4u) {
     dim3 grid(p.n_pad / 64, convert_rows(p.heads, p.heads_k, p.kv_split > 1), p.batch);
-    if (const int launched = launch_kernel(p.overlap != 0, bwd_dq_convert_kernel<kHeadDim, kBf16, kSoftcap, kParts>, grid, 256, 0, stream, p)) return launched;
+    return launch_kernel(p.overlap != 0, bwd_dq_convert_kernel<kHeadDim, kBf16, kSoftcap, kParts>, grid, 256, 0, stream, p);
   }
   return FDA_OK;
 }
@@ -964,7 +965,8 @@ constexpr double kLine = 240;
 // Samples of that many tokens a half, the longest and on average, and no chain of a key tile's steps over all heads of a group longer
 // than 1.23 times a CTA's share.
 bool bwd_chains_fit(const FdaProblem& pr, int tokens) {
-  if (pr.heads_k <= 0 || pr.batch <= 0 || pr.seqlen / 2 < tokens || pr.total / 2 < static_cast<int64_t>(pr.batch) * tokens) return false;
+  if (pr.heads_k <= 0 || pr.batch <= 0 || pr.seqlen / 2 < tokens) return false;
+  if (pr.total / 2 < static_cast<int64_t>(pr.batch) * tokens) return false;
   double longest, all, squares;
   known_tiles(pr, longest, all, squares);
   return pr.heads_k * (squares + 2 * all) >= kLine * longest;

@@ -1010,8 +1010,7 @@ int launch_dkdv(const BwdParams& p, int sm_count, cudaStream_t stream) {
   if (rc) return rc;
   const int items = bwd_item_bound(p, p.heads_k) * Cfg::kItems;
   const int grid = items < sm_count ? items : sm_count;
-  if (const int launched = launch_kernel(p.overlap != 0, kernel, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, p)) return launched;
-  return FDA_OK;
+  return launch_kernel(p.overlap != 0, kernel, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, p);
 }
 
 template <int kHeadDim, int kStagesKv, int kStagesQ, bool kBf16, bool kSoftcap>
@@ -1042,7 +1041,7 @@ int launch_bwd_instance(const BwdParams& p, int sm_count, unsigned stages, cudaS
     if (rc) return rc;
     const int items = bwd_item_bound(p, p.heads);
     const int grid = items < sm_count ? items : sm_count;
-    if (const int launched = launch_kernel(p.overlap != 0, kernel, grid, kBwdThreads, Cfg::kSmemBytes, stream, p)) return launched;
+    return launch_kernel(p.overlap != 0, kernel, grid, kBwdThreads, Cfg::kSmemBytes, stream, p);
   }
   return FDA_OK;
 }
@@ -1075,10 +1074,11 @@ constexpr int64_t kSmallAccBytes = 32 << 20;
 // The single-pass backward adds dQ partials in an order that depends on scheduling and needs head dim <= 128.
 bool bwd_single_pass(const FdaProblem& pr) { return pr.deterministic == 0 && pr.head_dim <= 128; }
 
-// Heads wider than 128, split form: dV items in a launch of their own have three dO slots, at the price of a second tail and of items
-// that cannot fill each other's gaps. Backward, together / apart, us, heads of 256: 16 x 2000 tokens, 8 heads, blocks of 16 820 / 789,
-// 16/8 heads, blocks of 512 1844 / 1721; 4 x 4096, 8 heads 679 / 641, 1 x 16384 2173 / 2000. Short ones and those whose longest
-// chain is more than a CTA's share stay together (32 x 512 tokens 246 / 264; 1 x 16384, 8/2 heads 2360 / 3140).
+// Heads wider than 128, split form: dV items in a launch of their own have three dO slots, at the price of a second
+// tail and of items that cannot fill each other's gaps. Backward, together / apart, us, heads of 256: 16 x 2000 tokens,
+// 8 heads, blocks of 16 820 / 789, 16/8 heads, blocks of 512 1844 / 1721; 4 x 4096, 8 heads 679 / 641, 1 x 16384 2173 /
+// 2000. Short ones and those whose longest chain is more than a CTA's share stay together (32 x 512 tokens 246 / 264; 1
+// x 16384, 8/2 heads 2360 / 3140).
 bool bwd_dv_apart(const FdaProblem& pr) { return pr.head_dim > 128 && bwd_chains_fit(pr, 700); }
 
 // The items that count for overlapped_launches, by what the host knows of the lengths.

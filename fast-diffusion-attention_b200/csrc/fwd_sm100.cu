@@ -234,7 +234,8 @@ struct FwdConfig {
 // has time, walks the geometry and leaves one word of flags beside every K slot. (A single thread that decoded items and
 // classified tiles between the products spent 1200 cycles a round on that while the pipe ran dry; the whole warp takes
 // part in waits and loop control, one elected lane issues, which keeps descriptors and counters in uniform registers.)
-constexpr uint32_t kInfoFirst = 16, kInfoLast = 32, kInfoHalf1 = 64, kInfoStop = 128, kInfoTile0 = 256, kInfoQ = 1024;  // bit 2 t + h: tile t sees half h
+// Bit 2 t + h: tile t sees half h.
+constexpr uint32_t kInfoFirst = 16, kInfoLast = 32, kInfoHalf1 = 64, kInfoStop = 128, kInfoTile0 = 256, kInfoQ = 1024;
 
 // kFullLoop: fully visible sub-steps have a loop of their own (see forward_full_loop).
 template <int kHeadDim, int kQTiles, int kType, bool kSoftcap, bool kQInTmem, bool kFullLoop>
@@ -261,7 +262,8 @@ __global__ void __launch_bounds__(kQTiles == 2 ? 384 : 128 * kQTiles + 64, 1) fw
   volatile uint32_t* slot_info = tmem_slot + 2;    // one word per pair
   SchedMailbox* mbox = reinterpret_cast<SchedMailbox*>(reinterpret_cast<uint8_t*>(bars) + 320);
   ItemDesc* desc = reinterpret_cast<ItemDesc*>(reinterpret_cast<uint8_t*>(bars) + 512);  // two slots
-  static_assert(Cfg::kMmaWarp + kQTiles <= Cfg::kThreads / 32 && sizeof(SchedMailbox) <= 192 && 2 * sizeof(ItemDesc) <= 512, "mailbox and item descriptions");
+  static_assert(Cfg::kMmaWarp + kQTiles <= Cfg::kThreads / 32, "roles");
+  static_assert(sizeof(SchedMailbox) <= 192 && 2 * sizeof(ItemDesc) <= 512, "mailbox and item descriptions");
 
   const int warp = ptx::uniform(static_cast<int>(threadIdx.x >> 5));
   const int lane = threadIdx.x & 31;
@@ -872,8 +874,7 @@ int launch_fwd_instance(const FwdParams& p, int grid, cudaStream_t stream) {
   static PerDeviceFlags smem_set;
   const int rc = set_dynamic_smem(kernel, Cfg::kSmemBytes, smem_set);
   if (rc) return rc;
-  if (const int launched = launch_kernel(p.overlap != 0, kernel, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, p)) return launched;
-  return FDA_OK;
+  return launch_kernel(p.overlap != 0, kernel, grid, Cfg::kThreads, Cfg::kSmemBytes, stream, p);
 }
 
 template <int kHeadDim, int kQTiles, int kType, bool kQInTmem>
@@ -900,20 +901,21 @@ size_t fwd_workspace_bytes(const FdaProblem& pr) {
   return 256 + (pr.cu_seqlens != nullptr ? varlen_list_bytes(pr.batch) : 0);
 }
 
-// Whether fully visible sub-steps get a loop of their own. It saves their classification and mask, and makes a second and a third
-// copy of a long body. Where CTAs take many items of few sub-steps each, or of few that the loop takes (noisy rows of large blocks
-// see no clean key in full), the warps run from one copy into another and wait for instructions. One loop / two, us, d = 64, e4m3, e4m3 of
-// 256 (16/8 heads, blocks of 64):
+// Whether fully visible sub-steps get a loop of their own. It saves their classification and mask, and makes a second
+// and a third copy of a long body. Where CTAs take many items of few sub-steps each, or of few that the loop takes
+// (noisy rows of large blocks see no clean key in full), the warps run from one copy into another and wait for
+// instructions. One loop / two, us, d = 64, e4m3, e4m3 of 256 (16/8 heads, blocks of 64):
 //   32 x 1024 tokens  111 / 142  135 / 188  238 / 277      4 x 6000   257 / 252  327 / 323  550 / 538
 //   8 x 3000          157 / 164  197 / 219  332 / 355      3 x 8192   323 / 303  409 / 384  688 / 642
 //   8 x 4096          248 / 252  314 / 331  535 / 550      1 x 16384  388 / 362  487 / 454  823 / 754
-// 3 x 8192 in blocks of 1024: 355 / 345, 470 / 440, 798 / 746; in one block: 558 / 580, 744 / 723, 1216 / 1181. Capped, 3 x 8192: 501 /
-// 486, 600 / 565, 892 / 828. With at most eight items a CTA the loop loses nothing from 600 tokens a half on (blocks of 16): 16 x 512, 16
-// heads 20.6 / 20.6, 21.0 / 22.7, 33.1 / 33.6; 1 x 1400, 16/4 heads 17.2 / 16.7, 20.3 / 19.5, 22.7 / 23.5; 4 x 1400 35.1 / 34.8, 39.4 /
-// 39.1, 63.5 / 62.4; 1 x 3000, 16 heads 35.7 / 33.1, 43.3 / 40.8, 55.9 / 55.4; 1 x 6000, 3 heads 38.8 / 35.2, 46.8 / 43.3, 49.7 / 49.9; 1 x
-// 4096, 16 heads in one block 69.1 / 69.9, 88.7 / 88.0, 141 / 137.
-// 16-bit heads of 128 have one loop (1 x 16384, 32/8 heads, blocks of 64, 256 and 1024 941 / 963, 953 / 984, 1033 / 1063; 3 x 8192, 16/8, blocks
-// of 1024 427 / 448), and those of 256, which wait for K and V (1 % the other way).
+// 3 x 8192 in blocks of 1024: 355 / 345, 470 / 440, 798 / 746; in one block: 558 / 580, 744 / 723, 1216 / 1181. Capped,
+// 3 x 8192: 501 / 486, 600 / 565, 892 / 828. With at most eight items a CTA the loop loses nothing from 600 tokens a
+// half on (blocks of 16): 16 x 512, 16 heads 20.6 / 20.6, 21.0 / 22.7, 33.1 / 33.6; 1 x 1400, 16/4 heads 17.2 / 16.7,
+// 20.3 / 19.5, 22.7 / 23.5; 4 x 1400 35.1 / 34.8, 39.4 / 39.1, 63.5 / 62.4; 1 x 3000, 16 heads 35.7 / 33.1, 43.3 /
+// 40.8, 55.9 / 55.4; 1 x 6000, 3 heads 38.8 / 35.2, 46.8 / 43.3, 49.7 / 49.9; 1 x 4096, 16 heads in one block 69.1 /
+// 69.9, 88.7 / 88.0, 141 / 137. 16-bit heads of 128 have one loop (1 x 16384, 32/8 heads, blocks of 64, 256 and 1024
+// 941 / 963, 953 / 984, 1033 / 1063; 3 x 8192, 16/8, blocks of 1024 427 / 448), and those of 256, which wait for K and
+// V (1 % the other way).
 bool forward_full_loop(const FdaProblem& pr) {
   const bool fp8 = pr.dtype == FDA_E4M3;
   if (pr.batch <= 0 || (!fp8 && pr.head_dim > 64)) return false;

@@ -111,9 +111,10 @@ int set_dynamic_smem(Kernel kernel, int bytes, PerDeviceFlags& flags) {
   return FDA_OK;
 }
 
-// Launches a kernel; with `overlap` its blocks may start, up to ptx::wait_for_stream, while the last blocks of the kernel ahead in the
-// stream are still running (if that is one of ours and has called ptx::let_next_start; behind anything else it starts as usual): the
-// launch, the set-up of barriers and the allocation of tensor memory come off the path.
+// Launches a kernel; with `overlap` its blocks may start, up to ptx::wait_for_stream, while the last blocks of the
+// kernel ahead in the stream are still running (if that is one of ours and has called ptx::let_next_start; behind
+// anything else it starts as usual): the launch, the set-up of barriers and the allocation of tensor memory come off
+// the path.
 template <typename... Params, typename... Args>
 int launch_kernel(bool overlap, void (*kernel)(Params...), dim3 grid, int threads, int smem_bytes, cudaStream_t stream,
                   const Args&... args) {
@@ -131,19 +132,20 @@ int launch_kernel(bool overlap, void (*kernel)(Params...), dim3 grid, int thread
   return FDA_OK;
 }
 
-// Where launches overlap: on little data and little work, where launches are a good part of the time. In one stream with nothing
-// else between them (step of 2 x 512 tokens, 4 heads of 64, 33.1 -> 26.4 us; 3 x 666, 12/4 heads of 96, 100 -> 94; 1 x 2048, 4 heads of
-// 256, 129 -> 120; forward of 1 x 1024, 16 heads of 128, 16.6 -> 14.3) a call overlaps the one before it, too. With another library's
-// kernel in between only the kernels of a call overlap each other: steps 1-5 % (1 x 1400 tokens, 16/4 heads of 128, 83.2 -> 80.1 us),
-// a forward of one kernel nothing. At twice the data, 16 x 512 tokens, 16/4 heads of 128, there is nothing left of it (150 / 152).
-// Beyond 2^36 = rows x length x heads x head dim nothing either (step of 1 x 16384 tokens, 8 heads of 64, 570 / 572; 1 x 32768, 2 heads of
-// 128, deterministic, 1088 / 1105; 1 x 8192, 4 heads of 256 400 / 398).
-// `items` is the number of items of a single-pass backward at head dims 65 to 128, else 0. With more than two a CTA that kernel gets
-// slower: its blocks land on other SMs, in the order in which these become free. 256 items: 1 x 3000 tokens, 8 heads of 128, 111 / 103; 1 x
-// 8192, 4 heads 234 / 228; 16 x 500, 8/2 heads 135 / 135. 384: 1 x 3000, 16 heads 122 / 130; 1 x 6000, 8/2 heads 207 / 224. 512: 4 x 1024, 16
-// heads 103 / 105; 1 x 8192, 8/2 heads 285 / 302; 1 x 16384, 4 heads 470 / 481. Head dim 64, 512 items: 602 / 605.
-// Nor with sm_margin: blocks that start early go first to the SMs that the caller wants free, and hold all tensor memory there while they
-// wait. (For the same reason the kernels of such a call do not let the next one start: next_early.)
+// Where launches overlap: on little data and little work, where launches are a good part of the time. In one stream
+// with nothing else between them (step of 2 x 512 tokens, 4 heads of 64, 33.1 -> 26.4 us; 3 x 666, 12/4 heads of 96,
+// 100 -> 94; 1 x 2048, 4 heads of 256, 129 -> 120; forward of 1 x 1024, 16 heads of 128, 16.6 -> 14.3) a call overlaps
+// the one before it, too. With another library's kernel in between only the kernels of a call overlap each other: steps
+// 1-5 % (1 x 1400 tokens, 16/4 heads of 128, 83.2 -> 80.1 us), a forward of one kernel nothing. At twice the data, 16 x
+// 512 tokens, 16/4 heads of 128, there is nothing left of it (150 / 152). From 2^36 = rows x length x heads x head
+// dim on nothing either (step of 1 x 16384 tokens, 8 heads of 64, 570 / 572; 1 x 32768, 2 heads of 128, deterministic,
+// 1088 / 1105; 1 x 8192, 4 heads of 256 400 / 398). `items` is the number of items of a single-pass backward at head
+// dims 65 to 128, else 0. With more than two a CTA that kernel gets slower: its blocks land on other SMs, in the order
+// in which these become free. 256 items: 1 x 3000 tokens, 8 heads of 128, 111 / 103; 1 x 8192, 4 heads 234 / 228; 16 x
+// 500, 8/2 heads 135 / 135. 384: 1 x 3000, 16 heads 122 / 130; 1 x 6000, 8/2 heads 207 / 224. 512: 4 x 1024, 16 heads
+// 103 / 105; 1 x 8192, 8/2 heads 285 / 302; 1 x 16384, 4 heads 470 / 481. Head dim 64, 512 items: 602 / 605. Nor with
+// sm_margin: blocks that start early go first to the SMs that the caller wants free, and hold all tensor memory there
+// while they wait. (For the same reason the kernels of such a call do not let the next one start: next_early.)
 inline bool overlapped_launches(const FdaProblem& pr, int64_t items) {
   if (pr.sm_margin > 0 || items > 2 * 148) return false;
   const int64_t q = static_cast<int64_t>(pr.total) * pr.heads * pr.head_dim;

@@ -33,8 +33,8 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
-// The value of lane 0, for values that are the same in every lane: what is computed from the result (loop control, barrier and
-// tensor-memory addresses) can then stay in uniform registers.
+// The value of lane 0, for values that are the same in every lane: what is computed from the result (loop control,
+// barrier and tensor-memory addresses) can then stay in uniform registers.
 __device__ __forceinline__ int uniform(int x) { return __shfl_sync(0xffffffffu, x, 0); }
 __device__ __forceinline__ uint32_t uniform(uint32_t x) { return __shfl_sync(0xffffffffu, x, 0); }
 
@@ -81,8 +81,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait of one thread. `abort_flag` lives in shared memory; once any thread of the CTA gives up, every later wait that would
-// have to wait returns at once so the CTA can drain, free its tensor memory and exit. Returns false when aborted.
+// Bounded wait of one thread. `abort_flag` lives in shared memory; once any thread of the CTA gives up, every later
+// wait that would have to wait returns at once so the CTA can drain, free its tensor memory and exit. Returns false
+// when aborted.
 constexpr long long kWaitLimitCycles = 4000000000LL;  // about two seconds at the boost clock
 
 __device__ __forceinline__ void note_expired_wait(uint32_t parity, volatile int* abort_flag, int code) {
@@ -112,14 +113,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return true;
 }
 
-// Whether a warp gives up a wait, with one answer for all its lanes. Behind a wait come operations that every lane has to take part in
-// (elections, shuffles, tensor-memory loads, the block's last barrier): were some lanes to see the phase complete and others only the
-// abort flag, each would wait for lanes that have left, without a bound. So a warp gives up as a whole, all its lanes here at once. While
-// lanes are missing they have seen the phase complete, and so will the others: the phase after it needs this warp's arrival. (Lanes that
-// run apart for another limit, with none through, leave one by one, which is all of them.)
-// Out of line: the dozens of waits of a kernel are then short, and its warps wait for instructions less (steps of 1 x 2000 to 4 x 4096
-// tokens 1-3 % faster than with all of it in line, forwards between 2 % and -1 %). A vote on every wait would do it as well, but costs
-// 1-2 % of a step and up to 7 % of a forward.
+// Whether a warp gives up a wait, with one answer for all its lanes. Behind a wait come operations that every lane has
+// to take part in (elections, shuffles, tensor-memory loads, the block's last barrier): were some lanes to see the
+// phase complete and others only the abort flag, each would wait for lanes that have left, without a bound. So a warp
+// gives up as a whole, all its lanes here at once. While lanes are missing they have seen the phase complete, and so
+// will the others: the phase after it needs this warp's arrival. (Lanes that run apart for another limit, with none
+// through, leave one by one, which is all of them.) Out of line: the dozens of waits of a kernel are then short, and
+// its warps wait for instructions less (steps of 1 x 2000 to 4 x 4096 tokens 1-3 % faster than with all of it in line,
+// forwards between 2 % and -1 %). A vote on every wait would do it as well, but costs 1-2 % of a step and up to 7 % of
+// a forward.
 static __device__ __noinline__ bool warp_gives_up(uint32_t parity, volatile int* abort_flag, int code, long long waited) {
   if ((*abort_flag != 0 || waited > kWaitLimitCycles) && (__activemask() == 0xffffffffu || waited > 2 * kWaitLimitCycles)) {
     note_expired_wait(parity, abort_flag, code);

@@ -66,9 +66,9 @@ __device__ __forceinline__ int sched_produce(SchedMailbox* m, uint32_t it, int* 
 template <bool kWholeWarp>
 __device__ __forceinline__ int sched_peek(SchedMailbox* m, uint32_t it, volatile int* abort_flag) {
   const uint32_t slot = it & 1u, parity = (it >> 1) & 1u;
-  if (!(kWholeWarp ? ptx::mbar_wait_warp(&m->full[slot], parity, abort_flag, 6) : ptx::mbar_wait(&m->full[slot], parity, abort_flag, 6))) {
-    return -1;
-  }
+  const bool ok = kWholeWarp ? ptx::mbar_wait_warp(&m->full[slot], parity, abort_flag, 6)
+                             : ptx::mbar_wait(&m->full[slot], parity, abort_flag, 6);
+  if (!ok) return -1;
   return m->idx[slot];
 }
 template <bool kWholeWarp>

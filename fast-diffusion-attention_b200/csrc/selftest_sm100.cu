@@ -138,9 +138,9 @@ __global__ void __launch_bounds__(128, 1) selftest_umma_kernel(const __grid_cons
 // A wait that nobody ends: one block allocates tensor memory the way the attention kernels do, one thread waits on a
 // barrier no one arrives at with a SHORT limit, the others see the abort flag in their own wait, and everybody takes
 // the kernels' exit path (drain, free the tensor memory, return). Exercises the give-up branches of ptx::mbar_wait and
-// ptx::mbar_wait_warp, which in the attention kernels are two seconds away. All of warp 1 waits on that barrier and has to give up
-// as a whole (code 112 otherwise); half of warp 2 waits on one that completes after the flag is up, the other half on one that is complete from the
-// start, and all of it has to see that (code 113).
+// ptx::mbar_wait_warp, which in the attention kernels are two seconds away. All of warp 1 waits on that barrier and has
+// to give up as a whole (code 112 otherwise); half of warp 2 waits on one that completes after the flag is up, the
+// other half on one that is complete from the start, and all of it has to see that (code 113).
 __global__ void __launch_bounds__(128, 1) selftest_wait_kernel(long long limit_cycles) {
   __shared__ uint64_t never, complete, late;
   __shared__ uint32_t tmem_base_s;

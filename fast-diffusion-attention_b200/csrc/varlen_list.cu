@@ -40,7 +40,8 @@ __global__ void __launch_bounds__(256) varlen_prepare_kernel(const int32_t* __re
 
 int launch_varlen_prepare(const int32_t* cu_seqlens, int batch, int unit_rows, int* out, int* tickets, void* stream,
                           bool overlap) {
-  return launch_kernel(overlap, varlen_prepare_kernel, 1, 256, 0, static_cast<cudaStream_t>(stream), cu_seqlens, batch, unit_rows, out, tickets);
+  return launch_kernel(overlap, varlen_prepare_kernel, 1, 256, 0, static_cast<cudaStream_t>(stream), cu_seqlens, batch,
+                       unit_rows, out, tickets);
 }
 
 }  // namespace fda
